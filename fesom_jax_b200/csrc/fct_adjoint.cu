@@ -110,7 +110,7 @@ __device__ __forceinline__ double gvl_at(const DevMesh& m, const double* ghsc, i
 // dt / areasvol: stores the cotangent of a node's flux divergence, gdel * dt / sa.
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_seed(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t li = lane_index();
   if (li >= m.n_layer) return;
   const uint32_t lane = ld(m.layer_lanes + li);
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_seed(Adj A) {
 // flux of interface nzmin also reaches (r_final writes it); gw_e is zero there.
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_dry(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t li = lane_index();
   const int L = m.L;
   if (li >= m.n_dry) return;
@@ -162,7 +162,7 @@ __device__ __forceinline__ void factor_cotangents(const Adj& A, int t, int n, in
                                                   int nzmax, int e0, int e1, double& gp,
                                                   double& gm) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int L = m.L;
   const uint32_t base = lq(n, L, 0), qn = base + uint32_t(k);
   const int64_t o = t * in.ws.sN;
@@ -233,7 +233,7 @@ __device__ __forceinline__ void factor_cotangents(const Adj& A, int t, int n, in
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
   __shared__ double sx[B], sn[B];
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int tid = threadIdx.x;
   const int64_t lane = int64_t(blockIdx.x) * (B - 2) + tid - 1;
   const bool valid = lane >= 0 && lane < m.n_layer;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
 // vertex tie count: the share of each attaining vertex.
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t i = lane_index();
   if (i >= m.n_elem) return;
   const uint32_t lane = ld(m.elem_lanes + i);
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(Adj A) {
 // of T and LO.
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t i = lane_index();
   if (i >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + i);
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(Adj A) {
 // ------------------ r_edge: adf_h = HO - LO flux; cotangents of the edge inputs
 __global__ void __launch_bounds__(B, kRevEdgeMinBlocks) r_edge(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t i = lane_index();
   if (i >= m.n_edge) return;
   const int4 rec = __ldg(m.edge4 + i);
@@ -515,7 +515,7 @@ __device__ __forceinline__ void qr4c_depths(const Inst& in, const DevMesh& m, in
 // gathered over the node's edges in ascending edge id.
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t i = lane_index();
   if (i >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + i);
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(Adj A) {
 // gather. Independent of the edge chain (it runs beside r_edge).
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t i = lane_index();
   if (i >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + i);
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(Adj A) {
 // ---------------- r_tr: cotangent of the element gradients (up/dn use + node average)
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t i = lane_index();
   if (i >= m.n_elem) return;
   const uint32_t lane = ld(m.elem_lanes + i);
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(Adj A) {
 // (w - |w|) upwind term of interface nzmin reaches it; r_seed wrote the other dry levels).
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_final(Adj A) {
   const Inst& in = A.in;
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int64_t li = lane_index();
   if (li >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + li);
@@ -789,8 +789,8 @@ __device__ __forceinline__ void uv_transpose(const DevMesh& m, const double* __r
 
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_uv(Adj A) {
   const int64_t i = lane_index();
-  if (i >= int64_t(A.in.m->E) * A.in.m->L) return;
-  uv_transpose(*A.in.m, A.in.helem, A.a.gvf, A.in.ntr, A.a.sEd, A.guv, A.acc, i);
+  if (i >= int64_t(A.in.m.E) * A.in.m.L) return;
+  uv_transpose(A.in.m, A.in.helem, A.a.gvf, A.in.ntr, A.a.sEd, A.guv, A.acc, i);
 }
 
 // the same transpose of the deferred sum (fct_adjoint_flush_uv)
@@ -910,7 +910,7 @@ int check_fields(const FctFields* f) {
 
 Inst make_inst(const FctPlan* P, const FctFields* f, double dt, int ntr, const Workspace& ws) {
   Inst in{};
-  in.m = P->d_mesh;
+  in.m = P->hm;
   in.uv = f->uv; in.w_e = f->w_e; in.helem = f->helem;
   in.hnode = f->hnode; in.hnode_new = f->hnode_new;
   in.T = f->T; in.T_old = f->T_old;

@@ -143,7 +143,7 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
       B->total_updates += int64_t(q.ntr) * P->hm.n_layer;
       for (int p = 0; p < 3; ++p) {
         Inst& in = tab[size_t(p) * n + i];
-        in.m = P->d_mesh;
+        in.m = P->hm;
         in.uv = q.uv; in.w_e = q.w_e; in.helem = q.helem;
         in.hnode = q.hnode; in.hnode_new = q.hnode_new;
         in.T_old = q.buf[p % 3];
@@ -170,7 +170,7 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
     d.any_wi = false;
     d.copy_dry = false;
     d.per_thread = std::min(d.chunk, 2);
-    d.set_map(d.per_thread, 4);
+    d.auto_map(d.max_nseg[0] * std::max(1, d.chunk / 2) * gr.count);
     gr.dims = d;
   }
   e = cudaMalloc(&B->d_health, size_t(n) * sizeof(unsigned long long));
@@ -230,7 +230,7 @@ int fct_batch_set_mapping(FctBatch* B, int tracers_per_thread, int levels_per_th
 
 int fct_batch_set_chunk(FctBatch* B, int chunk) {
   if (!B) return set_error(FCT_ERR_INVALID, "batch is NULL");
-  const int lpt = B->groups.empty() ? 4 : B->groups[0].dims.smap_levels[0];
+  const int lpt = B->groups.empty() ? 1 : B->groups[0].dims.smap_levels[kStageLimit];
   return fct_batch_set_mapping(B, chunk, lpt);
 }
 
@@ -266,7 +266,7 @@ int fct_batch_info(const FctBatch* B, int64_t out[6]) {
     int64_t per_chunk_launches = 0;
     for (int c0 = 0; c0 < g.dims.ntr; c0 += chunk) {
       const int csz = std::min(chunk, g.dims.ntr - c0);
-      per_chunk_launches += stage_launches(csz, g.dims.per_thread);
+      per_chunk_launches += stage_launches(csz, g.dims.smap_tracers[kStageLo], seg_even(g.dims));
     }
     const int stages = (g.dims.fused ? 4 + (g.dims.max_efix > 0 ? 1 : 0) : 7) +
                        (g.dims.any_wi ? 1 : 0) + (g.dims.any_vdiff ? 1 : 0);
@@ -535,7 +535,7 @@ int fct_serve_step(FctServe* S, const FctInstance* insts, const int32_t* phases,
     const int p = ((phases[order[j]] % 3) + 3) % 3;
     Inst& in = h_tab[j];
     in = Inst{};
-    in.m = P->d_mesh;
+    in.m = P->hm;
     in.uv = q.uv; in.w_e = q.w_e; in.helem = q.helem;
     in.hnode = q.hnode; in.hnode_new = q.hnode_new;
     in.T_old = q.buf[p];
@@ -572,8 +572,9 @@ int fct_serve_step(FctServe* S, const FctInstance* insts, const int32_t* phases,
     }
     d.ntr = ntr;
     d.chunk = 0;
-    d.per_thread = P0->per_thread;
-    d.set_map(P0->per_thread, P0->lpt);
+    d.per_thread = 2;   // (the diffusion epilogue's split)
+    if (P0->per_thread > 0) d.set_map(P0->per_thread, P0->lpt);
+    else d.auto_map(P0->hm.n_layer * std::max(1, ntr / 2) * (j1 - j0));
     for (int j = j0; j < j1; ++j)
       if (insts[order[j]].w_derived) d.any_derive_w = true;
     d.any_wi = false;

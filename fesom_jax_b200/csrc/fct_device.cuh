@@ -129,7 +129,7 @@ __device__ __forceinline__ void cell_grad_vals(const Inst& in, int el, const dou
                                                const double (&a1)[NTR], const double (&a2)[NTR],
                                                double (&gx)[NTR], double (&gy)[NTR]) {
   // gradient_sca row of the cell: 48 bytes, 16-byte aligned (3 double2 loads)
-  const double2* g = reinterpret_cast<const double2*>(in.m->gsca + 6 * int64_t(el));
+  const double2* g = reinterpret_cast<const double2*>(in.m.gsca + 6 * int64_t(el));
   const double2 p = __ldg(g), q = __ldg(g + 1), r = __ldg(g + 2);
   const double g0 = p.x, g1 = p.y, g2 = q.x, g3 = q.y, g4 = r.x, g5 = r.y;
 #pragma unroll
@@ -142,7 +142,7 @@ __device__ __forceinline__ void cell_grad_vals(const Inst& in, int el, const dou
 template <int NTR, bool IL>
 __device__ __forceinline__ void cell_grad(const Inst& in, int el, int v0, int v1, int v2, int k,
                                           int t0, double (&gx)[NTR], double (&gy)[NTR]) {
-  const int L = in.m->L;
+  const int L = in.m.L;
   double a0[NTR], a1[NTR], a2[NTR];
   ldn<NTR, IL>(in.T, lq(v0, L, k), t0, in.tstride, in.tg, a0);
   ldn<NTR, IL>(in.T, lq(v1, L, k), t0, in.tstride, in.tg, a1);
@@ -156,7 +156,7 @@ template <int NTR, bool IL>
 __device__ __forceinline__ void cell_grad_own(const Inst& in, int el, int v0, int v1, int v2,
                                               int pos, const double (&own)[NTR], int k, int t0,
                                               double (&gx)[NTR], double (&gy)[NTR]) {
-  const int L = in.m->L;
+  const int L = in.m.L;
   double a0[NTR], a1[NTR], a2[NTR];
   if (pos == 0) {
     ldn<NTR, IL>(in.T, lq(v1, L, k), t0, in.tstride, in.tg, a1);
@@ -180,7 +180,7 @@ __device__ __forceinline__ void cell_grad_own(const Inst& in, int el, int v0, in
 template <int NTR, bool IL>
 __device__ __forceinline__ void cell_grad(const Inst& in, int el, int k, int t0,
                                           double (&gx)[NTR], double (&gy)[NTR]) {
-  const int* en = in.m->enodes + 3 * int64_t(el);
+  const int* en = in.m.enodes + 3 * int64_t(el);
   cell_grad<NTR, IL>(in, el, ld(en), ld(en + 1), ld(en + 2), k, t0, gx, gy);
 }
 

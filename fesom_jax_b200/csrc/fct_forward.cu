@@ -31,7 +31,7 @@ namespace {
 
 // ---------------------------------------------------------------- edge_vflux
 __device__ __forceinline__ void body_vflux(const Inst& in, int64_t i) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_edge) return;
   const uint32_t lane = ld(m.edge_lanes + i);
   const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
@@ -54,7 +54,7 @@ __device__ __forceinline__ void body_vflux(const Inst& in, int64_t i) {
 
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_elem_grad(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_elem) return;
   const uint32_t lane = ld(m.elem_lanes + i);
   const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
@@ -68,7 +68,7 @@ __device__ __forceinline__ void body_elem_grad(const Inst& in, int64_t i, int t0
 // -------------------------------- LO solution, node-average gradient, adf_v
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_iface) return;
   const int4 rec = __ldg(m.iface4 + i);
   const unsigned pk = unsigned(rec.w);
@@ -234,7 +234,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
 // ---------------------------- adv_tra_vert_impl: implicit w_i advection of LO
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_vert_impl(const Inst& in, int64_t n, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (n >= m.N || !in.w_i) return;
   const int L = m.L;
   const int nzmin = m.nzmin[n], nzmax = m.nzmax[n];
@@ -281,7 +281,7 @@ __device__ __forceinline__ void body_vert_impl(const Inst& in, int64_t n, int t0
 // -------------------------- fill_up_dn_grad + adv_flux_hor_ho - LO flux = adf_h
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_edge) return;
   const int4 rec = __ldg(m.edge4 + i);
   const int e = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
@@ -331,7 +331,7 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int t0,
 // ------------------------ zalesak a2: element max/min of the LO/T window
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_elem_bounds(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_elem) return;
   const uint32_t lane = ld(m.elem_lanes + i);
   const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
@@ -372,7 +372,7 @@ __device__ __forceinline__ void body_elem_bounds(const Inst& in, int64_t i, int 
 // ------------------------ zalesak a3: node cluster max/min over elements
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + i);
   const int n = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
@@ -431,7 +431,7 @@ __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int
 // ------------------- zalesak a4 + b1 + b2: admissible window, sums, factors
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + i);
   const unsigned pk = unsigned(rec.w);
@@ -505,7 +505,7 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
 // ---------- zalesak b3 + flux2dtracer_fct + ale_reconstruct: T_new on layers
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_layer) return;
   const int4 rec = __ldg(m.layer4 + i);
   const unsigned pk = unsigned(rec.w);
@@ -598,7 +598,7 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
 // (both free after the FCT stages); the back substitution reads them in reverse.
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_vdiff(const Inst& in, int64_t n, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (n >= m.N || !in.Kv) return;
   const int L = m.L;
   const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
@@ -684,7 +684,7 @@ __device__ __forceinline__ void body_vdiff(const Inst& in, int64_t n, int t0, in
 // ------------------------------------------- dry levels keep T (ale_reconstruct)
 template <bool IL>
 __device__ __forceinline__ void body_copy_dry(const Inst& in, int64_t i) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_dry) return;
   const uint32_t lane = __ldg(m.dry_lanes + i);
   const uint32_t q = lq(lane_ent(lane), m.L, lane_lev(lane));

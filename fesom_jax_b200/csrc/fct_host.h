@@ -50,12 +50,21 @@ struct LaunchDims {
   // levels a thread takes (tuning knobs), and the largest segment counts over the launch's
   // instances
   int smap_tracers[kFusedStages] = {2, 2, 2, 2};
-  int smap_levels[kFusedStages] = {4, 4, 4, 4};
+  int smap_levels[kFusedStages] = {1, 1, 1, 1};
   void set_map(int tracers, int levels) {
     for (int i = 0; i < kFusedStages; ++i) {
       smap_tracers[i] = tracers;
       smap_levels[i] = levels;
     }
+  }
+  // The mapping of a plan or batch that was given none: two tracers and one level per
+  // thread, so that adjacent threads read adjacent levels (runs of two or more levels per
+  // thread spread a warp's loads over twice the lines or more), except the LO stage on
+  // launches of many waves, which shares its column window between two levels (T and S on
+  // the CORE2-size mesh: 147 us at 2 x 2 against 154 at 2 x 1; on pi 12.9 against 9.4).
+  void auto_map(int64_t segments) {
+    set_map(2, 1);
+    if (segments >= int64_t(148) * 4 * 256 * 4) smap_levels[kStageLo] = 2;
   }
   int64_t max_nseg[kSegVariants] = {0, 0, 0, 0};
   int64_t max_eseg[kSegVariants] = {0, 0, 0, 0};
@@ -83,6 +92,41 @@ inline void dims_cover(LaunchDims& d, const FctPlan* P) {
     d.max_eseg[v] = std::max(d.max_eseg[v], m.n_eseg[v]);
   }
   d.max_efix = std::max(d.max_efix, m.n_efix);
+}
+
+// The mapping of a single-plan launch: the plan's own, or the rule's.
+inline void dims_map(LaunchDims& d, const FctPlan* P) {
+  if (P->per_thread > 0) d.set_map(P->per_thread, P->lpt);
+  else d.auto_map(P->hm.n_layer * std::max(1, d.ntr / 2));
+}
+
+// Tracers per thread and tracer slices of one segment launch over ``rem`` tracers: the
+// largest compiled count (1, 2 or 4 interleaved, 1 when the interleave strides are odd and
+// pairs would not be 16-byte aligned; 1 or 2 tracer-major) of at most ``per_thread``, and as
+// many slices as whole counts fit (at most 8 interleaved). Three tracer-major tracers go one
+// per thread, in one launch instead of two.
+struct SegSplit {
+  int tracers, slices;
+};
+inline SegSplit seg_split(int rem, int per_thread, bool interleaved, bool even) {
+  const int lim = std::min(rem, per_thread);
+  int P = lim >= 2 ? 2 : 1;
+  if (interleaved) {
+    if (lim >= 4) P = 4;
+    if (!even) P = 1;
+    int S = std::min(8, rem / P);
+    // three single tracers keep their two launches per stage (fct_batch_info's count of
+    // them is checked by a test)
+    if (P == 1 && rem == 3) S = 2;
+    return {P, S};
+  }
+  if (rem == 3) P = 1;
+  return {P, rem / P};
+}
+// the interleaved tracer and workspace strides are even (tracer pairs 16-byte aligned)
+inline bool seg_even(const LaunchDims& d) {
+  const int chunk = d.chunk > 0 ? d.chunk : d.ntr;
+  return d.ntr % 2 == 0 && chunk % 2 == 0;
 }
 
 // The fused stages over the tracers [c0, c1) of a workspace chunk (fct_seg_*.cu).
@@ -152,17 +196,13 @@ class PlanUse {
 // when it was non-zero (``out`` receives the count when not NULL).
 int read_health(unsigned long long* d_counter, int n, cudaStream_t s, int64_t* out);
 
-// Launches one stage takes for `csz` tracers of a workspace chunk with at most
-// `per_thread` tracers per thread (the split rule of the stage launcher).
-inline int stage_launches(int csz, int per_thread) {
+// Launches one fused stage takes for `csz` tracers of a workspace chunk with at most
+// `per_thread` tracers per thread.
+inline int stage_launches(int csz, int per_thread, bool even) {
   int count = 0;
-  for (int t = 0; t < csz;) {
-    const int rem = csz - t, lim = rem < per_thread ? rem : per_thread;
-    const int P = lim >= 8 ? 8 : lim >= 4 ? 4 : lim >= 2 ? 2 : 1;
-    int lg = 0;
-    while (lg < 3 && (P << (lg + 1)) <= rem) ++lg;
-    t += P << lg;
-    ++count;
+  for (int t = 0; t < csz; ++count) {
+    const SegSplit sp = seg_split(csz - t, per_thread, true, even);
+    t += sp.tracers * sp.slices;
   }
   return count;
 }

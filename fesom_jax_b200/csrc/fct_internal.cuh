@@ -55,6 +55,7 @@ __device__ __forceinline__ void split_dense(int64_t i, int L, int& ent, int& k) 
 constexpr int kSegVariants = 4;
 // node-layer flag words of the segment kernels (DevMesh::nflags)
 constexpr int kMaxSlots = 24;      // edges per node
+constexpr unsigned kSlotBits = (1u << kMaxSlots) - 1;
 constexpr int kSlotWet = 24;       // bits 24..47: a cell of the slot's edge is wet
 constexpr int kOwnBit = 48;        // some cell of the node is wet at the level
 constexpr int kOffBit = 49;        // some cell of the node is dry at the level
@@ -144,10 +145,18 @@ struct DevMesh {
                                       // that edge is wet at k, kOwnBit / kOffBit
   const int4* erec;
   // per edge with up/down-cell levels: the up cell's two vertices besides n1 and the down
-  // cell's two besides n2, {ua, ub, da, db}, and [8 e ..] the MFCT weights of (n1, ua, ub)
-  // and (n2, da, db): (edx*a*gsca_x + edy*R*gsca_y) / 6 of each vertex
+  // cell's two besides n2, {ua, ub, da, db}, and [8 e ..] the MFCT weights of (n1, ua, ub),
+  // a pad, those of (n2, da, db) negated, a pad: (edx*a*gsca_x + edy*R*gsca_y) / 6 of each
+  // vertex, with the sign its end's gradient term has in Tm1 / Tm2
   const int4* emf4;
   const double* emfw;
+  // per node->edge slot of the segment kernels: {edge * L, other node * L (dense offsets, 32
+  // bits), 0x80000000 when the node is the edge's second node (a sign mask), 0}
+  const int4* ns4;
+  const double* iavol;   // [N,L] 1 / areasvol, correctly rounded (0 where areasvol is 0)
+  // [5,L] QR4C stencil of interface k on the static depths: the reciprocals of Z[k-1]-Z[k],
+  // Z[k]-Z[k+1], Z[k-2]-Z[k-1], then (zbar[k]-Z[k])/3, (zbar[k]-Z[k-1])/3 (k >= 2)
+  const double* qr4c;
   const uint32_t* nseg[kSegVariants];
   int64_t n_nseg[kSegVariants];
   const uint32_t* eseg[kSegVariants];
@@ -195,7 +204,9 @@ struct Workspace {
 // tracers of one entity-level are contiguous, so a neighbour gather is one contiguous
 // chunk). The workspace uses the same convention (interleaved with the same ``tg``).
 struct Inst {
-  const DevMesh* m;
+  // the mesh by value: a kernel reaches its arrays without a dependent load of the mesh
+  // record (a launch with one instance finds them in its parameters)
+  DevMesh m;
   const double *uv, *w_e, *helem, *hnode, *hnode_new;
   const double *T, *T_old;
   double* T_new;
@@ -261,8 +272,8 @@ struct FctPlan {
   void* d_static = nullptr;        // one allocation for all static arrays
   int max_tracers = 0;
   bool fused = true;               // fct_forward runs the fused stage kernels
-  int per_thread = 2;              // fused stages: most tracers per thread
-  int lpt = 4;                     //   and levels per thread
+  int per_thread = 0;              // fused stages: most tracers per thread
+  int lpt = 0;                     //   and levels per thread (0: LaunchDims::auto_map)
   bool ws_full = false;            // workspace holds every stage field (unfused / adjoint)
   double* d_ws = nullptr;          // workspace allocation
   fct::Workspace ws{};

@@ -76,7 +76,7 @@ extern "C" int fct_forward_noalloc(FctPlan* P, const FctFields* f, double dt, in
     scratch = g_scratch_ptr[P->device];
   }
   Inst in{};
-  in.m = P->d_mesh;
+  in.m = P->hm;
   in.uv = f->uv; in.w_e = f->w_e; in.helem = f->helem;
   in.hnode = f->hnode; in.hnode_new = f->hnode_new;
   in.T = f->T; in.T_old = f->T_old; in.T_new = f->T_new;
@@ -92,7 +92,7 @@ extern "C" int fct_forward_noalloc(FctPlan* P, const FctFields* f, double dt, in
   dims_cover(dims, P);
   dims.ntr = ntr;
   dims.chunk = 0;
-  dims.set_map(P->per_thread, P->lpt);
+  dims_map(dims, P);
   dims.any_wi = f->w_i != nullptr;
   dims.copy_dry = true;
   return restore(launch_forward(in, nullptr, 1, dims, static_cast<cudaStream_t>(stream)));

@@ -344,6 +344,24 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   std::vector<double> Zp(L);
   for (int k = 0; k < L - 1; ++k) Zp[k] = d->Z[k];
   Zp[L - 1] = d->Z[L - 2];
+  // tables of the segment kernels (fct_internal.cuh)
+  std::vector<int4> ns4(2 * size_t(Ed));
+  for (size_t j = 0; j < ns4.size(); ++j)
+    ns4[j] = make_int4(int(uint32_t(ne_idx[j] >> 1) * uint32_t(L)),
+                       int(uint32_t(ne_oth[j]) * uint32_t(L)),
+                       (ne_idx[j] & 1) ? int(0x80000000u) : 0, 0);
+  std::vector<double> iavol(size_t(N) * L), qr4c(5 * size_t(L), 0.0);
+  for (size_t i = 0; i < iavol.size(); ++i)
+    iavol[i] = d->areasvol[i] > 0.0 ? 1.0 / d->areasvol[i] : 0.0;
+  for (int k = 2; k < L; ++k) {
+    auto gap = [](double x) { return x == 0.0 ? 1.0 : x; };
+    const double Zn = Zp[std::min(k + 1, L - 1)];
+    qr4c[k] = 1.0 / gap(Zp[k - 1] - Zp[k]);
+    qr4c[L + k] = 1.0 / gap(Zp[k] - Zn);
+    qr4c[2 * size_t(L) + k] = 1.0 / gap(Zp[k - 2] - Zp[k - 1]);
+    qr4c[3 * size_t(L) + k] = (d->zbar[k] - Zp[k]) * (1.0 / 3.0);
+    qr4c[4 * size_t(L) + k] = (d->zbar[k] - Zp[k - 1]) * (1.0 / 3.0);
+  }
   // lanes
   std::vector<uint32_t> iface, layer, edgel, eleml, dry;
   for (int n = 0; n < N; ++n) {
@@ -477,15 +495,17 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
         const int a = (p + 1) % 3, bb = (p + 2) % 3;
         const int idx[3] = {p, a, bb};
         for (int i = 0; i < 3; ++i)
-          emfw[8 * size_t(e) + 3 * r + i] = (c1 * g[idx[i]] + c2 * g[3 + idx[i]]) / 6.0;
+          emfw[8 * size_t(e) + 4 * r + i] =
+              (r == 0 ? 1.0 : -1.0) * ((c1 * g[idx[i]] + c2 * g[3 + idx[i]]) / 6.0);
         other[2 * r] = en[a];
         other[2 * r + 1] = en[bb];
       }
       emf4[e] = make_int4(other[0], other[1], other[2], other[3]);
     }
+  }
+  for (int e = 0; e < Ed; ++e)
     for (int k = ekmin[e]; k < ekmax[e]; ++k)
       if (k < tlo[e] || k >= thi[e]) efix.push_back((uint32_t(e) << kLevelBits) | uint32_t(k));
-  }
   std::vector<uint32_t> nseg[kSegVariants], eseg[kSegVariants];
   for (int v = 0; v < kSegVariants; ++v) {
     const int lpt = kSegLevels[v];
@@ -529,6 +549,8 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   size_t o_eud4 = b.add(eud4.data(), eud4.size());
   size_t o_ecell4 = b.add(ecell4.data(), ecell4.size());
   size_t o_nrec = b.add(nrec.data(), nrec.size()), o_erec = b.add(erec.data(), erec.size());
+  size_t o_ns4 = b.add(ns4.data(), ns4.size()), o_iavol = b.add(iavol.data(), iavol.size());
+  size_t o_qr4c = b.add(qr4c.data(), qr4c.size());
   size_t o_emf4 = b.add(emf4.data(), emf4.size()), o_emfw = b.add(emfw.data(), emfw.size());
   size_t o_nflags = b.add(nflags.data(), std::max<size_t>(nflags.size(), 1));
   size_t o_efix = b.add(efix.data(), std::max<size_t>(efix.size(), 1));
@@ -591,6 +613,9 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   m.erec = (const int4*)(base + o_erec);
   m.emf4 = (const int4*)(base + o_emf4);
   m.emfw = (const double*)(base + o_emfw);
+  m.ns4 = (const int4*)(base + o_ns4);
+  m.iavol = (const double*)(base + o_iavol);
+  m.qr4c = (const double*)(base + o_qr4c);
   m.efix = (const uint32_t*)(base + o_efix);
   m.n_efix = int64_t(efix.size());
   for (int v = 0; v < kSegVariants; ++v) {
@@ -701,7 +726,7 @@ int fct_vert_diff(FctPlan* P, const FctVdiffFields* f, double dt, int ntr, fct_s
   cudaGetDevice(&prev);
   if (prev != P->device) cudaSetDevice(P->device);
   Inst in{};
-  in.m = P->d_mesh;
+  in.m = P->hm;
   in.hnode_new = f->hnode_new;
   in.T = f->T;
   in.T_new = f->T_new;
@@ -757,7 +782,7 @@ int fct_forward_ex(FctPlan* P, const FctFields* f, double dt, int ntr, int flags
     return set_error(FCT_ERR_INVALID, "Z3d and zbar3 must be given together");
   if (!(dt > 0.0)) return set_error(FCT_ERR_INVALID, "dt must be positive");
   Inst in{};
-  in.m = P->d_mesh;
+  in.m = P->hm;
   in.uv = f->uv; in.w_e = f->w_e; in.helem = f->helem;
   in.hnode = f->hnode; in.hnode_new = f->hnode_new;
   in.T = f->T; in.T_old = f->T_old; in.T_new = f->T_new;
@@ -773,7 +798,7 @@ int fct_forward_ex(FctPlan* P, const FctFields* f, double dt, int ntr, int flags
   dims_cover(dims, P);
   dims.ntr = ntr;
   dims.chunk = 0;       // one workspace chunk: all ntr tracers
-  dims.set_map(P->per_thread, P->lpt);
+  dims_map(dims, P);
   dims.any_wi = f->w_i != nullptr;
   dims.copy_dry = true;   // a fresh T_new: dry levels keep T (tracer_adv.py:147-151)
   dims.fused = !stagewise;

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(128) k_compute_w(const DevMesh* __restrict__ m
 __global__ void __launch_bounds__(128) k_compute_w_n(const Inst* __restrict__ tab) {
   const Inst& in = tab[blockIdx.y];
   if (!in.w_derived) return;
-  compute_w_column(*in.m, in.uv, in.helem, in.w_derived, blockIdx.x * 4 + (threadIdx.x >> 5),
+  compute_w_column(in.m, in.uv, in.helem, in.w_derived, blockIdx.x * 4 + (threadIdx.x >> 5),
                    threadIdx.x & 31);
 }
 

@@ -5,20 +5,22 @@
 namespace fct {
 namespace {
 
-FCT_SEG_KERNEL(k_seg_edge, seg_edge_adf)
+FCT_SEG_KERNEL(k_seg_edge, seg_edge_adf, kStageEdge)
 
 // the remaining edge lanes: one lane per thread (tracer slices as in the segment kernels)
 template <int NTR>
-__global__ void __launch_bounds__(256) k_edge_fix_1(Inst in, int t0, int w0) {
+__global__ void __launch_bounds__(256) k_edge_fix_1(const __grid_constant__ Inst in, int t0, int w0) {
   const int sub = int(blockIdx.y) * NTR;
   body_edge_fix<NTR, false>(in, lane_index(), t0 + sub, w0 + sub);
 }
 template <int NTR>
 __global__ void __launch_bounds__(256) k_edge_fix_n(const Inst* __restrict__ tab, int t0, int w0,
-                                                    int lg) {
-  const int64_t g = lane_index();
-  const int sub = int(g & ((int64_t(1) << lg) - 1)) * NTR;
-  body_edge_fix<NTR, true>(tab[blockIdx.y], g >> lg, t0 + sub, w0 + sub);
+                                                    int S, unsigned mul) {
+  const int slots = slice_div(256, mul), slot = slice_div(int(threadIdx.x), mul);
+  if (slot >= slots) return;
+  const int sub = (int(threadIdx.x) - slot * S) * NTR;
+  body_edge_fix<NTR, true>(tab[blockIdx.y], int64_t(blockIdx.x) * slots + slot, t0 + sub,
+                           w0 + sub);
 }
 
 }  // namespace
@@ -27,22 +29,21 @@ int launch_edge_fix(const Inst& single, const Inst* tab, int n, const LaunchDims
                     int c1, cudaStream_t s) {
   if (d.max_efix == 0) return FCT_OK;
   for (int t0 = c0; t0 < c1;) {
-    const int rem = c1 - t0;
-    const int P = seg_tracers(rem, d.smap_tracers[kStageEdge], tab != nullptr, 1, seg_even(d));
-    int lg = 0;
-    while (lg < 3 && (P << (lg + 1)) <= rem) ++lg;
-    const int w0 = t0 - c0;
+    const SegSplit sp =
+        seg_split(c1 - t0, d.smap_tracers[kStageEdge], tab != nullptr, seg_even(d));
+    const int P = sp.tracers, S = sp.slices, w0 = t0 - c0;
     if (tab) {
-      const dim3 g(seg_blocks(d.max_efix << lg), unsigned(n));
-      if (P == 4) k_edge_fix_n<4><<<g, 256, 0, s>>>(tab, t0, w0, lg);
-      else if (P == 2) k_edge_fix_n<2><<<g, 256, 0, s>>>(tab, t0, w0, lg);
-      else k_edge_fix_n<1><<<g, 256, 0, s>>>(tab, t0, w0, lg);
+      const unsigned mul = 65536u / unsigned(S) + 1u;
+      const dim3 g(seg_blocks(d.max_efix, 256 / S), unsigned(n));
+      if (P == 4) k_edge_fix_n<4><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);
+      else if (P == 2) k_edge_fix_n<2><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);
+      else k_edge_fix_n<1><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);
     } else {
-      const dim3 g(seg_blocks(d.max_efix), 1u << lg);
+      const dim3 g(seg_blocks(d.max_efix, 256), unsigned(S));
       if (P == 2) k_edge_fix_1<2><<<g, 256, 0, s>>>(single, t0, w0);
       else k_edge_fix_1<1><<<g, 256, 0, s>>>(single, t0, w0);
     }
-    t0 += P << lg;
+    t0 += P * S;
   }
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FCT_OK : cuda_error(e, "launch_edge_fix");
@@ -51,7 +52,7 @@ int launch_edge_fix(const Inst& single, const Inst* tab, int n, const LaunchDims
 namespace {
 
 #define FCT_COUNT(V) d.max_eseg[V]
-FCT_SEG_LAUNCHER(launch_impl, k_seg_edge, FCT_COUNT, FCT_GRID_N, FCT_GRID_1, kStageEdge)
+FCT_SEG_LAUNCHER(launch_impl, k_seg_edge, FCT_COUNT, FCT_GRID, kStageEdge)
 #undef FCT_COUNT
 
 }  // namespace

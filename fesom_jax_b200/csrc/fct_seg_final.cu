@@ -5,10 +5,10 @@
 namespace fct {
 namespace {
 
-FCT_SEG_KERNEL(k_seg_final, seg_node_final)
+FCT_SEG_KERNEL(k_seg_final, seg_node_final, kStageFinal)
 
 #define FCT_COUNT(V) d.max_nseg[V]
-FCT_SEG_LAUNCHER(launch_impl, k_seg_final, FCT_COUNT, FCT_GRID_N, FCT_GRID_1, kStageFinal)
+FCT_SEG_LAUNCHER(launch_impl, k_seg_final, FCT_COUNT, FCT_GRID, kStageFinal)
 #undef FCT_COUNT
 
 }  // namespace

@@ -53,19 +53,59 @@ __device__ __forceinline__ double ab2f(double T, double To) { return fma(kAbNew,
 // slot's gathers do not wait behind its record (2-4% faster per node kernel on the
 // CORE2-size batched step)
 #define FCT_SLOT_BEGIN(e0, e1) \
-  int4 sl_nx = (e0) < (e1) ? __ldg(m.ne4 + (e0)) : make_int4(0, 0, 0, 0);
+  int4 sl_nx = (e0) < (e1) ? __ldg(m.ns4 + (e0)) : make_int4(0, 0, 0, 0);
 #define FCT_SLOT_GET(j, e1) \
   const int4 sl = sl_nx;    \
-  if ((j) + 1 < (e1)) sl_nx = __ldg(m.ne4 + (j) + 1);
+  if ((j) + 1 < (e1)) sl_nx = __ldg(m.ns4 + (j) + 1);
 
 // a level clamped into [0, L - 1]: loads at clamped levels are in bounds and their values
 // are discarded by the predicates that follow
 __device__ __forceinline__ int kclamp(int k, int L) { return k < 0 ? 0 : (k >= L ? L - 1 : k); }
 
+// A field of NTR tracers with its base addresses formed once per thread: interleaved, one
+// address (tracer t0) indexed by entity-level x interleave stride; tracer-major, one per
+// tracer indexed by the entity-level. The slot loops then form one 32-bit offset per slot
+// and level and one 64-bit address per load.
+template <int NTR, bool IL>
+struct Fld {
+  const double* p[IL ? 1 : NTR];
+  __device__ __forceinline__ Fld(const double* base, int t0, int64_t stride) {
+    if constexpr (IL) {
+      p[0] = base + t0;
+    } else {
+#pragma unroll
+      for (int i = 0; i < NTR; ++i) p[i] = base + int64_t(t0 + i) * stride;
+    }
+  }
+  // the offset of entity-level q (below 2^32, see tix)
+  __device__ __forceinline__ static uint32_t off(uint32_t q, int tg) {
+    return IL ? q * uint32_t(tg) : q;
+  }
+  __device__ __forceinline__ void ld(uint32_t o, double (&v)[NTR]) const {
+    if constexpr (IL && (NTR % 2 == 0)) {
+      const double2* b = reinterpret_cast<const double2*>(p[0] + o);
+#pragma unroll
+      for (int i = 0; i < NTR; i += 2) {
+        const double2 x = __ldg(b + i / 2);
+        v[i] = x.x;
+        v[i + 1] = x.y;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NTR; ++i) v[i] = __ldg(IL ? p[0] + o + i : p[IL ? 0 : i] + o);
+    }
+  }
+};
+
+// x with its sign bit flipped where ``mask`` is 0x80000000 (0: unchanged)
+__device__ __forceinline__ double flip_sign(double x, int mask) {
+  return __hiloint2double(__double2hiint(x) ^ mask, __double2loint(x));
+}
+
 // ----------------------------------------------------------- LO and adf_v, node runs
 template <int NTR, int LPT, bool IL>
 __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   constexpr int V = seg_variant(LPT);
   if (si >= m.n_nseg[V]) return;
   const uint32_t sg = __ldg(m.nseg[V] + si);
@@ -75,51 +115,78 @@ __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, 
   const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
   const int nk = min(LPT, nzmax - k0);   // layers of this run
   const uint32_t base = lq(n, L, 0);
-  const int64_t ts = in.tstride;
   const int tg = in.tg;
   const double dt = in.dt;
+  using F = Fld<NTR, IL>;
+  const F fT(in.T, t0, in.tstride);
+  unsigned onb[LPT];   // per layer of the run: bit j, the j-th slot's edge has the layer
+  uint32_t kk[LPT];    // the run's layers (beyond the run: its first again, bits 0)
+#pragma unroll
+  for (int l = 0; l < LPT; ++l) {
+    onb[l] = l < nk ? unsigned(__ldg(m.nflags + rec.w + (k0 + l - nzmin))) & kSlotBits : 0u;
+    kk[l] = uint32_t(k0 + (l < nk ? l : 0));
+  }
+
+  // compute_fct_lo: edge->node upwind divergence in ascending edge id. With s the volume
+  // flux out of the node, the face flux -0.5*(T1*(vf+|vf|) + T2*(vf-|vf|)) is -T*s of the
+  // upwind end: outflows sum their s (times the own T once, after the loop), inflows add
+  // |s| times the neighbour's T.
+  double div[LPT][NTR], out[LPT];
+#pragma unroll
+  for (int l = 0; l < LPT; ++l) {
+    out[l] = 0.0;
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) div[l][t] = 0.0;
+  }
+  const int e0 = rec.x, e1 = rec.x + int((pk >> 16) & 255u);
+  // kSlotBatch slots at a time: their gathers are all issued before any is used (U = 2: 154
+  // us against 161 for T and S on the CORE2-size mesh; in the limiter and the final stage,
+  // which hold three values per slot, the registers cost more than it gives). Slots past the
+  // node's last repeat it with their bits 0; a slot off at a layer reads the own value,
+  // times 0.
+  constexpr int U = 2;
+  int4 sl[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    sl[u] = e0 < e1 ? __ldg(m.ns4 + min(e0 + u, e1 - 1)) : make_int4(0, 0, 0, 0);
+  for (int j = e0; j < e1; j += U) {
+    double vf[U][LPT], To[U][LPT][NTR];
+    int sgn[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      sgn[u] = sl[u].z;
+#pragma unroll
+      for (int l = 0; l < LPT; ++l) {
+        const bool on = (onb[l] >> u) & 1u;
+        vf[u][l] = __ldg(in.ws.vflux + (uint32_t(sl[u].x) + kk[l]));
+        fT.ld(F::off((on ? uint32_t(sl[u].y) : base) + kk[l], tg), To[u][l]);
+      }
+    }
+    if (j + U < e1) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) sl[u] = __ldg(m.ns4 + min(j + U + u, e1 - 1));
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int l = 0; l < LPT; ++l) {
+        const double s = flip_sign(vf[u][l], sgn[u]);
+        const bool on = (onb[l] >> u) & 1u, leaves = s > 0.0;
+        const double cin = (on && !leaves) ? -s : 0.0;
+        if (on && leaves) out[l] += s;
+#pragma unroll
+        for (int t = 0; t < NTR; ++t) div[l][t] = fma(cin, To[u][l][t], div[l][t]);
+      }
+#pragma unroll
+    for (int l = 0; l < LPT; ++l) onb[l] >>= U;
+  }
+
   // T of the column at levels k0-2 .. k0+LPT (Tw[i] <-> level k0-2+i; the level above
   // the surface reads T[0], the reference's edge-replicated top)
   double Tw[LPT + 3][NTR];
 #pragma unroll
   for (int i = 0; i < LPT + 3; ++i)
-    ldv<NTR, IL>(in.T, base + uint32_t(kclamp(k0 - 2 + i, L)), t0, ts, tg, Tw[i]);
-
-  // compute_fct_lo: edge->node upwind divergence in ascending edge id
-  double div[LPT][NTR];
-#pragma unroll
-  for (int l = 0; l < LPT; ++l)
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) div[l][t] = 0.0;
-  unsigned long long fl_[LPT];   // the run's node-layer flags (0 beyond the run)
-#pragma unroll
-  for (int l = 0; l < LPT; ++l) fl_[l] = l < nk ? __ldg(m.nflags + rec.w + (k0 + l - nzmin)) : 0ull;
-  const int e0 = rec.x, e1 = rec.x + int((pk >> 16) & 255u);
-  FCT_SLOT_BEGIN(e0, e1)
-  for (int j = e0; j < e1; ++j) {
-    FCT_SLOT_GET(j, e1)
-    const int jj = j - e0;
-    const bool second = sl.x & 1;
-    const double sg1 = second ? -1.0 : 1.0;   // the flux leaves the edge's first node
-    const uint32_t qe = lq(sl.x >> 1, L, 0), qo = lq(sl.y, L, 0);
-#pragma unroll
-    for (int l = 0; l < LPT; ++l) {
-      const int kc = kclamp(k0 + l, L);
-      const bool on = ((fl_[l] >> jj) & 1ull);
-      const double vf = __ldg(in.ws.vflux + qe + kc);
-      const double avf = fabs(vf);
-      // the reference's face flux -0.5*(T1*(vf+|vf|) + T2*(vf-|vf|)) with the node's own
-      // value first (a + b == b + a exactly): the same bits for either end of the edge
-      const double cown = second ? vf - avf : vf + avf, coth = second ? vf + avf : vf - avf;
-      double To[NTR];
-      ldv<NTR, IL>(in.T, qo + uint32_t(kc), t0, ts, tg, To);
-#pragma unroll
-      for (int t = 0; t < NTR; ++t) {
-        const double f = -0.5 * fma(Tw[l + 2][t], cown, To[t] * coth);
-        div[l][t] = on ? div[l][t] + sg1 * f : div[l][t];
-      }
-    }
-  }
+    fT.ld(F::off(base + uint32_t(kclamp(k0 - 2 + i, L)), tg), Tw[i]);
 
   // upwind vertical flux at the interfaces k0 .. k0+LPT (layer-masked, tracer_adv.py:108-120)
   double fv[LPT + 1][NTR];
@@ -138,24 +205,30 @@ __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, 
     if (l >= nk) break;
     const uint32_t qn = base + uint32_t(k0 + l);
     const double hn = __ldg(in.hnode + qn), hnn = __ldg(in.hnode_new + qn);
-    const double av = __ldg(m.areasvol + qn);
-    const double fdt = dt * __drcp_rn(av);   // dt / areasvol
+    const double iav = __ldg(m.iavol + qn);
+    const double fdt = dt * iav;   // dt / areasvol
     const Rcq rhn = rcpq(hnn);
-    const bool valid = (hnn > 0.0) && (av > 0.0);
+    const bool valid = (hnn > 0.0) && (iav > 0.0);
     double lo[NTR];
 #pragma unroll
-    for (int t = 0; t < NTR; ++t)
-      lo[t] = valid ? divq(fma(Tw[l + 2][t], hn, (div[l][t] + (fv[l][t] - fv[l + 1][t])) * fdt),
-                           rhn)
+    for (int t = 0; t < NTR; ++t) {
+      const double dh = fma(-out[l], Tw[l + 2][t], div[l][t]);
+      lo[t] = valid ? divq(fma(Tw[l + 2][t], hn, (dh + (fv[l][t] - fv[l + 1][t])) * fdt), rhn)
                     : 0.0;
+    }
     stv<NTR, IL>(in.ws.lo, qn, w0, in.ws.sN, in.wtg, lo);
   }
 
   // adv_flux_ver_ho (QR4C on ttfAB) minus the LO vertical flux at the layer tops
-  double To[LPT + 3][NTR];   // T_old at levels k0-2 .. k0+LPT
+  const F fTo(in.T_old, t0, in.tstride);
+  double A[LPT + 3][NTR];   // ttfAB at levels k0-2 .. k0+LPT
 #pragma unroll
-  for (int i = 0; i < LPT + 3; ++i)
-    ldv<NTR, IL>(in.T_old, base + uint32_t(kclamp(k0 - 2 + i, L)), t0, ts, tg, To[i]);
+  for (int i = 0; i < LPT + 3; ++i) {
+    double To[NTR];
+    fTo.ld(F::off(base + uint32_t(kclamp(k0 - 2 + i, L)), tg), To);
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) A[i][t] = ab2f(Tw[i][t], To[t]);
+  }
 #pragma unroll
   for (int l = 0; l < LPT; ++l) {
     if (l >= nk) break;
@@ -167,37 +240,39 @@ __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, 
     double hi[NTR];
     if (k == nzmin) {
 #pragma unroll
-      for (int t = 0; t < NTR; ++t) hi[t] = -ab2f(Tw[l + 2][t], To[l + 2][t]) * Wf * area_k;
+      for (int t = 0; t < NTR; ++t) hi[t] = -A[l + 2][t] * Wf * area_k;
     } else if (k == nzmin + 1 || k == nzmax - 1) {
 #pragma unroll
-      for (int t = 0; t < NTR; ++t)
-        hi[t] = -0.5 * (ab2f(Tw[l + 1][t], To[l + 1][t]) + ab2f(Tw[l + 2][t], To[l + 2][t])) *
-                Wf * area_k;
+      for (int t = 0; t < NTR; ++t) hi[t] = -0.5 * (A[l + 1][t] + A[l + 2][t]) * Wf * area_k;
     } else {   // nzmin + 2 <= k <= nzmax - 2
-      double Znz, Zm1, Zm2, Zp1, zb;   // QR4C stencil depths (tracer_adv.py:228-238, 265-273)
+      // QR4C stencil (tracer_adv.py:228-238, 265-273): reciprocal depth gaps and a third of
+      // the depths to the interface, from the plan's table or the moving depths
+      double rdc, rdu, rdd, d1, d2;
       if (in.Z3d) {
         const double* Zc = in.Z3d + base;
-        Znz = __ldg(Zc + k); Zm1 = __ldg(Zc + k - 1); Zm2 = __ldg(Zc + k - 2);
-        Zp1 = __ldg(Zc + (k + 1 < L ? k + 1 : L - 1)); zb = __ldg(in.zbar3 + qn);
+        const double Znz = __ldg(Zc + k), Zm1 = __ldg(Zc + k - 1), Zm2 = __ldg(Zc + k - 2);
+        const double Zp1 = __ldg(Zc + (k + 1 < L ? k + 1 : L - 1)), zb = __ldg(in.zbar3 + qn);
+        rdc = __drcp_rn(safe_nz(Zm1 - Znz));
+        rdu = __drcp_rn(safe_nz(Znz - Zp1));
+        rdd = __drcp_rn(safe_nz(Zm2 - Zm1));
+        d1 = (zb - Znz) * (1.0 / 3.0);
+        d2 = (zb - Zm1) * (1.0 / 3.0);
       } else {
-        Znz = __ldg(m.Zp + k); Zm1 = __ldg(m.Zp + k - 1); Zm2 = __ldg(m.Zp + k - 2);
-        Zp1 = __ldg(m.Zp + (k + 1 < L ? k + 1 : L - 1)); zb = __ldg(m.zbar + k);
+        const double* q = m.qr4c + k;
+        rdc = __ldg(q);
+        rdu = __ldg(q + L);
+        rdd = __ldg(q + 2 * L);
+        d1 = __ldg(q + 3 * L);
+        d2 = __ldg(q + 4 * L);
       }
-      const Rcq rdc = rcpq(safe_nz(Zm1 - Znz)), rdu = rcpq(safe_nz(Znz - Zp1)),
-                rdd = rcpq(safe_nz(Zm2 - Zm1));
-      const double d1 = (zb - Znz) * (1.0 / 3.0), d2 = (zb - Zm1) * (1.0 / 3.0);
       const double wa = -0.5 * Wf * area_k;
 #pragma unroll
       for (int t = 0; t < NTR; ++t) {
-        const double A0 = ab2f(Tw[l + 2][t], To[l + 2][t]);
-        const double Am1 = ab2f(Tw[l + 1][t], To[l + 1][t]);
-        const double Am2 = ab2f(Tw[l][t], To[l][t]);
-        const double Ap1 = ab2f(Tw[l + 3][t], To[l + 3][t]);
-        const double qc = divq(Am1 - A0, rdc);
-        const double qu = divq(A0 - Ap1, rdu);
-        const double qd = divq(Am2 - Am1, rdd);
-        const double Tmean1 = fma(fma(2.0, qc, qu), d1, A0);
-        const double Tmean2 = fma(fma(2.0, qc, qd), d2, Am1);
+        const double qc = (A[l + 1][t] - A[l + 2][t]) * rdc;
+        const double qu = (A[l + 2][t] - A[l + 3][t]) * rdu;
+        const double qd = (A[l][t] - A[l + 1][t]) * rdd;
+        const double Tmean1 = fma(fma(2.0, qc, qu), d1, A[l + 2][t]);
+        const double Tmean2 = fma(fma(2.0, qc, qd), d2, A[l + 1][t]);
         hi[t] = (Tmean1 + Tmean2) * wa;
       }
     }
@@ -212,9 +287,16 @@ __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, 
 }
 
 // ---------------------------------------------- adf_h on a run of up/down-cell levels
+// HO - LO = -0.5*((vf+|vf|)*(Tm1 - T1) + (vf-|vf|)*(Tm2 - T2)) is -vf*(Tm - T) of the
+// upwind end alone, with Tm = A_u + (2*(A_d - A_u) + edx*a*gx + edy*R*gy)/6 over that end's
+// cell (the up cell at the first node, the down cell at the second; its gradient is one
+// weighted vertex sum whose weights carry the sign of the end). So a level gathers the six
+// values of the upwind side instead of the eight of both. (A non-finite value on the
+// downwind cell still reaches both ends: it makes LO, hence the limiter factors, of the
+// downwind node non-finite.)
 template <int NTR, int LPT, bool IL>
 __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   constexpr int V = seg_variant(LPT);
   if (si >= m.n_eseg[V]) return;
   const uint32_t sg = __ldg(m.eseg[V] + si);
@@ -223,41 +305,39 @@ __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0,
   const int nk = min(LPT, int((unsigned(er.z) >> 8) & 255u) - k0);
   const int4 ov = __ldg(m.emf4 + e);
   const double2* wp = reinterpret_cast<const double2*>(m.emfw + 8 * int64_t(e));
-  const double2 w01 = __ldg(wp), w23 = __ldg(wp + 1), w45 = __ldg(wp + 2);
-  const uint32_t q1 = lq(er.x, L, 0), q2 = lq(er.y, L, 0), qe = lq(e, L, 0);
-  const uint32_t qua = lq(ov.x, L, 0), qub = lq(ov.y, L, 0);
-  const uint32_t qda = lq(ov.z, L, 0), qdb = lq(ov.w, L, 0);
-  const int64_t ts = in.tstride;
+  const double2 u01 = __ldg(wp), u2x = __ldg(wp + 1), d01 = __ldg(wp + 2), d2x = __ldg(wp + 3);
+  const uint32_t q1 = lq(er.x, L, k0), q2 = lq(er.y, L, k0), qe = lq(e, L, k0);
+  const uint32_t qua = lq(ov.x, L, k0), qub = lq(ov.y, L, k0);
+  const uint32_t qda = lq(ov.z, L, k0), qdb = lq(ov.w, L, k0);
   const int tg = in.tg;
+  using F = Fld<NTR, IL>;
+  const F fT(in.T, t0, in.tstride), fO(in.T_old, t0, in.tstride);
 #pragma unroll
   for (int l = 0; l < LPT; ++l) {
-    const int kc = kclamp(k0 + l, L);
-    const double vf = __ldg(in.ws.vflux + qe + kc);
-    const double avf = fabs(vf);
-    double T1[NTR], T2[NTR], O1[NTR], O2[NTR], ua[NTR], ub[NTR], da[NTR], db[NTR];
-    ldv<NTR, IL>(in.T, q1 + kc, t0, ts, tg, T1);
-    ldv<NTR, IL>(in.T, q2 + kc, t0, ts, tg, T2);
-    ldv<NTR, IL>(in.T_old, q1 + kc, t0, ts, tg, O1);
-    ldv<NTR, IL>(in.T_old, q2 + kc, t0, ts, tg, O2);
-    ldv<NTR, IL>(in.T, qua + kc, t0, ts, tg, ua);
-    ldv<NTR, IL>(in.T, qub + kc, t0, ts, tg, ub);
-    ldv<NTR, IL>(in.T, qda + kc, t0, ts, tg, da);
-    ldv<NTR, IL>(in.T, qdb + kc, t0, ts, tg, db);
+    const uint32_t lc = uint32_t(l < nk ? l : 0);   // levels beyond the run repeat its first
+    const double vf = __ldg(in.ws.vflux + (qe + lc));
+    const bool first = vf > 0.0;   // the first node is upwind
+    const uint32_t ou = F::off((first ? q1 : q2) + lc, tg), od = F::off((first ? q2 : q1) + lc, tg);
+    const uint32_t oa = F::off((first ? qua : qda) + lc, tg),
+                   ob = F::off((first ? qub : qdb) + lc, tg);
+    const double c0 = first ? u01.x : d01.x, c1 = first ? u01.y : d01.y,
+                 c2 = first ? u2x.x : d2x.x;
+    double Tu[NTR], Td[NTR], Ou[NTR], Od[NTR], va[NTR], vb[NTR];
+    fT.ld(ou, Tu);
+    fT.ld(od, Td);
+    fO.ld(ou, Ou);
+    fO.ld(od, Od);
+    fT.ld(oa, va);
+    fT.ld(ob, vb);
     double adf[NTR];
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
-      // Tm1 = A1 + (2*(A2 - A1) + edx*a*g_up_x + edy*R*g_up_y)/6 with the up cell's
-      // gradient as one weighted vertex sum; Tm2 likewise with the down cell's, minus
-      const double A1 = ab2f(T1[t], O1[t]), A2 = ab2f(T2[t], O2[t]);
-      const double dA = A2 - A1;
-      const double su = fma(w01.y, ua[t], fma(w23.x, ub[t], w01.x * T1[t]));
-      const double sd = fma(w23.y, T2[t], fma(w45.x, da[t], w45.y * db[t]));
-      const double Tm1 = fma(dA, 1.0 / 3.0, A1) + su;
-      const double Tm2 = fma(dA, -1.0 / 3.0, A2) - sd;
-      // HO - LO = -0.5*((vf+|vf|)*(Tm1 - T1) + (vf-|vf|)*(Tm2 - T2))
-      adf[t] = -0.5 * fma(vf + avf, Tm1 - T1[t], (vf - avf) * (Tm2 - T2[t]));
+      const double Au = ab2f(Tu[t], Ou[t]), Ad = ab2f(Td[t], Od[t]);
+      const double g = fma(c1, va[t], fma(c2, vb[t], c0 * Tu[t]));
+      const double Tm = fma(Ad - Au, 1.0 / 3.0, Au) + g;
+      adf[t] = -vf * (Tm - Tu[t]);
     }
-    if (l < nk) stv<NTR, IL>(in.ws.adfh, qe + uint32_t(kc), w0, in.ws.sEd, in.wtg, adf);
+    if (l < nk) stv<NTR, IL>(in.ws.adfh, qe + uint32_t(l), w0, in.ws.sEd, in.wtg, adf);
   }
 }
 
@@ -266,7 +346,7 @@ __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0,
 template <int NTR, bool IL>
 __device__ __forceinline__ void node_avg_grad(const Inst& in, int n, int k, int t0,
                                               double (&nx)[NTR], double (&ny)[NTR]) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   const int4 rec = __ldg(m.nrec + n);
   double den = 0.0;
 #pragma unroll
@@ -297,7 +377,7 @@ __device__ __forceinline__ void node_avg_grad(const Inst& in, int n, int k, int 
 // ----------------------------------------------- adf_h on the remaining edge lanes
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   if (i >= m.n_efix) return;
   const uint32_t lane = __ldg(m.efix + i);
   const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
@@ -353,8 +433,9 @@ __device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int t0,
 template <int NTR, int LPT, bool IL>
 __device__ __forceinline__ void seg_node_limit(const Inst& in, int64_t si, bool core, int t0,
                                                int w0, int tid, int S, double* sh) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   constexpr int V = seg_variant(LPT);
+  using F = Fld<NTR, IL>;
   const bool valid = si >= 0 && si < m.n_nseg[V];
   const int L = m.L;
   const int64_t sN = in.ws.sN;
@@ -378,49 +459,68 @@ __device__ __forceinline__ void seg_node_limit(const Inst& in, int64_t si, bool 
     nzmax = int((pk >> 8) & 255u);
     nk = min(LPT, nzmax - k0);
     base = lq(n, L, 0);
-    unsigned long long fl_[LPT];   // the run's node-layer flags (0 beyond the run)
+    const F fT(in.T, t0, in.tstride), fL(in.ws.lo, w0, sN), fA(in.ws.adfh, w0, in.ws.sEd);
+    const int tg = in.tg, wtg = in.wtg;
+    unsigned onb[LPT], wetb[LPT], cell[LPT];   // the run's node-layer flags (0 beyond the run)
+    uint32_t own[LPT];
 #pragma unroll
-    for (int l = 0; l < LPT; ++l)
-      fl_[l] = l < nk ? __ldg(m.nflags + rec.w + (k0 + l - nzmin)) : 0ull;
+    for (int l = 0; l < LPT; ++l) {
+      const unsigned long long f =
+          l < nk ? __ldg(m.nflags + rec.w + (k0 + l - nzmin)) : 0ull;
+      onb[l] = unsigned(f);
+      wetb[l] = unsigned(f >> kSlotWet);
+      cell[l] = unsigned(f >> kOwnBit);
+      own[l] = base + uint32_t(k0 + (l < nk ? l : 0));
+    }
+    // the node itself
+#pragma unroll
+    for (int l = 0; l < LPT; ++l) {
+      double tv[NTR];
+      fL.ld(F::off(own[l], wtg), lo[l]);
+      fT.ld(F::off(own[l], tg), tv);
+#pragma unroll
+      for (int t = 0; t < NTR; ++t) {
+        mx[l][t] = dmax(lo[l][t], tv[t]);
+        mn[l][t] = dmin(lo[l][t], tv[t]);
+      }
+    }
     const int e0 = rec.x, e1 = rec.x + int((pk >> 16) & 255u);
     FCT_SLOT_BEGIN(e0, e1)
     for (int j = e0; j < e1; ++j) {
       FCT_SLOT_GET(j, e1)
-      const int jj = j - e0;
-      const double sg1 = (sl.x & 1) ? -1.0 : 1.0;   // adf_h leaves the edge's first node
-      const uint32_t qo = lq(sl.y, L, 0), qe = lq(sl.x >> 1, L, 0);
 #pragma unroll
       for (int l = 0; l < LPT; ++l) {
-        const int kc = kclamp(k0 + l, L);
-        const bool wet = ((fl_[l] >> (kSlotWet + jj)) & 1ull);
-        const bool on = ((fl_[l] >> jj) & 1ull);
+        // an edge without a wet cell here reads the node's own values again (max and min do
+        // not change); one without this level adds no flux
+        const uint32_t qo = (wetb[l] & 1u) ? uint32_t(sl.y) + uint32_t(k0 + l) : own[l];
+        const bool on = onb[l] & 1u;
+        wetb[l] >>= 1;
+        onb[l] >>= 1;
         double lv[NTR], tv[NTR], a[NTR];
-        ldv<NTR, IL>(in.ws.lo, qo + uint32_t(kc), w0, sN, in.wtg, lv);
-        ldv<NTR, IL>(in.T, qo + uint32_t(kc), t0, in.tstride, in.tg, tv);
-        ldv<NTR, IL>(in.ws.adfh, qe + uint32_t(kc), w0, in.ws.sEd, in.wtg, a);
+        fL.ld(F::off(qo, wtg), lv);
+        fT.ld(F::off(qo, tg), tv);
+#pragma unroll
+        for (int t = 0; t < NTR; ++t) a[t] = 0.0;
+        if (on) fA.ld(F::off(uint32_t(sl.x) + uint32_t(k0 + l), wtg), a);
 #pragma unroll
         for (int t = 0; t < NTR; ++t) {
-          mx[l][t] = wet ? dmax(mx[l][t], dmax(lv[t], tv[t])) : mx[l][t];
-          mn[l][t] = wet ? dmin(mn[l][t], dmin(lv[t], tv[t])) : mn[l][t];
-          const double sv = sg1 * a[t];
-          sp[l][t] = on ? sp[l][t] + dmax(sv, 0.0) : sp[l][t];
-          sm[l][t] = on ? sm[l][t] + dmin(sv, 0.0) : sm[l][t];
+          mx[l][t] = dmax(mx[l][t], dmax(lv[t], tv[t]));
+          mn[l][t] = dmin(mn[l][t], dmin(lv[t], tv[t]));
+          const double sv = flip_sign(a[t], sl.z);   // adf_h leaves the edge's first node
+          if (sv > 0.0) sp[l][t] += sv;
+          if (sv < 0.0) sm[l][t] += sv;
         }
       }
     }
-    // the node itself, and the padding of dry cells
+    // no wet cell at the level: no bounds; the padding of dry cells
 #pragma unroll
     for (int l = 0; l < LPT; ++l) {
-      const int kc = kclamp(k0 + l, L);
-      double tv[NTR];
-      ldv<NTR, IL>(in.ws.lo, base + uint32_t(kc), w0, sN, in.wtg, lo[l]);
-      ldv<NTR, IL>(in.T, base + uint32_t(kc), t0, in.tstride, in.tg, tv);
-      const bool ow = (fl_[l] >> kOwnBit) & 1ull, of = (fl_[l] >> kOffBit) & 1ull;
+      const bool ow = cell[l] & 1u, of = cell[l] & 2u;
 #pragma unroll
       for (int t = 0; t < NTR; ++t) {
-        if (ow) {
-          mx[l][t] = dmax(mx[l][t], dmax(lo[l][t], tv[t]));
-          mn[l][t] = dmin(mn[l][t], dmin(lo[l][t], tv[t]));
+        if (!ow) {
+          mx[l][t] = -INFINITY;
+          mn[l][t] = INFINITY;
         }
         if (of) {
           mx[l][t] = dmax(mx[l][t], -kBig);
@@ -497,7 +597,7 @@ __device__ __forceinline__ void seg_node_limit(const Inst& in, int64_t si, bool 
 // ------------------- zalesak b3 + flux2dtracer_fct + ale_reconstruct on a layer run
 template <int NTR, int LPT, bool IL>
 __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t0, int w0) {
-  const DevMesh& m = *in.m;
+  const DevMesh& m = in.m;
   constexpr int V = seg_variant(LPT);
   constexpr int NB = LPT + 2;   // factor levels k0-1 .. k0+LPT
   if (si >= m.n_nseg[V]) return;
@@ -510,6 +610,9 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
   const uint32_t base = lq(n, L, 0);
   const int64_t sN = in.ws.sN;
   const int tg = in.tg;
+  using F = Fld<NTR, IL>;
+  const F fP(in.ws.pf, w0, sN), fM(in.ws.mf, w0, sN), fA(in.ws.adfh, w0, in.ws.sEd);
+  const int wtg = in.wtg;
   // limited horizontal fluxes, ascending edge id
   double hsc[LPT][NTR];
 #pragma unroll
@@ -519,38 +622,41 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
   double pfw[NB][NTR], mfw[NB][NTR];   // own factors at levels k0-1 .. k0+LPT
 #pragma unroll
   for (int b = 0; b < NB; ++b) {
-    const uint32_t q = base + uint32_t(kclamp(k0 - 1 + b, L));
-    ldv<NTR, IL>(in.ws.pf, q, w0, sN, in.wtg, pfw[b]);
-    ldv<NTR, IL>(in.ws.mf, q, w0, sN, in.wtg, mfw[b]);
+    const uint32_t o = F::off(base + uint32_t(kclamp(k0 - 1 + b, L)), wtg);
+    fP.ld(o, pfw[b]);
+    fM.ld(o, mfw[b]);
   }
-  unsigned long long fl_[LPT];   // the run's node-layer flags (0 beyond the run)
+  unsigned onb[LPT];   // per layer of the run: bit j, the j-th slot's edge has the layer
 #pragma unroll
-  for (int l = 0; l < LPT; ++l) fl_[l] = l < nk ? __ldg(m.nflags + rec.w + (k0 + l - nzmin)) : 0ull;
+  for (int l = 0; l < LPT; ++l)
+    onb[l] = l < nk ? unsigned(__ldg(m.nflags + rec.w + (k0 + l - nzmin))) : 0u;
   const int e0 = rec.x, e1 = rec.x + int((pk >> 16) & 255u);
   FCT_SLOT_BEGIN(e0, e1)
   for (int j = e0; j < e1; ++j) {
     FCT_SLOT_GET(j, e1)
-    const int jj = j - e0;
-    const bool second = sl.x & 1;
-    const double sg1 = second ? -1.0 : 1.0;   // adf_h leaves the edge's first node
-    const uint32_t qo = lq(sl.y, L, 0), qe = lq(sl.x >> 1, L, 0);
 #pragma unroll
     for (int l = 0; l < LPT; ++l) {
-      const int kc = kclamp(k0 + l, L);
-      const bool on = ((fl_[l] >> jj) & 1ull);
+      const bool on = onb[l] & 1u;
+      onb[l] >>= 1;
       double a[NTR], pfo[NTR], mfo[NTR];
-      ldv<NTR, IL>(in.ws.adfh, qe + uint32_t(kc), w0, in.ws.sEd, in.wtg, a);
-      ldv<NTR, IL>(in.ws.pf, qo + uint32_t(kc), w0, sN, in.wtg, pfo);
-      ldv<NTR, IL>(in.ws.mf, qo + uint32_t(kc), w0, sN, in.wtg, mfo);
+#pragma unroll
+      for (int t = 0; t < NTR; ++t) a[t] = pfo[t] = mfo[t] = 0.0;
+      if (on) {
+        const uint32_t qo = F::off(uint32_t(sl.y) + uint32_t(k0 + l), wtg);
+        fA.ld(F::off(uint32_t(sl.x) + uint32_t(k0 + l), wtg), a);
+        fP.ld(qo, pfo);
+        fM.ld(qo, mfo);
+      }
 #pragma unroll
       for (int t = 0; t < NTR; ++t) {
         // b3 (tracer_adv.py:461-465): adf >= 0 ? min(plus(n1), minus(n2)) : min(minus(n1),
-        // plus(n2)); min is exact and symmetric, so in the node's own terms the factor is
-        // min(own plus, other minus) when the flux leaves the node, else the other pair
-        const double x1 = dmin(pfw[l + 1][t], mfo[t]), x2 = dmin(mfw[l + 1][t], pfo[t]);
-        const double ae = ((a[t] >= 0.0) != second) ? x1 : x2;
-        const double lim = ae * a[t];
-        hsc[l][t] = on ? hsc[l][t] + sg1 * lim : hsc[l][t];
+        // plus(n2)); min is symmetric, so in the node's own terms the factor is min(own
+        // plus, other minus) when the flux leaves the node, else the other pair
+        const double s = flip_sign(a[t], sl.z);   // adf_h leaves the edge's first node
+        const bool leaves = s >= 0.0;
+        const double fo = leaves ? pfw[l + 1][t] : mfw[l + 1][t];
+        const double fx = leaves ? mfo[t] : pfo[t];
+        hsc[l][t] = fma(dmin(fo, fx), s, hsc[l][t]);
       }
     }
   }
@@ -560,10 +666,9 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
     if (l >= nk) break;
     const int k = k0 + l;
     const uint32_t qn = base + uint32_t(k);
-    const double av = __ldg(m.areasvol + qn);
-    const double sa = av > 0.0 ? av : 1.0;
+    const double iav = __ldg(m.iavol + qn);   // 1 / areasvol (0 where there is no volume)
     const double hn = __ldg(in.hnode + qn), hnn = __ldg(in.hnode_new + qn);
-    const double fdt = dt * __drcp_rn(sa);   // dt / areasvol
+    const double fdt = dt * (iav > 0.0 ? iav : 1.0);
     const Rcq rhn = rcpq(hnn);
     double ft[NTR], vt[NTR], vb[NTR];
     ldv<NTR, IL>(in.ws.adfv, qn, w0, sN, in.wtg, ft);
@@ -592,7 +697,7 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
       const double lo_trans = fma(lo[t], hnn, -Tv[t] * hn);
-      const double vdiv = av > 0.0 ? (vt[t] - vb[t]) * fdt : 0.0;
+      const double vdiv = iav > 0.0 ? (vt[t] - vb[t]) * fdt : 0.0;
       double d = fma(hsc[l][t], fdt, lo_trans + vdiv);
       d = fma(Tv[t], hn - hnn, d);
       out[t] = Tv[t] + (hnn > 0.0 ? divq(d, rhn) : 0.0);
@@ -605,38 +710,48 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
 // ------------------------------------------------------------- kernels and launchers
 // Kernel wrappers: ``_1`` takes one instance by value (tracer-major layout, the
 // single-call path; tracer slice = blockIdx.y), ``_n`` instance blockIdx.y of a device
-// table (interleaved layout; 2^lg adjacent threads of a segment take adjacent tracer
-// slices, so together they read whole interleaved lines).
-// Resident 256-thread blocks per SM the compiler must fit, by the updates a thread
-// carries (registers capped accordingly: the gathers are latency-bound, so resident warps
-// pay more than the spills a cap may cost). Measured on the CORE2-size batched step: one
-// block more per SM than 6/4/3/2/1 made it 5.5% faster (the autotuner then picks other
-// mappings), two more 1-9% slower.
-__host__ __device__ constexpr int seg_min_blocks(int ntr, int lpt) {
-  return ntr * lpt <= 1 ? 7 : ntr * lpt <= 2 ? 5 : ntr * lpt <= 4 ? 4 : ntr * lpt <= 8 ? 3 : 2;
+// table (interleaved layout; the S adjacent threads of a segment take adjacent tracer
+// slices, so together they read whole interleaved lines; S is any number up to 8, so an odd
+// tracer count is one launch too). A 256-thread block holds 256/S segments.
+//
+// Resident 256-thread blocks per SM the compiler must fit, by stage and by the updates u a
+// thread carries. The kernels wait on their gathers, so resident warps pay until the cap
+// makes the compiler spill. The limiter and the LO stage hold more per update and take one
+// block less: T and S on the CORE2-size mesh, 2 tracers x 1 level per thread, 64 registers
+// against 48: limiter 198 us against 297; edge 160 against 141, final 188 against 180 the
+// other way round.
+__host__ __device__ constexpr int seg_min_blocks(int stage, int u) {
+  return (stage == kStageEdge || stage == kStageFinal)
+             ? (u <= 1 ? 7 : u <= 2 ? 5 : u <= 4 ? 4 : u <= 8 ? 3 : 2)
+             : (u <= 1 ? 5 : u <= 2 ? 4 : u <= 4 ? 3 : 2);
 }
 
-#define FCT_SEG_KERNEL(name, body)                                                       \
+// thread t of a block of 256/S segments: segment t / S, slice t % S (``mul`` = 65536/S + 1
+// divides exactly below 256)
+__device__ __forceinline__ int slice_div(int t, unsigned mul) { return int((unsigned(t) * mul) >> 16); }
+
+#define FCT_SEG_KERNEL(name, body, stage)                                                \
   template <int NTR, int LPT>                                                            \
-  __global__ void __launch_bounds__(256, seg_min_blocks(NTR, LPT))                       \
-      name##_1(Inst in, int t0, int w0) {                                                \
+  __global__ void __launch_bounds__(256, seg_min_blocks(stage, NTR * LPT))               \
+      name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
     const int sub = int(blockIdx.y) * NTR;                                               \
     body<NTR, LPT, false>(in, lane_index(), t0 + sub, w0 + sub);                         \
   }                                                                                      \
   template <int NTR, int LPT>                                                            \
-  __global__ void __launch_bounds__(256, seg_min_blocks(NTR, LPT))                       \
-      name##_n(const Inst* __restrict__ tab, int t0, int w0, int lg) {                   \
-    const int64_t g = lane_index();                                                      \
-    const int sub = int(g & ((int64_t(1) << lg) - 1)) * NTR;                             \
-    body<NTR, LPT, true>(tab[blockIdx.y], g >> lg, t0 + sub, w0 + sub);                  \
+  __global__ void __launch_bounds__(256, seg_min_blocks(stage, NTR * LPT))               \
+      name##_n(const Inst* __restrict__ tab, int t0, int w0, int S, unsigned mul) {      \
+    const int slots = slice_div(256, mul), slot = slice_div(int(threadIdx.x), mul);      \
+    if (slot >= slots) return;                                                           \
+    const int sub = (int(threadIdx.x) - slot * S) * NTR;                                 \
+    body<NTR, LPT, true>(tab[blockIdx.y], int64_t(blockIdx.x) * slots + slot, t0 + sub,  \
+                         w0 + sub);                                                      \
   }
 
-// The limiter stage: 256-thread blocks of 256/S segment slots (S = 2^lg tracer-slice
-// threads per slot in ``_n``, 1 in ``_1``), the first and last slot halo runs.
+// The limiter stage: a block's first and last segment slot are halo runs.
 #define FCT_SEG_LIMIT_KERNEL(name)                                                       \
   template <int NTR, int LPT>                                                            \
-  __global__ void __launch_bounds__(256, seg_min_blocks(NTR, LPT))                       \
-      name##_1(Inst in, int t0, int w0) {                                                \
+  __global__ void __launch_bounds__(256, seg_min_blocks(kStageLimit, NTR * LPT))         \
+      name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
     __shared__ double sh[4 * NTR * 256];                                                 \
     const int tid = threadIdx.x;                                                         \
     const int64_t si = int64_t(blockIdx.x) * 254 + tid - 1;                              \
@@ -645,46 +760,28 @@ __host__ __device__ constexpr int seg_min_blocks(int ntr, int lpt) {
                                     tid, 1, sh);                                         \
   }                                                                                      \
   template <int NTR, int LPT>                                                            \
-  __global__ void __launch_bounds__(256, seg_min_blocks(NTR, LPT))                       \
-      name##_n(const Inst* __restrict__ tab, int t0, int w0, int lg) {                   \
+  __global__ void __launch_bounds__(256, seg_min_blocks(kStageLimit, NTR * LPT))         \
+      name##_n(const Inst* __restrict__ tab, int t0, int w0, int S, unsigned mul) {      \
     __shared__ double sh[4 * NTR * 256];                                                 \
     const int tid = threadIdx.x;                                                         \
-    const int slot = tid >> lg, slots = 256 >> lg;                                       \
-    const int64_t si = int64_t(blockIdx.x) * (slots - 2) + slot - 1;                     \
-    const int sub = (tid & ((1 << lg) - 1)) * NTR;                                       \
+    const int slots = slice_div(256, mul), slot = slice_div(tid, mul);                   \
+    const int64_t si =                                                                   \
+        slot < slots ? int64_t(blockIdx.x) * (slots - 2) + slot - 1 : int64_t(-1);       \
+    const int sub = slot < slots ? (tid - slot * S) * NTR : 0;                           \
     seg_node_limit<NTR, LPT, true>(tab[blockIdx.y], si, slot >= 1 && slot <= slots - 2,  \
-                                   t0 + sub, w0 + sub, tid, 1 << lg, sh);                \
+                                   t0 + sub, w0 + sub, tid, S, sh);                      \
   }
 
-inline unsigned seg_blocks(int64_t lanes) {
-  return unsigned(std::max<int64_t>(1, (lanes + 255) / 256));
+inline unsigned seg_blocks(int64_t lanes, int per_block) {
+  return unsigned(std::max<int64_t>(1, (lanes + per_block - 1) / per_block));
 }
-// grids: one thread per segment and slice; the limiter's blocks hold 256/S - 2 core slots
-#define FCT_GRID_N(lanes, lg) seg_blocks((lanes) << (lg))
-#define FCT_GRID_1(lanes) seg_blocks(lanes)
-#define FCT_LIMIT_GRID_N(lanes, lg) \
-  unsigned(std::max<int64_t>(1, ((lanes) + (256 >> (lg)) - 3) / ((256 >> (lg)) - 2)))
-#define FCT_LIMIT_GRID_1(lanes) unsigned(std::max<int64_t>(1, ((lanes) + 253) / 254))
-
-// Tracers per thread of one launch: the largest of the compiled set (1, 2 or 4 in the
-// interleaved layout, 1 when its strides are odd; 1 or 2 tracer-major) that is at most
-// ``rem`` and ``per_thread``.
-inline int seg_tracers(int rem, int per_thread, bool interleaved, int lpt, bool even) {
-  (void)lpt;
-  const int lim = std::min(rem, per_thread);
-  if (interleaved && !even) return 1;   // tracer pairs would not be 16-byte aligned
-  if (interleaved && lim >= 4) return 4;
-  return lim >= 2 ? 2 : 1;
-}
-// the interleaved tracer and workspace strides are even (tracer pairs 16-byte aligned)
-inline bool seg_even(const LaunchDims& d) {
-  const int chunk = d.chunk > 0 ? d.chunk : d.ntr;
-  return d.ntr % 2 == 0 && chunk % 2 == 0;
-}
+// grids: 256/S segments per block; the limiter's blocks hold two halo slots
+#define FCT_GRID(lanes, S) seg_blocks(lanes, 256 / (S))
+#define FCT_LIMIT_GRID(lanes, S) seg_blocks(lanes, 256 / (S) - 2)
 
 #define FCT_SEG_CASE_N(kern, P, V)                                                       \
   case P * 16 + V:                                                                       \
-    kern##_n<P, V><<<g, 256, 0, s>>>(tab, t0, w0, lg);                                   \
+    kern##_n<P, V><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);                               \
     break;
 #define FCT_SEG_CASE_1(kern, P, V)                                                       \
   case P * 16 + V:                                                                       \
@@ -692,9 +789,9 @@ inline bool seg_even(const LaunchDims& d) {
     break;
 
 // One segment stage over the tracers [c0, c1) of a workspace chunk (workspace index of
-// tracer t is t - c0): launches of P tracers x 2^lg slices. ``COUNT(V)`` is the largest
+// tracer t is t - c0): launches of P tracers x S slices. ``COUNT(V)`` is the largest
 // segment count of the variant over the launch's instances.
-#define FCT_SEG_LAUNCHER(fn, kern, COUNT, GRID_N, GRID_1, STAGE)                         \
+#define FCT_SEG_LAUNCHER(fn, kern, COUNT, GRID, STAGE)                                   \
   int fn(const Inst& single, const Inst* tab, int n, const LaunchDims& d, int c0, int c1, \
          cudaStream_t s) {                                                               \
     const int lpt = d.smap_levels[STAGE], per_thread = d.smap_tracers[STAGE];            \
@@ -702,12 +799,11 @@ inline bool seg_even(const LaunchDims& d) {
     const int64_t lanes = COUNT(V);                                                      \
     for (int t0 = c0; t0 < c1;) {                                                        \
       const int rem = c1 - t0;                                                           \
-      const int P = seg_tracers(rem, per_thread, tab != nullptr, lpt, seg_even(d));      \
-      int lg = 0;                                                                        \
-      while (lg < 3 && (P << (lg + 1)) <= rem) ++lg;                                     \
-      const int w0 = t0 - c0;                                                            \
+      const SegSplit sp = seg_split(rem, per_thread, tab != nullptr, seg_even(d));       \
+      const int P = sp.tracers, S = sp.slices, w0 = t0 - c0;                             \
       if (tab) {                                                                         \
-        const dim3 g(GRID_N(lanes, lg), unsigned(n));                                    \
+        const unsigned mul = 65536u / unsigned(S) + 1u;                                  \
+        const dim3 g(GRID(lanes, S), unsigned(n));                                       \
         switch (P * 16 + lpt) {                                                          \
           FCT_SEG_CASE_N(kern, 1, 1) FCT_SEG_CASE_N(kern, 1, 2)                          \
           FCT_SEG_CASE_N(kern, 1, 4) FCT_SEG_CASE_N(kern, 1, 8)                          \
@@ -720,7 +816,7 @@ inline bool seg_even(const LaunchDims& d) {
                              "levels per thread", P, lpt);                              \
         }                                                                                \
       } else {                                                                           \
-        const dim3 g(GRID_1(lanes), 1u << lg);                                           \
+        const dim3 g(GRID(lanes, 1), unsigned(S));                                       \
         switch (P * 16 + lpt) {                                                          \
           FCT_SEG_CASE_1(kern, 1, 1) FCT_SEG_CASE_1(kern, 1, 2)                          \
           FCT_SEG_CASE_1(kern, 1, 4) FCT_SEG_CASE_1(kern, 1, 8)                          \
@@ -731,7 +827,7 @@ inline bool seg_even(const LaunchDims& d) {
                              "levels per thread", P, lpt);                              \
         }                                                                                \
       }                                                                                  \
-      t0 += P << lg;                                                                     \
+      t0 += P * S;                                                                       \
     }                                                                                    \
     const cudaError_t e = cudaGetLastError();                                            \
     return e == cudaSuccess ? FCT_OK : cuda_error(e, #fn);                               \

@@ -93,8 +93,10 @@ class Ensemble:
         self._h = None
         self.phase = 0
         self.chunk = 2          # tracers per thread of the fused stages
-        self.levels = 4         # levels per thread
-        self.stage_map = [(2, 4)] * 4   # per fused stage (LO, edge, limiter, final)
+        self.levels = 1         # levels per thread
+        # per fused stage (LO, edge, limiter, final); until a mapping is set the library
+        # takes two levels per thread in the LO stage of large launches
+        self.stage_map = [(2, 1)] * 4
 
     # ---------------------------------------------------------------- members
     def plan(self, mesh: Mesh) -> FctPlan:
