@@ -41,11 +41,18 @@ struct FctBatch {
   Fork fork{};   // the edge stage beside the LO stage (graph capture and fct_batch_step)
 };
 
-static int batch_launch_step(FctBatch* b, int phase, cudaStream_t s) {
+// ``steps`` consecutive steps, group by group (instances are independent): a group's volume
+// fluxes, and the w it derives, depend only on inputs that a run does not change, so its first
+// step forms them and the others find them in the group's workspace.
+static int batch_launch_steps(FctBatch* b, int phase, int steps, cudaStream_t s) {
   for (auto& g : b->groups) {
-    Inst dummy{};
-    const int st = launch_forward(dummy, g.d_tab[phase % 3], g.count, g.dims, s);
-    if (st) return st;
+    LaunchDims d = g.dims;
+    for (int k = 0; k < steps; ++k) {
+      Inst dummy{};
+      d.skip_vflux = k > 0;
+      const int st = launch_forward(dummy, g.d_tab[(phase + k) % 3], g.count, d, s);
+      if (st) return st;
+    }
   }
   return FCT_OK;
 }
@@ -298,7 +305,7 @@ int fct_batch_step(FctBatch* B, int phase, fct_stream_t stream) {
   int prev = -1;
   cudaGetDevice(&prev);
   cudaSetDevice(B->device);
-  const int st = batch_launch_step(B, phase, static_cast<cudaStream_t>(stream));
+  const int st = batch_launch_steps(B, phase, 1, static_cast<cudaStream_t>(stream));
   if (prev >= 0) cudaSetDevice(prev);
   return st;
 }
@@ -320,8 +327,7 @@ int fct_batch_run(FctBatch* B, int first_phase, int steps, fct_stream_t stream) 
     } else {
       cudaError_t e = cudaStreamBeginCapture(B->cap_stream, cudaStreamCaptureModeThreadLocal);
       if (e != cudaSuccess) return restore(cuda_error(e, "cudaStreamBeginCapture"));
-      int st = FCT_OK;
-      for (int k = 0; k < steps && !st; ++k) st = batch_launch_step(B, first_phase + k, B->cap_stream);
+      const int st = batch_launch_steps(B, first_phase, steps, B->cap_stream);
       cudaGraph_t graph = nullptr;
       e = cudaStreamEndCapture(B->cap_stream, &graph);
       if (st) { if (graph) cudaGraphDestroy(graph); return restore(st); }

@@ -1,0 +1,210 @@
+// Column solves staged through shared memory: the implicit vertical diffusion and the
+// implicit part of the split vertical velocity. A tridiagonal recursion is sequential in the
+// level, so one thread walks a column; read straight from memory every step of that walk
+// waits for a strided load (T of 60,000 columns x 48 levels: 212 us per tracer at 32% of the
+// memory rate with 11% of the issue slots used). Here a block takes kColumns columns:
+//   1. all threads form the rows' coefficients and right-hand sides, levels adjacent (whole
+//      lines), into shared memory;
+//   2. one thread per column and tracer eliminates and substitutes back in shared memory
+//      (rows padded to an odd length, so that neighbouring columns use different banks);
+//   3. all threads write the result, levels adjacent.
+#pragma once
+
+#include "fct_device.cuh"
+
+namespace fct {
+namespace {
+
+constexpr int kColThreads = 128;
+constexpr int kColMaxSmem = 227 << 10;   // opt-in shared memory of a block
+
+// Shared rows of a block: a, b, c, cp of the matrix and one right-hand side per tracer, each
+// [columns][stride].
+struct ColRows {
+  double *a, *b, *c, *cp, *r;
+  int stride, columns;
+  __device__ __forceinline__ ColRows(double* sh, int columns_, int L)
+      : stride(L | 1), columns(columns_) {
+    const int n = columns * stride;
+    a = sh;
+    b = sh + n;
+    c = sh + 2 * n;
+    cp = sh + 3 * n;
+    r = sh + 4 * n;
+  }
+  __device__ __forceinline__ int at(int col, int k) const { return col * stride + k; }
+  __device__ __forceinline__ double* rhs(int t) const { return r + t * columns * stride; }
+};
+
+inline size_t col_smem(int columns, int L, int nt) {
+  return size_t(columns) * size_t(L | 1) * size_t(4 + nt) * sizeof(double);
+}
+// Columns per block: as many (32, 16 or 8) as keep about four blocks on an SM and one
+// thread per column and tracer.
+inline int col_columns(int L, int nt) {
+  for (int c : {32, 16})
+    if (col_smem(c, L, nt) <= size_t(56) << 10 && c * nt <= kColThreads) return c;
+  return 8;
+}
+
+// Thomas algorithm over the rows [nzmin, nzmax) of every column of the block (fesom_jax/
+// ops.py:121-168; the padded rows above and below solve to exactly 0). The solution
+// replaces the right-hand side. Every thread of the block calls it, after a barrier.
+__device__ __forceinline__ void col_solve(const DevMesh& m, const ColRows& s, int n0, int nt) {
+  const int tid = threadIdx.x, col = tid % s.columns, t = tid / s.columns, n = n0 + col;
+  const bool on = t < nt && n < m.N;
+  const int nzmin = on ? ld(m.nzmin + n) : 0, nzmax = on ? ld(m.nzmax + n) : 0;
+  double* r = s.rhs(on ? t : 0);
+  double cprev = 0.0, dprev = 0.0;
+  for (int k = nzmin; k < nzmax; ++k) {
+    const int i = s.at(col, k);
+    const double a = s.a[i];
+    const Rcp rm = rcp(s.b[i] - a * cprev);
+    cprev = divr(s.c[i], rm);
+    if (t == 0) s.cp[i] = cprev;
+    dprev = divr(r[i] - a * dprev, rm);
+    r[i] = dprev;
+  }
+  __syncthreads();
+  double x = 0.0;
+  for (int k = nzmax - 1; k >= nzmin; --k) {
+    const int i = s.at(col, k);
+    x = r[i] - s.cp[i] * x;
+    r[i] = x;
+  }
+  __syncthreads();
+}
+
+// ------------- implicit vertical diffusion (tracer_diff.py:68-123, ops.py:121-168) of the
+// tracers [t0, t0 + nt) of the columns [n0, n0 + columns)
+template <bool IL>
+__device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns, int t0, int nt,
+                                            double* sh) {
+  const DevMesh& m = in.m;
+  if (!in.Kv || n0 >= m.N) return;   // block-uniform
+  const int L = m.L;
+  const ColRows s(sh, columns, L);
+  const int64_t ts = in.tstride;
+  const int tg = in.tg;
+  const double* Tin = in.vd_T;
+  const double dt = in.dt;
+  for (int i = threadIdx.x; i < columns * L; i += kColThreads) {
+    const int col = i / L, k = i - col * L, n = n0 + col;
+    if (n >= m.N) break;
+    const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
+    if (k < nzmin || k >= nzmax) continue;
+    const uint32_t base = lq(n, L, 0), q = base + uint32_t(k);
+    const double* Zc = in.vd_Z3d ? in.vd_Z3d + base : m.Zp;
+    const bool last = k + 1 >= L;
+    double dzu = k == 0 ? 0.0 : ld(Zc + k - 1) - ld(Zc + k);
+    double dzd = ld(Zc + k) - (last ? 0.0 : ld(Zc + k + 1));
+    dzu = dzu == 0.0 ? 1.0 : dzu;
+    dzd = dzd == 0.0 ? 1.0 : dzd;
+    const double av = ld(m.areasvol + q);
+    const double sav = av > 0.0 ? av : 1.0;
+    const double ar = ld(m.area + q), arp = last ? 0.0 : ld(m.area + q + 1);
+    const double kv = ld(in.Kv + q), kvp = last ? 0.0 : ld(in.Kv + q + 1);
+    const double a_full = -kv * dt / dzu * (ar / sav);
+    const double c_full = -kvp * dt / dzd * (arp / sav);
+    const double a = k == nzmin ? 0.0 : a_full;
+    const double c = k == nzmax - 1 ? 0.0 : c_full;
+    const int j = s.at(col, k);
+    s.a[j] = a;
+    s.c[j] = c;
+    s.b[j] = -a - c + ld(in.hnode_new + q);
+    double swd = 0.0;
+    if (in.sw_3d) {
+      const double sw = ld(in.sw_3d + q), swp = last ? 0.0 : ld(in.sw_3d + q + 1);
+      swd = (sw - swp * (arp / sav)) * dt;
+    }
+    for (int t = 0; t < nt; ++t) {
+      const double Tc = Tin[tix<IL>(q, t0 + t, ts, tg)];
+      const double Tm = Tin[tix<IL>(k > 0 ? q - 1 : q, t0 + t, ts, tg)];
+      const double Tp = last ? 0.0 : Tin[tix<IL>(q + 1, t0 + t, ts, tg)];
+      double rhs = a * (Tc - Tm) + c * (Tc - Tp);
+      if (in.bc_surf)
+        rhs = rhs + (k == nzmin ? ld(in.bc_surf + (t0 + t) * in.bc_stride + n) : 0.0);
+      if (in.sw_3d && t0 + t == in.sw_tracer) rhs = rhs + swd;
+      s.rhs(t)[j] = rhs;
+    }
+  }
+  __syncthreads();
+  col_solve(m, s, n0, nt);
+  const bool copy = Tin != in.T_new;   // out of place: dry levels keep T
+  if constexpr (IL) {
+    for (int i = threadIdx.x; i < columns * L * nt; i += kColThreads) {
+      const int e = i / nt, t = i - e * nt, col = e / L, k = e - col * L, n = n0 + col;
+      if (n >= m.N) break;
+      const int64_t o = tix<IL>(lq(n, L, k), t0 + t, ts, tg);
+      if (k >= ld(m.nzmin + n) && k < ld(m.nzmax + n)) in.T_new[o] = Tin[o] + s.rhs(t)[s.at(col, k)];
+      else if (copy) in.T_new[o] = Tin[o];
+    }
+  } else {
+    for (int t = 0; t < nt; ++t)
+      for (int i = threadIdx.x; i < columns * L; i += kColThreads) {
+        const int col = i / L, k = i - col * L, n = n0 + col;
+        if (n >= m.N) break;
+        const int64_t o = tix<IL>(lq(n, L, k), t0 + t, ts, tg);
+        if (k >= ld(m.nzmin + n) && k < ld(m.nzmax + n))
+          in.T_new[o] = Tin[o] + s.rhs(t)[s.at(col, k)];
+        else if (copy) in.T_new[o] = Tin[o];
+      }
+  }
+}
+
+// ---------------------------- adv_tra_vert_impl (tracer_adv.py:487-529): implicit w_i
+// advection of LO, the tracers' workspace slots [w0, w0 + nt)
+template <bool IL>
+__device__ __forceinline__ void block_vert_impl(const Inst& in, int n0, int columns, int w0,
+                                                int nt, double* sh) {
+  const DevMesh& m = in.m;
+  if (!in.w_i || n0 >= m.N) return;   // block-uniform
+  const int L = m.L;
+  const ColRows s(sh, columns, L);
+  const int64_t sN = in.ws.sN;
+  const double dt = in.dt;
+  double* LO = in.ws.lo;
+  for (int i = threadIdx.x; i < columns * L; i += kColThreads) {
+    const int col = i / L, k = i - col * L, n = n0 + col;
+    if (n >= m.N) break;
+    const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
+    if (k < nzmin || k >= nzmax) continue;
+    const uint32_t q = lq(n, L, k);
+    const double av = ld(m.areasvol + q);
+    const double sa = av > 0.0 ? av : 1.0;
+    const double v_top = dt * ld(m.area + q) / sa;
+    const double v_bot = dt * (k + 1 < L ? ld(m.area + q + 1) : 0.0) / sa;
+    const double wu = ld(in.w_i + q), wd = k + 1 < L ? ld(in.w_i + q + 1) : 0.0;
+    const bool surf = k == nzmin, bot = k == nzmax - 1;
+    const double a = (surf ? 0.0 : fmin(0.0, wu)) * v_top;
+    const double b_top = (surf ? wu : fmax(0.0, wu)) * v_top;
+    const double b_bot = (bot ? 0.0 : -fmin(0.0, wd)) * v_bot;
+    const double c = (bot ? 0.0 : -fmax(0.0, wd)) * v_bot;
+    const double b_adv = b_top + b_bot;
+    const int j = s.at(col, k);
+    s.a[j] = a;
+    s.c[j] = c;
+    s.b[j] = ld(in.hnode_new + q) + b_adv;
+    for (int t = 0; t < nt; ++t) {
+      // the neighbours above the surface and below the bottom enter with a zero
+      // coefficient; LO is 0 there in the reference, and this step never wrote them
+      const double Tm = surf ? 0.0 : LO[tix<IL>(q - 1, w0 + t, sN, in.wtg)];
+      const double T0 = LO[tix<IL>(q, w0 + t, sN, in.wtg)];
+      const double Tp = bot ? 0.0 : LO[tix<IL>(q + 1, w0 + t, sN, in.wtg)];
+      s.rhs(t)[j] = -(a * Tm + b_adv * T0 + c * Tp);
+    }
+  }
+  __syncthreads();
+  col_solve(m, s, n0, nt);
+  for (int t = 0; t < nt; ++t)
+    for (int i = threadIdx.x; i < columns * L; i += kColThreads) {
+      const int col = i / L, k = i - col * L, n = n0 + col;
+      if (n >= m.N) break;
+      if (k < ld(m.nzmin + n) || k >= ld(m.nzmax + n)) continue;
+      const int64_t o = tix<IL>(lq(n, L, k), w0 + t, sN, in.wtg);
+      LO[o] = LO[o] + s.rhs(t)[s.at(col, k)];
+    }
+}
+
+}  // namespace
+}  // namespace fct

@@ -23,7 +23,7 @@
 // contiguous chunk in the interleaved layout), so the gathers overlap.
 #include <algorithm>
 
-#include "fct_device.cuh"
+#include "fct_columns.cuh"
 
 namespace fct {
 
@@ -229,53 +229,6 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
     adf[t] = hi[t] - lo_v;
   }
   stn<NTR, IL>(in.ws.adfv, qn, w0, in.ws.sN, in.wtg, adf);
-}
-
-// ---------------------------- adv_tra_vert_impl: implicit w_i advection of LO
-template <int NTR, bool IL>
-__device__ __forceinline__ void body_vert_impl(const Inst& in, int64_t n, int t0, int w0) {
-  const DevMesh& m = in.m;
-  if (n >= m.N || !in.w_i) return;
-  const int L = m.L;
-  const int nzmin = m.nzmin[n], nzmax = m.nzmax[n];
-  if (nzmax <= nzmin) return;
-  const uint32_t base = lq(int(n), L, 0);
-  const double dt = in.dt;
-  double cp[kMaxLevels], dp[kMaxLevels];
-  for (int tw = w0; tw < w0 + NTR; ++tw) {
-    auto LO = [&](int k) -> double& { return in.ws.lo[tix<IL>(base + k, tw, in.ws.sN, in.wtg)]; };
-    double cprev = 0.0, dprev = 0.0;
-    for (int k = nzmin; k < nzmax; ++k) {
-      const double av = m.areasvol[base + k];
-      const double sa = av > 0.0 ? av : 1.0;
-      const double v_top = dt * m.area[base + k] / sa;
-      const double v_bot = dt * (k + 1 < L ? m.area[base + k + 1] : 0.0) / sa;
-      const double wu = in.w_i[base + k];
-      const double wd = k + 1 < L ? in.w_i[base + k + 1] : 0.0;
-      const bool surf = (k == nzmin), bot = (k == nzmax - 1);
-      const double a = (surf ? 0.0 : fmin(0.0, wu)) * v_top;
-      const double b_top = (surf ? wu : fmax(0.0, wu)) * v_top;
-      const double b_bot = (bot ? 0.0 : -fmin(0.0, wd)) * v_bot;
-      const double c = (bot ? 0.0 : -fmax(0.0, wd)) * v_bot;
-      const double b_adv = b_top + b_bot;
-      const double b = in.hnode_new[base + k] + b_adv;
-      // the neighbours above the surface and below the bottom enter with a zero
-      // coefficient; LO is 0 there in the reference, and this step never wrote them
-      const double Tm = surf ? 0.0 : LO(k - 1), T0 = LO(k), Tp = bot ? 0.0 : LO(k + 1);
-      const double rhs = -(a * Tm + b_adv * T0 + c * Tp);
-      const double md = b - a * cprev;
-      cprev = c / md;
-      dprev = (rhs - a * dprev) / md;
-      cp[k] = cprev;
-      dp[k] = dprev;
-    }
-    double x = 0.0;
-    for (int k = nzmax - 1; k >= nzmin; --k) {
-      x = dp[k] - cp[k] * x;
-      dp[k] = x;
-    }
-    for (int k = nzmin; k < nzmax; ++k) LO(k) = LO(k) + dp[k];
-  }
 }
 
 // -------------------------- fill_up_dn_grad + adv_flux_hor_ho - LO flux = adf_h
@@ -589,98 +542,6 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
   count_nonfinite<NTR>(in.nonfinite, out);
 }
 
-// ------------- implicit vertical diffusion (tracer_diff.py:68-123, ops.py:121-168)
-// One thread per node column and NTR tracers: the Thomas algorithm over the column's wet
-// layers [nzmin, nzmax) (the reference's padded rows above and below solve to exactly 0,
-// so starting and ending the recursions there gives the same numbers). The elimination
-// factors m and cp do not depend on the tracer: one reciprocal of m serves c/m and every
-// tracer's dp/m. cp goes to workspace slot w0 of adfv, dp to the tracer's slots of lo
-// (both free after the FCT stages); the back substitution reads them in reverse.
-template <int NTR, bool IL>
-__device__ __forceinline__ void body_vdiff(const Inst& in, int64_t n, int t0, int w0) {
-  const DevMesh& m = in.m;
-  if (n >= m.N || !in.Kv) return;
-  const int L = m.L;
-  const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
-  const uint32_t base = lq(int(n), L, 0);
-  const int64_t ts = in.tstride, sN = in.ws.sN;
-  const int tg = in.tg;
-  const double* Tin = in.vd_T;
-  if (Tin != in.T_new) {   // out of place: dry levels keep T
-    for (int k = 0; k < L; ++k) {
-      if (k >= nzmin && k < nzmax) continue;
-      double v[NTR];
-      ldn<NTR, IL>(Tin, base + k, t0, ts, tg, v);
-      stn<NTR, IL>(in.T_new, base + k, t0, ts, tg, v);
-    }
-  }
-  if (nzmax <= nzmin) return;
-  const double dt = in.dt;
-  const double* Zc = in.vd_Z3d ? in.vd_Z3d + base : m.Zp;
-  double cprev = 0.0, dprev[NTR], Tm[NTR], Tc[NTR], Tp[NTR];
-#pragma unroll
-  for (int t = 0; t < NTR; ++t) dprev[t] = 0.0;
-  ldn<NTR, IL>(Tin, base + nzmin, t0, ts, tg, Tc);
-  ldn<NTR, IL>(Tin, base + (nzmin > 0 ? nzmin - 1 : 0), t0, ts, tg, Tm);
-  for (int k = nzmin; k < nzmax; ++k) {
-    const uint32_t q = base + uint32_t(k);
-    const bool last = k + 1 >= L;
-    if (last) {
-#pragma unroll
-      for (int t = 0; t < NTR; ++t) Tp[t] = 0.0;
-    } else {
-      ldn<NTR, IL>(Tin, q + 1, t0, ts, tg, Tp);
-    }
-    double dzu = k == 0 ? 0.0 : ld(Zc + k - 1) - ld(Zc + k);
-    double dzd = ld(Zc + k) - (last ? 0.0 : ld(Zc + k + 1));
-    dzu = dzu == 0.0 ? 1.0 : dzu;
-    dzd = dzd == 0.0 ? 1.0 : dzd;
-    const double av = ld(m.areasvol + q);
-    const double sav = av > 0.0 ? av : 1.0;
-    const double ar = ld(m.area + q), arp = last ? 0.0 : ld(m.area + q + 1);
-    const double kv = ld(in.Kv + q), kvp = last ? 0.0 : ld(in.Kv + q + 1);
-    const double a_full = -kv * dt / dzu * (ar / sav);
-    const double c_full = -kvp * dt / dzd * (arp / sav);
-    const double a = k == nzmin ? 0.0 : a_full;
-    const double c = k == nzmax - 1 ? 0.0 : c_full;
-    const double b = -a - c + ld(in.hnode_new + q);
-    const Rcp rm = rcp(b - a * cprev);
-    cprev = divr(c, rm);
-    in.ws.adfv[tix<IL>(q, w0, sN, in.wtg)] = cprev;
-    double swd = 0.0;
-    if (in.sw_3d) {
-      const double sw = ld(in.sw_3d + q), swp = last ? 0.0 : ld(in.sw_3d + q + 1);
-      swd = (sw - swp * (arp / sav)) * dt;
-    }
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) {
-      double rhs = a * (Tc[t] - Tm[t]) + c * (Tc[t] - Tp[t]);
-      if (in.bc_surf) rhs = rhs + (k == nzmin ? ld(in.bc_surf + (t0 + t) * in.bc_stride + n) : 0.0);
-      if (in.sw_3d && t0 + t == in.sw_tracer) rhs = rhs + swd;
-      dprev[t] = divr(rhs - a * dprev[t], rm);
-      Tm[t] = Tc[t];
-      Tc[t] = Tp[t];
-    }
-    stn<NTR, IL>(in.ws.lo, q, w0, sN, in.wtg, dprev);
-  }
-  double x[NTR];
-#pragma unroll
-  for (int t = 0; t < NTR; ++t) x[t] = 0.0;
-  for (int k = nzmax - 1; k >= nzmin; --k) {
-    const uint32_t q = base + uint32_t(k);
-    const double cp = in.ws.adfv[tix<IL>(q, w0, sN, in.wtg)];
-    double dp[NTR], Tv[NTR];
-    ldn<NTR, IL>(in.ws.lo, q, w0, sN, in.wtg, dp);
-    ldn<NTR, IL>(Tin, q, t0, ts, tg, Tv);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) {
-      x[t] = dp[t] - cp * x[t];
-      Tv[t] = Tv[t] + x[t];
-    }
-    stn<NTR, IL>(in.T_new, q, t0, ts, tg, Tv);
-  }
-}
-
 // ------------------------------------------- dry levels keep T (ale_reconstruct)
 template <bool IL>
 __device__ __forceinline__ void body_copy_dry(const Inst& in, int64_t i) {
@@ -709,8 +570,8 @@ constexpr int kMinBlocks = NTR == 1 ? 7 : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
 
 #define FCT_KERNEL_T(name, body)                                                        \
   template <int NTR>                                                                    \
-  __global__ void __launch_bounds__(256, kMinBlocks<NTR>) name##_1(Inst in, int t0,     \
-                                                                   int w0) {            \
+  __global__ void __launch_bounds__(256, kMinBlocks<NTR>) name##_1(                       \
+      const __grid_constant__ Inst in, int t0, int w0) {                                \
     const int sub = int(blockIdx.y) * NTR;                                              \
     body<NTR, false>(in, lane_index(), t0 + sub, w0 + sub);                             \
   }                                                                                     \
@@ -727,20 +588,38 @@ constexpr int kMinBlocks = NTR == 1 ? 7 : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
 // unfused stages (every intermediate in the workspace; the reverse pass reads them)
 FCT_KERNEL_T(k_elem_grad, body_elem_grad)
 FCT_KERNEL_T(k_node_lo, body_node_lo)
-FCT_KERNEL_T(k_vert_impl, body_vert_impl)
 FCT_KERNEL_T(k_edge_adf, body_edge_adf)
 FCT_KERNEL_T(k_elem_bounds, body_elem_bounds)
 FCT_KERNEL_T(k_node_cluster, body_node_cluster)
 FCT_KERNEL_T(k_node_factors, body_node_factors)
 FCT_KERNEL_T(k_node_final, body_node_final)
-// implicit vertical diffusion (the epilogue of the batched step and fct_vert_diff)
-FCT_KERNEL_T(k_vdiff, body_vdiff)
 
-__global__ void __launch_bounds__(256) k_vflux_1(Inst in) { body_vflux(in, lane_index()); }
+// column solves (fct_columns.cuh): blockIdx.y the instance (batched), blockIdx.z the group of
+// at most ``group`` tracers
+#define FCT_KERNEL_COL(name, block_body)                                                 \
+  __global__ void __launch_bounds__(kColThreads) name##_1(                               \
+      const __grid_constant__ Inst in, int columns, int t0, int nt, int group) {         \
+    extern __shared__ double col_sh[];                                                   \
+    const int g = int(blockIdx.z) * group;                                               \
+    block_body<false>(in, int(blockIdx.x) * columns, columns, t0 + g, min(group, nt - g), \
+                      col_sh);                                                           \
+  }                                                                                      \
+  __global__ void __launch_bounds__(kColThreads) name##_n(                               \
+      const Inst* __restrict__ tab, int columns, int t0, int nt, int group) {            \
+    extern __shared__ double col_sh[];                                                   \
+    const int g = int(blockIdx.z) * group;                                               \
+    block_body<true>(tab[blockIdx.y], int(blockIdx.x) * columns, columns, t0 + g,        \
+                     min(group, nt - g), col_sh);                                        \
+  }
+// implicit vertical diffusion (the epilogue of the batched step and fct_vert_diff)
+FCT_KERNEL_COL(k_vdiff, block_vdiff)
+FCT_KERNEL_COL(k_vert_impl, block_vert_impl)
+
+__global__ void __launch_bounds__(256) k_vflux_1(const __grid_constant__ Inst in) { body_vflux(in, lane_index()); }
 __global__ void __launch_bounds__(256) k_vflux_n(const Inst* __restrict__ tab) {
   body_vflux(tab[blockIdx.y], lane_index());
 }
-__global__ void __launch_bounds__(256) k_copy_dry_1(Inst in) {
+__global__ void __launch_bounds__(256) k_copy_dry_1(const __grid_constant__ Inst in) {
   body_copy_dry<false>(in, lane_index());
 }
 __global__ void __launch_bounds__(256) k_copy_dry_n(const Inst* __restrict__ tab) {
@@ -803,6 +682,32 @@ void fork_destroy(Fork& f) {
   f = Fork{};
 }
 
+namespace {
+
+// One column solve over ``nt`` tracers from ``t0``, all of them in one launch: up to 8 of an
+// interleaved instance share a block's matrix rows; tracer-major ones go up to 2 per block.
+template <class K1, class KN>
+int launch_columns(K1 k1, KN kn, const Inst& single, const Inst* tab, int n, int64_t nodes, int L,
+                   int t0, int nt, cudaStream_t s, const char* what) {
+  const int group = std::min(nt, tab ? 8 : 2);
+  const int columns = col_columns(L, group);
+  const size_t sh = col_smem(columns, L, group);
+  cudaError_t e = cudaSuccess;
+  // the opt-in limit is the same value every time, so concurrent callers do not disturb it
+  if (sh > size_t(48) << 10)
+    e = tab ? cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, kColMaxSmem)
+            : cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, kColMaxSmem);
+  if (e != cudaSuccess) return cuda_error(e, what);
+  const dim3 g(unsigned(std::max<int64_t>(1, (nodes + columns - 1) / columns)),
+               tab ? unsigned(n) : 1u, unsigned((nt + group - 1) / group));
+  if (tab) kn<<<g, kColThreads, sh, s>>>(tab, columns, t0, nt, group);
+  else k1<<<g, kColThreads, sh, s>>>(single, columns, t0, nt, group);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? FCT_OK : cuda_error(e, what);
+}
+
+}  // namespace
+
 int launch_forward_events(const Inst& single, const Inst* tab, int n, const LaunchDims& d,
                           cudaStream_t s, cudaEvent_t* after, bool stop_before_final,
                           int chunk_sel) {
@@ -813,6 +718,10 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
   auto grid = [&](int64_t lanes) { return dim3(xblocks(lanes), unsigned(n), 1); };
   const int chunk = d.chunk > 0 ? d.chunk : d.ntr;
   const int nchunks = (d.ntr + chunk - 1) / chunk;
+  // the dry-level copy on the side stream, beside the stages (190 of 9,200 us of a step of
+  // 300,000 nodes x 70 levels x 4 tracers when it ran after them)
+  const bool dry_aside = d.fused && kForkEdge && d.fork && !after && d.copy_dry &&
+                         !stop_before_final && !d.any_vdiff && chunk_sel < 0;
   for (int ci = 0; ci < nchunks; ++ci) {
     if (chunk_sel >= 0 && ci != chunk_sel) continue;
     const int c0 = ci * chunk, c1 = std::min(d.ntr, c0 + chunk);
@@ -822,7 +731,7 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
       ++stage;
     };
     if (ci == 0) {   // the volume flux is shared by all tracers
-      if (tab && d.any_derive_w) {   // producer: w_e from continuity, in the same graph
+      if (tab && d.any_derive_w && !d.skip_vflux) {   // producer: w_e from continuity, in the same graph
         const int st = launch_compute_w_tab(tab, n, d.max_nodes, s);
         if (st) return st;
       }
@@ -847,10 +756,18 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
         if ((st = launch_seg_edge(single, tab, n, d, c0, c1, fk->side))) return st;
         if ((st = launch_edge_fix(single, tab, n, d, c0, c1, fk->side))) return st;
         FCT_CUDA(cudaEventRecord(fk->ev[1], fk->side));
+        if (dry_aside && ci == 0) {   // reads T's, writes T_new's dry levels: no stage does
+          if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, fk->side>>>(tab);
+          else k_copy_dry_1<<<grid(d.max_dry), B, 0, fk->side>>>(single);
+          FCT_CUDA(cudaEventRecord(fk->ev[2], fk->side));
+        }
       }
       if ((st = launch_seg_lo(single, tab, n, d, c0, c1, s))) return st;
       mark();
-      if (d.any_wi) FCT_STAGE(k_vert_impl, d.max_nodes);
+      if (d.any_wi && (st = launch_columns(k_vert_impl_1, k_vert_impl_n, single, tab, n,
+                                           d.max_nodes, d.max_levels, 0, c1 - c0, s,
+                                           "split vertical velocity launch")))
+        return st;
       mark();
       if (fk) {
         FCT_CUDA(cudaStreamWaitEvent(s, fk->ev[1], 0));
@@ -870,7 +787,9 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
           if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, s>>>(tab);
           else k_copy_dry_1<<<grid(d.max_dry), B, 0, s>>>(single);
         }
-        FCT_STAGE(k_vdiff, d.max_nodes);
+        if ((st = launch_columns(k_vdiff_1, k_vdiff_n, single, tab, n, d.max_nodes, d.max_levels,
+                                 c0, c1 - c0, s, "vertical diffusion launch")))
+          return st;
       }
       mark();
       continue;
@@ -879,7 +798,12 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
     mark();
     FCT_STAGE(k_node_lo, d.max_iface);
     mark();
-    if (d.any_wi) FCT_STAGE(k_vert_impl, d.max_nodes);
+    if (d.any_wi) {
+      const int st = launch_columns(k_vert_impl_1, k_vert_impl_n, single, tab, n, d.max_nodes,
+                                    d.max_levels, 0, c1 - c0, s,
+                                    "split vertical velocity launch");
+      if (st) return st;
+    }
     mark();
     FCT_STAGE(k_edge_adf, d.max_edge);
     mark();
@@ -893,7 +817,9 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
     FCT_STAGE(k_node_final, d.max_layer);
     mark();
   }
-  if (d.copy_dry && !stop_before_final && (chunk_sel < 0 || chunk_sel == nchunks - 1)) {
+  if (dry_aside) {
+    FCT_CUDA(cudaStreamWaitEvent(s, d.fork->ev[2], 0));
+  } else if (d.copy_dry && !stop_before_final && (chunk_sel < 0 || chunk_sel == nchunks - 1)) {
     if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, s>>>(tab);
     else k_copy_dry_1<<<grid(d.max_dry), B, 0, s>>>(single);
   }
@@ -914,16 +840,8 @@ int launch_forward_stages(const Inst& single, const LaunchDims& d, cudaStream_t 
 }
 
 int launch_vdiff(const Inst& single, const LaunchDims& d, cudaStream_t s) {
-  constexpr int B = 256;
-  auto xblocks = [&](int64_t lanes) {
-    return unsigned(std::max<int64_t>(1, (lanes + B - 1) / B));
-  };
-  const Inst* tab = nullptr;
-  const int n = 1;
-  const int c0 = 0, c1 = d.ntr;
-  FCT_STAGE(k_vdiff, d.max_nodes);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? FCT_OK : cuda_error(e, "vertical diffusion launch");
+  return launch_columns(k_vdiff_1, k_vdiff_n, single, nullptr, 1, d.max_nodes, d.max_levels, 0,
+                        d.ntr, s, "vertical diffusion launch");
 }
 
 int launch_copy_dry(const Inst* tab, int n, int64_t max_dry, cudaStream_t s) {

@@ -35,6 +35,7 @@ enum { kStageLo = 0, kStageEdge = 1, kStageLimit = 2, kStageFinal = 3 };
 struct LaunchDims {
   int64_t max_iface, max_layer, max_edge, max_elem, max_dense, max_nodes;
   int64_t max_dry = 0;   // dry node levels (kept from T)
+  int max_levels = 0;    // nl
   int ntr;           // tracers per instance (every instance of a launch has the same)
   int chunk = 0;     // tracers whose intermediates share the workspace (0 = all ntr);
                      // stages run chunk by chunk
@@ -43,7 +44,8 @@ struct LaunchDims {
   bool copy_dry;    // launch the dry-level copy
   bool any_vdiff = false;  // launch the implicit vertical diffusion after each chunk
   bool any_derive_w = false;  // derive w_e from uv (compute_w) before the step
-  bool skip_vflux = false;    // the workspace already holds this step's volume fluxes
+  bool skip_vflux = false;    // the workspace already holds this step's volume fluxes (and
+                              // w_derived its w)
   bool fused = true;  // fused stages (lean workspace); false: every stage kernel writes its
                       // intermediates (what the reverse pass reads)
   // fused (segment) stages: per stage (LO, edge, limiter, final) the most tracers and the
@@ -87,6 +89,7 @@ inline void dims_cover(LaunchDims& d, const FctPlan* P) {
   d.max_dense = std::max(d.max_dense, int64_t(P->N) * P->L);
   d.max_dry = std::max(d.max_dry, P->hm.n_dry);
   d.max_nodes = std::max(d.max_nodes, int64_t(P->N));
+  d.max_levels = std::max(d.max_levels, P->L);
   for (int v = 0; v < kSegVariants; ++v) {
     d.max_nseg[v] = std::max(d.max_nseg[v], m.n_nseg[v]);
     d.max_eseg[v] = std::max(d.max_eseg[v], m.n_eseg[v]);

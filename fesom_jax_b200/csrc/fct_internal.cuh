@@ -69,6 +69,7 @@ __host__ __device__ constexpr int seg_variant(int lpt) {
 // Static mesh on the device (pointers into one plan allocation).
 struct DevMesh {
   int N, E, Ed, L;
+  int edges_outside;     // some edge has a level outside its end nodes' layers
   // nodes
   const int* nzmin;      // ulevels_nod2D - 1
   const int* nzmax;      // nlevels_nod2D - 1 (exclusive layer bound; bottom interface)
@@ -165,13 +166,13 @@ struct DevMesh {
   int64_t n_efix;
 };
 
-// A side stream and two events (fork, join) with which the fused step runs its edge stage
-// beside the LO stage: both read only the step's inputs and the volume fluxes, and they
+// A side stream and its events (fork, joins) with which the fused step runs its edge stage
+// beside the LO stage and the dry-level copy beside the others: both read only the step's inputs and the volume fluxes, and they
 // write disjoint workspace fields (adf_h; LO and adf_v), so the two latency-bound kernels
 // can share the SMs. Owned by a plan or a batch and used under its lock.
 struct Fork {
   cudaStream_t side = nullptr;
-  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
 };
 
 // Per-tracer intermediates of one instance (dense [entity, L]; tracer t at +t*stride).

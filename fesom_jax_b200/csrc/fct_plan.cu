@@ -566,6 +566,12 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   char* base = static_cast<char*>(P->d_static);
   DevMesh& m = P->hm;
   m.N = N; m.E = E; m.Ed = Ed; m.L = L;
+  m.edges_outside = 0;
+  for (int e = 0; e < Ed; ++e)
+    for (int r = 0; r < 2; ++r) {
+      const int n = d->edges[2 * e + r];
+      if (ekmax[e] > ekmin[e] && (ekmin[e] < nzmin[n] || ekmax[e] > nzmax[n])) m.edges_outside = 1;
+    }
   m.nzmin = (const int*)(base + o_nzmin);
   m.nzmax = (const int*)(base + o_nzmax);
   m.ulmax = (const int*)(base + o_ulmax);
@@ -745,9 +751,9 @@ int fct_vert_diff(FctPlan* P, const FctVdiffFields* f, double dt, int ntr, fct_s
   in.ntr = ntr;
   LaunchDims dims{};
   dims.max_nodes = P->N;
+  dims.max_levels = P->L;
   dims.ntr = ntr;
   dims.chunk = 0;
-  dims.per_thread = 8;
   int st;
   {
     PlanUse use(P, static_cast<cudaStream_t>(stream));

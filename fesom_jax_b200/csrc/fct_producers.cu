@@ -16,70 +16,87 @@ using namespace fct;
 
 namespace {
 
-// One warp per node column, the levels in its lanes (32 at a time, bottom block first):
-// every lane gathers its level's divergence, then the bottom-up running sum is added in
-// the sequential order (level L-1 first) through shuffles, so the result is the same as a
-// per-column loop's.
-__device__ __forceinline__ void compute_w_column(const DevMesh& m, const double* __restrict__ uv,
-                                                 const double* __restrict__ helem,
-                                                 double* __restrict__ w, int n, int lane) {
-  if (n >= m.N) return;   // warp-uniform
-  const int L = m.L;
-  const int64_t base = int64_t(n) * L;
-  const int nzmin = __ldg(m.nzmin + n), nzmax = __ldg(m.nzmax + n);
-  const int e0 = __ldg(m.ne_off + n), e1 = __ldg(m.ne_off + n + 1);
-  double carry = 0.0;
-  for (int kb = ((L - 1) / 32) * 32; kb >= 0; kb -= 32) {
-    const int k = kb + lane;
+// A block takes kWColumns node columns: all threads gather the divergence of the columns' wet
+// levels (levels adjacent), one thread per column adds them bottom to top in shared memory (in
+// the sequential order, so the sum is the reference's), and all threads write w. (With a warp
+// per column and the running sum through shuffles the kernel executed 1,700 warp-instructions
+// per column, half of them shuffles and idle levels, and was issue-bound: 340 us on the
+// CORE2-size mesh.)
+constexpr int kWColumns = 16, kWThreads = 256;
+
+__device__ __forceinline__ void compute_w_columns(const DevMesh& m, const double* __restrict__ uv,
+                                                  const double* __restrict__ helem,
+                                                  double* __restrict__ w, int n0, double* sh) {
+  if (n0 >= m.N) return;   // block-uniform
+  const int L = m.L, stride = L | 1;
+  const double2* uv2 = reinterpret_cast<const double2*>(uv);
+  for (int i = threadIdx.x; i < kWColumns * L; i += kWThreads) {
+    const int col = i / L, k = i - col * L, n = n0 + col;
+    if (n >= m.N) break;
+    const int4 rec = __ldg(m.nrec + n);
+    const unsigned pk = unsigned(rec.z);
+    if (!m.edges_outside && (k < int(pk & 255u) || k >= int((pk >> 8) & 255u)))
+      continue;   // no edge has the level
+    const int e1 = rec.x + int((pk >> 16) & 255u);
     double div = 0.0;
-    if (k < L) {
-      for (int j = e0; j < e1; ++j) {
-        const int idx = __ldg(m.ne_idx + j), e = idx >> 1;
-        if (k < __ldg(m.ekmin + e) || k >= __ldg(m.ekmax + e)) continue;
-        const int el1 = __ldg(m.etri + 2 * e), el2 = __ldg(m.etri + 2 * e + 1);
-        const double* cr = m.cross + 4 * int64_t(e);
-        double t1 = 0.0, t2 = 0.0;
-        if (k >= __ldg(m.eul + el1) && k < __ldg(m.enl + el1)) {
-          const int64_t q = int64_t(el1) * L + k;
-          t1 = (__ldg(uv + 2 * q + 1) * __ldg(cr) - __ldg(uv + 2 * q) * __ldg(cr + 1)) *
-               __ldg(helem + q);
-        }
-        if (el2 >= 0 && k >= __ldg(m.eul + el2) && k < __ldg(m.enl + el2)) {
-          const int64_t q = int64_t(el2) * L + k;
-          t2 = (__ldg(uv + 2 * q + 1) * __ldg(cr + 2) - __ldg(uv + 2 * q) * __ldg(cr + 3)) *
-               __ldg(helem + q);
-        }
-        const double c = t1 - t2;
-        div += (idx & 1) ? -c : c;
+    for (int j = rec.x; j < e1; ++j) {
+      const int4 sl = __ldg(m.ne4 + j);
+      const unsigned rg = unsigned(sl.z), tr = unsigned(sl.w);
+      if (k < int(rg & 255u) || k >= int((rg >> 8) & 255u)) continue;
+      const int e = sl.x >> 1;
+      const int4 ec = __ldg(m.ecell4 + e);
+      const double2* cr = reinterpret_cast<const double2*>(m.cross + 4 * int64_t(e));
+      double t1 = 0.0, t2 = 0.0;
+      if (k >= int(tr & 255u) && k < int((tr >> 8) & 255u)) {
+        const uint32_t q = lq(ec.x, L, k);
+        const double2 U = __ldg(uv2 + q), x = __ldg(cr);
+        t1 = (U.y * x.x - U.x * x.y) * __ldg(helem + q);
       }
+      if (((tr >> 16) & 255u) != kNoCell && k >= int((tr >> 16) & 255u) && k < int(tr >> 24)) {
+        const uint32_t q = lq(ec.y, L, k);
+        const double2 U = __ldg(uv2 + q), x = __ldg(cr + 1);
+        t2 = (U.y * x.x - U.x * x.y) * __ldg(helem + q);
+      }
+      const double c = t1 - t2;
+      div += (sl.x & 1) ? -c : c;
     }
-    double acc = carry, mine = 0.0;
-    for (int s = 31; s >= 0; --s) {   // acc += div[kb + s], top of the block last
-      const double ds = __shfl_sync(0xffffffffu, div, s);
-      if (kb + s < L) acc += ds;
-      if (lane == s) mine = acc;
-    }
-    carry = acc;
-    if (k < L) {
-      const double a = __ldg(m.area + base + k);
-      w[base + k] = (k >= nzmin && k <= nzmax) ? mine / (a > 0.0 ? a : 1.0) : 0.0;
-    }
+    sh[col * stride + k] = div;
+  }
+  __syncthreads();
+  if (threadIdx.x < kWColumns && n0 + int(threadIdx.x) < m.N) {
+    const int n = n0 + threadIdx.x;
+    const int lo = m.edges_outside ? 0 : __ldg(m.nzmin + n);
+    const int hi = m.edges_outside ? L : __ldg(m.nzmax + n);
+    double* s = sh + threadIdx.x * stride;
+    double acc = 0.0;
+    for (int k = hi - 1; k >= lo; --k) s[k] = acc += s[k];
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kWColumns * L; i += kWThreads) {
+    const int col = i / L, k = i - col * L, n = n0 + col;
+    if (n >= m.N) break;
+    const int nzmin = __ldg(m.nzmin + n), nzmax = __ldg(m.nzmax + n);
+    const int64_t q = int64_t(n) * L + k;
+    const double a = __ldg(m.area + q);
+    // the bottom interface nzmax carries 0 unless an edge reaches below it
+    w[q] = (k >= nzmin && (k < nzmax || (m.edges_outside && k == nzmax))) ? sh[col * stride + k] / (a > 0.0 ? a : 1.0) : 0.0;
   }
 }
 
-__global__ void __launch_bounds__(128) k_compute_w(const DevMesh* __restrict__ mp,
-                                                   const double* __restrict__ uv,
-                                                   const double* __restrict__ helem,
-                                                   double* __restrict__ w) {
-  compute_w_column(*mp, uv, helem, w, blockIdx.x * 4 + (threadIdx.x >> 5), threadIdx.x & 31);
+__global__ void __launch_bounds__(kWThreads) k_compute_w(const DevMesh* __restrict__ mp,
+                                                         const double* __restrict__ uv,
+                                                         const double* __restrict__ helem,
+                                                         double* __restrict__ w) {
+  __shared__ double sh[kWColumns * (kMaxLevels + 1)];
+  compute_w_columns(*mp, uv, helem, w, int(blockIdx.x) * kWColumns, sh);
 }
 
 // batched: instance blockIdx.y of a device table derives its w into w_derived
-__global__ void __launch_bounds__(128) k_compute_w_n(const Inst* __restrict__ tab) {
+__global__ void __launch_bounds__(kWThreads) k_compute_w_n(const Inst* __restrict__ tab) {
+  __shared__ double sh[kWColumns * (kMaxLevels + 1)];
   const Inst& in = tab[blockIdx.y];
   if (!in.w_derived) return;
-  compute_w_column(in.m, in.uv, in.helem, in.w_derived, blockIdx.x * 4 + (threadIdx.x >> 5),
-                   threadIdx.x & 31);
+  compute_w_columns(in.m, in.uv, in.helem, in.w_derived, int(blockIdx.x) * kWColumns, sh);
 }
 
 }  // namespace
@@ -87,8 +104,9 @@ __global__ void __launch_bounds__(128) k_compute_w_n(const Inst* __restrict__ ta
 namespace fct {
 
 int launch_compute_w_tab(const Inst* tab, int n, int64_t max_nodes, cudaStream_t s) {
-  const dim3 g(unsigned(std::max<int64_t>(1, (max_nodes + 3) / 4)), unsigned(n), 1);
-  k_compute_w_n<<<g, 128, 0, s>>>(tab);   // 4 warps = 4 node columns per block
+  const dim3 g(unsigned(std::max<int64_t>(1, (max_nodes + kWColumns - 1) / kWColumns)),
+               unsigned(n), 1);
+  k_compute_w_n<<<g, kWThreads, 0, s>>>(tab);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FCT_OK : cuda_error(e, "compute_w (batched) launch");
 }
@@ -101,8 +119,8 @@ extern "C" int fct_compute_w(FctPlan* P, const double* uv, const double* helem, 
   int prev = -1;
   cudaGetDevice(&prev);
   if (prev != P->device) cudaSetDevice(P->device);
-  k_compute_w<<<(P->N + 3) / 4, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      P->d_mesh, uv, helem, w);   // 4 warps = 4 node columns per block
+  k_compute_w<<<(P->N + kWColumns - 1) / kWColumns, kWThreads, 0,
+                static_cast<cudaStream_t>(stream)>>>(P->d_mesh, uv, helem, w);
   cudaError_t e = cudaGetLastError();
   if (prev >= 0 && prev != P->device) cudaSetDevice(prev);
   return e == cudaSuccess ? FCT_OK : cuda_error(e, "compute_w launch");

@@ -341,36 +341,66 @@ __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0,
   }
 }
 
-// node-average gradient of T at node n, level k (_node_avg_grad, tracer_adv.py:329-341):
-// the area-weighted mean over n's cells wet at k, in the node's cell order
+// node-average gradients of T at the two nodes n[0], n[1], level k (_node_avg_grad,
+// tracer_adv.py:329-341): the area-weighted mean over a node's cells wet at k, in the node's
+// cell order. The two nodes' cells go side by side, their records one ahead: the loop is a
+// chain of dependent loads, and one loop for both halves it.
 template <int NTR, bool IL>
-__device__ __forceinline__ void node_avg_grad(const Inst& in, int n, int k, int t0,
-                                              double (&nx)[NTR], double (&ny)[NTR]) {
+__device__ __forceinline__ void node_avg_grads(const Inst& in, int n1, int n2, int k, int t0,
+                                               double (&nx)[2][NTR], double (&ny)[2][NTR]) {
   const DevMesh& m = in.m;
-  const int4 rec = __ldg(m.nrec + n);
-  double den = 0.0;
+  int c[2], left[2];
+  double den[2] = {0.0, 0.0};
 #pragma unroll
-  for (int t = 0; t < NTR; ++t) nx[t] = ny[t] = 0.0;
-  const int c0 = rec.y, c1 = rec.y + int(unsigned(rec.z) >> 24);
-  for (int j = c0; j < c1; ++j) {
-    const unsigned r = unsigned(__ldg(m.nelr + j));
-    const int4 sl = __ldg(m.nel4 + j);
-    if (!in_range(k, r)) continue;
-    const double a = __ldg(m.earea + sl.x);
-    double gx[NTR], gy[NTR];
-    cell_grad<NTR, IL>(in, sl.x, sl.y, sl.z, sl.w, k, t0, gx, gy);
+  for (int i = 0; i < 2; ++i) {
+    const int4 rec = __ldg(m.nrec + (i == 0 ? n1 : n2));
+    c[i] = rec.y;
+    left[i] = int(unsigned(rec.z) >> 24);
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) nx[i][t] = ny[i][t] = 0.0;
+  }
+  const int count = max(left[0], left[1]);
+  int4 sl[2];
+  unsigned r[2];
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const bool some = j < left[i];
+      r[i] = some ? unsigned(__ldg(m.nelr + c[i] + j)) : 0u;   // 0: no level
+      sl[i] = __ldg(m.nel4 + (some ? c[i] + j : 0));   // (a cell whose values are not used)
+    }
+  };
+  if (count > 0) fetch(0);
+  for (int j = 0; j < count; ++j) {
+    const int4 s0[2] = {sl[0], sl[1]};
+    const bool on[2] = {in_range(k, r[0]), in_range(k, r[1])};
+    if (j + 1 < count) fetch(j + 1);
+    double gx[2][NTR], gy[2][NTR], a[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      a[i] = __ldg(m.earea + s0[i].x);
+      cell_grad<NTR, IL>(in, s0[i].x, s0[i].y, s0[i].z, s0[i].w, k, t0, gx[i], gy[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (on[i]) {
+#pragma unroll
+        for (int t = 0; t < NTR; ++t) {
+          nx[i][t] += gx[i][t] * a[i];
+          ny[i][t] += gy[i][t] * a[i];
+        }
+        den[i] += a[i];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const Rcp rdd = rcp(den[i] > 0.0 ? den[i] : 1.0);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
-      nx[t] += gx[t] * a;
-      ny[t] += gy[t] * a;
+      nx[i][t] = divr(nx[i][t], rdd);
+      ny[i][t] = divr(ny[i][t], rdd);
     }
-    den += a;
-  }
-  const Rcp rdd = rcp(den > 0.0 ? den : 1.0);
-#pragma unroll
-  for (int t = 0; t < NTR; ++t) {
-    nx[t] = divr(nx[t], rdd);
-    ny[t] = divr(ny[t], rdd);
   }
 }
 
@@ -390,18 +420,17 @@ __device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int t0,
   const uint32_t q1 = lq(n1, L, k), q2 = lq(n2, L, k);
   const int64_t ts = in.tstride;
   const int tg = in.tg;
-  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], g0[NTR], g1[NTR], g2[NTR], g3[NTR];
+  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[2][NTR], gy[2][NTR];
   ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
   ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
   ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
   ldn<NTR, IL>(in.T_old, q2, t0, ts, tg, O2);
   if (use_tri) {   // a mesh whose up/down cells do not hold the edge's nodes
     const int4 cu = __ldg(m.eud4 + 2 * e), cd = __ldg(m.eud4 + 2 * e + 1);
-    cell_grad<NTR, IL>(in, cu.x, cu.y, cu.z, cu.w, k, t0, g0, g2);
-    cell_grad<NTR, IL>(in, cd.x, cd.y, cd.z, cd.w, k, t0, g1, g3);
+    cell_grad<NTR, IL>(in, cu.x, cu.y, cu.z, cu.w, k, t0, gx[0], gy[0]);
+    cell_grad<NTR, IL>(in, cd.x, cd.y, cd.z, cd.w, k, t0, gx[1], gy[1]);
   } else {
-    node_avg_grad<NTR, IL>(in, n1, k, t0, g0, g2);
-    node_avg_grad<NTR, IL>(in, n2, k, t0, g1, g3);
+    node_avg_grads<NTR, IL>(in, n1, n2, k, t0, gx, gy);
   }
   double adf[NTR];
   const Rcp r6{6.0, 1.0 / 6.0, true};
@@ -410,8 +439,8 @@ __device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int t0,
     const double fl = -0.5 * (T1[t] * (vf + avf) + T2[t] * (vf - avf));
     const double A1 = ab2(T1[t], O1[t]), A2 = ab2(T2[t], O2[t]);
     const double diff = A2 - A1;
-    const double Tm1 = A1 + divr(2.0 * diff + c1 * g0[t] + c2 * g2[t], r6);
-    const double Tm2 = A2 - divr(2.0 * diff + c1 * g1[t] + c2 * g3[t], r6);
+    const double Tm1 = A1 + divr(2.0 * diff + c1 * gx[0][t] + c2 * gy[0][t], r6);
+    const double Tm2 = A2 - divr(2.0 * diff + c1 * gx[1][t] + c2 * gy[1][t], r6);
     const double ho = -0.5 * ((vf + avf) * Tm1 + (vf - avf) * Tm2);
     adf[t] = ho - fl;
   }
