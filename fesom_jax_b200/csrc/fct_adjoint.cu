@@ -54,8 +54,12 @@ constexpr int B = 256;
 // pay more than the spills the cap costs: on the CORE2-size 10-step chain the reverse
 // passes took 28.7 ms unconstrained (r_edge at 3 blocks), 23.3 ms at 4 blocks, 20.2 ms at
 // 6 (r_edge 5) and 20.0 ms at 8.
-constexpr int kRevMinBlocks = 6;
-constexpr int kRevEdgeMinBlocks = 5;
+#ifndef FCT_RMB
+#define FCT_RMB 6
+#define FCT_REB 5
+#endif
+constexpr int kRevMinBlocks = FCT_RMB;
+constexpr int kRevEdgeMinBlocks = FCT_REB;
 
 __device__ __forceinline__ int64_t lane_index() {
   return int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -108,7 +112,7 @@ __device__ __forceinline__ double gvl_at(const DevMesh& m, const double* ghsc, i
 // ------------------------------------------------------------------ r_seed
 // T_new = T + d / hnn (d = del + T (hn - hnn)) and del holds the flux divergence times
 // dt / areasvol: stores the cotangent of a node's flux divergence, gdel * dt / sa.
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_seed(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_seed(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t li = lane_index();
@@ -129,7 +133,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_seed(Adj A) {
 // Dry levels keep T (T_new = T, ale_reconstruct): their outputs depend only on dT_new and
 // are final here, except dT at the level above a cavity's first layer, which the upwind
 // flux of interface nzmin also reaches (r_final writes it); gw_e is zero there.
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_dry(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_dry(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t li = lane_index();
@@ -159,8 +163,8 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_dry(Adj A) {
 // (zalesak_limit b3, tracer_adv.py:453-465): the limited vertical fluxes at interfaces k
 // and k+1 and the limited horizontal fluxes of the incident edges in ascending edge id.
 __device__ __forceinline__ void factor_cotangents(const Adj& A, int t, int n, int k, int nzmin,
-                                                  int nzmax, int e0, int e1, double& gp,
-                                                  double& gm) {
+                                                  int nzmax, int e0, int e1, unsigned onb,
+                                                  double& gp, double& gm) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int L = m.L;
@@ -192,34 +196,25 @@ __device__ __forceinline__ void factor_cotangents(const Adj& A, int t, int n, in
     if (f >= 0.0) gm += g_ae * smin_a(mfk, pf[qn + 1]);
     else gp += g_ae * smin_a(pfk, mf[qn + 1]);
   }
-  // horizontal limited fluxes of the incident edges, ascending edge id; the loads are
-  // unconditional (all in bounds) and edges without a flux at k are selected away
+  // horizontal limited fluxes of the incident edges, ascending edge id. In the node's own
+  // terms (s the flux out of the node, lim = ae * s, ae = min(own plus, other minus) when it
+  // leaves, else min(own minus, other plus)) the cotangent of ae is (ghsc - ghsc_other) * s,
+  // and the own factor gets its share of the min. The loads are unconditional (all in bounds)
+  // and edges without a flux at k are selected away.
   const double ghsc0 = ghsc[qn];
   const double* adfh = in.ws.adfh + t * in.ws.sEd;
 #pragma unroll 2
   for (int j = e0; j < e1; ++j) {
-    const int4 sl = __ldg(m.ne4 + j);
-    const bool on = in_range(k, unsigned(sl.z));
-    const bool second = sl.x & 1;
-    const uint32_t qo = lq(sl.y, L, k);
-    const double ghsco = ghsc[qo];
-    const double glim = second ? (ghsco - ghsc0) : (ghsc0 - ghsco);
-    const double a = adfh[lq(sl.x >> 1, L, k)];
-    const double g_ae = glim * a;
+    const int4 sl = __ldg(m.ns4 + j);
+    const bool on = (onb >> (j - e0)) & 1u;
+    const uint32_t qo = uint32_t(sl.y) + uint32_t(k);
+    const double a = adfh[uint32_t(sl.x) + uint32_t(k)];
+    const double g_ae = sl.z ? (ghsc[qo] - ghsc0) * a : (ghsc0 - ghsc[qo]) * a;
     const double pfo = pf[qo], mfo = mf[qo];
-    const double pf1 = second ? pfo : pfk, mf1 = second ? mfo : mfk;
-    const double pf2 = second ? pfk : pfo, mf2 = second ? mfk : mfo;
-    double dp = 0.0, dm = 0.0;
-    bool tp = false, tm = false;
-    if (a >= 0.0) {   // ae = min(pf[n1], mf[n2])
-      if (!second) { dp = g_ae * smin_a(pf1, mf2); tp = true; }
-      else { dm = g_ae * smin_b(pf1, mf2); tm = true; }
-    } else {          // ae = min(mf[n1], pf[n2])
-      if (!second) { dm = g_ae * smin_a(mf1, pf2); tm = true; }
-      else { dp = g_ae * smin_b(mf1, pf2); tp = true; }
-    }
-    gp = (on && tp) ? gp + dp : gp;
-    gm = (on && tm) ? gm + dm : gm;
+    const bool leaves = (a >= 0.0) != (sl.z != 0);
+    const double d = g_ae * smin_a(leaves ? pfk : mfk, leaves ? mfo : pfo);
+    gp = (on && leaves) ? gp + d : gp;
+    gm = (on && !leaves) ? gm + d : gm;
   }
 }
 
@@ -230,7 +225,7 @@ __device__ __forceinline__ void factor_cotangents(const Adj& A, int t, int n, in
 // Blocks of B threads cover B - 2 lanes plus one halo lane on each side: every thread
 // computes its lane's window cotangents (gtmax, gtmin) into shared memory, and the core
 // lanes spread them back over the window's three levels (lanes i-1, i, i+1).
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(const __grid_constant__ Adj A) {
   __shared__ double sx[B], sn[B];
   const Inst& in = A.in;
   const DevMesh& m = in.m;
@@ -242,6 +237,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
   int n = 0, k = 0, nzmin = 0, nzmax = 0, e0 = 0, e1 = 0;
   uint32_t base = 0, qn = 0;
   bool valid_n = false, use_own = true;
+  unsigned onb = 0;   // bit j: the j-th slot's edge has the layer (flag words in lane order)
   Rcp rsa{1.0, 1.0, true}, rsh{1.0, 1.0, true};
   if (valid) {
     const int4 rec = __ldg(m.layer4 + lane);
@@ -256,7 +252,8 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
     qn = base + uint32_t(k);
     const double av = ld(m.areasvol + qn), hnn = ld(in.hnode_new + qn);
     valid_n = (av > 0.0) && (hnn > 0.0);
-    rsa = rcp(av > 0.0 ? av : 1.0);
+    onb = unsigned(__ldg(m.nflags + lane));
+    if (av > 0.0) rsa = rcp_known(av, ld(m.iavol + qn));
     rsh = rcp(hnn > 0.0 ? hnn : 1.0);
     use_own = (k == nzmin) || (k == nzmax - 1);
   }
@@ -268,7 +265,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
     double gtmax = 0.0, gtmin = 0.0;
     if (valid) {
       double gpf, gmf;
-      factor_cotangents(A, t, n, k, nzmin, nzmax, e0, e1, gpf, gmf);
+      factor_cotangents(A, t, n, k, nzmin, nzmax, e0, e1, onb, gpf, gmf);
       double gplus = 0.0, gminus = 0.0;
       if (valid_n) {
         double tmax = tv[qn], tmin = tn[qn];
@@ -341,7 +338,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(Adj A) {
 // the tied vertices, of the a3 shares of the vertices whose cluster bound the element
 // attains (tie counts come from the forward). Stored already divided by the element's
 // vertex tie count: the share of each attaining vertex.
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t i = lane_index();
@@ -377,7 +374,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(Adj A) {
 // ------- r_bounds_lo: a1 (max/min of LO and T) gathering the element shares of the
 // node's cells whose bound this node attains, then LO = numer / hnn and the seed terms
 // of T and LO.
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t i = lane_index();
@@ -428,7 +425,13 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(Adj A) {
 }
 
 // ------------------ r_edge: adf_h = HO - LO flux; cotangents of the edge inputs
-__global__ void __launch_bounds__(B, kRevEdgeMinBlocks) r_edge(Adj A) {
+// Both fluxes take the upwind end alone ((vf + |vf|) or (vf - |vf|) is 0), so an edge level
+// keeps two cotangents, of the upwind T through the LO flux (gT) and of the upwind Tm through
+// the HO flux (gM), where it kept six per-end terms before (390 us on the CORE2-size mesh,
+// its traffic twice what it is now); the readers tell the ends by the sign of vf
+// (edge_terms). The MFCT gradients are read at the upwind end, or at both where vf is 0 and
+// the subgradient of |vf| weighs the ends equally.
+__global__ void __launch_bounds__(B, kRevEdgeMinBlocks) r_edge(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t i = lane_index();
@@ -438,14 +441,17 @@ __global__ void __launch_bounds__(B, kRevEdgeMinBlocks) r_edge(Adj A) {
   const int n1 = rec.y, n2 = rec.z;
   const bool use_tri = in_range(k, unsigned(rec.w));
   const uint32_t qe = lq(e, L, k), q1 = lq(n1, L, k), q2 = lq(n2, L, k);
-  uint32_t qa = q1, qb = q2;   // where the MFCT gradients are read
+  const double vf = ld(in.ws.vflux + qe), avf = fabs(vf);
+  const bool first = vf > 0.0, both = !(avf > 0.0);
+  // where the MFCT gradients of the upwind (and the other) end are read
+  uint32_t qu = first ? q1 : q2, qd = first ? q2 : q1;
   if (use_tri) {
-    qa = lq(ld(m.eupdn + 2 * e), L, k);
-    qb = lq(ld(m.eupdn + 2 * e + 1), L, k);
+    qu = lq(ld(m.eupdn + 2 * e + (first ? 0 : 1)), L, k);
+    qd = lq(ld(m.eupdn + 2 * e + (first ? 1 : 0)), L, k);
   }
-  const double vf = ld(in.ws.vflux + qe), avf = fabs(vf), s = sgn(vf);
   const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
   const Rcp r6{6.0, 1.0 / 6.0, true};
+  const double cu = -0.5 * (first ? vf + avf : vf - avf);
   double gvf_t = 0.0;   // summed over tracers in tracer order, as r_uv sums them
   for (int t = 0; t < in.ntr; ++t) {
     const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * A.a.sEd;
@@ -469,29 +475,45 @@ __global__ void __launch_bounds__(B, kRevEdgeMinBlocks) r_edge(Adj A) {
     // MFCT gradients: the up/down cells' (use_tri) or the two nodes' averages
     const double* gxp = use_tri ? in.ws.gx + t * in.ws.sE : in.ws.gnx + o;
     const double* gyp = use_tri ? in.ws.gy + t * in.ws.sE : in.ws.gny + o;
-    const double g0 = gxp[qa], g1 = gxp[qb], g2 = gyp[qa], g3 = gyp[qb];
     const double diff = A2 - A1;
-    const double Tm1 = A1 + divr(2.0 * diff + c1 * g0 + c2 * g2, r6);
-    const double Tm2 = A2 - divr(2.0 * diff + c1 * g1 + c2 * g3, r6);
+    const double X = divr(2.0 * diff + c1 * gxp[qu] + c2 * gyp[qu], r6);
     // HO = -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2); fl = -0.5 (T1 (vf + |vf|) + T2 (vf - |vf|))
-    double gvf = -0.5 * ((1.0 + s) * Tm1 + (1.0 - s) * Tm2) * gHO;
-    gvf += -0.5 * (T1 * (1.0 + s) + T2 * (1.0 - s)) * gfl;
+    const double Tu = first ? A1 + X : A2 - X;
+    double gvf;
+    if (both) {   // vf == 0: Tu is the second end's
+      const double Xd = divr(2.0 * diff + c1 * gxp[qd] + c2 * gyp[qd], r6);
+      gvf = -0.5 * ((A1 + Xd) + Tu) * gHO;
+      gvf += -0.5 * (T1 + T2) * gfl;
+    } else {
+      gvf = -Tu * gHO;
+      gvf += -(first ? T1 : T2) * gfl;
+    }
     if (!(A.acc & kDeferUV)) A.a.gvf[oe + qe] = gvf;   // r_uv's input (not run when deferred)
     gvf_t += gvf;
-    // per-end terms for the node and element gathers: T1/T2 through the upwind flux;
-    // ttfAB at the ends through Tm1 = A1 + X1 / 6 and Tm2 = A2 - X2 / 6 with
-    // X = 2 (A2 - A1) + c1 gx + c2 gy (so the gradients' factors are c1 gX, c2 gX)
-    const double gTm1 = -0.5 * (vf + avf) * gHO, gTm2 = -0.5 * (vf - avf) * gHO;
-    const double gX1 = divr(gTm1, r6), gX2 = divr(-gTm2, r6);
-    const double gdiff = 2.0 * gX1 + 2.0 * gX2;
-    A.a.gT1[oe + qe] = -0.5 * (vf + avf) * gfl;
-    A.a.gT2[oe + qe] = -0.5 * (vf - avf) * gfl;
-    A.a.gA1[oe + qe] = gTm1 - gdiff;
-    A.a.gA2[oe + qe] = gTm2 + gdiff;
-    A.a.gX1[oe + qe] = gX1;
-    A.a.gX2[oe + qe] = gX2;
+    A.a.gT[oe + qe] = cu * gfl;
+    A.a.gM[oe + qe] = cu * gHO;
   }
   if (A.acc & kDeferUV) A.a.gvf_sum[qe] += gvf_t;   // one thread per edge level: no race
+}
+
+// x / 6, correctly rounded
+__device__ __forceinline__ double div6(double x) { return divr(x, Rcp{6.0, 1.0 / 6.0, true}); }
+
+// A node's terms of an edge level: T through the LO flux, ttfAB through Tm. With X = 2 (A2 -
+// A1) + c1 gx + c2 gy, Tm1 = A1 + X1 / 6 and Tm2 = A2 - X2 / 6, the upwind end's A takes gM -
+// 2 gM / 6 and the other end's 2 gM / 6.
+__device__ __forceinline__ void edge_terms(bool upwind, double gT, double gM, double& vT,
+                                           double& vA) {
+  const double d = 2.0 * div6(gM);
+  vT = upwind ? gT : 0.0 * gT;
+  vA = upwind ? gM - d : d;
+}
+
+// The factor of the MFCT gradient at the edge's first (second) end: gM / 6, its sign turned at
+// the second end, where that end is upwind.
+__device__ __forceinline__ double grad_factor(bool second, double vf, double gM) {
+  const double x = div6(second ? -gM : gM);
+  return (second ? vf < 0.0 : vf > 0.0) ? x : 0.0 * x;
 }
 
 // QR4C stencil depths of interface j (tracer_adv.py:228-238, 265-273)
@@ -513,7 +535,7 @@ __device__ __forceinline__ void qr4c_depths(const Inst& in, const DevMesh& m, in
 
 // ------- r_gnode: cotangent of the node-average gradient (fill_up_dn_grad's node branch),
 // gathered over the node's edges in ascending edge id.
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t i = lane_index();
@@ -524,8 +546,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(Adj A) {
   const uint32_t qn = lq(n, L, k);
   const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
   // no edge of the node takes the node-average gradient at k (kGradBit): its cotangent is 0
-  const int nzmin = int(pk & 255u);
-  const bool grad = (__ldg(m.nflags + __ldg(m.nrec + n).w + (k - nzmin)) >> kGradBit) & 1ull;
+  const bool grad = (__ldg(m.nflags + i) >> kGradBit) & 1ull;   // (flag words in lane order)
   for (int t = 0; t < in.ntr; ++t) {
     const int64_t oa = t * A.a.sN, oe = t * A.a.sEd;
     double gx = 0.0, gy = 0.0;
@@ -535,7 +556,8 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(Adj A) {
       const int e = sl.x >> 1;
       const bool on = in_range(k, unsigned(sl.z)) && !in_range(k, unsigned(ld(m.etr + e)));
       const bool second = sl.x & 1;
-      const double x = (second ? A.a.gX2 : A.a.gX1)[oe + lq(e, L, k)];
+      const uint32_t qe = lq(e, L, k);
+      const double x = grad_factor(second, ld(in.ws.vflux + qe), A.a.gM[oe + qe]);
       const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
       gx = on ? gx + c1 * x : gx;
       gy = on ? gy + c2 * x : gy;
@@ -550,7 +572,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(Adj A) {
 // flux (gfv = -gf + gdiv terms); gw[j] is complete here (only interface j feeds it), and
 // the QR4C flux's terms for ttfAB at levels j, j-1, j-2 and j+1 are stored for r_final to
 // gather. Independent of the edge chain (it runs beside r_edge).
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t i = lane_index();
@@ -568,9 +590,15 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(Adj A) {
   Rcp rdc{1.0, 1.0, true}, rdu{1.0, 1.0, true}, rdd{1.0, 1.0, true};
   if (interior) {
     qr4c_depths(in, m, base, j, Znz, Zm1, Zm2, Zp1, zb);
-    rdc = rcp(safe_nz(Zm1 - Znz));
-    rdu = rcp(safe_nz(Znz - Zp1));
-    rdd = rcp(safe_nz(Zm2 - Zm1));
+    if (in.Z3d) {
+      rdc = rcp(safe_nz(Zm1 - Znz));
+      rdu = rcp(safe_nz(Znz - Zp1));
+      rdd = rcp(safe_nz(Zm2 - Zm1));
+    } else {   // the static depths' reciprocals come from the plan
+      rdc = rcp_known(safe_nz(Zm1 - Znz), ld(m.qr4c + j));
+      rdu = rcp_known(safe_nz(Znz - Zp1), ld(m.qr4c + L + j));
+      rdd = rcp_known(safe_nz(Zm2 - Zm1), ld(m.qr4c + 2 * L + j));
+    }
   }
   for (int t = 0; t < in.ntr; ++t) {
     const int64_t o = t * in.ws.sN, oa = t * A.a.sN;
@@ -627,7 +655,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(Adj A) {
 }
 
 // ---------------- r_tr: cotangent of the element gradients (up/dn use + node average)
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t i = lane_index();
@@ -647,7 +675,8 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(Adj A) {
       const int idx = ld(m.eud_idx + j), e = idx >> 1;
       const bool on = in_range(k, unsigned(ld(m.etr + e)));
       // the down (slot 1) / up (slot 0) cell's gradient enters Tm2 / Tm1
-      const double x = ((idx & 1) ? A.a.gX2 : A.a.gX1)[oe + lq(e, L, k)];
+      const uint32_t qe = lq(e, L, k);
+      const double x = grad_factor(idx & 1, ld(in.ws.vflux + qe), A.a.gM[oe + qe]);
       const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
       gx = on ? gx + c1 * x : gx;
       gy = on ? gy + c2 * x : gy;
@@ -675,7 +704,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(Adj A) {
 // ascending interface order; the edge terms in ascending edge id. Also sums gw_e over the
 // tracers, and writes dT at the dry level above a cavity's first layer (only the
 // (w - |w|) upwind term of interface nzmin reaches it; r_seed wrote the other dry levels).
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_final(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_final(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
   const int64_t li = lane_index();
@@ -687,6 +716,7 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_final(Adj A) {
   const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
   const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
   const int c0 = rec.z, c1 = rec.z + int(pk >> 24);
+  const unsigned onb = unsigned(__ldg(m.nflags + li));   // (flag words in lane order)
   for (int t = 0; t < in.ntr; ++t) {
     const int64_t oa = t * A.a.sN;
     const double* gfv = A.a.gfv + oa;
@@ -731,11 +761,13 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_final(Adj A) {
     double gT = A.a.gTp[oa + i] + gTtr + gTv;
 #pragma unroll 2
     for (int j = e0; j < e1; ++j) {
-      const int4 sl = __ldg(m.ne4 + j);
-      const bool on = in_range(k, unsigned(sl.z));
-      const bool second = sl.x & 1;
-      const int64_t q = t * A.a.sEd + lq(sl.x >> 1, L, k);
-      const double vT = (second ? A.a.gT2 : A.a.gT1)[q], vA = (second ? A.a.gA2 : A.a.gA1)[q];
+      const int4 sl = __ldg(m.ns4 + j);
+      const bool on = (onb >> (j - e0)) & 1u;
+      const uint32_t qe = uint32_t(sl.x) + uint32_t(k);
+      const double vf = ld(in.ws.vflux + qe);
+      double vT, vA;
+      edge_terms(sl.z ? vf < 0.0 : vf > 0.0, A.a.gT[t * A.a.sEd + qe], A.a.gM[t * A.a.sEd + qe],
+                 vT, vA);
       gT = on ? gT + vT : gT;
       gA = on ? gA + vA : gA;
     }
@@ -787,7 +819,7 @@ __device__ __forceinline__ void uv_transpose(const DevMesh& m, const double* __r
   }
 }
 
-__global__ void __launch_bounds__(B, kRevMinBlocks) r_uv(Adj A) {
+__global__ void __launch_bounds__(B, kRevMinBlocks) r_uv(const __grid_constant__ Adj A) {
   const int64_t i = lane_index();
   if (i >= int64_t(A.in.m.E) * A.in.m.L) return;
   uv_transpose(A.in.m, A.in.helem, A.a.gvf, A.in.ntr, A.a.sEd, A.guv, A.acc, i);
@@ -888,7 +920,7 @@ int reserve_adj_ws(FctPlan* P, int max_tracers) {
                      &a.gzm1, &a.gzm2, &a.gzp1};
   static_assert(sizeof(node) / sizeof(node[0]) == kAdjNodeFields, "node field count");
   for (double** f : node) *f = take(sN);
-  double** edge[] = {&a.gT1, &a.gT2, &a.gA1, &a.gA2, &a.gX1, &a.gX2, &a.gvf};
+  double** edge[] = {&a.gT, &a.gM, &a.gvf};
   static_assert(sizeof(edge) / sizeof(edge[0]) == kAdjEdgeFields, "edge field count");
   for (double** f : edge) *f = take(sEd);
   double** elem[] = {&a.gax, &a.gan, &a.gtrx, &a.gtry};

@@ -41,6 +41,9 @@ __device__ __forceinline__ Rcp rcp(double y) {
   return c;
 }
 
+// the same for a divisor whose correctly rounded reciprocal is at hand
+__device__ __forceinline__ Rcp rcp_known(double y, double r) { return Rcp{y, r, div_exp_ok(y)}; }
+
 // The native division for the operands the fast path does not take. Kept out of line so
 // that the compiler branches around it instead of evaluating it under a predicate at
 // every call site.

@@ -94,7 +94,8 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
   if (layer) {
     const double hn = ld(in.hnode + qn), hnn = ld(in.hnode_new + qn);
     const double av = ld(m.areasvol + qn);
-    const Rcp rav = rcp(av), rhn = rcp(hnn);   // shared by the NTR quotients below
+    const Rcp rav = rcp_known(av, ld(m.iavol + qn)), rhn = rcp(hnn);   // shared by the NTR
+                                                                       // quotients below
     const double dt = in.dt;
     double fvk1[NTR];
     if (layer1) {
@@ -112,19 +113,21 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
 #pragma unroll
     for (int t = 0; t < NTR; ++t) div[t] = 0.0;
     const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
-    for (int j = e0; j < e1; ++j) {
-      const int idx = ld(m.ne_idx + j), e = idx >> 1;
-      if (k < ld(m.ekmin + e) || k >= ld(m.ekmax + e)) continue;   // vflux == 0 there
-      const int oth = ld(m.ne_oth + j);
-      const double vf = ld(in.ws.vflux + lq(e, L, k));
+    const unsigned long long flags = __ldg(m.nflags + __ldg(m.nrec + n).w + (k - nzmin));
+    unsigned onb = unsigned(flags);   // bit j: the j-th slot's edge has the layer
+    for (int j = e0; j < e1; ++j, onb >>= 1) {
+      const int4 sl = __ldg(m.ns4 + j);
+      if (!(onb & 1u)) continue;   // vflux == 0 there
+      const double vf = ld(in.ws.vflux + (uint32_t(sl.x) + uint32_t(k)));
       const double avf = fabs(vf);
+      // the face flux with the node's own value first (a + b == b + a exactly)
+      const double cown = sl.z ? vf - avf : vf + avf, coth = sl.z ? vf + avf : vf - avf;
       double To[NTR];
-      ldn<NTR, IL>(in.T, lq(oth, L, k), t0, ts, tg, To);
+      ldn<NTR, IL>(in.T, uint32_t(sl.y) + uint32_t(k), t0, ts, tg, To);
 #pragma unroll
       for (int t = 0; t < NTR; ++t) {
-        const double T1 = (idx & 1) ? To[t] : Tc[t], T2 = (idx & 1) ? Tc[t] : To[t];
-        const double fl = -0.5 * (T1 * (vf + avf) + T2 * (vf - avf));
-        div[t] += (idx & 1) ? -fl : fl;
+        const double fl = -0.5 * (Tc[t] * cown + To[t] * coth);
+        div[t] += sl.z ? -fl : fl;
       }
     }
   
@@ -138,8 +141,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
     // _node_avg_grad: area-weighted mean over the node's active elements, at the levels
     // where an edge of the node takes it (kGradBit; its readers, the edge stage's and the
     // reverse pass's node-gradient lanes, read no other level)
-    const int fw = __ldg(m.nrec + n).w;
-    if ((__ldg(m.nflags + fw + (k - nzmin)) >> kGradBit) & 1ull) {
+    if ((flags >> kGradBit) & 1ull) {
       double nx[NTR], ny[NTR], den = 0.0;
 #pragma unroll
       for (int t = 0; t < NTR; ++t) nx[t] = ny[t] = 0.0;
@@ -200,8 +202,16 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
       Znz = ld(m.Zp + k); Zm1 = ld(m.Zp + k - 1); Zm2 = ld(m.Zp + k - 2);
       Zp1 = ld(m.Zp + (k + 1 < L ? k + 1 : L - 1)); zb = ld(m.zbar + k);
     }
-    const Rcp rdc = rcp(safe_nz(Zm1 - Znz)), rdu = rcp(safe_nz(Znz - Zp1)),
-              rdd = rcp(safe_nz(Zm2 - Zm1));
+    Rcp rdc, rdu, rdd;
+    if (in.Z3d) {
+      rdc = rcp(safe_nz(Zm1 - Znz));
+      rdu = rcp(safe_nz(Znz - Zp1));
+      rdd = rcp(safe_nz(Zm2 - Zm1));
+    } else {   // the static depths' reciprocals come from the plan
+      rdc = rcp_known(safe_nz(Zm1 - Znz), ld(m.qr4c + k));
+      rdu = rcp_known(safe_nz(Znz - Zp1), ld(m.qr4c + L + k));
+      rdd = rcp_known(safe_nz(Zm2 - Zm1), ld(m.qr4c + 2 * L + k));
+    }
     const Rcp r3{3.0, 1.0 / 3.0, true};
     double To[NTR], Tom[NTR], Tm2[NTR], Tom2[NTR], Tp[NTR], Top[NTR];
     ldn<NTR, IL>(in.T_old, qn, t0, ts, tg, To);
@@ -246,36 +256,35 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int t0,
   const uint32_t q1 = lq(n1, L, k), q2 = lq(n2, L, k);
   const int64_t ts = in.tstride;
   const int tg = in.tg;
-  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], g0[NTR], g1[NTR], g2[NTR], g3[NTR];
+  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[NTR], gy[NTR];
   ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
   ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
   ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
   ldn<NTR, IL>(in.T_old, q2, t0, ts, tg, O2);
+  // -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2) is exactly -0.5 times the upwind end's term (the
+  // other one is 0), so only that end's gradient is read
+  const bool first = vf > 0.0;
   if (use_tri) {
     // both cells are wet at k here (k is above every adjacent cell's bottom)
-    const int up = ld(m.eupdn + 2 * e), dn = ld(m.eupdn + 2 * e + 1);
-    const uint32_t qu = lq(up, L, k), qd = lq(dn, L, k);
-    ldn<NTR, IL>(in.ws.gx, qu, w0, in.ws.sE, in.wtg, g0);
-    ldn<NTR, IL>(in.ws.gx, qd, w0, in.ws.sE, in.wtg, g1);
-    ldn<NTR, IL>(in.ws.gy, qu, w0, in.ws.sE, in.wtg, g2);
-    ldn<NTR, IL>(in.ws.gy, qd, w0, in.ws.sE, in.wtg, g3);
-  
+    const uint32_t q = lq(ld(m.eupdn + 2 * e + (first ? 0 : 1)), L, k);
+    ldn<NTR, IL>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
+    ldn<NTR, IL>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
   } else {
-    ldn<NTR, IL>(in.ws.gnx, q1, w0, in.ws.sN, in.wtg, g0);
-    ldn<NTR, IL>(in.ws.gnx, q2, w0, in.ws.sN, in.wtg, g1);
-    ldn<NTR, IL>(in.ws.gny, q1, w0, in.ws.sN, in.wtg, g2);
-    ldn<NTR, IL>(in.ws.gny, q2, w0, in.ws.sN, in.wtg, g3);
+    const uint32_t q = first ? q1 : q2;
+    ldn<NTR, IL>(in.ws.gnx, q, w0, in.ws.sN, in.wtg, gx);
+    ldn<NTR, IL>(in.ws.gny, q, w0, in.ws.sN, in.wtg, gy);
   }
   double adf[NTR];
   const Rcp r6{6.0, 1.0 / 6.0, true};
+  const double cu = first ? vf + avf : vf - avf;
 #pragma unroll
   for (int t = 0; t < NTR; ++t) {
     const double fl = -0.5 * (T1[t] * (vf + avf) + T2[t] * (vf - avf));
     const double A1 = ab2(T1[t], O1[t]), A2 = ab2(T2[t], O2[t]);
     const double diff = A2 - A1;
-    const double Tm1 = A1 + divr(2.0 * diff + c1 * g0[t] + c2 * g2[t], r6);
-    const double Tm2 = A2 - divr(2.0 * diff + c1 * g1[t] + c2 * g3[t], r6);
-    const double ho = -0.5 * ((vf + avf) * Tm1 + (vf - avf) * Tm2);
+    const double X = divr(2.0 * diff + c1 * gx[t] + c2 * gy[t], r6);
+    const double Tm = first ? A1 + X : A2 - X;
+    const double ho = -0.5 * (cu * Tm);
     adf[t] = ho - fl;
   }
   stn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);
@@ -394,8 +403,9 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
   const bool use_own = (k == nzmin) || (k == nzmax - 1);
   const double av = ld(m.areasvol + qn), hnn = ld(in.hnode_new + qn);
   const bool valid = (av > 0.0) && (hnn > 0.0);
-  const double sa = av > 0.0 ? av : 1.0, sh = hnn > 0.0 ? hnn : 1.0;
-  const Rcp rsa = rcp(sa), rsh = rcp(sh);
+  const double sh = hnn > 0.0 ? hnn : 1.0;
+  const Rcp rsa = av > 0.0 ? rcp_known(av, ld(m.iavol + qn)) : Rcp{1.0, 1.0, true};
+  const Rcp rsh = rcp(sh);
   const double dt = in.dt;
   const int64_t sN = in.ws.sN;
   double tmax[NTR], tmin[NTR];
@@ -421,14 +431,15 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
 #pragma unroll
   for (int t = 0; t < NTR; ++t) sp[t] = sm[t] = 0.0;
   const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
-  for (int j = e0; j < e1; ++j) {
-    const int idx = ld(m.ne_idx + j), e = idx >> 1;
-    if (k < ld(m.ekmin + e) || k >= ld(m.ekmax + e)) continue;   // no flux on this level
+  unsigned onb = unsigned(__ldg(m.nflags + i));   // (flag words in lane order)
+  for (int j = e0; j < e1; ++j, onb >>= 1) {
+    const int4 sl = __ldg(m.ns4 + j);
+    if (!(onb & 1u)) continue;   // no flux on this level
     double a[NTR];
-    ldn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, a);
+    ldn<NTR, IL>(in.ws.adfh, uint32_t(sl.x) + uint32_t(k), w0, in.ws.sEd, in.wtg, a);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
-      const double s = (idx & 1) ? -a[t] : a[t];
+      const double s = sl.z ? -a[t] : a[t];
       sp[t] += fmax(s, 0.0);
       sm[t] += fmin(s, 0.0);
     }
@@ -466,9 +477,9 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
   const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
   const uint32_t base = lq(n, L, 0), qn = base + uint32_t(k);
   const double av = ld(m.areasvol + qn);
-  const double sa = av > 0.0 ? av : 1.0;
   const double hn = ld(in.hnode + qn), hnn = ld(in.hnode_new + qn);
-  const Rcp rsa = rcp(sa), rhn = rcp(hnn);
+  const Rcp rsa = av > 0.0 ? rcp_known(av, ld(m.iavol + qn)) : Rcp{1.0, 1.0, true};
+  const Rcp rhn = rcp(hnn);
   const double dt = in.dt;
   const int tg = in.tg;
   const int64_t sN = in.ws.sN;
@@ -509,22 +520,23 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
 #pragma unroll
   for (int t = 0; t < NTR; ++t) hsc[t] = 0.0;
   const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
-  for (int j = e0; j < e1; ++j) {
-    const int idx = ld(m.ne_idx + j), e = idx >> 1;
-    if (k < ld(m.ekmin + e) || k >= ld(m.ekmax + e)) continue;   // no flux on this level
-    const uint32_t qo = lq(ld(m.ne_oth + j), L, k);
+  unsigned onb = unsigned(__ldg(m.nflags + i));   // (flag words in lane order)
+  for (int j = e0; j < e1; ++j, onb >>= 1) {
+    const int4 sl = __ldg(m.ns4 + j);
+    if (!(onb & 1u)) continue;   // no flux on this level
+    const uint32_t qo = uint32_t(sl.y) + uint32_t(k);
     double a[NTR], pfo[NTR], mfo[NTR];
-    ldn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, a);
+    ldn<NTR, IL>(in.ws.adfh, uint32_t(sl.x) + uint32_t(k), w0, in.ws.sEd, in.wtg, a);
     ldn<NTR, IL>(in.ws.pf, qo, w0, sN, in.wtg, pfo);
     ldn<NTR, IL>(in.ws.mf, qo, w0, sN, in.wtg, mfo);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
-      // (pf, mf) at the edge's first node n1 and second node n2
-      const double pf1 = (idx & 1) ? pfo[t] : pf0[t], mf1 = (idx & 1) ? mfo[t] : mf0[t];
-      const double pf2 = (idx & 1) ? pf0[t] : pfo[t], mf2 = (idx & 1) ? mf0[t] : mfo[t];
-      const double ae = a[t] >= 0.0 ? fmin(pf1, mf2) : fmin(mf1, pf2);
+      // ae = a >= 0 ? min(plus(n1), minus(n2)) : min(minus(n1), plus(n2)): the own plus and
+      // the other's minus when the flux leaves the node, else the other pair
+      const bool leaves = (a[t] >= 0.0) != (sl.z != 0);
+      const double ae = fmin(leaves ? pf0[t] : mf0[t], leaves ? mfo[t] : pfo[t]);
       const double lim = ae * a[t];
-      hsc[t] += (idx & 1) ? -lim : lim;
+      hsc[t] += sl.z ? -lim : lim;
     }
   }
   double Tv[NTR], lo[NTR], out[NTR];
@@ -565,8 +577,11 @@ __device__ __forceinline__ void body_copy_dry(const Inst& in, int64_t i) {
 // accordingly): latency hiding pays more than the spills it costs (one tracer, the
 // adjoint's taped forward on the CORE2-size mesh: 11.1 ms for 10 steps at 6 blocks,
 // 10.6 ms at 7, no gain at 8).
+#ifndef FCT_KMB
+#define FCT_KMB 7
+#endif
 template <int NTR>
-constexpr int kMinBlocks = NTR == 1 ? 7 : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
+constexpr int kMinBlocks = NTR == 1 ? FCT_KMB : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
 
 #define FCT_KERNEL_T(name, body)                                                        \
   template <int NTR>                                                                    \

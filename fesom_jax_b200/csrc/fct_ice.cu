@@ -3,9 +3,13 @@
 //
 // The reference scatters element contributions to nodes; here every node gathers over
 // its cells (node->element CSR in the reference's nod_in_elem2D order, the node's vertex
-// index packed in the slot) so sums are deterministic and no atomics are needed. One
-// thread per node carries all three tracers: the tracer-independent cell terms (the
-// Taylor-Galerkin matrix row, the mass-matrix weight) are formed once per cell.
+// index packed in the slot) so sums are deterministic and no atomics are needed. A thread
+// takes a node and one tracer (blockIdx.y); the right-hand side, whose matrix row is the same
+// for all tracers, a node and all three. The kernels wait on their gathers: with all three
+// tracers in one thread the CORE2-size mesh filled a third of the warp slots, and every flux
+// divided by 12 through the full division sequence. Now the mesh's quotients come from the
+// plan, quotients by 12 and 9 are correctly rounded products (fct_div.cuh), and a cell's slot
+// is loaded one ahead.
 //
 //   k_ice_rhs    _tg_rhs (:47-75), _mm_times (:37-44), _solve_low_order (:78-89),
 //                first high-order approximation (:103)
@@ -14,18 +18,18 @@
 //   k_ice_apply  _fem_fct limited flux application (:162-172)
 #include <algorithm>
 
+#include "fct_div.cuh"
 #include "fct_host.h"
 
 using namespace fct;
 
 namespace {
 
-constexpr double kIceScaleArea = 2.0e8;   // ice_adv.py:33
 constexpr double kIceFluxEps = 1.0e-12;   // ice_adv.py:34
 constexpr int B = 128;
 
 struct IceArgs {
-  const DevMesh* m;
+  DevMesh m;
   const double* X[3];   // a_ice, m_ice, m_snow
   const double *u, *v;
   double* out[3];
@@ -36,55 +40,73 @@ struct IceArgs {
 __device__ __forceinline__ int64_t node_index() {
   return int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
 }
-__device__ __forceinline__ bool cell_on(const DevMesh& m, int el) { return __ldg(m.eul + el) <= 0; }
-__device__ __forceinline__ double inv_area(const DevMesh& m, int n) {
-  const double a = __ldg(m.area + int64_t(n) * m.L);   // surface level
-  return 1.0 / (a > 0.0 ? a : 1.0);
+// x / 12 and x / 9, correctly rounded
+__device__ __forceinline__ double div12(double x) { return divr(x, Rcp{12.0, 1.0 / 12.0, true}); }
+__device__ __forceinline__ double div9(double x) { return divr(x, Rcp{9.0, 1.0 / 9.0, true}); }
+
+// A node's cells in order, the slot records one ahead: ``sl`` {cell, its vertices}, ``p`` the
+// node's place among them, ``on`` not a cavity cell.
+#define ICE_FOR_CELLS(c0, c1)                                                     \
+  int4 sl_nx = (c0) < (c1) ? __ldg(m.nel4 + (c0)) : make_int4(0, 0, 0, 0);        \
+  int r_nx = (c0) < (c1) ? __ldg(m.nelr + (c0)) : 0;                              \
+  for (int j = (c0); j < (c1); ++j)
+#define ICE_CELL(c1)                                                              \
+  const int4 sl = sl_nx;                                                          \
+  const int p = (r_nx >> 16) & 3;                                                 \
+  const bool on = (r_nx & 255) == 0;                                              \
+  if (j + 1 < (c1)) {                                                             \
+    sl_nx = __ldg(m.nel4 + j + 1);                                                \
+    r_nx = __ldg(m.nelr + j + 1);                                                 \
+  }                                                                               \
+  const int vq[3] = {sl.y, sl.z, sl.w};
+
+__device__ __forceinline__ double pick(const double (&x)[3], int p) {
+  return p == 0 ? x[0] : (p == 1 ? x[1] : x[2]);
 }
 
-__global__ void __launch_bounds__(B) k_ice_rhs(IceArgs A) {
-  const DevMesh& m = *A.m;
+__global__ void __launch_bounds__(B) k_ice_rhs(const __grid_constant__ IceArgs A) {
+  const DevMesh& m = A.m;
   const int64_t n = node_index();
   if (n >= m.N) return;
   const int N = m.N;
   double rhs[3] = {0.0, 0.0, 0.0}, mmx[3] = {0.0, 0.0, 0.0};
   const int c0 = __ldg(m.nel_off + n), c1 = __ldg(m.nel_off + n + 1);
-  for (int j = c0; j < c1; ++j) {
-    const int4 sl = __ldg(m.nel4 + j);
-    if (!cell_on(m, sl.x)) continue;   // cavity cells contribute 0
-    const int p = (__ldg(m.nelr + j) >> 16) & 3;
-    const int vq[3] = {sl.y, sl.z, sl.w};
-    const double* gs = m.gsca + 6 * int64_t(sl.x);
-    const double dx[3] = {__ldg(gs), __ldg(gs + 1), __ldg(gs + 2)};
-    const double dy[3] = {__ldg(gs + 3), __ldg(gs + 4), __ldg(gs + 5)};
-    const double vol = __ldg(m.earea + sl.x);
-    double U[3], V[3];
+  ICE_FOR_CELLS(c0, c1) {
+    ICE_CELL(c1)
+    if (!on) continue;   // cavity cells contribute 0
+    const double2* gs = reinterpret_cast<const double2*>(m.gsca + 6 * int64_t(sl.x));
+    const double2 g0 = __ldg(gs), g1 = __ldg(gs + 1), g2 = __ldg(gs + 2);
+    const double dx[3] = {g0.x, g0.y, g1.x}, dy[3] = {g1.y, g2.x, g2.y};
+    const double vol = __ldg(m.earea + sl.x), vol12 = __ldg(m.earea12 + sl.x);
+    double U[3], V[3], x[3][3];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) { U[q] = __ldg(A.u + vq[q]); V[q] = __ldg(A.v + vq[q]); }
+    for (int q = 0; q < 3; ++q) {
+      U[q] = __ldg(A.u + vq[q]);
+      V[q] = __ldg(A.v + vq[q]);
+#pragma unroll
+      for (int t = 0; t < 3; ++t) x[t][q] = __ldg(A.X[t] + vq[q]);
+    }
     const double um = U[0] + U[1] + U[2], vm = V[0] + V[1] + V[2];
-    const double diff = A.diff * sqrt(vol / kIceScaleArea);
-    const double dxp = dx[p], dyp = dy[p];
+    const double diff = A.diff * __ldg(m.ediff + sl.x);
+    const double dxp = pick(dx, p), dyp = pick(dy, p);
     const double udnp = um * dxp + vm * dyp;
     double E[3];
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double a = (dxp * (um + U[q]) + dyp * (vm + V[q])) / 12.0;
+      const double a = div12(dxp * (um + U[q]) + dyp * (vm + V[q]));
       const double b = diff * (dxp * dx[q] + dyp * dy[q]);
       const double udnq = um * dx[q] + vm * dy[q];
-      const double c = 0.5 * A.dt * (udnp * udnq) / 9.0;
+      const double c = div9(0.5 * A.dt * (udnp * udnq));
       E[q] = vol * A.dt * (a - b - c);
     }
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
-      const double x0 = __ldg(A.X[t] + vq[0]), x1 = __ldg(A.X[t] + vq[1]),
-                   x2 = __ldg(A.X[t] + vq[2]);
-      rhs[t] += E[0] * x0 + E[1] * x1 + E[2] * x2;
-      const double xs[3] = {x0, x1, x2};
-      mmx[t] += vol / 12.0 * (xs[p] + (x0 + x1 + x2));
+      rhs[t] += E[0] * x[t][0] + E[1] * x[t][1] + E[2] * x[t][2];
+      mmx[t] += vol12 * (pick(x[t], p) + (x[t][0] + x[t][1] + x[t][2]));
     }
   }
   const bool nc = __ldg(m.nzmin + n) <= 0;   // ulevels_nod2D <= 1
-  const double ia = inv_area(m, int(n));
+  const double ia = __ldg(m.iarea0 + n);
 #pragma unroll
   for (int t = 0; t < 3; ++t) {
     const double X = __ldg(A.X[t] + n);
@@ -95,121 +117,103 @@ __global__ void __launch_bounds__(B) k_ice_rhs(IceArgs A) {
 }
 
 // d_out = d_in + (rhs - mm d_in) / area on open-water/ice nodes
-__global__ void __launch_bounds__(B) k_ice_hi(IceArgs A, const double* __restrict__ din,
+__global__ void __launch_bounds__(B) k_ice_hi(const __grid_constant__ IceArgs A,
+                                              const double* __restrict__ din_,
                                               double* __restrict__ dout) {
-  const DevMesh& m = *A.m;
+  const DevMesh& m = A.m;
   const int64_t n = node_index();
   if (n >= m.N) return;
-  const int N = m.N;
-  double mmd[3] = {0.0, 0.0, 0.0};
+  const int64_t o = int64_t(blockIdx.y) * m.N;
+  const double* __restrict__ din = din_ + o;
+  double mmd = 0.0;
   const int c0 = __ldg(m.nel_off + n), c1 = __ldg(m.nel_off + n + 1);
-  for (int j = c0; j < c1; ++j) {
-    const int4 sl = __ldg(m.nel4 + j);
-    if (!cell_on(m, sl.x)) continue;
-    const int p = (__ldg(m.nelr + j) >> 16) & 3;
-    const double vol = __ldg(m.earea + sl.x);
-#pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      const double x0 = din[t * N + sl.y], x1 = din[t * N + sl.z], x2 = din[t * N + sl.w];
-      const double xs[3] = {x0, x1, x2};
-      mmd[t] += vol / 12.0 * (xs[p] + (x0 + x1 + x2));
-    }
+  ICE_FOR_CELLS(c0, c1) {
+    ICE_CELL(c1)
+    const double x[3] = {__ldg(din + vq[0]), __ldg(din + vq[1]), __ldg(din + vq[2])};
+    const double s = __ldg(m.earea12 + sl.x) * (pick(x, p) + (x[0] + x[1] + x[2]));
+    mmd = on ? mmd + s : mmd;
   }
   const bool nc = __ldg(m.nzmin + n) <= 0;
-  const double ia = inv_area(m, int(n));
-#pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    const double d = din[t * N + n];
-    dout[t * N + n] = nc ? d + (A.rhs[t * N + n] - mmd[t]) * ia : d;
-  }
+  const double ia = __ldg(m.iarea0 + n), d = din[n];
+  dout[o + n] = nc ? d + (A.rhs[o + n] - mmd) * ia : d;
 }
 
 // the cell's antidiffusive flux at vertex q: -s_q (vol / area_q) / 12, s_q = sum w - 3 w_q
 __device__ __forceinline__ double ice_flux(double sw, double wq, double vol, double iaq) {
-  return -(sw - 3.0 * wq) * (vol * iaq) / 12.0;
+  return div12(-(sw - 3.0 * wq) * (vol * iaq));
 }
 
-__global__ void __launch_bounds__(B) k_ice_limit(IceArgs A, const double* __restrict__ dv) {
-  const DevMesh& m = *A.m;
+__global__ void __launch_bounds__(B) k_ice_limit(const __grid_constant__ IceArgs A,
+                                                 const double* __restrict__ dv_) {
+  const DevMesh& m = A.m;
   const int64_t n = node_index();
   if (n >= m.N) return;
-  const int N = m.N;
-  const double ia_n = inv_area(m, int(n));
-  double fp[3] = {0.0, 0.0, 0.0}, fm[3] = {0.0, 0.0, 0.0};
-  double hi[3] = {-INFINITY, -INFINITY, -INFINITY}, lo[3] = {INFINITY, INFINITY, INFINITY};
+  const int64_t o = int64_t(blockIdx.y) * m.N;
+  const double* __restrict__ X = A.X[blockIdx.y];
+  const double* __restrict__ dv = dv_ + o;
+  const double* __restrict__ XL = A.xl + o;
+  const double ia_n = __ldg(m.iarea0 + n);
+  double fp = 0.0, fm = 0.0, hi = -INFINITY, lo = INFINITY;
   const int c0 = __ldg(m.nel_off + n), c1 = __ldg(m.nel_off + n + 1);
-  for (int j = c0; j < c1; ++j) {
-    const int4 sl = __ldg(m.nel4 + j);
-    const bool on = cell_on(m, sl.x);
-    const int p = (__ldg(m.nelr + j) >> 16) & 3;
-    const int vq[3] = {sl.y, sl.z, sl.w};
+  ICE_FOR_CELLS(c0, c1) {
+    ICE_CELL(c1)
     const double vol = __ldg(m.earea + sl.x);
+    double w[3], xl[3], xv[3];
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      double w[3], xl[3], xv[3];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        xv[q] = __ldg(A.X[t] + vq[q]);
-        w[q] = A.gamma * xv[q] + dv[t * N + vq[q]];
-        xl[q] = A.xl[t * N + vq[q]];
-      }
-      const double sw = w[0] + w[1] + w[2];
-      const double f = on ? ice_flux(sw, w[p], vol, ia_n) : 0.0;
-      fp[t] += fmax(f, 0.0);
-      fm[t] += fmin(f, 0.0);
-      if (on) {
-        const double ehi = fmax(fmax(fmax(xl[0], xl[1]), xl[2]), fmax(fmax(xv[0], xv[1]), xv[2]));
-        const double elo = fmin(fmin(fmin(xl[0], xl[1]), xl[2]), fmin(fmin(xv[0], xv[1]), xv[2]));
-        hi[t] = fmax(hi[t], ehi);
-        lo[t] = fmin(lo[t], elo);
-      }
+    for (int q = 0; q < 3; ++q) {
+      xv[q] = __ldg(X + vq[q]);
+      w[q] = A.gamma * xv[q] + __ldg(dv + vq[q]);
+      xl[q] = __ldg(XL + vq[q]);
     }
+    if (!on) continue;
+    const double sw = w[0] + w[1] + w[2];
+    const double f = ice_flux(sw, pick(w, p), vol, ia_n);
+    fp += fmax(f, 0.0);
+    fm += fmin(f, 0.0);
+    const double ehi = fmax(fmax(fmax(xl[0], xl[1]), xl[2]), fmax(fmax(xv[0], xv[1]), xv[2]));
+    const double elo = fmin(fmin(fmin(xl[0], xl[1]), xl[2]), fmin(fmin(xv[0], xv[1]), xv[2]));
+    hi = fmax(hi, ehi);
+    lo = fmin(lo, elo);
   }
   const bool nc = __ldg(m.nzmin + n) <= 0;
-#pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    const double h = isfinite(hi[t]) ? hi[t] : 0.0, l = isfinite(lo[t]) ? lo[t] : 0.0;
-    const double xl = A.xl[t * N + n];
-    const double tmax = h - xl, tmin = l - xl;
-    double pp = fp[t] > 0.0 ? fmin(tmax / (fp[t] > kIceFluxEps ? fp[t] : kIceFluxEps), 1.0) : 0.0;
-    double pm = fm[t] < 0.0 ? fmin(tmin / (fm[t] < -kIceFluxEps ? fm[t] : -kIceFluxEps), 1.0) : 0.0;
-    A.pp[t * N + n] = nc ? pp : 0.0;
-    A.pm[t * N + n] = nc ? pm : 0.0;
-  }
+  const double h = isfinite(hi) ? hi : 0.0, l = isfinite(lo) ? lo : 0.0;
+  const double xl = XL[n];
+  const double tmax = h - xl, tmin = l - xl;
+  const double pp = fp > 0.0 ? fmin(tmax / (fp > kIceFluxEps ? fp : kIceFluxEps), 1.0) : 0.0;
+  const double pm = fm < 0.0 ? fmin(tmin / (fm < -kIceFluxEps ? fm : -kIceFluxEps), 1.0) : 0.0;
+  A.pp[o + n] = nc ? pp : 0.0;
+  A.pm[o + n] = nc ? pm : 0.0;
 }
 
-__global__ void __launch_bounds__(B) k_ice_apply(IceArgs A, const double* __restrict__ dv) {
-  const DevMesh& m = *A.m;
+__global__ void __launch_bounds__(B) k_ice_apply(const __grid_constant__ IceArgs A,
+                                                 const double* __restrict__ dv_) {
+  const DevMesh& m = A.m;
   const int64_t n = node_index();
   if (n >= m.N) return;
-  const int N = m.N;
-  double acc[3] = {0.0, 0.0, 0.0};
+  const int64_t o = int64_t(blockIdx.y) * m.N;
+  const double* __restrict__ X = A.X[blockIdx.y];
+  const double* __restrict__ dv = dv_ + o;
+  const double* __restrict__ pp = A.pp + o;
+  const double* __restrict__ pm = A.pm + o;
+  double acc = 0.0;
   const int c0 = __ldg(m.nel_off + n), c1 = __ldg(m.nel_off + n + 1);
-  for (int j = c0; j < c1; ++j) {
-    const int4 sl = __ldg(m.nel4 + j);
-    if (!cell_on(m, sl.x)) continue;   // limited fluxes of cavity cells are 0
-    const int p = (__ldg(m.nelr + j) >> 16) & 3;
-    const int vq[3] = {sl.y, sl.z, sl.w};
+  ICE_FOR_CELLS(c0, c1) {
+    ICE_CELL(c1)
     const double vol = __ldg(m.earea + sl.x);
-    const double ia[3] = {inv_area(m, vq[0]), inv_area(m, vq[1]), inv_area(m, vq[2])};
+    double w[3], f[3], cand[3];
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-      double w[3];
+    for (int q = 0; q < 3; ++q) w[q] = A.gamma * __ldg(X + vq[q]) + __ldg(dv + vq[q]);
+    const double sw = w[0] + w[1] + w[2];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) w[q] = A.gamma * __ldg(A.X[t] + vq[q]) + dv[t * N + vq[q]];
-      const double sw = w[0] + w[1] + w[2];
-      double f[3], cand[3];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        f[q] = ice_flux(sw, w[q], vol, ia[q]);
-        cand[q] = f[q] >= 0.0 ? A.pp[t * N + vq[q]] : A.pm[t * N + vq[q]];
-      }
-      const double ae = fmin(fmin(cand[0], cand[1]), cand[2]);
-      acc[t] += f[p] * ae;
+    for (int q = 0; q < 3; ++q) {
+      const double a = __ldg(pp + vq[q]), b = __ldg(pm + vq[q]);
+      f[q] = ice_flux(sw, w[q], vol, __ldg(m.iarea0 + vq[q]));
+      cand[q] = f[q] >= 0.0 ? a : b;
     }
+    const double ae = fmin(fmin(cand[0], cand[1]), cand[2]);
+    acc = on ? acc + pick(f, p) * ae : acc;   // limited fluxes of cavity cells are 0
   }
-#pragma unroll
-  for (int t = 0; t < 3; ++t) A.out[t][n] = A.xl[t * N + n] + acc[t];
+  A.out[blockIdx.y][n] = A.xl[o + n] + acc;
 }
 
 }  // namespace
@@ -232,7 +236,7 @@ extern "C" int fct_ice_solve(FctPlan* P, const FctIceFields* f, const FctIceConf
   cudaGetDevice(&prev);
   if (prev != P->device) cudaSetDevice(P->device);
   IceArgs A{};
-  A.m = P->d_mesh;
+  A.m = P->hm;
   for (int t = 0; t < 3; ++t) { A.X[t] = f->tracer[t]; A.out[t] = f->tracer_new[t]; }
   A.u = f->u_ice;
   A.v = f->v_ice;
@@ -248,10 +252,11 @@ extern "C" int fct_ice_solve(FctPlan* P, const FctIceFields* f, const FctIceConf
     st = use.status();
     if (!st) {
       k_ice_rhs<<<g, B, 0, s>>>(A);
-      k_ice_hi<<<g, B, 0, s>>>(A, A.d0, A.d1);   // two residual corrections (ice_adv.py:104)
-      k_ice_hi<<<g, B, 0, s>>>(A, A.d1, A.d0);
-      k_ice_limit<<<g, B, 0, s>>>(A, A.d0);
-      k_ice_apply<<<g, B, 0, s>>>(A, A.d0);
+      const dim3 g3(g, 3);
+      k_ice_hi<<<g3, B, 0, s>>>(A, A.d0, A.d1);   // two residual corrections (ice_adv.py:104)
+      k_ice_hi<<<g3, B, 0, s>>>(A, A.d1, A.d0);
+      k_ice_limit<<<g3, B, 0, s>>>(A, A.d0);
+      k_ice_apply<<<g3, B, 0, s>>>(A, A.d0);
       const cudaError_t e = cudaGetLastError();
       st = e == cudaSuccess ? use.release() : cuda_error(e, "ice FCT launch");
     }

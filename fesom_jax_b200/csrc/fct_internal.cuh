@@ -24,6 +24,7 @@ constexpr double kAbOld = -(0.5 + 0.1);  // tracer_adv.py:44-46
 constexpr double kAbNew = (1.5 + 0.1);
 constexpr double kFluxEps = 1e-16;       // tracer_adv.py:192
 constexpr double kBig = 1e3;             // tracer_adv.py:193
+constexpr double kIceScaleArea = 2.0e8;  // ice_adv.py:33
 
 __host__ __device__ inline int lane_ent(uint32_t lane) { return int(lane >> kLevelBits); }
 // The layer ranges [eul, enl) of an edge's two cells in one word: cell 1 in the low
@@ -154,6 +155,8 @@ struct DevMesh {
   // per node->edge slot of the segment kernels: {edge * L, other node * L (dense offsets, 32
   // bits), 0x80000000 when the node is the edge's second node (a sign mask), 0}
   const int4* ns4;
+  // sea-ice tables: 1 / surface area (safe), cell area / 12, sqrt(cell area / 2e8)
+  const double *iarea0, *earea12, *ediff;
   const double* iavol;   // [N,L] 1 / areasvol, correctly rounded (0 where areasvol is 0)
   // [5,L] QR4C stencil of interface k on the static depths: the reciprocals of Z[k-1]-Z[k],
   // Z[k]-Z[k+1], Z[k-2]-Z[k-1], then (zbar[k]-Z[k])/3, (zbar[k]-Z[k-1])/3 (k >= 2)
@@ -240,10 +243,9 @@ struct AdjWorkspace {
   double *ggnx, *ggny;        // node-average gradients
   double *gfv, *gw;           // vertical LO flux, w_e (per tracer)
   double *gz0, *gzm1, *gzm2, *gzp1;  // interface j's QR4C flux into ttfAB at j, j-1, j-2, j+1
-  // edge [Ed, L] per tracer: the per-end cotangents of the edge's fluxes (T at the first /
-  // second node through the upwind flux, ttfAB through MFCT, the MFCT gradient factor
-  // of each end) and of its volume flux
-  double *gT1, *gT2, *gA1, *gA2, *gX1, *gX2, *gvf;
+  // edge [Ed, L] per tracer: the cotangents of the edge's upwind T through the LO flux and of
+  // its upwind Tm through the HO flux (the other end's are 0), and of its volume flux
+  double *gT, *gM, *gvf;
   // element [E, L] per tracer: the element bounds' shares (divided by the vertex tie
   // counts) and the element gradients
   double *gax, *gan, *gtrx, *gtry;
@@ -252,7 +254,7 @@ struct AdjWorkspace {
   double* gvf_sum;
   int64_t sN, sE, sEd;
 };
-constexpr int kAdjNodeFields = 16, kAdjEdgeFields = 7, kAdjElemFields = 4;
+constexpr int kAdjNodeFields = 16, kAdjEdgeFields = 3, kAdjElemFields = 4;
 
 }  // namespace fct
 

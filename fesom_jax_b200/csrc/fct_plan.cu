@@ -10,6 +10,7 @@
 //   * per-edge MFCT coefficients (edx*a, edy*R) with a = R*cos averaged over the edge's
 //     cells, evaluated with the reference's expression (tracer_adv.py:216-220).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <unordered_set>
@@ -353,6 +354,15 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   std::vector<double> iavol(size_t(N) * L), qr4c(5 * size_t(L), 0.0);
   for (size_t i = 0; i < iavol.size(); ++i)
     iavol[i] = d->areasvol[i] > 0.0 ? 1.0 / d->areasvol[i] : 0.0;
+  std::vector<double> iarea0(N), earea12(E), ediff(E);
+  for (int n = 0; n < N; ++n) {
+    const double a = d->area[size_t(n) * L];
+    iarea0[n] = 1.0 / (a > 0.0 ? a : 1.0);
+  }
+  for (int e = 0; e < E; ++e) {
+    earea12[e] = d->elem_area[e] / 12.0;
+    ediff[e] = std::sqrt(d->elem_area[e] / kIceScaleArea);
+  }
   for (int k = 2; k < L; ++k) {
     auto gap = [](double x) { return x == 0.0 ? 1.0 : x; };
     const double Zn = Zp[std::min(k + 1, L - 1)];
@@ -551,6 +561,8 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   size_t o_nrec = b.add(nrec.data(), nrec.size()), o_erec = b.add(erec.data(), erec.size());
   size_t o_ns4 = b.add(ns4.data(), ns4.size()), o_iavol = b.add(iavol.data(), iavol.size());
   size_t o_qr4c = b.add(qr4c.data(), qr4c.size());
+  size_t o_iarea0 = b.add(iarea0.data(), N), o_earea12 = b.add(earea12.data(), E);
+  size_t o_ediff = b.add(ediff.data(), E);
   size_t o_emf4 = b.add(emf4.data(), emf4.size()), o_emfw = b.add(emfw.data(), emfw.size());
   size_t o_nflags = b.add(nflags.data(), std::max<size_t>(nflags.size(), 1));
   size_t o_efix = b.add(efix.data(), std::max<size_t>(efix.size(), 1));
@@ -622,6 +634,9 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   m.ns4 = (const int4*)(base + o_ns4);
   m.iavol = (const double*)(base + o_iavol);
   m.qr4c = (const double*)(base + o_qr4c);
+  m.iarea0 = (const double*)(base + o_iarea0);
+  m.earea12 = (const double*)(base + o_earea12);
+  m.ediff = (const double*)(base + o_ediff);
   m.efix = (const uint32_t*)(base + o_efix);
   m.n_efix = int64_t(efix.size());
   for (int v = 0; v < kSegVariants; ++v) {
