@@ -59,14 +59,17 @@ struct LaunchDims {
       smap_levels[i] = levels;
     }
   }
-  // The mapping of a plan or batch that was given none: two tracers and one level per
-  // thread, so that adjacent threads read adjacent levels (runs of two or more levels per
-  // thread spread a warp's loads over twice the lines or more), except the LO stage on
-  // launches of many waves, which shares its column window between two levels (T and S on
-  // the CORE2-size mesh: 147 us at 2 x 2 against 154 at 2 x 1; on pi 12.9 against 9.4).
-  void auto_map(int64_t segments) {
+  // The mapping of a plan or batch that was given none: one level per thread (the stream
+  // kernels; runs of two or more levels per thread spread a warp's loads over twice the lines
+  // or more) and two tracers. Interleaved instances of 4 tracers or more take 4 per thread,
+  // and the run kernel at 2 x 2 in the final stage (fct_seg_final.cu), if that still leaves
+  // ``threads`` (wet node layers x tracers of the launch / 4) for two blocks on every SM.
+  void auto_map(bool interleaved, int64_t threads) {
     set_map(2, 1);
-    if (segments >= int64_t(148) * 4 * 256 * 4) smap_levels[kStageLo] = 2;
+    if (interleaved && ntr >= 4 && threads >= int64_t(148) * 2 * 256) {
+      for (int i : {kStageLo, kStageEdge, kStageLimit}) smap_tracers[i] = 4;
+      smap_levels[kStageFinal] = 2;
+    }
   }
   int64_t max_nseg[kSegVariants] = {0, 0, 0, 0};
   int64_t max_eseg[kSegVariants] = {0, 0, 0, 0};
@@ -100,7 +103,7 @@ inline void dims_cover(LaunchDims& d, const FctPlan* P) {
 // The mapping of a single-plan launch: the plan's own, or the rule's.
 inline void dims_map(LaunchDims& d, const FctPlan* P) {
   if (P->per_thread > 0) d.set_map(P->per_thread, P->lpt);
-  else d.auto_map(P->hm.n_layer * std::max(1, d.ntr / 2));
+  else d.auto_map(false, 0);
 }
 
 // Tracers per thread and tracer slices of one segment launch over ``rem`` tracers: the

@@ -51,7 +51,12 @@ int launch_edge_fix(const Inst& single, const Inst* tab, int n, const LaunchDims
 
 namespace {
 
+__host__ __device__ constexpr int edge_blocks(int ntr) { return ntr == 1 ? 5 : ntr == 2 ? 3 : 2; }
+__host__ __device__ constexpr int edge_batch(int) { return 1; }
+FCT_STREAM_KERNEL(k_edge_stream, stream_edge_adf, edge_blocks, edge_batch)
+
 #define FCT_COUNT(V) d.max_eseg[V]
+FCT_STREAM_LAUNCHER(launch_stream, k_edge_stream, FCT_COUNT, FCT_GRID, kStageEdge, edge_blocks)
 FCT_SEG_LAUNCHER(launch_impl, k_seg_edge, FCT_COUNT, FCT_GRID, kStageEdge)
 #undef FCT_COUNT
 
@@ -59,6 +64,7 @@ FCT_SEG_LAUNCHER(launch_impl, k_seg_edge, FCT_COUNT, FCT_GRID, kStageEdge)
 
 int launch_seg_edge(const Inst& single, const Inst* tab, int n, const LaunchDims& d, int c0, int c1,
                     cudaStream_t s) {
+  if (d.smap_levels[kStageEdge] == 1) return launch_stream(single, tab, n, d, c0, c1, s);
   return launch_impl(single, tab, n, d, c0, c1, s);
 }
 

@@ -7,7 +7,16 @@ namespace {
 
 FCT_SEG_KERNEL(k_seg_final, seg_node_final, kStageFinal)
 
+// Blocks per SM and slots per batch by tracers per thread, against the run kernel at its best
+// mapping: 1 tracer 90 us against 102, T and S 155 against 179 (CORE2-size mesh); 8 tracers of
+// two members 1.15 ms against 1.08 of the run kernel at 2 x 2, which interleaved instances of 4
+// tracers or more therefore keep.
+__host__ __device__ constexpr int stream_blocks(int ntr) { return ntr == 1 ? 4 : ntr == 2 ? 2 : 1; }
+__host__ __device__ constexpr int slot_batch(int) { return 3; }
+FCT_STREAM_KERNEL(k_stream_final, stream_node_final, stream_blocks, slot_batch)
+
 #define FCT_COUNT(V) d.max_nseg[V]
+FCT_STREAM_LAUNCHER(launch_stream, k_stream_final, FCT_COUNT, FCT_GRID, kStageFinal, stream_blocks)
 FCT_SEG_LAUNCHER(launch_impl, k_seg_final, FCT_COUNT, FCT_GRID, kStageFinal)
 #undef FCT_COUNT
 
@@ -15,6 +24,7 @@ FCT_SEG_LAUNCHER(launch_impl, k_seg_final, FCT_COUNT, FCT_GRID, kStageFinal)
 
 int launch_seg_final(const Inst& single, const Inst* tab, int n, const LaunchDims& d, int c0, int c1,
                      cudaStream_t s) {
+  if (d.smap_levels[kStageFinal] == 1) return launch_stream(single, tab, n, d, c0, c1, s);
   return launch_impl(single, tab, n, d, c0, c1, s);
 }
 

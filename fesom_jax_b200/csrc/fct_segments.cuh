@@ -1,7 +1,9 @@
 // Segment kernels of the fused forward step: the product path of fct_forward, the
 // batched engine and the serving engine (fesom_jax/tracer_adv.py:532-578).
 //
-// A thread takes a *segment*: a run of up to LPT consecutive levels of one node (or one
+// One level per thread (the default), NTR tracers: the stream kernels, whose threads walk the
+// layers or edge levels with adjacent threads on adjacent levels. Two or more levels per
+// thread: a thread takes a *segment*, a run of up to LPT consecutive levels of one node (or one
 // edge) and NTR tracers. The entity's neighbour slots, level range and static geometry
 // are decoded once per segment and every neighbour gather issues LPT x NTR independent
 // loads (consecutive levels of one column), instead of one level per thread re-decoding
@@ -139,11 +141,10 @@ __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, 
     for (int t = 0; t < NTR; ++t) div[l][t] = 0.0;
   }
   const int e0 = rec.x, e1 = rec.x + int((pk >> 16) & 255u);
-  // kSlotBatch slots at a time: their gathers are all issued before any is used (U = 2: 154
-  // us against 161 for T and S on the CORE2-size mesh; in the limiter and the final stage,
-  // which hold three values per slot, the registers cost more than it gives). Slots past the
-  // node's last repeat it with their bits 0; a slot off at a layer reads the own value,
-  // times 0.
+  // U slots at a time: their gathers are all issued before any is used (in the limiter and the
+  // final stage, which hold three values per slot and level, the registers cost more than it
+  // gives). Slots past the node's last repeat it with their bits 0; a slot off at a layer reads
+  // the own value, times 0.
   constexpr int U = 2;
   int4 sl[U];
 #pragma unroll
@@ -338,6 +339,63 @@ __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0,
       adf[t] = -vf * (Tm - Tu[t]);
     }
     if (l < nk) stv<NTR, IL>(in.ws.adfh, qe + uint32_t(l), w0, in.ws.sEd, in.wtg, adf);
+  }
+}
+
+// The same, one level at a time (T and S on the CORE2-size mesh: 139 -> 107 us; 8 tracers of
+// two members, 4 per thread: 0.82 -> 0.66 ms), for a thread that walks the segments si, si + stride, ...: the
+// next level's records and volume flux are loaded while this level's gathers are under way, so
+// a level costs one memory round trip instead of three in a row (segment, records, gathers).
+template <int NTR, bool IL, int U>
+__device__ __forceinline__ void stream_edge_adf(const Inst& in, int64_t si, int64_t stride, int t0,
+                                                int w0) {
+  const DevMesh& m = in.m;
+  const int64_t count = m.n_eseg[0];
+  if (si >= count) return;
+  const int L = m.L, tg = in.tg;
+  using F = Fld<NTR, IL>;
+  const F fT(in.T, t0, in.tstride), fO(in.T_old, t0, in.tstride);
+  const uint32_t* __restrict__ list = m.eseg[0];
+  const int4* __restrict__ erec = m.erec;
+  const int4* __restrict__ emf4 = m.emf4;
+  const double* __restrict__ emfw = m.emfw;
+  const double* __restrict__ vflux = in.ws.vflux;
+  uint32_t sg = __ldg(list + si);
+  uint32_t sg1 = si + stride < count ? __ldg(list + si + stride) : sg;
+  int4 er = __ldg(erec + lane_ent(sg)), ov = __ldg(emf4 + lane_ent(sg));
+  double vf = __ldg(vflux + lq(lane_ent(sg), L, lane_lev(sg)));
+  for (; si < count; si += stride) {
+    const int e = lane_ent(sg), k = lane_lev(sg);
+    const bool first = vf > 0.0;   // the first node is upwind
+    const uint32_t ou = F::off(lq(first ? er.x : er.y, L, k), tg);
+    const uint32_t od = F::off(lq(first ? er.y : er.x, L, k), tg);
+    const uint32_t oa = F::off(lq(first ? ov.x : ov.z, L, k), tg);
+    const uint32_t ob = F::off(lq(first ? ov.y : ov.w, L, k), tg);
+    const double* wp = emfw + (8 * int64_t(e) + (first ? 0 : 4));
+    double Tu[NTR], Td[NTR], Ou[NTR], Od[NTR], va[NTR], vb[NTR];
+    fT.ld(ou, Tu);
+    fT.ld(od, Td);
+    fO.ld(ou, Ou);
+    fO.ld(od, Od);
+    fT.ld(oa, va);
+    fT.ld(ob, vb);
+    const double2 c01 = __ldg(reinterpret_cast<const double2*>(wp));
+    const double c2 = __ldg(wp + 2), v = vf;
+    // the next level's records, and the segment after it
+    sg = sg1;
+    er = __ldg(erec + lane_ent(sg));
+    ov = __ldg(emf4 + lane_ent(sg));
+    vf = __ldg(vflux + lq(lane_ent(sg), L, lane_lev(sg)));
+    sg1 = si + 2 * stride < count ? __ldg(list + si + 2 * stride) : sg;
+    double adf[NTR];
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) {
+      const double Au = ab2f(Tu[t], Ou[t]), Ad = ab2f(Td[t], Od[t]);
+      const double g = fma(c01.y, va[t], fma(c2, vb[t], c01.x * Tu[t]));
+      const double Tm = fma(Ad - Au, 1.0 / 3.0, Au) + g;
+      adf[t] = -v * (Tm - Tu[t]);
+    }
+    stv<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);
   }
 }
 
@@ -736,6 +794,397 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
   }
 }
 
+// ------------------------------------------- node stages, threads that walk the layers
+// What bounds these stages is the wait for their gathers (L2 answers in 300 to 650 cycles on
+// an idle chip, DRAM in 840), and what a thread waits for first used to be the chain segment ->
+// record -> slots. So a thread walks the layers si, si + stride, ... (nseg[0], one layer per segment, in the order
+// of the flag words). The next layer's record, flag word and first slots are loaded while this
+// layer's gathers are under way, and a batch of U slots issues all its gathers before it uses
+// any, so the memory round trips of a layer are those of its gathers alone. Blocks per SM and U
+// per stage (fct_seg_*.cu) were swept together, 1 to 6 blocks and U of 1 to 3: fewer blocks
+// with more registers and longer batches win except where they start to spill.
+template <int U>
+struct NodeWalk {
+  const uint32_t* __restrict__ list;
+  const int4* __restrict__ nrec;
+  const int4* __restrict__ ns4;
+  const unsigned long long* __restrict__ flags;
+  int64_t count;
+  uint32_t sg, sg1;
+  int4 rec, rec1, sl[U];
+  unsigned long long fl, fl1;
+  __device__ __forceinline__ NodeWalk(const DevMesh& m, int64_t si, int64_t stride)
+      : list(m.nseg[0]), nrec(m.nrec), ns4(m.ns4), flags(m.nflags), count(m.n_nseg[0]) {
+    const int64_t i = si < 0 ? 0 : (si < count ? si : count - 1);
+    const int64_t j = si + stride < count ? si + stride : i;
+    sg = __ldg(list + i);
+    sg1 = __ldg(list + j);
+    fl = __ldg(flags + i);
+    rec = __ldg(nrec + lane_ent(sg));
+    first_slots(rec);
+  }
+  __device__ __forceinline__ int degree() const { return int((unsigned(rec.z) >> 16) & 255u); }
+  __device__ __forceinline__ void first_slots(const int4& r) {
+    const int e1 = r.x + int((unsigned(r.z) >> 16) & 255u);
+#pragma unroll
+    for (int u = 0; u < U; ++u) sl[u] = __ldg(ns4 + max(min(r.x + u, e1 - 1), 0));
+  }
+  // the records of the batch after the one at j (the last batch keeps what it has)
+  __device__ __forceinline__ void more_slots(int j) {
+    const int e1 = rec.x + degree();
+    if (j + U < e1) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) sl[u] = __ldg(ns4 + min(j + U + u, e1 - 1));
+    }
+  }
+  // the next layer's record and flags, and the segment after it
+  __device__ __forceinline__ void ahead(int64_t si, int64_t stride) {
+    const int64_t j = si + stride < count ? si + stride : (si < 0 ? 0 : min(si, count - 1));
+    rec1 = __ldg(nrec + lane_ent(sg1));
+    fl1 = __ldg(flags + j);
+  }
+  // the first slots of the next layer (its record has arrived)
+  __device__ __forceinline__ void ahead_slots() { first_slots(rec1); }
+  __device__ __forceinline__ void next(int64_t si, int64_t stride) {
+    rec = rec1;
+    fl = fl1;
+    sg = sg1;
+    const int64_t j = si + 2 * stride;
+    sg1 = j < count ? __ldg(list + j) : sg1;
+  }
+};
+
+template <int NTR, bool IL, int U>
+__device__ __forceinline__ void stream_node_final(const Inst& in, int64_t si, int64_t stride,
+                                                  int t0, int w0) {
+  const DevMesh& m = in.m;
+  if (si >= m.n_nseg[0]) return;
+  using F = Fld<NTR, IL>;
+  const int64_t sN = in.ws.sN;
+  const F fP(in.ws.pf, w0, sN), fM(in.ws.mf, w0, sN), fA(in.ws.adfh, w0, in.ws.sEd);
+  const F fV(in.ws.adfv, w0, sN), fL(in.ws.lo, w0, sN), fT(in.T, t0, in.tstride);
+  const int L = m.L, tg = in.tg, wtg = in.wtg;
+  const double dt = in.dt;
+  NodeWalk<U> nw(m, si, stride);
+  for (; si < nw.count; si += stride) {
+    const int n = lane_ent(nw.sg), k = lane_lev(nw.sg);
+    const unsigned pk = unsigned(nw.rec.z);
+    const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
+    const uint32_t base = lq(n, L, 0), qn = base + uint32_t(k), on_ = F::off(qn, wtg);
+    double pf0[NTR], mf0[NTR], hsc[NTR];
+    fP.ld(on_, pf0);
+    fM.ld(on_, mf0);
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) hsc[t] = 0.0;
+    unsigned onb = unsigned(nw.fl) & kSlotBits;
+    const int e1 = nw.rec.x + nw.degree();
+    for (int j = nw.rec.x; j < e1; j += U) {
+      double a[U][NTR], pfo[U][NTR], mfo[U][NTR];
+      int sgn[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t qo = F::off(uint32_t(nw.sl[u].y) + uint32_t(k), wtg);
+        sgn[u] = nw.sl[u].z;
+        fA.ld(F::off(uint32_t(nw.sl[u].x) + uint32_t(k), wtg), a[u]);
+        fP.ld(qo, pfo[u]);
+        fM.ld(qo, mfo[u]);
+      }
+      if (j == nw.rec.x) nw.ahead(si, stride);
+      nw.more_slots(j);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool on = (onb >> u) & 1u;
+#pragma unroll
+        for (int t = 0; t < NTR; ++t) {
+          const double s = flip_sign(a[u][t], sgn[u]);   // adf_h leaves the edge's first node
+          const bool leaves = s >= 0.0;
+          const double h = fma(dmin(leaves ? pf0[t] : mf0[t], leaves ? mfo[u][t] : pfo[u][t]), s,
+                               hsc[t]);
+          hsc[t] = on ? h : hsc[t];
+        }
+      }
+      onb >>= U;
+    }
+    if (e1 == nw.rec.x) nw.ahead(si, stride);
+    nw.ahead_slots();
+    const double iav = __ldg(m.iavol + qn);   // 1 / areasvol (0 where there is no volume)
+    const double hn = __ldg(in.hnode + qn), hnn = __ldg(in.hnode_new + qn);
+    double ft[NTR], fb[NTR], Tv[NTR], lo[NTR], pu[NTR], mu[NTR], pd[NTR], md[NTR];
+    const bool below = k + 1 < nzmax, above = k > nzmin;
+    const uint32_t oa = F::off(above ? qn - 1 : qn, wtg), ob = F::off(below ? qn + 1 : qn, wtg);
+    fV.ld(on_, ft);
+    fV.ld(ob, fb);
+    fT.ld(F::off(qn, tg), Tv);
+    fL.ld(on_, lo);
+    fP.ld(oa, pu);
+    fM.ld(oa, mu);
+    fP.ld(ob, pd);
+    fM.ld(ob, md);
+    nw.next(si, stride);
+    const double fdt = dt * (iav > 0.0 ? iav : 1.0);
+    const Rcq rhn = rcpq(hnn);
+    double out[NTR];
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) {
+      // limited vertical fluxes at the top (k) and bottom (k + 1) interfaces
+      const double vt = above ? (ft[t] >= 0.0 ? dmin(mu[t], pf0[t]) : dmin(pu[t], mf0[t])) * ft[t]
+                              : (ft[t] >= 0.0 ? pf0[t] : mf0[t]) * ft[t];
+      const double vb =
+          below ? (fb[t] >= 0.0 ? dmin(mf0[t], pd[t]) : dmin(pf0[t], md[t])) * fb[t] : 0.0;
+      const double lo_trans = fma(lo[t], hnn, -Tv[t] * hn);
+      const double vdiv = iav > 0.0 ? (vt - vb) * fdt : 0.0;
+      double d = fma(hsc[t], fdt, lo_trans + vdiv);
+      d = fma(Tv[t], hn - hnn, d);
+      out[t] = Tv[t] + (hnn > 0.0 ? divq(d, rhn) : 0.0);
+    }
+    stv<NTR, IL>(in.T_new, qn, t0, in.tstride, tg, out);
+    count_nonfinite<NTR>(in.nonfinite, out);
+  }
+}
+
+template <int NTR, bool IL, int U>
+__device__ __forceinline__ void stream_node_lo(const Inst& in, int64_t si, int64_t stride, int t0,
+                                               int w0) {
+  const DevMesh& m = in.m;
+  if (si >= m.n_nseg[0]) return;
+  using F = Fld<NTR, IL>;
+  const F fT(in.T, t0, in.tstride), fTo(in.T_old, t0, in.tstride);
+  const int L = m.L, tg = in.tg;
+  const double dt = in.dt;
+  NodeWalk<U> nw(m, si, stride);
+  for (; si < nw.count; si += stride) {
+    const int n = lane_ent(nw.sg), k = lane_lev(nw.sg);
+    const unsigned pk = unsigned(nw.rec.z);
+    const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
+    const uint32_t base = lq(n, L, 0), qn = base + uint32_t(k);
+    double div[NTR], out = 0.0;
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) div[t] = 0.0;
+    unsigned onb = unsigned(nw.fl) & kSlotBits;
+    const int e1 = nw.rec.x + nw.degree();
+    for (int j = nw.rec.x; j < e1; j += U) {
+      double vf[U], To[U][NTR];
+      int sgn[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool on = (onb >> u) & 1u;
+        sgn[u] = nw.sl[u].z;
+        vf[u] = __ldg(in.ws.vflux + (uint32_t(nw.sl[u].x) + uint32_t(k)));
+        fT.ld(F::off((on ? uint32_t(nw.sl[u].y) : base) + uint32_t(k), tg), To[u]);
+      }
+      if (j == nw.rec.x) nw.ahead(si, stride);
+      nw.more_slots(j);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const double s = flip_sign(vf[u], sgn[u]);
+        const bool on = (onb >> u) & 1u, leaves = s > 0.0;
+        const double cin = (on && !leaves) ? -s : 0.0;
+        if (on && leaves) out += s;
+#pragma unroll
+        for (int t = 0; t < NTR; ++t) div[t] = fma(cin, To[u][t], div[t]);
+      }
+      onb >>= U;
+    }
+    if (e1 == nw.rec.x) nw.ahead(si, stride);
+    nw.ahead_slots();
+    // the column at k-2 .. k+1 (the level above the surface reads the top again), w and areas
+    const uint32_t q0 = base + uint32_t(kclamp(k - 2, L)), q1 = base + uint32_t(kclamp(k - 1, L));
+    const uint32_t q3 = base + uint32_t(kclamp(k + 1, L));
+    double T0[NTR], T1[NTR], T2[NTR], T3[NTR], O0[NTR], O1[NTR], O2[NTR], O3[NTR];
+    fT.ld(F::off(q0, tg), T0);
+    fT.ld(F::off(q1, tg), T1);
+    fT.ld(F::off(qn, tg), T2);
+    fT.ld(F::off(q3, tg), T3);
+    fTo.ld(F::off(q0, tg), O0);
+    fTo.ld(F::off(q1, tg), O1);
+    fTo.ld(F::off(qn, tg), O2);
+    fTo.ld(F::off(q3, tg), O3);
+    const double w = __ldg(in.w_e + qn), area = __ldg(m.area + qn);
+    const double wb = __ldg(in.w_e + q3), areab = __ldg(m.area + q3);
+    const double hn = __ldg(in.hnode + qn), hnn = __ldg(in.hnode_new + qn);
+    const double iav = __ldg(m.iavol + qn);
+    nw.next(si, stride);
+    const bool below = k + 1 < nzmax;
+    const double fdt = dt * iav;   // dt / areasvol
+    const Rcq rhn = rcpq(hnn);
+    const bool valid = (hnn > 0.0) && (iav > 0.0);
+    double lo[NTR], fv[NTR];
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) {
+      fv[t] = vflux_up(T2[t], T1[t], w, area);
+      const double fvb = below ? vflux_up(T3[t], T2[t], wb, areab) : 0.0;
+      const double dh = fma(-out, T2[t], div[t]);
+      lo[t] = valid ? divq(fma(T2[t], hn, (dh + (fv[t] - fvb)) * fdt), rhn) : 0.0;
+    }
+    stv<NTR, IL>(in.ws.lo, qn, w0, in.ws.sN, in.wtg, lo);
+    // adv_flux_ver_ho (QR4C on ttfAB) minus the LO vertical flux at the layer top
+    const double Wf = in.w_i ? w + __ldg(in.w_i + qn) : w;
+    double hi[NTR];
+    if (k == nzmin) {
+#pragma unroll
+      for (int t = 0; t < NTR; ++t) hi[t] = -ab2f(T2[t], O2[t]) * Wf * area;
+    } else if (k == nzmin + 1 || k == nzmax - 1) {
+#pragma unroll
+      for (int t = 0; t < NTR; ++t)
+        hi[t] = -0.5 * (ab2f(T1[t], O1[t]) + ab2f(T2[t], O2[t])) * Wf * area;
+    } else {
+      double rdc, rdu, rdd, d1, d2;
+      if (in.Z3d) {
+        const double* Zc = in.Z3d + base;
+        const double Znz = __ldg(Zc + k), Zm1 = __ldg(Zc + k - 1), Zm2 = __ldg(Zc + k - 2);
+        const double Zp1 = __ldg(Zc + (k + 1 < L ? k + 1 : L - 1)), zb = __ldg(in.zbar3 + qn);
+        rdc = __drcp_rn(safe_nz(Zm1 - Znz));
+        rdu = __drcp_rn(safe_nz(Znz - Zp1));
+        rdd = __drcp_rn(safe_nz(Zm2 - Zm1));
+        d1 = (zb - Znz) * (1.0 / 3.0);
+        d2 = (zb - Zm1) * (1.0 / 3.0);
+      } else {
+        const double* q = m.qr4c + k;
+        rdc = __ldg(q);
+        rdu = __ldg(q + L);
+        rdd = __ldg(q + 2 * L);
+        d1 = __ldg(q + 3 * L);
+        d2 = __ldg(q + 4 * L);
+      }
+      const double wa = -0.5 * Wf * area;
+#pragma unroll
+      for (int t = 0; t < NTR; ++t) {
+        const double A0 = ab2f(T2[t], O2[t]), Am1 = ab2f(T1[t], O1[t]);
+        const double Am2 = ab2f(T0[t], O0[t]), Ap1 = ab2f(T3[t], O3[t]);
+        const double qc = (Am1 - A0) * rdc, qu = (A0 - Ap1) * rdu, qd = (Am2 - Am1) * rdd;
+        const double Tmean1 = fma(fma(2.0, qc, qu), d1, A0);
+        const double Tmean2 = fma(fma(2.0, qc, qd), d2, Am1);
+        hi[t] = (Tmean1 + Tmean2) * wa;
+      }
+    }
+    double adf[NTR];
+#pragma unroll
+    for (int t = 0; t < NTR; ++t)
+      adf[t] = hi[t] - (in.w_i ? vflux_up(T2[t], T1[t], Wf, area) : fv[t]);
+    stv<NTR, IL>(in.ws.adfv, qn, w0, in.ws.sN, in.wtg, adf);
+  }
+}
+
+// The limiter: a block's segment slots hold consecutive layers, the first and the last one
+// halo layers that only publish their bounds; ``sh`` holds two sets (alternate rounds, so one
+// barrier a round is enough) of [2][NTR][256] doubles.
+template <int NTR, bool IL, int U>
+__device__ __forceinline__ void stream_node_limit(const Inst& in, int64_t si, int64_t stride,
+                                                  int64_t rounds, bool core, int t0, int w0,
+                                                  int tid, int S, double* sh) {
+  if (rounds <= 0) return;   // block-uniform
+  const DevMesh& m = in.m;
+  using F = Fld<NTR, IL>;
+  const int64_t sN = in.ws.sN;
+  const F fT(in.T, t0, in.tstride), fL(in.ws.lo, w0, sN), fA(in.ws.adfh, w0, in.ws.sEd);
+  const F fV(in.ws.adfv, w0, sN);
+  const int L = m.L, tg = in.tg, wtg = in.wtg;
+  const double dt = in.dt;
+  NodeWalk<U> nw(m, si, stride);
+  for (int64_t r = 0; r < rounds; ++r, si += stride) {
+    const bool valid = si >= 0 && si < nw.count;
+    const int n = lane_ent(nw.sg), k = lane_lev(nw.sg);
+    const unsigned pk = unsigned(nw.rec.z);
+    const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
+    const uint32_t base = lq(n, L, 0), qn = base + uint32_t(k);
+    double mx[NTR], mn[NTR], sp[NTR], sm[NTR], lo[NTR];
+    {
+      double tv[NTR];
+      fL.ld(F::off(qn, wtg), lo);
+      fT.ld(F::off(qn, tg), tv);
+#pragma unroll
+      for (int t = 0; t < NTR; ++t) {
+        mx[t] = dmax(lo[t], tv[t]);
+        mn[t] = dmin(lo[t], tv[t]);
+        sp[t] = sm[t] = 0.0;
+      }
+    }
+    unsigned onb = unsigned(nw.fl) & kSlotBits;
+    unsigned wetb = unsigned(nw.fl >> kSlotWet) & kSlotBits;
+    const bool ow = (nw.fl >> kOwnBit) & 1ull, of = (nw.fl >> kOffBit) & 1ull;
+    const int e1 = nw.rec.x + nw.degree();
+    for (int j = nw.rec.x; j < e1; j += U) {
+      double lv[U][NTR], tv[U][NTR], a[U][NTR];
+      int sgn[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        // an edge without a wet cell here reads the node's own values again
+        const uint32_t qo = ((wetb >> u) & 1u) ? uint32_t(nw.sl[u].y) + uint32_t(k) : qn;
+        sgn[u] = nw.sl[u].z;
+        fL.ld(F::off(qo, wtg), lv[u]);
+        fT.ld(F::off(qo, tg), tv[u]);
+        fA.ld(F::off(uint32_t(nw.sl[u].x) + uint32_t(k), wtg), a[u]);
+      }
+      if (j == nw.rec.x) nw.ahead(si, stride);
+      nw.more_slots(j);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool on = (onb >> u) & 1u;
+#pragma unroll
+        for (int t = 0; t < NTR; ++t) {
+          mx[t] = dmax(mx[t], dmax(lv[u][t], tv[u][t]));
+          mn[t] = dmin(mn[t], dmin(lv[u][t], tv[u][t]));
+          const double sv = flip_sign(a[u][t], sgn[u]);   // adf_h leaves the first node
+          if (on && sv > 0.0) sp[t] += sv;
+          if (on && sv < 0.0) sm[t] += sv;
+        }
+      }
+      onb >>= U;
+      wetb >>= U;
+    }
+    if (e1 == nw.rec.x) nw.ahead(si, stride);
+    nw.ahead_slots();
+    double* shr = sh + (r & 1) * (2 * NTR * 256);
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) {
+      if (!ow) {   // no wet cell at the level: no bounds
+        mx[t] = -INFINITY;
+        mn[t] = INFINITY;
+      }
+      if (of) {   // the padding of dry cells
+        mx[t] = dmax(mx[t], -kBig);
+        mn[t] = dmin(mn[t], kBig);
+      }
+      shr[t * 256 + tid] = mx[t];
+      shr[(NTR + t) * 256 + tid] = mn[t];
+    }
+    const bool below = k + 1 < nzmax;
+    double ft[NTR], fb[NTR];
+    fV.ld(F::off(qn, wtg), ft);
+    fV.ld(F::off(below ? qn + 1 : qn, wtg), fb);
+    const double av = __ldg(m.areasvol + qn), hnn = __ldg(in.hnode_new + qn);
+    nw.next(si, stride);
+    __syncthreads();
+    if (!valid || !core) continue;
+    const bool interior = k != nzmin && k != nzmax - 1;   // a4: window over k-1, k, k+1
+    const bool valid_n = (av > 0.0) && (hnn > 0.0);
+    const double sa = av > 0.0 ? av : 1.0, shn = hnn > 0.0 ? hnn : 1.0;
+    const double fdt = dt * __drcp_rn(sa * shn);   // dt / (areasvol * hnode_new)
+    double pf[NTR], mf[NTR];
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) {
+      double wmx = mx[t], wmn = mn[t];
+      if (interior) {
+        wmx = dmax(dmax(shr[t * 256 + tid - S], wmx), shr[t * 256 + tid + S]);
+        wmn = dmin(dmin(shr[(NTR + t) * 256 + tid - S], wmn), shr[(NTR + t) * 256 + tid + S]);
+      }
+      const double vb = below ? fb[t] : 0.0;   // the bottom interface carries no flux
+      const double plus = (dmax(ft[t], 0.0) + dmax(-vb, 0.0)) + sp[t];
+      const double minus = (dmin(ft[t], 0.0) + dmin(-vb, 0.0)) + sm[t];
+      pf[t] = 1.0;
+      mf[t] = 1.0;
+      if (valid_n) {
+        const double flux_pos = fma(plus, fdt, kFluxEps);
+        const double flux_neg = fma(minus, fdt, -kFluxEps);
+        pf[t] = dmin(1.0, (wmx - lo[t]) * __drcp_rn(flux_pos));
+        mf[t] = dmin(1.0, (wmn - lo[t]) * __drcp_rn(flux_neg));
+      }
+    }
+    stv<NTR, IL>(in.ws.pf, qn, w0, sN, in.wtg, pf);
+    stv<NTR, IL>(in.ws.mf, qn, w0, sN, in.wtg, mf);
+  }
+}
+
 // ------------------------------------------------------------- kernels and launchers
 // Kernel wrappers: ``_1`` takes one instance by value (tracer-major layout, the
 // single-call path; tracer slice = blockIdx.y), ``_n`` instance blockIdx.y of a device
@@ -743,16 +1192,15 @@ __device__ __forceinline__ void seg_node_final(const Inst& in, int64_t si, int t
 // slices, so together they read whole interleaved lines; S is any number up to 8, so an odd
 // tracer count is one launch too). A 256-thread block holds 256/S segments.
 //
-// Resident 256-thread blocks per SM the compiler must fit, by stage and by the updates u a
-// thread carries. The kernels wait on their gathers, so resident warps pay until the cap
-// makes the compiler spill. The limiter and the LO stage hold more per update and take one
-// block less: T and S on the CORE2-size mesh, 2 tracers x 1 level per thread, 64 registers
-// against 48: limiter 198 us against 297; edge 160 against 141, final 188 against 180 the
-// other way round.
+// Resident 256-thread blocks per SM the compiler must fit (runs of two or more levels), by
+// stage and by the updates u a thread carries. The kernels wait on their gathers, so resident
+// warps pay until the cap makes the compiler spill; the limiter and the LO stage hold more per
+// update and take one block less (T and S on the CORE2-size mesh, 2 tracers x 4 levels: limiter
+// 384 us against 638; edge 221 against 195 the other way round).
 __host__ __device__ constexpr int seg_min_blocks(int stage, int u) {
   return (stage == kStageEdge || stage == kStageFinal)
-             ? (u <= 1 ? 7 : u <= 2 ? 5 : u <= 4 ? 4 : u <= 8 ? 3 : 2)
-             : (u <= 1 ? 5 : u <= 2 ? 4 : u <= 4 ? 3 : 2);
+             ? (u <= 2 ? 5 : u <= 4 ? 4 : u <= 8 ? 3 : 2)
+             : (u <= 2 ? 4 : u <= 4 ? 3 : 2);
 }
 
 // thread t of a block of 256/S segments: segment t / S, slice t % S (``mul`` = 65536/S + 1
@@ -834,12 +1282,11 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
         const unsigned mul = 65536u / unsigned(S) + 1u;                                  \
         const dim3 g(GRID(lanes, S), unsigned(n));                                       \
         switch (P * 16 + lpt) {                                                          \
-          FCT_SEG_CASE_N(kern, 1, 1) FCT_SEG_CASE_N(kern, 1, 2)                          \
-          FCT_SEG_CASE_N(kern, 1, 4) FCT_SEG_CASE_N(kern, 1, 8)                          \
-          FCT_SEG_CASE_N(kern, 2, 1) FCT_SEG_CASE_N(kern, 2, 2)                          \
+          FCT_SEG_CASE_N(kern, 1, 2) FCT_SEG_CASE_N(kern, 1, 4)                          \
+          FCT_SEG_CASE_N(kern, 1, 8) FCT_SEG_CASE_N(kern, 2, 2)                          \
           FCT_SEG_CASE_N(kern, 2, 4) FCT_SEG_CASE_N(kern, 2, 8)                          \
-          FCT_SEG_CASE_N(kern, 4, 1) FCT_SEG_CASE_N(kern, 4, 2)                          \
-          FCT_SEG_CASE_N(kern, 4, 4) FCT_SEG_CASE_N(kern, 4, 8)                          \
+          FCT_SEG_CASE_N(kern, 4, 2) FCT_SEG_CASE_N(kern, 4, 4)                          \
+          FCT_SEG_CASE_N(kern, 4, 8)                                                     \
           default:                                                                       \
             return set_error(FCT_ERR_INVALID, "no segment kernel for %d tracers x %d "  \
                              "levels per thread", P, lpt);                              \
@@ -847,14 +1294,87 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
       } else {                                                                           \
         const dim3 g(GRID(lanes, 1), unsigned(S));                                       \
         switch (P * 16 + lpt) {                                                          \
-          FCT_SEG_CASE_1(kern, 1, 1) FCT_SEG_CASE_1(kern, 1, 2)                          \
-          FCT_SEG_CASE_1(kern, 1, 4) FCT_SEG_CASE_1(kern, 1, 8)                          \
-          FCT_SEG_CASE_1(kern, 2, 1) FCT_SEG_CASE_1(kern, 2, 2)                          \
+          FCT_SEG_CASE_1(kern, 1, 2) FCT_SEG_CASE_1(kern, 1, 4)                          \
+          FCT_SEG_CASE_1(kern, 1, 8) FCT_SEG_CASE_1(kern, 2, 2)                          \
           FCT_SEG_CASE_1(kern, 2, 4) FCT_SEG_CASE_1(kern, 2, 8)                          \
           default:                                                                       \
             return set_error(FCT_ERR_INVALID, "no segment kernel for %d tracers x %d "  \
                              "levels per thread", P, lpt);                              \
         }                                                                                \
+      }                                                                                  \
+      t0 += P * S;                                                                       \
+    }                                                                                    \
+    const cudaError_t e = cudaGetLastError();                                            \
+    return e == cudaSuccess ? FCT_OK : cuda_error(e, #fn);                               \
+  }
+
+// Kernels whose threads walk the segments (one level per thread): as many blocks as are
+// resident at once; the batched ones go through the instances one after the other, so the
+// gathers of all blocks stay within a few columns of each other.
+#define FCT_STREAM_KERNEL(name, body, blocks, batch)                                         \
+  template <int NTR>                                                                     \
+  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+      name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
+    const int sub = int(blockIdx.y) * NTR;                                               \
+    body<NTR, false, batch(NTR)>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub); \
+  }                                                                                      \
+  template <int NTR>                                                                     \
+  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+      name##_n(const Inst* __restrict__ tab, int n, int t0, int w0, int S, unsigned mul) { \
+    const int slots = slice_div(256, mul), slot = slice_div(int(threadIdx.x), mul);      \
+    if (slot >= slots) return;                                                           \
+    const int sub = (int(threadIdx.x) - slot * S) * NTR;                                 \
+    for (int i = 0; i < n; ++i)                                                          \
+      body<NTR, true, batch(NTR)>(tab[i], int64_t(blockIdx.x) * slots + slot,                     \
+                         int64_t(gridDim.x) * slots, t0 + sub, w0 + sub);                \
+  }
+#define FCT_STREAM_LIMIT_KERNEL(name, blocks, batch)                                         \
+  template <int NTR>                                                                     \
+  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+      name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
+    __shared__ double sh[4 * NTR * 256];                                                 \
+    const int tid = threadIdx.x, sub = int(blockIdx.y) * NTR;                            \
+    const int64_t stride = int64_t(gridDim.x) * 254, b0 = int64_t(blockIdx.x) * 254;     \
+    const int64_t rounds = (in.m.n_nseg[0] - b0 + stride - 1) / stride;                  \
+    stream_node_limit<NTR, false, batch(NTR)>(in, b0 + tid - 1, stride, rounds,                   \
+                                     tid >= 1 && tid <= 254, t0 + sub, w0 + sub, tid, 1, sh); \
+  }                                                                                      \
+  template <int NTR>                                                                     \
+  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+      name##_n(const Inst* __restrict__ tab, int n, int t0, int w0, int S, unsigned mul) { \
+    __shared__ double sh[4 * NTR * 256];                                                 \
+    const int tid = threadIdx.x;                                                         \
+    const int slots = slice_div(256, mul), slot = slice_div(tid, mul);                   \
+    const int sub = slot < slots ? (tid - slot * S) * NTR : 0;                           \
+    const int64_t stride = int64_t(gridDim.x) * (slots - 2);                             \
+    const int64_t b0 = int64_t(blockIdx.x) * (slots - 2);                                \
+    for (int i = 0; i < n; ++i) {                                                        \
+      const int64_t rounds = (tab[i].m.n_nseg[0] - b0 + stride - 1) / stride;            \
+      stream_node_limit<NTR, true, batch(NTR)>(tab[i], b0 + slot - 1, stride, rounds,             \
+                                      slot >= 1 && slot <= slots - 2, t0 + sub, w0 + sub, \
+                                      tid, S, sh);                                       \
+      __syncthreads();                                                                   \
+    }                                                                                    \
+  }
+#define FCT_STREAM_LAUNCHER(fn, kern, COUNT, GRID, STAGE, blocks)                        \
+  int fn(const Inst& single, const Inst* tab, int n, const LaunchDims& d, int c0, int c1, \
+         cudaStream_t s) {                                                               \
+    for (int t0 = c0; t0 < c1;) {                                                        \
+      const SegSplit sp =                                                                \
+          seg_split(c1 - t0, d.smap_tracers[STAGE], tab != nullptr, seg_even(d));        \
+      const int P = sp.tracers, S = sp.slices, w0 = t0 - c0;                             \
+      const int64_t need = GRID(COUNT(0), tab ? S : 1), full = int64_t(148) * blocks(P); \
+      if (tab) {                                                                         \
+        const unsigned mul = 65536u / unsigned(S) + 1u;                                  \
+        const unsigned g = unsigned(std::max<int64_t>(1, std::min(need, full)));         \
+        if (P == 4) kern##_n<4><<<g, 256, 0, s>>>(tab, n, t0, w0, S, mul);               \
+        else if (P == 2) kern##_n<2><<<g, 256, 0, s>>>(tab, n, t0, w0, S, mul);          \
+        else kern##_n<1><<<g, 256, 0, s>>>(tab, n, t0, w0, S, mul);                      \
+      } else {                                                                           \
+        const int64_t per = std::max<int64_t>(1, full / S);                              \
+        const dim3 g(unsigned(std::max<int64_t>(1, std::min(need, per))), unsigned(S));  \
+        if (P == 2) kern##_1<2><<<g, 256, 0, s>>>(single, t0, w0);                       \
+        else kern##_1<1><<<g, 256, 0, s>>>(single, t0, w0);                              \
       }                                                                                  \
       t0 += P * S;                                                                       \
     }                                                                                    \

@@ -95,7 +95,7 @@ class Ensemble:
         self.chunk = 2          # tracers per thread of the fused stages
         self.levels = 1         # levels per thread
         # per fused stage (LO, edge, limiter, final); until a mapping is set the library
-        # takes two levels per thread in the LO stage of large launches
+        # takes four tracers per thread where a large launch has them
         self.stage_map = [(2, 1)] * 4
 
     # ---------------------------------------------------------------- members
