@@ -50,16 +50,12 @@ namespace {
 
 constexpr int B = 256;
 // Resident 256-thread blocks per SM the reverse kernels' register allocation must allow
-// (40 registers; 48 for r_edge). The kernels are latency-bound gathers, so resident warps
-// pay more than the spills the cap costs: on the CORE2-size 10-step chain the reverse
-// passes took 28.7 ms unconstrained (r_edge at 3 blocks), 23.3 ms at 4 blocks, 20.2 ms at
-// 6 (r_edge 5) and 20.0 ms at 8.
-#ifndef FCT_RMB
-#define FCT_RMB 6
-#define FCT_REB 5
-#endif
-constexpr int kRevMinBlocks = FCT_RMB;
-constexpr int kRevEdgeMinBlocks = FCT_REB;
+// (40 registers; 128 for r_edge, whose walk keeps some 20 gathers under way: 247 us against 316
+// at 3 blocks and 390 with one lane per thread, CORE2-size mesh). The others are
+// latency-bound gathers, so resident warps pay more than the spills the cap costs: 10-step
+// chain, all at 6 blocks 26.2 ms, at 5 27.4, at 4 29.9, at 3 33.8.
+constexpr int kRevMinBlocks = 6;
+constexpr int kRevEdgeMinBlocks = 2;
 
 __device__ __forceinline__ int64_t lane_index() {
   return int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -95,6 +91,21 @@ struct Adj {
   double *gT, *gTo, *guv, *gw;
   int acc;               // kAcc* bits: add into the output instead of overwriting it
 };
+
+// The reverse kernels walk their lanes (lane_index(), + the grid's threads, ...) with the next
+// lane's record loaded one ahead.
+template <class T>
+__device__ __forceinline__ T first_record(const T* p, int64_t count) {
+  const int64_t i = lane_index();
+  return __ldg(p + (i < count ? i : 0));
+}
+template <class T>
+__device__ __forceinline__ T next_record(const T* p, int64_t count, int64_t i, int64_t stride,
+                                         T& next) {
+  const T r = next;
+  if (i + stride < count) next = __ldg(p + i + stride);
+  return r;
+}
 
 // Cotangent reaching the limited vertical flux at interface j of a node column, from the
 // stored divergence cotangents ghsc = gdel * dt / sa (sa = areasvol, 1 where it is 0): the
@@ -341,33 +352,35 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_ratio_window(const __grid_
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
-  const int64_t i = lane_index();
-  if (i >= m.n_elem) return;
-  const uint32_t lane = ld(m.elem_lanes + i);
-  const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
-  const uint32_t qe = lq(e, L, k);
-  const uint32_t qv[3] = {lq(ld(m.enodes + 3 * e), L, k),
-                         lq(ld(m.enodes + 3 * e + 1), L, k),
-                         lq(ld(m.enodes + 3 * e + 2), L, k)};
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * in.ws.sE;
-    const double vx = in.ws.amax[oe + qe], vn = in.ws.amin[oe + qe];
-    double tx[3], tn[3], qx[3], qn[3];
+  const int64_t stride = int64_t(gridDim.x) * B;
+  uint32_t next = first_record(m.elem_lanes, m.n_elem);
+  for (int64_t i = lane_index(); i < m.n_elem; i += stride) {
+    const uint32_t lane = next_record(m.elem_lanes, m.n_elem, i, stride, next);
+    const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
+    const uint32_t qe = lq(e, L, k);
+    const uint32_t qv[3] = {lq(ld(m.enodes + 3 * e), L, k),
+                           lq(ld(m.enodes + 3 * e + 1), L, k),
+                           lq(ld(m.enodes + 3 * e + 2), L, k)};
+    for (int t = 0; t < in.ntr; ++t) {
+      const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * in.ws.sE;
+      const double vx = in.ws.amax[oe + qe], vn = in.ws.amin[oe + qe];
+      double tx[3], tn[3], qx[3], qn[3];
 #pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      tx[v] = in.ws.tvmax[o + qv[v]];
-      tn[v] = in.ws.tvmin[o + qv[v]];
-      qx[v] = A.a.gqx[oa + qv[v]];
-      qn[v] = A.a.gqn[oa + qv[v]];
-    }
-    double gx = 0.0, gn = 0.0;
+      for (int v = 0; v < 3; ++v) {
+        tx[v] = in.ws.tvmax[o + qv[v]];
+        tn[v] = in.ws.tvmin[o + qv[v]];
+        qx[v] = A.a.gqx[oa + qv[v]];
+        qn[v] = A.a.gqn[oa + qv[v]];
+      }
+      double gx = 0.0, gn = 0.0;
 #pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      gx = vx == tx[v] ? gx + qx[v] : gx;
-      gn = vn == tn[v] ? gn + qn[v] : gn;
+      for (int v = 0; v < 3; ++v) {
+        gx = vx == tx[v] ? gx + qx[v] : gx;
+        gn = vn == tn[v] ? gn + qn[v] : gn;
+      }
+      A.a.gax[t * A.a.sE + qe] = divr(gx, rcp(double(int(in.ws.ecx[oe + qe]))));
+      A.a.gan[t * A.a.sE + qe] = divr(gn, rcp(double(int(in.ws.ecn[oe + qe]))));
     }
-    A.a.gax[t * A.a.sE + qe] = divr(gx, rcp(double(int(in.ws.ecx[oe + qe]))));
-    A.a.gan[t * A.a.sE + qe] = divr(gn, rcp(double(int(in.ws.ecn[oe + qe]))));
   }
 }
 
@@ -377,52 +390,57 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_cluster(const __grid_const
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
-  const int64_t i = lane_index();
-  if (i >= m.n_layer) return;
-  const int4 rec = __ldg(m.layer4 + i);
-  const unsigned pk = unsigned(rec.w);
-  const int n = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
-  const uint32_t qn = lq(n, L, k);
-  const double hn = ld(in.hnode + qn), hnn = ld(in.hnode_new + qn), av = ld(m.areasvol + qn);
-  const bool valid = (hnn > 0.0) && (av > 0.0);
-  const int c0 = rec.z, c1 = rec.z + int(pk >> 24);
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * in.ws.sE, ae = t * A.a.sE;
-    const double lo = in.ws.lo[o + qn], T = ld(in.T + t * in.tstride + qn);
-    const double mxv = fmax(lo, T), mnv = fmin(lo, T);
-    double gx = 0.0, gn = 0.0;
-    // the node's cells in nod_in_elem2D order; loads are unconditional (in bounds) and
-    // cells dry at k are selected away
+  const int64_t stride = int64_t(gridDim.x) * B;
+  int4 next = first_record(m.layer4, m.n_layer);
+  for (int64_t i = lane_index(); i < m.n_layer; i += stride) {
+    const int4 rec = next_record(m.layer4, m.n_layer, i, stride, next);
+    const unsigned pk = unsigned(rec.w);
+    const int n = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
+    const uint32_t qn = lq(n, L, k);
+    const double hn = ld(in.hnode + qn), hnn = ld(in.hnode_new + qn), av = ld(m.areasvol + qn);
+    const bool valid = (hnn > 0.0) && (av > 0.0);
+    const int c0 = rec.z, c1 = rec.z + int(pk >> 24);
+    for (int t = 0; t < in.ntr; ++t) {
+      const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * in.ws.sE, ae = t * A.a.sE;
+      const double lo = in.ws.lo[o + qn], T = ld(in.T + t * in.tstride + qn);
+      const double mxv = fmax(lo, T), mnv = fmin(lo, T);
+      double gx = 0.0, gn = 0.0;
+      // the node's cells in nod_in_elem2D order; loads are unconditional (in bounds) and
+      // cells dry at k are selected away
 #pragma unroll 2
-    for (int j = c0; j < c1; ++j) {
-      const bool on = in_range(k, unsigned(ld(m.nelr + j)));
-      const uint32_t qe = lq(ld(m.nel_idx + j), L, k);
-      const double ex = in.ws.amax[oe + qe], en = in.ws.amin[oe + qe];
-      const double sx = A.a.gax[ae + qe], sn = A.a.gan[ae + qe];
-      gx = (on && mxv == ex) ? gx + sx : gx;
-      gn = (on && mnv == en) ? gn + sn : gn;
+      for (int j = c0; j < c1; ++j) {
+        const bool on = in_range(k, unsigned(ld(m.nelr + j)));
+        const uint32_t qe = lq(ld(m.nel_idx + j), L, k);
+        const double ex = in.ws.amax[oe + qe], en = in.ws.amin[oe + qe];
+        const double sx = A.a.gax[ae + qe], sn = A.a.gan[ae + qe];
+        gx = (on && mxv == ex) ? gx + sx : gx;
+        gn = (on && mnv == en) ? gn + sn : gn;
+      }
+      const double gLOb = gx * smax_a(lo, T) + gn * smin_a(lo, T);
+      const double gTb = gx * smax_b(lo, T) + gn * smin_b(lo, T);
+      // seed: T_new = T + d / hnn, d = (-T hn + LO hnn) + fluxes + T (hn - hnn)
+      const double g = ld(A.gTn + t * in.tstride + qn);
+      double gTs = g, gdel = 0.0;
+      if (hnn > 0.0) {
+        gdel = g / hnn;
+        gTs += gdel * (hn - hnn);
+      }
+      gTs += -gdel * hn;
+      const double gLO = gdel * hnn + A.a.gLOl[oa + qn] + gLOb;
+      double gdiv = 0.0, gT = gTs + gTb;
+      if (valid) {
+        const double gnum = gLO / hnn;
+        gT += gnum * hn;
+        gdiv = gnum * in.dt / av;
+      }
+      A.a.gdiv[oa + qn] = gdiv;
+      A.a.gTp[oa + qn] = gT;
     }
-    const double gLOb = gx * smax_a(lo, T) + gn * smin_a(lo, T);
-    const double gTb = gx * smax_b(lo, T) + gn * smin_b(lo, T);
-    // seed: T_new = T + d / hnn, d = (-T hn + LO hnn) + fluxes + T (hn - hnn)
-    const double g = ld(A.gTn + t * in.tstride + qn);
-    double gTs = g, gdel = 0.0;
-    if (hnn > 0.0) {
-      gdel = g / hnn;
-      gTs += gdel * (hn - hnn);
-    }
-    gTs += -gdel * hn;
-    const double gLO = gdel * hnn + A.a.gLOl[oa + qn] + gLOb;
-    double gdiv = 0.0, gT = gTs + gTb;
-    if (valid) {
-      const double gnum = gLO / hnn;
-      gT += gnum * hn;
-      gdiv = gnum * in.dt / av;
-    }
-    A.a.gdiv[oa + qn] = gdiv;
-    A.a.gTp[oa + qn] = gT;
   }
 }
+
+// x / 6, correctly rounded
+__device__ __forceinline__ double div6(double x) { return divr(x, Rcp{6.0, 1.0 / 6.0, true}); }
 
 // ------------------ r_edge: adf_h = HO - LO flux; cotangents of the edge inputs
 // Both fluxes take the upwind end alone ((vf + |vf|) or (vf - |vf|) is 0), so an edge level
@@ -431,73 +449,90 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_bounds_lo(const __grid_con
 // its traffic twice what it is now); the readers tell the ends by the sign of vf
 // (edge_terms). The MFCT gradients are read at the upwind end, or at both where vf is 0 and
 // the subgradient of |vf| weighs the ends equally.
+// A thread walks the lanes, the next lane's record, volume flux and cells loaded while this
+// lane's gathers are under way.
 __global__ void __launch_bounds__(B, kRevEdgeMinBlocks) r_edge(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
-  const int64_t i = lane_index();
-  if (i >= m.n_edge) return;
-  const int4 rec = __ldg(m.edge4 + i);
-  const int e = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
-  const int n1 = rec.y, n2 = rec.z;
-  const bool use_tri = in_range(k, unsigned(rec.w));
-  const uint32_t qe = lq(e, L, k), q1 = lq(n1, L, k), q2 = lq(n2, L, k);
-  const double vf = ld(in.ws.vflux + qe), avf = fabs(vf);
-  const bool first = vf > 0.0, both = !(avf > 0.0);
-  // where the MFCT gradients of the upwind (and the other) end are read
-  uint32_t qu = first ? q1 : q2, qd = first ? q2 : q1;
-  if (use_tri) {
-    qu = lq(ld(m.eupdn + 2 * e + (first ? 0 : 1)), L, k);
-    qd = lq(ld(m.eupdn + 2 * e + (first ? 1 : 0)), L, k);
-  }
-  const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
-  const Rcp r6{6.0, 1.0 / 6.0, true};
-  const double cu = -0.5 * (first ? vf + avf : vf - avf);
-  double gvf_t = 0.0;   // summed over tracers in tracer order, as r_uv sums them
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * A.a.sEd;
-    const double a = in.ws.adfh[t * in.ws.sEd + qe];
-    // limited flux lim = ae * a, with hsc(n1) += lim, hsc(n2) -= lim
-    const double glim = A.a.ghsc[oa + q1] - A.a.ghsc[oa + q2];
-    const double pf1 = in.ws.pf[o + q1], mf1 = in.ws.mf[o + q1];
-    const double pf2 = in.ws.pf[o + q2], mf2 = in.ws.mf[o + q2];
-    const double ae = a >= 0.0 ? fmin(pf1, mf2) : fmin(mf1, pf2);
-    double ga = glim * ae;
-    // fct_plus / fct_minus sums at both ends
-    ga += A.a.gplus[oa + q1] * dmax0(a) + A.a.gminus[oa + q1] * dmin0(a);
-    ga -= A.a.gplus[oa + q2] * dmax0(-a) + A.a.gminus[oa + q2] * dmin0(-a);
-    // adf_h = HO - fl; fl also feeds LO through the divergence
-    const double gHO = ga;
-    const double gfl = -ga + (A.a.gdiv[oa + q1] - A.a.gdiv[oa + q2]);
-    const double* T = in.T + t * in.tstride;
-    const double* To = in.T_old + t * in.tstride;
-    const double T1 = ld(T + q1), T2 = ld(T + q2);
-    const double A1 = ab2(T1, ld(To + q1)), A2 = ab2(T2, ld(To + q2));
-    // MFCT gradients: the up/down cells' (use_tri) or the two nodes' averages
-    const double* gxp = use_tri ? in.ws.gx + t * in.ws.sE : in.ws.gnx + o;
-    const double* gyp = use_tri ? in.ws.gy + t * in.ws.sE : in.ws.gny + o;
-    const double diff = A2 - A1;
-    const double X = divr(2.0 * diff + c1 * gxp[qu] + c2 * gyp[qu], r6);
-    // HO = -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2); fl = -0.5 (T1 (vf + |vf|) + T2 (vf - |vf|))
-    const double Tu = first ? A1 + X : A2 - X;
-    double gvf;
-    if (both) {   // vf == 0: Tu is the second end's
-      const double Xd = divr(2.0 * diff + c1 * gxp[qd] + c2 * gyp[qd], r6);
-      gvf = -0.5 * ((A1 + Xd) + Tu) * gHO;
-      gvf += -0.5 * (T1 + T2) * gfl;
-    } else {
-      gvf = -Tu * gHO;
-      gvf += -(first ? T1 : T2) * gfl;
+  const int64_t count = m.n_edge, stride = int64_t(gridDim.x) * B;
+  int64_t i = lane_index();
+  if (i >= count) return;
+  const int L = m.L;
+  const int2* updn = reinterpret_cast<const int2*>(m.eupdn);
+  const double2* coef = reinterpret_cast<const double2*>(m.ecoef);
+  int4 rec = __ldg(m.edge4 + i);
+  int4 rec1 = i + stride < count ? __ldg(m.edge4 + i + stride) : rec;
+  double vf1 = ld(in.ws.vflux + lq(lane_ent(uint32_t(rec.x)), L, lane_lev(uint32_t(rec.x))));
+  int2 ud1 = __ldg(updn + lane_ent(uint32_t(rec.x)));
+  for (; i < count; i += stride) {
+    const int e = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x));
+    const bool use_tri = in_range(k, unsigned(rec.w));
+    const uint32_t qe = lq(e, L, k), q1 = lq(rec.y, L, k), q2 = lq(rec.z, L, k);
+    const double vf = vf1, avf = fabs(vf);
+    const bool first = vf > 0.0, both = !(avf > 0.0);
+    // where the MFCT gradients of the upwind (and the other) end are read
+    uint32_t qu = first ? q1 : q2, qd = first ? q2 : q1;
+    if (use_tri) {
+      qu = lq(first ? ud1.x : ud1.y, L, k);
+      qd = lq(first ? ud1.y : ud1.x, L, k);
     }
-    if (!(A.acc & kDeferUV)) A.a.gvf[oe + qe] = gvf;   // r_uv's input (not run when deferred)
-    gvf_t += gvf;
-    A.a.gT[oe + qe] = cu * gfl;
-    A.a.gM[oe + qe] = cu * gHO;
+    rec = rec1;
+    const double2 c = __ldg(coef + e);
+    const double cu = -0.5 * (first ? vf + avf : vf - avf);
+    double gvf_t = 0.0;   // summed over tracers in tracer order, as r_uv sums them
+    for (int t = 0; t < in.ntr; ++t) {
+      const int64_t o = t * in.ws.sN, oa = t * A.a.sN, oe = t * A.a.sEd;
+      const double a = ld(in.ws.adfh + t * in.ws.sEd + qe);
+      const double gh1 = ld(A.a.ghsc + oa + q1), gh2 = ld(A.a.ghsc + oa + q2);
+      const double pf1 = ld(in.ws.pf + o + q1), mf1 = ld(in.ws.mf + o + q1);
+      const double pf2 = ld(in.ws.pf + o + q2), mf2 = ld(in.ws.mf + o + q2);
+      const double gp1 = ld(A.a.gplus + oa + q1), gm1 = ld(A.a.gminus + oa + q1);
+      const double gp2 = ld(A.a.gplus + oa + q2), gm2 = ld(A.a.gminus + oa + q2);
+      const double gd1 = ld(A.a.gdiv + oa + q1), gd2 = ld(A.a.gdiv + oa + q2);
+      const double* T = in.T + t * in.tstride;
+      const double* To = in.T_old + t * in.tstride;
+      const double T1 = ld(T + q1), T2 = ld(T + q2), O1 = ld(To + q1), O2 = ld(To + q2);
+      // MFCT gradients: the up/down cells' (use_tri) or the two nodes' averages
+      const double* gxp = use_tri ? in.ws.gx + t * in.ws.sE : in.ws.gnx + o;
+      const double* gyp = use_tri ? in.ws.gy + t * in.ws.sE : in.ws.gny + o;
+      const double gxu = ld(gxp + qu), gyu = ld(gyp + qu);
+      if (t == 0) {
+        vf1 = ld(in.ws.vflux + lq(lane_ent(uint32_t(rec.x)), L, lane_lev(uint32_t(rec.x))));
+        ud1 = __ldg(updn + lane_ent(uint32_t(rec.x)));
+        rec1 = i + 2 * stride < count ? __ldg(m.edge4 + i + 2 * stride) : rec;
+      }
+      // limited flux lim = ae * a, with hsc(n1) += lim, hsc(n2) -= lim
+      const double glim = gh1 - gh2;
+      const double ae = a >= 0.0 ? fmin(pf1, mf2) : fmin(mf1, pf2);
+      double ga = glim * ae;
+      // fct_plus / fct_minus sums at both ends
+      ga += gp1 * dmax0(a) + gm1 * dmin0(a);
+      ga -= gp2 * dmax0(-a) + gm2 * dmin0(-a);
+      // adf_h = HO - fl; fl also feeds LO through the divergence
+      const double gHO = ga;
+      const double gfl = -ga + (gd1 - gd2);
+      const double A1 = ab2(T1, O1), A2 = ab2(T2, O2);
+      const double diff = A2 - A1;
+      const double X = div6(2.0 * diff + c.x * gxu + c.y * gyu);
+      // HO = -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2); fl = -0.5 (T1 (vf + |vf|) + T2 (vf - |vf|))
+      const double Tu = first ? A1 + X : A2 - X;
+      double gvf;
+      if (both) {   // vf == 0: Tu is the second end's
+        const double Xd = div6(2.0 * diff + c.x * ld(gxp + qd) + c.y * ld(gyp + qd));
+        gvf = -0.5 * ((A1 + Xd) + Tu) * gHO;
+        gvf += -0.5 * (T1 + T2) * gfl;
+      } else {
+        gvf = -Tu * gHO;
+        gvf += -(first ? T1 : T2) * gfl;
+      }
+      if (!(A.acc & kDeferUV)) A.a.gvf[oe + qe] = gvf;   // r_uv's input (not run when deferred)
+      gvf_t += gvf;
+      A.a.gT[oe + qe] = cu * gfl;
+      A.a.gM[oe + qe] = cu * gHO;
+    }
+    if (A.acc & kDeferUV) A.a.gvf_sum[qe] += gvf_t;   // one thread per edge level: no race
   }
-  if (A.acc & kDeferUV) A.a.gvf_sum[qe] += gvf_t;   // one thread per edge level: no race
 }
-
-// x / 6, correctly rounded
-__device__ __forceinline__ double div6(double x) { return divr(x, Rcp{6.0, 1.0 / 6.0, true}); }
 
 // A node's terms of an edge level: T through the LO flux, ttfAB through Tm. With X = 2 (A2 -
 // A1) + c1 gx + c2 gy, Tm1 = A1 + X1 / 6 and Tm2 = A2 - X2 / 6, the upwind end's A takes gM -
@@ -575,82 +610,84 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_gnode(const __grid_constan
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
-  const int64_t i = lane_index();
-  if (i >= m.n_layer) return;
-  const int4 rec = __ldg(m.layer4 + i);
-  const unsigned pk = unsigned(rec.w);
-  const int n = lane_ent(uint32_t(rec.x)), j = lane_lev(uint32_t(rec.x)), L = m.L;
-  const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
-  const uint32_t base = lq(n, L, 0), qn = base + uint32_t(j);
-  const double w = ld(in.w_e + qn), area = ld(m.area + qn);
-  const int jm = j > 0 ? j - 1 : 0;
-  const Rcp r3{3.0, 1.0 / 3.0, true};
-  const bool interior = j >= nzmin + 2 && j <= nzmax - 2;
-  double Znz = 0.0, Zm1 = 0.0, Zm2 = 0.0, Zp1 = 0.0, zb = 0.0;
-  Rcp rdc{1.0, 1.0, true}, rdu{1.0, 1.0, true}, rdd{1.0, 1.0, true};
-  if (interior) {
-    qr4c_depths(in, m, base, j, Znz, Zm1, Zm2, Zp1, zb);
-    if (in.Z3d) {
-      rdc = rcp(safe_nz(Zm1 - Znz));
-      rdu = rcp(safe_nz(Znz - Zp1));
-      rdd = rcp(safe_nz(Zm2 - Zm1));
-    } else {   // the static depths' reciprocals come from the plan
-      rdc = rcp_known(safe_nz(Zm1 - Znz), ld(m.qr4c + j));
-      rdu = rcp_known(safe_nz(Znz - Zp1), ld(m.qr4c + L + j));
-      rdd = rcp_known(safe_nz(Zm2 - Zm1), ld(m.qr4c + 2 * L + j));
+  const int64_t stride = int64_t(gridDim.x) * B;
+  int4 next = first_record(m.layer4, m.n_layer);
+  for (int64_t i = lane_index(); i < m.n_layer; i += stride) {
+    const int4 rec = next_record(m.layer4, m.n_layer, i, stride, next);
+    const unsigned pk = unsigned(rec.w);
+    const int n = lane_ent(uint32_t(rec.x)), j = lane_lev(uint32_t(rec.x)), L = m.L;
+    const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
+    const uint32_t base = lq(n, L, 0), qn = base + uint32_t(j);
+    const double w = ld(in.w_e + qn), area = ld(m.area + qn);
+    const int jm = j > 0 ? j - 1 : 0;
+    const Rcp r3{3.0, 1.0 / 3.0, true};
+    const bool interior = j >= nzmin + 2 && j <= nzmax - 2;
+    double Znz = 0.0, Zm1 = 0.0, Zm2 = 0.0, Zp1 = 0.0, zb = 0.0;
+    Rcp rdc{1.0, 1.0, true}, rdu{1.0, 1.0, true}, rdd{1.0, 1.0, true};
+    if (interior) {
+      qr4c_depths(in, m, base, j, Znz, Zm1, Zm2, Zp1, zb);
+      if (in.Z3d) {
+        rdc = rcp(safe_nz(Zm1 - Znz));
+        rdu = rcp(safe_nz(Znz - Zp1));
+        rdd = rcp(safe_nz(Zm2 - Zm1));
+      } else {   // the static depths' reciprocals come from the plan
+        rdc = rcp_known(safe_nz(Zm1 - Znz), ld(m.qr4c + j));
+        rdu = rcp_known(safe_nz(Znz - Zp1), ld(m.qr4c + L + j));
+        rdd = rcp_known(safe_nz(Zm2 - Zm1), ld(m.qr4c + 2 * L + j));
+      }
     }
-  }
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t o = t * in.ws.sN, oa = t * A.a.sN;
-    const double* T = in.T + t * in.tstride + base;
-    const double* To = in.T_old + t * in.tstride + base;
-    const double* pf = in.ws.pf + o + base;
-    const double* mf = in.ws.mf + o + base;
-    const double* gplus = A.a.gplus + oa + base;
-    const double* gminus = A.a.gminus + oa + base;
-    const double* gdiv = A.a.gdiv + oa + base;
-    const double f = in.ws.adfv[o + qn];
-    double ae;
-    if (j == nzmin) ae = f >= 0.0 ? pf[j] : mf[j];
-    else ae = f >= 0.0 ? fmin(mf[j - 1], pf[j]) : fmin(pf[j - 1], mf[j]);
-    double gf = gvl_at(m, A.a.ghsc + oa, base, j, nzmin, nzmax) * ae;
-    gf += gplus[j] * dmax0(f) + gminus[j] * dmin0(f);
-    if (j - 1 >= nzmin) gf -= gplus[j - 1] * dmax0(-f) + gminus[j - 1] * dmin0(-f);
-    const double ghi = gf;
-    double gfv = -gf + gdiv[j];
-    if (j - 1 >= nzmin) gfv -= gdiv[j - 1];
-    A.a.gfv[oa + qn] = gfv;
-    double gw = 0.0;
-    gw += -0.5 * (ld(T + j) * (1.0 + sgn(w)) + ld(T + jm) * (1.0 - sgn(w))) * area * gfv;
-    // QR4C (tracer_adv.py:241-295): surface, next-to-surface / next-to-bottom, interior
-    double z0 = 0.0, zm1 = 0.0, zm2 = 0.0, zp1 = 0.0;
-    if (j == nzmin) {
-      gw += -ab2(ld(T + j), ld(To + j)) * area * ghi;
-      z0 = -w * area * ghi;
-    } else if (j == nzmin + 1 || j == nzmax - 1) {
-      gw += -0.5 * (ab2(ld(T + j - 1), ld(To + j - 1)) + ab2(ld(T + j), ld(To + j))) * area * ghi;
-      z0 = zm1 = -0.5 * w * area * ghi;
-    } else if (interior) {
-      const double A0 = ab2(ld(T + j), ld(To + j)), Am1 = ab2(ld(T + j - 1), ld(To + j - 1));
-      const double Am2 = ab2(ld(T + j - 2), ld(To + j - 2)), Ap1 = ab2(ld(T + j + 1), ld(To + j + 1));
-      const double qc = divr(Am1 - A0, rdc), qu = divr(A0 - Ap1, rdu), qd = divr(Am2 - Am1, rdd);
-      const double Tmean1 = A0 + divr((2.0 * qc + qu) * (zb - Znz), r3);
-      const double Tmean2 = Am1 + divr((2.0 * qc + qd) * (zb - Zm1), r3);
-      gw += -0.5 * (Tmean1 + Tmean2) * area * ghi;
-      // Tmean1 = A0 + (2 qc + qu) (zb - Z[j]) / 3, Tmean2 = Am1 + (2 qc + qd) (zb - Z[j-1]) / 3
-      const double gS = -0.5 * w * area * ghi;
-      const double gq1 = divr(gS * (zb - Znz), r3), gq2 = divr(gS * (zb - Zm1), r3);
-      const double gqc = 2.0 * gq1 + 2.0 * gq2, gqu = gq1, gqd = gq2;
-      z0 = gS - divr(gqc, rdc) + divr(gqu, rdu);
-      zm1 = gS + divr(gqc, rdc) - divr(gqd, rdd);
-      zm2 = divr(gqd, rdd);
-      zp1 = -divr(gqu, rdu);
+    for (int t = 0; t < in.ntr; ++t) {
+      const int64_t o = t * in.ws.sN, oa = t * A.a.sN;
+      const double* T = in.T + t * in.tstride + base;
+      const double* To = in.T_old + t * in.tstride + base;
+      const double* pf = in.ws.pf + o + base;
+      const double* mf = in.ws.mf + o + base;
+      const double* gplus = A.a.gplus + oa + base;
+      const double* gminus = A.a.gminus + oa + base;
+      const double* gdiv = A.a.gdiv + oa + base;
+      const double f = in.ws.adfv[o + qn];
+      double ae;
+      if (j == nzmin) ae = f >= 0.0 ? pf[j] : mf[j];
+      else ae = f >= 0.0 ? fmin(mf[j - 1], pf[j]) : fmin(pf[j - 1], mf[j]);
+      double gf = gvl_at(m, A.a.ghsc + oa, base, j, nzmin, nzmax) * ae;
+      gf += gplus[j] * dmax0(f) + gminus[j] * dmin0(f);
+      if (j - 1 >= nzmin) gf -= gplus[j - 1] * dmax0(-f) + gminus[j - 1] * dmin0(-f);
+      const double ghi = gf;
+      double gfv = -gf + gdiv[j];
+      if (j - 1 >= nzmin) gfv -= gdiv[j - 1];
+      A.a.gfv[oa + qn] = gfv;
+      double gw = 0.0;
+      gw += -0.5 * (ld(T + j) * (1.0 + sgn(w)) + ld(T + jm) * (1.0 - sgn(w))) * area * gfv;
+      // QR4C (tracer_adv.py:241-295): surface, next-to-surface / next-to-bottom, interior
+      double z0 = 0.0, zm1 = 0.0, zm2 = 0.0, zp1 = 0.0;
+      if (j == nzmin) {
+        gw += -ab2(ld(T + j), ld(To + j)) * area * ghi;
+        z0 = -w * area * ghi;
+      } else if (j == nzmin + 1 || j == nzmax - 1) {
+        gw += -0.5 * (ab2(ld(T + j - 1), ld(To + j - 1)) + ab2(ld(T + j), ld(To + j))) * area * ghi;
+        z0 = zm1 = -0.5 * w * area * ghi;
+      } else if (interior) {
+        const double A0 = ab2(ld(T + j), ld(To + j)), Am1 = ab2(ld(T + j - 1), ld(To + j - 1));
+        const double Am2 = ab2(ld(T + j - 2), ld(To + j - 2)), Ap1 = ab2(ld(T + j + 1), ld(To + j + 1));
+        const double qc = divr(Am1 - A0, rdc), qu = divr(A0 - Ap1, rdu), qd = divr(Am2 - Am1, rdd);
+        const double Tmean1 = A0 + divr((2.0 * qc + qu) * (zb - Znz), r3);
+        const double Tmean2 = Am1 + divr((2.0 * qc + qd) * (zb - Zm1), r3);
+        gw += -0.5 * (Tmean1 + Tmean2) * area * ghi;
+        // Tmean1 = A0 + (2 qc + qu) (zb - Z[j]) / 3, Tmean2 = Am1 + (2 qc + qd) (zb - Z[j-1]) / 3
+        const double gS = -0.5 * w * area * ghi;
+        const double gq1 = divr(gS * (zb - Znz), r3), gq2 = divr(gS * (zb - Zm1), r3);
+        const double gqc = 2.0 * gq1 + 2.0 * gq2, gqu = gq1, gqd = gq2;
+        z0 = gS - divr(gqc, rdc) + divr(gqu, rdu);
+        zm1 = gS + divr(gqc, rdc) - divr(gqd, rdd);
+        zm2 = divr(gqd, rdd);
+        zp1 = -divr(gqu, rdu);
+      }
+      A.a.gw[oa + qn] = gw;
+      A.a.gz0[oa + qn] = z0;
+      A.a.gzm1[oa + qn] = zm1;
+      A.a.gzm2[oa + qn] = zm2;
+      A.a.gzp1[oa + qn] = zp1;
     }
-    A.a.gw[oa + qn] = gw;
-    A.a.gz0[oa + qn] = z0;
-    A.a.gzm1[oa + qn] = zm1;
-    A.a.gzm2[oa + qn] = zm2;
-    A.a.gzp1[oa + qn] = zp1;
   }
 }
 
@@ -658,42 +695,44 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_vert(const __grid_constant
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
-  const int64_t i = lane_index();
-  if (i >= m.n_elem) return;
-  const uint32_t lane = ld(m.elem_lanes + i);
-  const int el = lane_ent(lane), k = lane_lev(lane), L = m.L;
-  const double aw = ld(m.earea + el);
-  const int u0 = ld(m.eud_off + el), u1 = ld(m.eud_off + el + 1);
-  const uint32_t qv[3] = {lq(ld(m.enodes + 3 * el), L, k),
-                         lq(ld(m.enodes + 3 * el + 1), L, k),
-                         lq(ld(m.enodes + 3 * el + 2), L, k)};
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t oa = t * A.a.sN, oe = t * A.a.sEd;
-    double gx = 0.0, gy = 0.0;
+  const int64_t stride = int64_t(gridDim.x) * B;
+  uint32_t next = first_record(m.elem_lanes, m.n_elem);
+  for (int64_t i = lane_index(); i < m.n_elem; i += stride) {
+    const uint32_t lane = next_record(m.elem_lanes, m.n_elem, i, stride, next);
+    const int el = lane_ent(lane), k = lane_lev(lane), L = m.L;
+    const double aw = ld(m.earea + el);
+    const int u0 = ld(m.eud_off + el), u1 = ld(m.eud_off + el + 1);
+    const uint32_t qv[3] = {lq(ld(m.enodes + 3 * el), L, k),
+                           lq(ld(m.enodes + 3 * el + 1), L, k),
+                           lq(ld(m.enodes + 3 * el + 2), L, k)};
+    for (int t = 0; t < in.ntr; ++t) {
+      const int64_t oa = t * A.a.sN, oe = t * A.a.sEd;
+      double gx = 0.0, gy = 0.0;
 #pragma unroll 2
-    for (int j = u0; j < u1; ++j) {   // edges using el as up (slot 0) or down (1) cell
-      const int idx = ld(m.eud_idx + j), e = idx >> 1;
-      const bool on = in_range(k, unsigned(ld(m.etr + e)));
-      // the down (slot 1) / up (slot 0) cell's gradient enters Tm2 / Tm1
-      const uint32_t qe = lq(e, L, k);
-      const double x = grad_factor(idx & 1, ld(in.ws.vflux + qe), A.a.gM[oe + qe]);
-      const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
-      gx = on ? gx + c1 * x : gx;
-      gy = on ? gy + c2 * x : gy;
-    }
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {   // gnode(n) = sum_e a_e tr_e / den(n)
-      // the cotangent is nonzero only at levels where an edge of the vertex takes the
-      // node-average gradient, the only levels whose denominator the forward stored
-      const double cx = A.a.ggnx[oa + qv[v]], cy = A.a.ggny[oa + qv[v]];
-      if (cx != 0.0 || cy != 0.0) {
-        const double dd = in.ws.nden[qv[v]];   // the forward's (safe) denominator
-        gx += cx * aw / dd;
-        gy += cy * aw / dd;
+      for (int j = u0; j < u1; ++j) {   // edges using el as up (slot 0) or down (1) cell
+        const int idx = ld(m.eud_idx + j), e = idx >> 1;
+        const bool on = in_range(k, unsigned(ld(m.etr + e)));
+        // the down (slot 1) / up (slot 0) cell's gradient enters Tm2 / Tm1
+        const uint32_t qe = lq(e, L, k);
+        const double x = grad_factor(idx & 1, ld(in.ws.vflux + qe), A.a.gM[oe + qe]);
+        const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
+        gx = on ? gx + c1 * x : gx;
+        gy = on ? gy + c2 * x : gy;
       }
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {   // gnode(n) = sum_e a_e tr_e / den(n)
+        // the cotangent is nonzero only at levels where an edge of the vertex takes the
+        // node-average gradient, the only levels whose denominator the forward stored
+        const double cx = A.a.ggnx[oa + qv[v]], cy = A.a.ggny[oa + qv[v]];
+        if (cx != 0.0 || cy != 0.0) {
+          const double dd = in.ws.nden[qv[v]];   // the forward's (safe) denominator
+          gx += cx * aw / dd;
+          gy += cy * aw / dd;
+        }
+      }
+      A.a.gtrx[t * A.a.sE + lq(el, L, k)] = gx;
+      A.a.gtry[t * A.a.sE + lq(el, L, k)] = gy;
     }
-    A.a.gtrx[t * A.a.sE + lq(el, L, k)] = gx;
-    A.a.gtry[t * A.a.sE + lq(el, L, k)] = gy;
   }
 }
 
@@ -707,78 +746,80 @@ __global__ void __launch_bounds__(B, kRevMinBlocks) r_tr(const __grid_constant__
 __global__ void __launch_bounds__(B, kRevMinBlocks) r_final(const __grid_constant__ Adj A) {
   const Inst& in = A.in;
   const DevMesh& m = in.m;
-  const int64_t li = lane_index();
-  if (li >= m.n_layer) return;
-  const int4 rec = __ldg(m.layer4 + li);
-  const unsigned pk = unsigned(rec.w);
-  const int n = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
-  const int64_t i = lq(n, L, k);
-  const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
-  const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
-  const int c0 = rec.z, c1 = rec.z + int(pk >> 24);
-  const unsigned onb = unsigned(__ldg(m.nflags + li));   // (flag words in lane order)
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t oa = t * A.a.sN;
-    const double* gfv = A.a.gfv + oa;
-    if (k == nzmin && k > 0) {   // the dry level above a cavity
-      const double w = ld(in.w_e + i), area = ld(m.area + i);
-      double g = 0.0;
-      g += -0.5 * (w - fabs(w)) * area * gfv[i];
-      const int64_t oT = t * in.tstride + i - 1;
-      const double vT = (ld(A.gTn + oT) + g) + kAbNew * 0.0;
+  const int64_t stride = int64_t(gridDim.x) * B;
+  int4 next = first_record(m.layer4, m.n_layer);
+  for (int64_t li = lane_index(); li < m.n_layer; li += stride) {
+    const int4 rec = next_record(m.layer4, m.n_layer, li, stride, next);
+    const unsigned pk = unsigned(rec.w);
+    const int n = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
+    const int64_t i = lq(n, L, k);
+    const int nzmin = int(pk & 255u), nzmax = int((pk >> 8) & 255u);
+    const int e0 = rec.y, e1 = rec.y + int((pk >> 16) & 255u);
+    const int c0 = rec.z, c1 = rec.z + int(pk >> 24);
+    const unsigned onb = unsigned(__ldg(m.nflags + li));   // (flag words in lane order)
+    for (int t = 0; t < in.ntr; ++t) {
+      const int64_t oa = t * A.a.sN;
+      const double* gfv = A.a.gfv + oa;
+      if (k == nzmin && k > 0) {   // the dry level above a cavity
+        const double w = ld(in.w_e + i), area = ld(m.area + i);
+        double g = 0.0;
+        g += -0.5 * (w - fabs(w)) * area * gfv[i];
+        const int64_t oT = t * in.tstride + i - 1;
+        const double vT = (ld(A.gTn + oT) + g) + kAbNew * 0.0;
+        A.gT[oT] = (A.acc & kAccT) ? A.gT[oT] + vT : vT;
+      }
+      double gA = 0.0;
+      // vertical upwind fluxes of interfaces k and k+1
+      double gTv = 0.0;
+      {
+        const double w = ld(in.w_e + i), area = ld(m.area + i);
+        gTv += -0.5 * (w + fabs(w)) * area * gfv[i];
+        if (k == 0) gTv += -0.5 * (w - fabs(w)) * area * gfv[i];
+      }
+      if (k + 1 < nzmax) {
+        const double w = ld(in.w_e + i + 1), area = ld(m.area + i + 1);
+        gTv += -0.5 * (w - fabs(w)) * area * gfv[i + 1];
+      }
+      // QR4C terms of interfaces k-1 .. k+2 in ascending order (a term that does not
+      // reach k is +0.0; gA starts at +0.0, so adding it changes no bit)
+      if (k - 1 >= nzmin) gA += A.a.gzp1[oa + i - 1];
+      gA += A.a.gz0[oa + i];
+      if (k + 1 < nzmax) gA += A.a.gzm1[oa + i + 1];
+      if (k + 2 < nzmax) gA += A.a.gzm2[oa + i + 2];
+      // element gradients on T: the node's cells in nod_in_elem2D order
+      double gTtr = 0.0;
+#pragma unroll 2
+      for (int j = c0; j < c1; ++j) {
+        const unsigned r = unsigned(ld(m.nelr + j));
+        const bool on = in_range(k, r);
+        const int el = ld(m.nel_idx + j), iv = int((r >> 16) & 3u);
+        const int64_t qe = t * A.a.sE + lq(el, L, k);
+        const double v = ld(m.gsca + 6 * el + iv) * A.a.gtrx[qe] +
+                         ld(m.gsca + 6 * el + 3 + iv) * A.a.gtry[qe];
+        gTtr = on ? gTtr + v : gTtr;
+      }
+      double gT = A.a.gTp[oa + i] + gTtr + gTv;
+#pragma unroll 2
+      for (int j = e0; j < e1; ++j) {
+        const int4 sl = __ldg(m.ns4 + j);
+        const bool on = (onb >> (j - e0)) & 1u;
+        const uint32_t qe = uint32_t(sl.x) + uint32_t(k);
+        const double vf = ld(in.ws.vflux + qe);
+        double vT, vA;
+        edge_terms(sl.z ? vf < 0.0 : vf > 0.0, A.a.gT[t * A.a.sEd + qe], A.a.gM[t * A.a.sEd + qe],
+                   vT, vA);
+        gT = on ? gT + vT : gT;
+        gA = on ? gA + vA : gA;
+      }
+      const int64_t oT = t * in.tstride + i;
+      const double vT = gT + kAbNew * gA, vTo = kAbOld * gA;
       A.gT[oT] = (A.acc & kAccT) ? A.gT[oT] + vT : vT;
+      A.gTo[oT] = (A.acc & kAccTo) ? A.gTo[oT] + vTo : vTo;
     }
-    double gA = 0.0;
-    // vertical upwind fluxes of interfaces k and k+1
-    double gTv = 0.0;
-    {
-      const double w = ld(in.w_e + i), area = ld(m.area + i);
-      gTv += -0.5 * (w + fabs(w)) * area * gfv[i];
-      if (k == 0) gTv += -0.5 * (w - fabs(w)) * area * gfv[i];
-    }
-    if (k + 1 < nzmax) {
-      const double w = ld(in.w_e + i + 1), area = ld(m.area + i + 1);
-      gTv += -0.5 * (w - fabs(w)) * area * gfv[i + 1];
-    }
-    // QR4C terms of interfaces k-1 .. k+2 in ascending order (a term that does not
-    // reach k is +0.0; gA starts at +0.0, so adding it changes no bit)
-    if (k - 1 >= nzmin) gA += A.a.gzp1[oa + i - 1];
-    gA += A.a.gz0[oa + i];
-    if (k + 1 < nzmax) gA += A.a.gzm1[oa + i + 1];
-    if (k + 2 < nzmax) gA += A.a.gzm2[oa + i + 2];
-    // element gradients on T: the node's cells in nod_in_elem2D order
-    double gTtr = 0.0;
-#pragma unroll 2
-    for (int j = c0; j < c1; ++j) {
-      const unsigned r = unsigned(ld(m.nelr + j));
-      const bool on = in_range(k, r);
-      const int el = ld(m.nel_idx + j), iv = int((r >> 16) & 3u);
-      const int64_t qe = t * A.a.sE + lq(el, L, k);
-      const double v = ld(m.gsca + 6 * el + iv) * A.a.gtrx[qe] +
-                       ld(m.gsca + 6 * el + 3 + iv) * A.a.gtry[qe];
-      gTtr = on ? gTtr + v : gTtr;
-    }
-    double gT = A.a.gTp[oa + i] + gTtr + gTv;
-#pragma unroll 2
-    for (int j = e0; j < e1; ++j) {
-      const int4 sl = __ldg(m.ns4 + j);
-      const bool on = (onb >> (j - e0)) & 1u;
-      const uint32_t qe = uint32_t(sl.x) + uint32_t(k);
-      const double vf = ld(in.ws.vflux + qe);
-      double vT, vA;
-      edge_terms(sl.z ? vf < 0.0 : vf > 0.0, A.a.gT[t * A.a.sEd + qe], A.a.gM[t * A.a.sEd + qe],
-                 vT, vA);
-      gT = on ? gT + vT : gT;
-      gA = on ? gA + vA : gA;
-    }
-    const int64_t oT = t * in.tstride + i;
-    const double vT = gT + kAbNew * gA, vTo = kAbOld * gA;
-    A.gT[oT] = (A.acc & kAccT) ? A.gT[oT] + vT : vT;
-    A.gTo[oT] = (A.acc & kAccTo) ? A.gTo[oT] + vTo : vTo;
+    double g = 0.0;   // dL/dw_e summed over tracers
+    for (int t = 0; t < in.ntr; ++t) g += A.a.gw[t * A.a.sN + i];
+    A.gw[i] = (A.acc & kAccW) ? A.gw[i] + g : g;
   }
-  double g = 0.0;   // dL/dw_e summed over tracers
-  for (int t = 0; t < in.ntr; ++t) g += A.a.gw[t * A.a.sN + i];
-  A.gw[i] = (A.acc & kAccW) ? A.gw[i] + g : g;
 }
 
 // -------------------------- r_uv: edge_vflux transposed, summed over tracers
@@ -1143,6 +1184,10 @@ int fct_adjoint_ex(FctPlan* P, const FctFields* f, const double* gT_new, double 
   auto grid = [](int64_t lanes, int b) {
     return dim3(unsigned(std::max<int64_t>(1, (lanes + b - 1) / b)));
   };
+  // walking kernels: as many blocks as are resident at once
+  auto walk = [&](int64_t lanes) {
+    return dim3(std::min(grid(lanes, B).x, unsigned(148 * kRevMinBlocks)));
+  };
   const DevMesh& hm = P->hm;
   // Side stream: r_dry (dry levels, needs nothing) from the start; r_vert (needs the
   // node kernels up to r_bounds_lo) beside r_edge; r_uv (needs r_edge's volume-flux
@@ -1153,13 +1198,14 @@ int fct_adjoint_ex(FctPlan* P, const FctFields* f, const double* gT_new, double 
   r_dry<<<grid(hm.n_dry, B), B, 0, P->adj_side>>>(A);
   r_seed<<<grid(hm.n_layer, B), B, 0, s>>>(A);
   r_ratio_window<<<dim3(unsigned(std::max<int64_t>(1, (hm.n_layer + B - 3) / (B - 2)))), B, 0, s>>>(A);
-  r_cluster<<<grid(hm.n_elem, B), B, 0, s>>>(A);
-  r_bounds_lo<<<grid(hm.n_layer, B), B, 0, s>>>(A);
+  r_cluster<<<walk(hm.n_elem), B, 0, s>>>(A);
+  r_bounds_lo<<<walk(hm.n_layer), B, 0, s>>>(A);
   FCT_CUDA(cudaEventRecord(P->adj_ev[4], s));
   FCT_CUDA(cudaStreamWaitEvent(P->adj_side, P->adj_ev[4], 0));
-  r_vert<<<grid(hm.n_layer, B), B, 0, P->adj_side>>>(A);
+  r_vert<<<walk(hm.n_layer), B, 0, P->adj_side>>>(A);
   FCT_CUDA(cudaEventRecord(P->adj_ev[1], P->adj_side));
-  r_edge<<<grid(hm.n_edge, B), B, 0, s>>>(A);
+  r_edge<<<dim3(unsigned(std::min<int64_t>(std::max<int64_t>(1, (hm.n_edge + B - 1) / B),
+                                           148 * kRevEdgeMinBlocks))), B, 0, s>>>(A);
   if (!defer_uv) {
     FCT_CUDA(cudaEventRecord(P->adj_ev[2], s));
     FCT_CUDA(cudaStreamWaitEvent(P->adj_side, P->adj_ev[2], 0));
@@ -1167,9 +1213,9 @@ int fct_adjoint_ex(FctPlan* P, const FctFields* f, const double* gT_new, double 
   }
   FCT_CUDA(cudaEventRecord(P->adj_ev[3], P->adj_side));
   r_gnode<<<grid(hm.n_layer, B), B, 0, s>>>(A);
-  r_tr<<<grid(hm.n_elem, B), B, 0, s>>>(A);
+  r_tr<<<walk(hm.n_elem), B, 0, s>>>(A);
   FCT_CUDA(cudaStreamWaitEvent(s, P->adj_ev[1], 0));
-  r_final<<<grid(hm.n_layer, B), B, 0, s>>>(A);
+  r_final<<<walk(hm.n_layer), B, 0, s>>>(A);
   FCT_CUDA(cudaStreamWaitEvent(s, P->adj_ev[3], 0));
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "adjoint kernel launch");
