@@ -177,7 +177,7 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
     d.any_wi = false;
     d.copy_dry = false;
     d.per_thread = std::min(d.chunk, 2);
-    d.auto_map(true, d.max_nseg[0] * d.chunk / 4 * gr.count);
+    d.auto_map(true, seg_even(d), d.max_nseg[0] * d.chunk / 4 * gr.count);
     gr.dims = d;
   }
   e = cudaMalloc(&B->d_health, size_t(n) * sizeof(unsigned long long));
@@ -580,7 +580,7 @@ int fct_serve_step(FctServe* S, const FctInstance* insts, const int32_t* phases,
     d.chunk = 0;
     d.per_thread = 2;   // (the diffusion epilogue's split)
     if (P0->per_thread > 0) d.set_map(P0->per_thread, P0->lpt);
-    else d.auto_map(true, P0->hm.n_layer * ntr / 4 * (j1 - j0));
+    else d.auto_map(true, seg_even(d), P0->hm.n_layer * ntr / 4 * (j1 - j0));
     for (int j = j0; j < j1; ++j)
       if (insts[order[j]].w_derived) d.any_derive_w = true;
     d.any_wi = false;

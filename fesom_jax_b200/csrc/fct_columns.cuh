@@ -2,12 +2,16 @@
 // implicit part of the split vertical velocity. A tridiagonal recursion is sequential in the
 // level, so one thread walks a column; read straight from memory every step of that walk
 // waits for a strided load (T of 60,000 columns x 48 levels: 212 us per tracer at 32% of the
-// memory rate with 11% of the issue slots used). Here a block takes kColumns columns:
+// memory rate with 11% of the issue slots used). Here a block takes a few columns:
 //   1. all threads form the rows' coefficients and right-hand sides, levels adjacent (whole
 //      lines), into shared memory;
-//   2. one thread per column and tracer eliminates and substitutes back in shared memory
-//      (rows padded to an odd length, so that neighbouring columns use different banks);
+//   2. one thread per column eliminates and substitutes back in shared memory (rows padded to
+//      an odd length, so that neighbouring columns use different banks), all tracers of the
+//      block in its registers: the walk's chain is the matrix recursion's, and the tracers'
+//      and the next row's loads fit beside it;
 //   3. all threads write the result, levels adjacent.
+// What bounds it is that chain (about 20 dependent operations a level), so the blocks are
+// small and many: 3 + (tracers) values per row and column.
 #pragma once
 
 #include "fct_device.cuh"
@@ -15,13 +19,14 @@
 namespace fct {
 namespace {
 
-constexpr int kColThreads = 128;
+constexpr int kColThreads = 256;
+constexpr int kColMaxTracers = 8;        // right-hand sides of a block
 constexpr int kColMaxSmem = 227 << 10;   // opt-in shared memory of a block
 
-// Shared rows of a block: a, b, c, cp of the matrix and one right-hand side per tracer, each
-// [columns][stride].
+// Shared rows of a block: a, b, c (then cp) of the matrix and one right-hand side per tracer,
+// each [columns][stride].
 struct ColRows {
-  double *a, *b, *c, *cp, *r;
+  double *a, *b, *c, *r;
   int stride, columns;
   __device__ __forceinline__ ColRows(double* sh, int columns_, int L)
       : stride(L | 1), columns(columns_) {
@@ -29,56 +34,93 @@ struct ColRows {
     a = sh;
     b = sh + n;
     c = sh + 2 * n;
-    cp = sh + 3 * n;
-    r = sh + 4 * n;
+    r = sh + 3 * n;
   }
   __device__ __forceinline__ int at(int col, int k) const { return col * stride + k; }
   __device__ __forceinline__ double* rhs(int t) const { return r + t * columns * stride; }
 };
 
 inline size_t col_smem(int columns, int L, int nt) {
-  return size_t(columns) * size_t(L | 1) * size_t(4 + nt) * sizeof(double);
+  return size_t(columns) * size_t(L | 1) * size_t(3 + nt) * sizeof(double);
 }
-// Columns per block: as many (32, 16 or 8) as keep about four blocks on an SM and one
-// thread per column and tracer.
-inline int col_columns(int L, int nt) {
-  for (int c : {32, 16})
-    if (col_smem(c, L, nt) <= size_t(56) << 10 && c * nt <= kColThreads) return c;
-  return 8;
+// Columns per block: 16, or 8 where 16 would leave fewer than four blocks on an SM.
+inline int col_columns(int L, int nt) { return col_smem(16, L, nt) <= size_t(56) << 10 ? 16 : 8; }
+
+// x / y for the NT + 1 dividends of a row, correctly rounded (fct_div.cuh) and without a branch
+// per quotient; operands outside the products' range take the native division.
+__device__ __noinline__ double col_div_slow(double x, double y) { return x / y; }
+__device__ __forceinline__ bool col_div_ok(double x) { return x == 0.0 || div_exp_ok(x); }
+__device__ __forceinline__ double col_div(double x, double y, double r) {
+  const double q0 = x * r;
+  const double q1 = fma(fma(-y, q0, x), r, q0);
+  const double q2 = fma(fma(-y, q1, x), r, q1);
+  return x == 0.0 ? q0 : q2;
 }
 
 // Thomas algorithm over the rows [nzmin, nzmax) of every column of the block (fesom_jax/
-// ops.py:121-168; the padded rows above and below solve to exactly 0). The solution
-// replaces the right-hand side. Every thread of the block calls it, after a barrier.
-__device__ __forceinline__ void col_solve(const DevMesh& m, const ColRows& s, int n0, int nt) {
-  const int tid = threadIdx.x, col = tid % s.columns, t = tid / s.columns, n = n0 + col;
-  const bool on = t < nt && n < m.N;
-  const int nzmin = on ? ld(m.nzmin + n) : 0, nzmax = on ? ld(m.nzmax + n) : 0;
-  double* r = s.rhs(on ? t : 0);
-  double cprev = 0.0, dprev = 0.0;
-  for (int k = nzmin; k < nzmax; ++k) {
-    const int i = s.at(col, k);
-    const double a = s.a[i];
-    const Rcp rm = rcp(s.b[i] - a * cprev);
-    cprev = divr(s.c[i], rm);
-    if (t == 0) s.cp[i] = cprev;
-    dprev = divr(r[i] - a * dprev, rm);
-    r[i] = dprev;
-  }
-  __syncthreads();
-  double x = 0.0;
-  for (int k = nzmax - 1; k >= nzmin; --k) {
-    const int i = s.at(col, k);
-    x = r[i] - s.cp[i] * x;
-    r[i] = x;
+// ops.py:121-168; the padded rows above and below solve to exactly 0). The solutions replace
+// the right-hand sides. Every thread of the block calls it, after a barrier.
+template <int NT>
+__device__ __forceinline__ void col_solve(const DevMesh& m, const ColRows& s, int n0) {
+  const int col = threadIdx.x, n = n0 + col;
+  if (col < s.columns && n < m.N) {
+    const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
+    const int rs = s.columns * s.stride;
+    double cp = 0.0, dp[NT], an = 0.0, bn = 1.0, cn = 0.0, rn[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) dp[t] = rn[t] = 0.0;
+    int i = s.at(col, nzmin);
+    if (nzmin < nzmax) {
+      an = s.a[i]; bn = s.b[i]; cn = s.c[i];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) rn[t] = s.r[t * rs + i];
+    }
+    for (int k = nzmin; k < nzmax; ++k, ++i) {
+      const double a = an, c = cn, y = bn - a * cp;
+      double x[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) x[t] = rn[t] - a * dp[t];
+      if (k + 1 < nzmax) {   // the next row beside this one's chain
+        an = s.a[i + 1]; bn = s.b[i + 1]; cn = s.c[i + 1];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) rn[t] = s.r[t * rs + i + 1];
+      }
+      bool ok = div_exp_ok(y) && col_div_ok(c);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) ok = ok && col_div_ok(x[t]);
+      const double r = __drcp_rn(y);
+      cp = col_div(c, y, r);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) dp[t] = col_div(x[t], y, r);
+      if (!ok) {
+        cp = col_div_slow(c, y);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) dp[t] = col_div_slow(x[t], y);
+      }
+      s.c[i] = cp;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) s.r[t * rs + i] = dp[t];
+    }
+    double v[NT];
+#pragma unroll
+    for (int t = 0; t < NT; ++t) v[t] = 0.0;
+    for (int k = nzmax - 1; k >= nzmin; --k) {
+      --i;
+      const double q = s.c[i];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        v[t] = s.r[t * rs + i] - q * v[t];
+        s.r[t * rs + i] = v[t];
+      }
+    }
   }
   __syncthreads();
 }
 
 // ------------- implicit vertical diffusion (tracer_diff.py:68-123, ops.py:121-168) of the
 // tracers [t0, t0 + nt) of the columns [n0, n0 + columns)
-template <bool IL>
-__device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns, int t0, int nt,
+template <int nt, bool IL>
+__device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns, int t0,
                                             double* sh) {
   const DevMesh& m = in.m;
   if (!in.Kv || n0 >= m.N) return;   // block-uniform
@@ -129,7 +171,7 @@ __device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns,
     }
   }
   __syncthreads();
-  col_solve(m, s, n0, nt);
+  col_solve<nt>(m, s, n0);
   const bool copy = Tin != in.T_new;   // out of place: dry levels keep T
   if constexpr (IL) {
     for (int i = threadIdx.x; i < columns * L * nt; i += kColThreads) {
@@ -154,9 +196,9 @@ __device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns,
 
 // ---------------------------- adv_tra_vert_impl (tracer_adv.py:487-529): implicit w_i
 // advection of LO, the tracers' workspace slots [w0, w0 + nt)
-template <bool IL>
+template <int nt, bool IL>
 __device__ __forceinline__ void block_vert_impl(const Inst& in, int n0, int columns, int w0,
-                                                int nt, double* sh) {
+                                                double* sh) {
   const DevMesh& m = in.m;
   if (!in.w_i || n0 >= m.N) return;   // block-uniform
   const int L = m.L;
@@ -195,7 +237,7 @@ __device__ __forceinline__ void block_vert_impl(const Inst& in, int n0, int colu
     }
   }
   __syncthreads();
-  col_solve(m, s, n0, nt);
+  col_solve<nt>(m, s, n0);
   for (int t = 0; t < nt; ++t)
     for (int i = threadIdx.x; i < columns * L; i += kColThreads) {
       const int col = i / L, k = i - col * L, n = n0 + col;

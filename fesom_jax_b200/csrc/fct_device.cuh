@@ -192,5 +192,18 @@ __device__ __forceinline__ double vflux_up(double Tb, double Ta, double w, doubl
   return -0.5 * (Tb * (w + aw) + Ta * (w - aw)) * area;
 }
 
+// ------------------------------------------- dry levels keep T (ale_reconstruct)
+template <bool IL>
+__device__ __forceinline__ void body_copy_dry(const Inst& in, int64_t i) {
+  const DevMesh& m = in.m;
+  if (i >= m.n_dry) return;
+  const uint32_t lane = __ldg(m.dry_lanes + i);
+  const uint32_t q = lq(lane_ent(lane), m.L, lane_lev(lane));
+  for (int t = 0; t < in.ntr; ++t) {
+    const int64_t a = tix<IL>(q, t, in.tstride, in.tg);
+    in.T_new[a] = in.T[a];
+  }
+}
+
 }  // namespace
 }  // namespace fct

@@ -30,26 +30,44 @@ namespace fct {
 namespace {
 
 // ---------------------------------------------------------------- edge_vflux
-__device__ __forceinline__ void body_vflux(const Inst& in, int64_t i) {
+// A thread walks the edge lanes i, i + stride, ...: the next lane's cells are loaded while this
+// lane's velocities are under way (82 us on the CORE2-size mesh when each thread took one lane
+// and waited for its lane, its cells and its velocities in a row).
+__device__ __forceinline__ void body_vflux(const Inst& in, int64_t i, int64_t stride) {
   const DevMesh& m = in.m;
-  if (i >= m.n_edge) return;
-  const uint32_t lane = ld(m.edge_lanes + i);
-  const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
-  const int4 ec = __ldg(m.ecell4 + e);   // cells and their layer ranges in one load
-  const unsigned tr = unsigned(ec.z);
-  const double* cr = m.cross + 4 * int64_t(e);
-  double t1 = 0.0, t2 = 0.0;
-  if (in_range(k, tr & 0xffffu)) {
-    const uint32_t q = lq(ec.x, L, k);
-    const double2 U = __ldg(reinterpret_cast<const double2*>(in.uv) + q);
-    t1 = (U.x * ld(cr + 1) - U.y * ld(cr + 0)) * ld(in.helem + q);
+  const int64_t count = m.n_edge;
+  if (i >= count) return;
+  const int L = m.L;
+  const double2* uv = reinterpret_cast<const double2*>(in.uv);
+  uint32_t lane = ld(m.edge_lanes + i);
+  uint32_t lane1 = i + stride < count ? ld(m.edge_lanes + i + stride) : lane;
+  int4 ec = __ldg(m.ecell4 + lane_ent(lane));   // cells and their layer ranges in one load
+  for (; i < count; i += stride) {
+    const int e = lane_ent(lane), k = lane_lev(lane);
+    const unsigned tr = unsigned(ec.z);
+    const bool on1 = in_range(k, tr & 0xffffu);
+    const bool on2 = ((tr >> 16) & 255u) != kNoCell && in_range(k, tr >> 16);
+    const double2* cr = reinterpret_cast<const double2*>(m.cross + 4 * int64_t(e));
+    const double2 c1 = __ldg(cr), c2 = __ldg(cr + 1);
+    double2 U1 = make_double2(0.0, 0.0), U2 = U1;
+    double h1 = 0.0, h2 = 0.0;
+    if (on1) {
+      const uint32_t q = lq(ec.x, L, k);
+      U1 = __ldg(uv + q);
+      h1 = ld(in.helem + q);
+    }
+    if (on2) {
+      const uint32_t q = lq(ec.y, L, k);
+      U2 = __ldg(uv + q);
+      h2 = ld(in.helem + q);
+    }
+    lane = lane1;
+    ec = __ldg(m.ecell4 + lane_ent(lane));
+    lane1 = i + 2 * stride < count ? ld(m.edge_lanes + i + 2 * stride) : lane;
+    const double t1 = on1 ? (U1.x * c1.y - U1.y * c1.x) * h1 : 0.0;
+    const double t2 = on2 ? (U2.y * c2.x - U2.x * c2.y) * h2 : 0.0;
+    in.ws.vflux[lq(e, L, k)] = t1 + t2;
   }
-  if (((tr >> 16) & 255u) != kNoCell && in_range(k, tr >> 16)) {
-    const uint32_t q = lq(ec.y, L, k);
-    const double2 U = __ldg(reinterpret_cast<const double2*>(in.uv) + q);
-    t2 = (U.y * ld(cr + 2) - U.x * ld(cr + 3)) * ld(in.helem + q);
-  }
-  in.ws.vflux[lq(e, L, k)] = t1 + t2;
 }
 
 template <int NTR, bool IL>
@@ -242,52 +260,66 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
 }
 
 // -------------------------- fill_up_dn_grad + adv_flux_hor_ho - LO flux = adf_h
+// -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2) is exactly -0.5 times the upwind end's term (the
+// other one is 0), so only that end's gradient is read. A thread walks the lanes i, i + stride,
+// ...: the next lane's record, volume flux and cells are loaded while this lane's gathers are
+// under way.
 template <int NTR, bool IL>
-__device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int t0, int w0) {
+__device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t stride, int t0,
+                                              int w0) {
   const DevMesh& m = in.m;
-  if (i >= m.n_edge) return;
-  const int4 rec = __ldg(m.edge4 + i);
-  const int e = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x)), L = m.L;
-  const int n1 = rec.y, n2 = rec.z;
-  const bool use_tri = in_range(k, unsigned(rec.w));
-  const double vf = ld(in.ws.vflux + lq(e, L, k));
-  const double avf = fabs(vf);
-  const double c1 = ld(m.ecoef + 2 * e), c2 = ld(m.ecoef + 2 * e + 1);
-  const uint32_t q1 = lq(n1, L, k), q2 = lq(n2, L, k);
+  const int64_t count = m.n_edge;
+  if (i >= count) return;
+  const int L = m.L;
   const int64_t ts = in.tstride;
   const int tg = in.tg;
-  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[NTR], gy[NTR];
-  ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
-  ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
-  ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
-  ldn<NTR, IL>(in.T_old, q2, t0, ts, tg, O2);
-  // -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2) is exactly -0.5 times the upwind end's term (the
-  // other one is 0), so only that end's gradient is read
-  const bool first = vf > 0.0;
-  if (use_tri) {
-    // both cells are wet at k here (k is above every adjacent cell's bottom)
-    const uint32_t q = lq(ld(m.eupdn + 2 * e + (first ? 0 : 1)), L, k);
-    ldn<NTR, IL>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
-    ldn<NTR, IL>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
-  } else {
-    const uint32_t q = first ? q1 : q2;
-    ldn<NTR, IL>(in.ws.gnx, q, w0, in.ws.sN, in.wtg, gx);
-    ldn<NTR, IL>(in.ws.gny, q, w0, in.ws.sN, in.wtg, gy);
-  }
-  double adf[NTR];
-  const Rcp r6{6.0, 1.0 / 6.0, true};
-  const double cu = first ? vf + avf : vf - avf;
+  const int2* updn = reinterpret_cast<const int2*>(m.eupdn);
+  const double2* coef = reinterpret_cast<const double2*>(m.ecoef);
+  int4 rec = __ldg(m.edge4 + i);
+  int4 rec1 = i + stride < count ? __ldg(m.edge4 + i + stride) : rec;
+  double vf1 = ld(in.ws.vflux + lq(lane_ent(uint32_t(rec.x)), L, lane_lev(uint32_t(rec.x))));
+  int2 ud1 = __ldg(updn + lane_ent(uint32_t(rec.x)));
+  for (; i < count; i += stride) {
+    const int e = lane_ent(uint32_t(rec.x)), k = lane_lev(uint32_t(rec.x));
+    const bool use_tri = in_range(k, unsigned(rec.w));
+    const double vf = vf1, avf = fabs(vf);
+    const uint32_t q1 = lq(rec.y, L, k), q2 = lq(rec.z, L, k);
+    const bool first = vf > 0.0;
+    double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[NTR], gy[NTR];
+    ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
+    ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
+    ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
+    ldn<NTR, IL>(in.T_old, q2, t0, ts, tg, O2);
+    if (use_tri) {
+      // both cells are wet at k here (k is above every adjacent cell's bottom)
+      const uint32_t q = lq(first ? ud1.x : ud1.y, L, k);
+      ldn<NTR, IL>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
+      ldn<NTR, IL>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
+    } else {
+      const uint32_t q = first ? q1 : q2;
+      ldn<NTR, IL>(in.ws.gnx, q, w0, in.ws.sN, in.wtg, gx);
+      ldn<NTR, IL>(in.ws.gny, q, w0, in.ws.sN, in.wtg, gy);
+    }
+    const double2 c = __ldg(coef + e);
+    rec = rec1;
+    vf1 = ld(in.ws.vflux + lq(lane_ent(uint32_t(rec.x)), L, lane_lev(uint32_t(rec.x))));
+    ud1 = __ldg(updn + lane_ent(uint32_t(rec.x)));
+    rec1 = i + 2 * stride < count ? __ldg(m.edge4 + i + 2 * stride) : rec;
+    double adf[NTR];
+    const Rcp r6{6.0, 1.0 / 6.0, true};
+    const double cu = first ? vf + avf : vf - avf;
 #pragma unroll
-  for (int t = 0; t < NTR; ++t) {
-    const double fl = -0.5 * (T1[t] * (vf + avf) + T2[t] * (vf - avf));
-    const double A1 = ab2(T1[t], O1[t]), A2 = ab2(T2[t], O2[t]);
-    const double diff = A2 - A1;
-    const double X = divr(2.0 * diff + c1 * gx[t] + c2 * gy[t], r6);
-    const double Tm = first ? A1 + X : A2 - X;
-    const double ho = -0.5 * (cu * Tm);
-    adf[t] = ho - fl;
+    for (int t = 0; t < NTR; ++t) {
+      const double fl = -0.5 * (T1[t] * (vf + avf) + T2[t] * (vf - avf));
+      const double A1 = ab2(T1[t], O1[t]), A2 = ab2(T2[t], O2[t]);
+      const double diff = A2 - A1;
+      const double X = divr(2.0 * diff + c.x * gx[t] + c.y * gy[t], r6);
+      const double Tm = first ? A1 + X : A2 - X;
+      const double ho = -0.5 * (cu * Tm);
+      adf[t] = ho - fl;
+    }
+    stn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);
   }
-  stn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);
 }
 
 // ------------------------ zalesak a2: element max/min of the LO/T window
@@ -554,19 +586,6 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
   count_nonfinite<NTR>(in.nonfinite, out);
 }
 
-// ------------------------------------------- dry levels keep T (ale_reconstruct)
-template <bool IL>
-__device__ __forceinline__ void body_copy_dry(const Inst& in, int64_t i) {
-  const DevMesh& m = in.m;
-  if (i >= m.n_dry) return;
-  const uint32_t lane = __ldg(m.dry_lanes + i);
-  const uint32_t q = lq(lane_ent(lane), m.L, lane_lev(lane));
-  for (int t = 0; t < in.ntr; ++t) {
-    const int64_t a = tix<IL>(q, t, in.tstride, in.tg);
-    in.T_new[a] = in.T[a];
-  }
-}
-
 // Kernel wrappers: ``_1`` takes one instance by value (tracer-major layout, the
 // single-call path); ``_n`` reads instance blockIdx.y of a device table (interleaved
 // layout, the batched path). A launch covers S = 2^lg tracer slices of NTR tracers each:
@@ -577,11 +596,8 @@ __device__ __forceinline__ void body_copy_dry(const Inst& in, int64_t i) {
 // accordingly): latency hiding pays more than the spills it costs (one tracer, the
 // adjoint's taped forward on the CORE2-size mesh: 11.1 ms for 10 steps at 6 blocks,
 // 10.6 ms at 7, no gain at 8).
-#ifndef FCT_KMB
-#define FCT_KMB 7
-#endif
 template <int NTR>
-constexpr int kMinBlocks = NTR == 1 ? FCT_KMB : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
+constexpr int kMinBlocks = NTR == 1 ? 7 : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
 
 #define FCT_KERNEL_T(name, body)                                                        \
   template <int NTR>                                                                    \
@@ -603,36 +619,46 @@ constexpr int kMinBlocks = NTR == 1 ? FCT_KMB : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
 // unfused stages (every intermediate in the workspace; the reverse pass reads them)
 FCT_KERNEL_T(k_elem_grad, body_elem_grad)
 FCT_KERNEL_T(k_node_lo, body_node_lo)
-FCT_KERNEL_T(k_edge_adf, body_edge_adf)
+// (a walk over the edge lanes)
+template <int NTR>
+constexpr int kWalkBlocks = NTR == 1 ? 5 : NTR == 2 ? 4 : NTR == 4 ? 2 : 1;
+template <int NTR>
+__global__ void __launch_bounds__(256, kWalkBlocks<NTR>) k_edge_adf_1(
+    const __grid_constant__ Inst in, int t0, int w0) {
+  const int sub = int(blockIdx.y) * NTR;
+  body_edge_adf<NTR, false>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub);
+}
 FCT_KERNEL_T(k_elem_bounds, body_elem_bounds)
 FCT_KERNEL_T(k_node_cluster, body_node_cluster)
 FCT_KERNEL_T(k_node_factors, body_node_factors)
 FCT_KERNEL_T(k_node_final, body_node_final)
 
-// column solves (fct_columns.cuh): blockIdx.y the instance (batched), blockIdx.z the group of
-// at most ``group`` tracers
+// column solves (fct_columns.cuh) of NT tracers: blockIdx.y the instance (batched)
 #define FCT_KERNEL_COL(name, block_body)                                                 \
+  template <int NT>                                                                      \
   __global__ void __launch_bounds__(kColThreads) name##_1(                               \
-      const __grid_constant__ Inst in, int columns, int t0, int nt, int group) {         \
+      const __grid_constant__ Inst in, int columns, int t0) {                            \
     extern __shared__ double col_sh[];                                                   \
-    const int g = int(blockIdx.z) * group;                                               \
-    block_body<false>(in, int(blockIdx.x) * columns, columns, t0 + g, min(group, nt - g), \
-                      col_sh);                                                           \
+    block_body<NT, false>(in, int(blockIdx.x) * columns, columns, t0, col_sh);           \
   }                                                                                      \
+  template <int NT>                                                                      \
   __global__ void __launch_bounds__(kColThreads) name##_n(                               \
-      const Inst* __restrict__ tab, int columns, int t0, int nt, int group) {            \
+      const Inst* __restrict__ tab, int columns, int t0) {                               \
     extern __shared__ double col_sh[];                                                   \
-    const int g = int(blockIdx.z) * group;                                               \
-    block_body<true>(tab[blockIdx.y], int(blockIdx.x) * columns, columns, t0 + g,        \
-                     min(group, nt - g), col_sh);                                        \
+    block_body<NT, true>(tab[blockIdx.y], int(blockIdx.x) * columns, columns, t0, col_sh); \
   }
 // implicit vertical diffusion (the epilogue of the batched step and fct_vert_diff)
 FCT_KERNEL_COL(k_vdiff, block_vdiff)
 FCT_KERNEL_COL(k_vert_impl, block_vert_impl)
 
-__global__ void __launch_bounds__(256) k_vflux_1(const __grid_constant__ Inst in) { body_vflux(in, lane_index()); }
-__global__ void __launch_bounds__(256) k_vflux_n(const Inst* __restrict__ tab) {
-  body_vflux(tab[blockIdx.y], lane_index());
+constexpr int kVfluxBlocks = 5;
+__global__ void __launch_bounds__(256, kVfluxBlocks) k_vflux_1(const __grid_constant__ Inst in) {
+  body_vflux(in, lane_index(), int64_t(gridDim.x) * 256);
+}
+__global__ void __launch_bounds__(256, kVfluxBlocks) k_vflux_n(const Inst* __restrict__ tab,
+                                                               int n) {
+  for (int i = int(blockIdx.y); i < n; i += int(gridDim.y))
+    body_vflux(tab[i], lane_index(), int64_t(gridDim.x) * 256);
 }
 __global__ void __launch_bounds__(256) k_copy_dry_1(const __grid_constant__ Inst in) {
   body_copy_dry<false>(in, lane_index());
@@ -677,6 +703,10 @@ const char* const kStageNames[kNumStages] = {
     }                                                                                   \
   } while (0)
 #define FCT_STAGE(name, lanes) FCT_SPLIT(FCT_STAGE_AS, name, lanes)
+// a stage whose threads walk its lanes (single instances: the reverse pass's stages)
+#define FCT_WALK_AS(name, lanes, P)                                                     \
+  name##_1<P><<<dim3(unsigned(std::min<int64_t>(xblocks(lanes), 148 * kWalkBlocks<P>)),  \
+                     1u << lg), B, 0, s>>>(single, t0, w0)
 
 // the fused step's edge stage beside its LO stage when the caller provides a fork
 constexpr bool kForkEdge = true;
@@ -699,25 +729,41 @@ void fork_destroy(Fork& f) {
 
 namespace {
 
-// One column solve over ``nt`` tracers from ``t0``, all of them in one launch: up to 8 of an
-// interleaved instance share a block's matrix rows; tracer-major ones go up to 2 per block.
-template <class K1, class KN>
-int launch_columns(K1 k1, KN kn, const Inst& single, const Inst* tab, int n, int64_t nodes, int L,
-                   int t0, int nt, cudaStream_t s, const char* what) {
-  const int group = std::min(nt, tab ? 8 : 2);
-  const int columns = col_columns(L, group);
-  const size_t sh = col_smem(columns, L, group);
-  cudaError_t e = cudaSuccess;
-  // the opt-in limit is the same value every time, so concurrent callers do not disturb it
-  if (sh > size_t(48) << 10)
-    e = tab ? cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, kColMaxSmem)
-            : cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, kColMaxSmem);
-  if (e != cudaSuccess) return cuda_error(e, what);
-  const dim3 g(unsigned(std::max<int64_t>(1, (nodes + columns - 1) / columns)),
-               tab ? unsigned(n) : 1u, unsigned((nt + group - 1) / group));
-  if (tab) kn<<<g, kColThreads, sh, s>>>(tab, columns, t0, nt, group);
-  else k1<<<g, kColThreads, sh, s>>>(single, columns, t0, nt, group);
-  e = cudaGetLastError();
+using ColKernel1 = void (*)(Inst, int, int);
+using ColKernelN = void (*)(const Inst*, int, int);
+struct ColKernels {
+  ColKernel1 one[kColMaxTracers];
+  ColKernelN many[kColMaxTracers];
+};
+#define FCT_COL_TABLE(name)                                                              \
+  ColKernels{{name##_1<1>, name##_1<2>, name##_1<3>, name##_1<4>, name##_1<5>, name##_1<6>, \
+              name##_1<7>, name##_1<8>},                                                 \
+             {name##_n<1>, name##_n<2>, name##_n<3>, name##_n<4>, name##_n<5>, name##_n<6>, \
+              name##_n<7>, name##_n<8>}}
+
+// One column solve over the tracers [t0, t0 + nt): launches of up to kColMaxTracers tracers,
+// which share a block's matrix rows.
+int launch_columns(const ColKernels& K, const Inst& single, const Inst* tab, int n, int64_t nodes,
+                   int L, int t0, int nt, cudaStream_t s, const char* what) {
+  for (int t = t0; t < t0 + nt;) {
+    const int g = std::min(t0 + nt - t, kColMaxTracers);
+    const int columns = col_columns(L, g);
+    const size_t sh = col_smem(columns, L, g);
+    cudaError_t e = cudaSuccess;
+    // the opt-in limit is the same value every time, so concurrent callers do not disturb it
+    if (sh > size_t(48) << 10)
+      e = tab ? cudaFuncSetAttribute(K.many[g - 1], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kColMaxSmem)
+              : cudaFuncSetAttribute(K.one[g - 1], cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     kColMaxSmem);
+    if (e != cudaSuccess) return cuda_error(e, what);
+    const dim3 grid(unsigned(std::max<int64_t>(1, (nodes + columns - 1) / columns)),
+                    tab ? unsigned(n) : 1u);
+    if (tab) K.many[g - 1]<<<grid, kColThreads, sh, s>>>(tab, columns, t);
+    else K.one[g - 1]<<<grid, kColThreads, sh, s>>>(single, columns, t);
+    t += g;
+  }
+  const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? FCT_OK : cuda_error(e, what);
 }
 
@@ -735,8 +781,10 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
   const int nchunks = (d.ntr + chunk - 1) / chunk;
   // the dry-level copy on the side stream, beside the stages (190 of 9,200 us of a step of
   // 300,000 nodes x 70 levels x 4 tracers when it ran after them)
-  const bool dry_aside = d.fused && kForkEdge && d.fork && !after && d.copy_dry &&
-                         !stop_before_final && !d.any_vdiff && chunk_sel < 0;
+  const bool dry_early = d.fused && !after && d.copy_dry && !stop_before_final &&
+                         !d.any_vdiff && chunk_sel < 0;
+  const bool dry_first = dry_early && !tab && seg_first_fits(d, 0, std::min(chunk, d.ntr));
+  const bool dry_aside = dry_early && !dry_first && kForkEdge && d.fork;
   for (int ci = 0; ci < nchunks; ++ci) {
     if (chunk_sel >= 0 && ci != chunk_sel) continue;
     const int c0 = ci * chunk, c1 = std::min(d.ntr, c0 + chunk);
@@ -751,8 +799,9 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
         if (st) return st;
       }
       if (!d.skip_vflux) {
-        if (tab) k_vflux_n<<<grid(d.max_edge), B, 0, s>>>(tab);
-        else k_vflux_1<<<grid(d.max_edge), B, 0, s>>>(single);
+        const dim3 g = stream_grid(xblocks(d.max_edge), int64_t(148) * kVfluxBlocks, n);
+        if (tab) k_vflux_n<<<g, B, 0, s>>>(tab, n);
+        else k_vflux_1<<<g, B, 0, s>>>(single);
       }
     }
     mark();
@@ -762,9 +811,14 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
       // where MFCT needs them, in the edge stage; elem_bounds and node_cluster: the factors
       // stage). With a fork (and no stage timing) the edge stage runs on the side stream
       // beside the LO stage and the limiter waits for both.
-      const Fork* fk = (kForkEdge && d.fork && !after) ? d.fork : nullptr;
+      // A small single instance takes all of these in one launch (launch_seg_first).
+      const bool first = !tab && !after && seg_first_fits(d, c0, c1);
+      const Fork* fk = (kForkEdge && d.fork && !after && !first) ? d.fork : nullptr;
       mark();
       int st;
+      if (first) {
+        if ((st = launch_seg_first(single, d, c0, c1, dry_first && ci == 0, s))) return st;
+      }
       if (fk) {
         FCT_CUDA(cudaEventRecord(fk->ev[0], s));
         FCT_CUDA(cudaStreamWaitEvent(fk->side, fk->ev[0], 0));
@@ -777,16 +831,16 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
           FCT_CUDA(cudaEventRecord(fk->ev[2], fk->side));
         }
       }
-      if ((st = launch_seg_lo(single, tab, n, d, c0, c1, s))) return st;
+      if (!first && (st = launch_seg_lo(single, tab, n, d, c0, c1, s))) return st;
       mark();
-      if (d.any_wi && (st = launch_columns(k_vert_impl_1, k_vert_impl_n, single, tab, n,
+      if (d.any_wi && (st = launch_columns(FCT_COL_TABLE(k_vert_impl), single, tab, n,
                                            d.max_nodes, d.max_levels, 0, c1 - c0, s,
                                            "split vertical velocity launch")))
         return st;
       mark();
       if (fk) {
         FCT_CUDA(cudaStreamWaitEvent(s, fk->ev[1], 0));
-      } else {
+      } else if (!first) {
         if ((st = launch_seg_edge(single, tab, n, d, c0, c1, s))) return st;
         if ((st = launch_edge_fix(single, tab, n, d, c0, c1, s))) return st;
       }
@@ -802,7 +856,7 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
           if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, s>>>(tab);
           else k_copy_dry_1<<<grid(d.max_dry), B, 0, s>>>(single);
         }
-        if ((st = launch_columns(k_vdiff_1, k_vdiff_n, single, tab, n, d.max_nodes, d.max_levels,
+        if ((st = launch_columns(FCT_COL_TABLE(k_vdiff), single, tab, n, d.max_nodes, d.max_levels,
                                  c0, c1 - c0, s, "vertical diffusion launch")))
           return st;
       }
@@ -814,13 +868,13 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
     FCT_STAGE(k_node_lo, d.max_iface);
     mark();
     if (d.any_wi) {
-      const int st = launch_columns(k_vert_impl_1, k_vert_impl_n, single, tab, n, d.max_nodes,
+      const int st = launch_columns(FCT_COL_TABLE(k_vert_impl), single, tab, n, d.max_nodes,
                                     d.max_levels, 0, c1 - c0, s,
                                     "split vertical velocity launch");
       if (st) return st;
     }
     mark();
-    FCT_STAGE(k_edge_adf, d.max_edge);
+    FCT_SPLIT(FCT_WALK_AS, k_edge_adf, d.max_edge);
     mark();
     FCT_STAGE(k_elem_bounds, d.max_elem);
     mark();
@@ -834,7 +888,7 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
   }
   if (dry_aside) {
     FCT_CUDA(cudaStreamWaitEvent(s, d.fork->ev[2], 0));
-  } else if (d.copy_dry && !stop_before_final && (chunk_sel < 0 || chunk_sel == nchunks - 1)) {
+  } else if (!dry_first && d.copy_dry && !stop_before_final && (chunk_sel < 0 || chunk_sel == nchunks - 1)) {
     if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, s>>>(tab);
     else k_copy_dry_1<<<grid(d.max_dry), B, 0, s>>>(single);
   }
@@ -855,7 +909,7 @@ int launch_forward_stages(const Inst& single, const LaunchDims& d, cudaStream_t 
 }
 
 int launch_vdiff(const Inst& single, const LaunchDims& d, cudaStream_t s) {
-  return launch_columns(k_vdiff_1, k_vdiff_n, single, nullptr, 1, d.max_nodes, d.max_levels, 0,
+  return launch_columns(FCT_COL_TABLE(k_vdiff), single, nullptr, 1, d.max_nodes, d.max_levels, 0,
                         d.ntr, s, "vertical diffusion launch");
 }
 

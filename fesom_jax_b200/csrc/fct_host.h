@@ -25,6 +25,11 @@ inline int cuda_error(cudaError_t e, const char* what) {
     if (e_ != cudaSuccess) return ::fct::cuda_error(e_, #call); \
   } while (0)
 
+// most blocks of the one launch of a small instance's first stages: eight waves of two blocks on
+// every SM (pi, T and S, 6 waves: 46.5 us a step against 50.9 with a launch per stage; 600 nodes
+// 33.8 against 46.1; 20,000 nodes x 3 tracers, 44 waves, no difference)
+constexpr int64_t kFirstBlocks = 8 * 2 * 148;
+
 // fused stages with their own thread mapping: LO, edge, limiter, final
 constexpr int kFusedStages = 4;
 enum { kStageLo = 0, kStageEdge = 1, kStageLimit = 2, kStageFinal = 3 };
@@ -59,16 +64,22 @@ struct LaunchDims {
       smap_levels[i] = levels;
     }
   }
-  // The mapping of a plan or batch that was given none: one level per thread (the stream
-  // kernels; runs of two or more levels per thread spread a warp's loads over twice the lines
-  // or more) and two tracers. Interleaved instances of 4 tracers or more take 4 per thread,
-  // and the run kernel at 2 x 2 in the final stage (fct_seg_final.cu), if that still leaves
-  // ``threads`` (wet node layers x tracers of the launch / 4) for two blocks on every SM.
-  void auto_map(bool interleaved, int64_t threads) {
+  // The mapping of a plan or batch that was given none. Tracer-major: two tracers and one level
+  // per thread everywhere (the stream kernels; runs of two or more levels per thread spread a
+  // warp's loads over twice the lines or more). Interleaved, from sweeps over 8 tracers of two
+  // CORE2-size members: the final stage's run kernel at two levels (1.08 ms, stream 1.14); 4
+  // tracers per thread in the others where ``threads`` (wet node layers x tracers of the launch
+  // / 4) leaves two blocks for every SM (LO 0.76 ms against 0.90 at 2 tracers, edge 0.66 / 0.80,
+  // limiter 1.25 / 1.37); odd tracer counts, whose loads are single values, the run kernels at
+  // two levels except in the edge stage (LO 1.21 against 1.54, limiter 1.68 / 1.75).
+  void auto_map(bool interleaved, bool even, int64_t threads) {
     set_map(2, 1);
-    if (interleaved && ntr >= 4 && threads >= int64_t(148) * 2 * 256) {
+    if (!interleaved) return;
+    smap_levels[kStageFinal] = 2;
+    if (!even) {
+      smap_levels[kStageLo] = smap_levels[kStageLimit] = 2;
+    } else if (ntr >= 4 && threads >= int64_t(148) * 2 * 256) {
       for (int i : {kStageLo, kStageEdge, kStageLimit}) smap_tracers[i] = 4;
-      smap_levels[kStageFinal] = 2;
     }
   }
   int64_t max_nseg[kSegVariants] = {0, 0, 0, 0};
@@ -103,7 +114,20 @@ inline void dims_cover(LaunchDims& d, const FctPlan* P) {
 // The mapping of a single-plan launch: the plan's own, or the rule's.
 inline void dims_map(LaunchDims& d, const FctPlan* P) {
   if (P->per_thread > 0) d.set_map(P->per_thread, P->lpt);
-  else d.auto_map(false, 0);
+  else d.auto_map(false, true, 0);
+}
+
+// Grid of a kernel whose threads walk its lanes, for ``n`` instances of at most ``need`` blocks
+// when ``full`` blocks are resident at once. Large instances go one after the other, so that
+// the gathers of all blocks stay within a few columns of each other; where one gives a thread
+// fewer than kWalk lanes they go side by side (grid.y), with as many blocks each as fill the
+// chip together (16 pi-size members x 30 steps: 17.3 ms one after the other, 14.8 with every
+// block of every instance in the grid and no walk, 12.8 so).
+constexpr int kWalk = 4;
+inline dim3 stream_grid(int64_t need, int64_t full, int n) {
+  if (need >= kWalk * full) return dim3(unsigned(full), 1);
+  const int64_t x = std::max<int64_t>(1, std::min(need, (full + n - 1) / n));
+  return dim3(unsigned(x), unsigned(n));
 }
 
 // Tracers per thread and tracer slices of one segment launch over ``rem`` tracers: the
@@ -146,6 +170,23 @@ int launch_seg_limit(const Inst& single, const Inst* tab, int n, const LaunchDim
                      int c1, cudaStream_t s);
 int launch_seg_final(const Inst& single, const Inst* tab, int n, const LaunchDims& d, int c0,
                      int c1, cudaStream_t s);
+// The LO stage, the edge stage with its remaining lanes and (``dry``) the dry-level copy of a
+// single instance in one launch, where all their blocks are resident at once (seg_first_fits):
+// they depend only on the volume fluxes, and on a small mesh each of them is shorter than the
+// gap between two launches (fct_seg_first.cu).
+int launch_seg_first(const Inst& single, const LaunchDims& d, int c0, int c1, bool dry,
+                     cudaStream_t s);
+inline int64_t seg_first_blocks(const LaunchDims& d, int tracers_per_thread, int rem) {
+  const int64_t slices = rem / tracers_per_thread;
+  auto blocks = [](int64_t threads) { return (threads + 255) / 256; };
+  return (blocks(d.max_nseg[0]) + blocks(d.max_eseg[0]) + blocks(d.max_efix * 2)) * slices;
+}
+inline bool seg_first_fits(const LaunchDims& d, int c0, int c1) {
+  const SegSplit sp = seg_split(c1 - c0, d.smap_tracers[kStageLo], false, false);
+  return d.smap_levels[kStageLo] == 1 && d.smap_levels[kStageEdge] == 1 &&
+         d.smap_tracers[kStageEdge] == d.smap_tracers[kStageLo] &&
+         seg_first_blocks(d, sp.tracers, c1 - c0) <= kFirstBlocks;
+}
 int launch_forward(const Inst& single, const Inst* tab, int n, const LaunchDims& d,
                    cudaStream_t s);
 // Same, recording ``after[i]`` on ``s`` after stage i of a chunk (skipped stages record

@@ -157,6 +157,9 @@ struct DevMesh {
   const int4* ns4;
   // sea-ice tables: 1 / surface area (safe), cell area / 12, sqrt(cell area / 2e8)
   const double *iarea0, *earea12, *ediff;
+  // per node->edge slot of compute_w: {first cell * L, second cell * L (dense offsets), the
+  // cells' layer ranges (pack_tri), 2*edge + (node is the edge's second node)}
+  const int4* nw4;
   const double* iavol;   // [N,L] 1 / areasvol, correctly rounded (0 where areasvol is 0)
   // [5,L] QR4C stencil of interface k on the static depths: the reciprocals of Z[k-1]-Z[k],
   // Z[k]-Z[k+1], Z[k-2]-Z[k-1], then (zbar[k]-Z[k])/3, (zbar[k]-Z[k-1])/3 (k >= 2)

@@ -351,6 +351,12 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
     ns4[j] = make_int4(int(uint32_t(ne_idx[j] >> 1) * uint32_t(L)),
                        int(uint32_t(ne_oth[j]) * uint32_t(L)),
                        (ne_idx[j] & 1) ? int(0x80000000u) : 0, 0);
+  std::vector<int4> nw4(2 * size_t(Ed));
+  for (size_t j = 0; j < nw4.size(); ++j) {
+    const int e = ne_idx[j] >> 1, el1 = d->edge_tri[2 * e], el2 = d->edge_tri[2 * e + 1];
+    nw4[j] = make_int4(int(uint32_t(el1) * uint32_t(L)),
+                       int(uint32_t(el2 >= 0 ? el2 : 0) * uint32_t(L)), ne4[j].w, ne_idx[j]);
+  }
   std::vector<double> iavol(size_t(N) * L), qr4c(5 * size_t(L), 0.0);
   for (size_t i = 0; i < iavol.size(); ++i)
     iavol[i] = d->areasvol[i] > 0.0 ? 1.0 / d->areasvol[i] : 0.0;
@@ -560,7 +566,7 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   size_t o_ecell4 = b.add(ecell4.data(), ecell4.size());
   size_t o_nrec = b.add(nrec.data(), nrec.size()), o_erec = b.add(erec.data(), erec.size());
   size_t o_ns4 = b.add(ns4.data(), ns4.size()), o_iavol = b.add(iavol.data(), iavol.size());
-  size_t o_qr4c = b.add(qr4c.data(), qr4c.size());
+  size_t o_qr4c = b.add(qr4c.data(), qr4c.size()), o_nw4 = b.add(nw4.data(), nw4.size());
   size_t o_iarea0 = b.add(iarea0.data(), N), o_earea12 = b.add(earea12.data(), E);
   size_t o_ediff = b.add(ediff.data(), E);
   size_t o_emf4 = b.add(emf4.data(), emf4.size()), o_emfw = b.add(emfw.data(), emfw.size());
@@ -634,6 +640,7 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   m.ns4 = (const int4*)(base + o_ns4);
   m.iavol = (const double*)(base + o_iavol);
   m.qr4c = (const double*)(base + o_qr4c);
+  m.nw4 = (const int4*)(base + o_nw4);
   m.iarea0 = (const double*)(base + o_iarea0);
   m.earea12 = (const double*)(base + o_earea12);
   m.ediff = (const double*)(base + o_ediff);

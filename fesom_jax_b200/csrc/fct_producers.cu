@@ -39,26 +39,29 @@ __device__ __forceinline__ void compute_w_columns(const DevMesh& m, const double
       continue;   // no edge has the level
     const int e1 = rec.x + int((pk >> 16) & 255u);
     double div = 0.0;
+#pragma unroll 2
     for (int j = rec.x; j < e1; ++j) {
-      const int4 sl = __ldg(m.ne4 + j);
-      const unsigned rg = unsigned(sl.z), tr = unsigned(sl.w);
-      if (k < int(rg & 255u) || k >= int((rg >> 8) & 255u)) continue;
-      const int e = sl.x >> 1;
-      const int4 ec = __ldg(m.ecell4 + e);
-      const double2* cr = reinterpret_cast<const double2*>(m.cross + 4 * int64_t(e));
-      double t1 = 0.0, t2 = 0.0;
-      if (k >= int(tr & 255u) && k < int((tr >> 8) & 255u)) {
-        const uint32_t q = lq(ec.x, L, k);
-        const double2 U = __ldg(uv2 + q), x = __ldg(cr);
-        t1 = (U.y * x.x - U.x * x.y) * __ldg(helem + q);
+      const int4 sl = __ldg(m.nw4 + j);
+      const unsigned tr = unsigned(sl.z);
+      const bool on1 = k >= int(tr & 255u) && k < int((tr >> 8) & 255u);
+      const bool on2 = ((tr >> 16) & 255u) != kNoCell && k >= int((tr >> 16) & 255u) &&
+                       k < int(tr >> 24);
+      const double2* cr = reinterpret_cast<const double2*>(m.cross + 4 * int64_t(sl.w >> 1));
+      const double2 x1 = __ldg(cr), x2 = __ldg(cr + 1);
+      double2 U1 = make_double2(0.0, 0.0), U2 = U1;
+      double h1 = 0.0, h2 = 0.0;
+      if (on1) {
+        U1 = __ldg(uv2 + (uint32_t(sl.x) + uint32_t(k)));
+        h1 = __ldg(helem + (uint32_t(sl.x) + uint32_t(k)));
       }
-      if (((tr >> 16) & 255u) != kNoCell && k >= int((tr >> 16) & 255u) && k < int(tr >> 24)) {
-        const uint32_t q = lq(ec.y, L, k);
-        const double2 U = __ldg(uv2 + q), x = __ldg(cr + 1);
-        t2 = (U.y * x.x - U.x * x.y) * __ldg(helem + q);
+      if (on2) {
+        U2 = __ldg(uv2 + (uint32_t(sl.y) + uint32_t(k)));
+        h2 = __ldg(helem + (uint32_t(sl.y) + uint32_t(k)));
       }
+      const double t1 = on1 ? (U1.y * x1.x - U1.x * x1.y) * h1 : 0.0;
+      const double t2 = on2 ? (U2.y * x2.x - U2.x * x2.y) * h2 : 0.0;
       const double c = t1 - t2;
-      div += (sl.x & 1) ? -c : c;
+      if (on1 || on2) div += (sl.w & 1) ? -c : c;
     }
     sh[col * stride + k] = div;
   }

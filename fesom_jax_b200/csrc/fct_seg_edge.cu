@@ -7,19 +7,20 @@ namespace {
 
 FCT_SEG_KERNEL(k_seg_edge, seg_edge_adf, kStageEdge)
 
-// the remaining edge lanes: one lane per thread (tracer slices as in the segment kernels)
+// the remaining edge lanes: kFixThreads threads per lane (and slice of NTR tracers)
 template <int NTR>
-__global__ void __launch_bounds__(256) k_edge_fix_1(const __grid_constant__ Inst in, int t0, int w0) {
+__global__ void __launch_bounds__(256) k_edge_fix_1(const __grid_constant__ Inst in, int t0,
+                                                    int w0) {
   const int sub = int(blockIdx.y) * NTR;
-  body_edge_fix<NTR, false>(in, lane_index(), t0 + sub, w0 + sub);
+  body_edge_fix<NTR, false>(in, lane_index() / kFixThreads, int(threadIdx.x) % kFixThreads,
+                            t0 + sub, w0 + sub);
 }
 template <int NTR>
 __global__ void __launch_bounds__(256) k_edge_fix_n(const Inst* __restrict__ tab, int t0, int w0,
-                                                    int S, unsigned mul) {
-  const int slots = slice_div(256, mul), slot = slice_div(int(threadIdx.x), mul);
-  if (slot >= slots) return;
-  const int sub = (int(threadIdx.x) - slot * S) * NTR;
-  body_edge_fix<NTR, true>(tab[blockIdx.y], int64_t(blockIdx.x) * slots + slot, t0 + sub,
+                                                    int S) {
+  const unsigned q = unsigned(lane_index() / kFixThreads), lane = q / unsigned(S);
+  const int sub = int(q - lane * unsigned(S)) * NTR;
+  body_edge_fix<NTR, true>(tab[blockIdx.y], lane, int(threadIdx.x) % kFixThreads, t0 + sub,
                            w0 + sub);
 }
 
@@ -29,17 +30,16 @@ int launch_edge_fix(const Inst& single, const Inst* tab, int n, const LaunchDims
                     int c1, cudaStream_t s) {
   if (d.max_efix == 0) return FCT_OK;
   for (int t0 = c0; t0 < c1;) {
-    const SegSplit sp =
-        seg_split(c1 - t0, d.smap_tracers[kStageEdge], tab != nullptr, seg_even(d));
+    // two tracers per thread at most: the lanes are few, and a thread's chain is what counts
+    const SegSplit sp = seg_split(c1 - t0, std::min(2, d.smap_tracers[kStageEdge]),
+                                  tab != nullptr, seg_even(d));
     const int P = sp.tracers, S = sp.slices, w0 = t0 - c0;
     if (tab) {
-      const unsigned mul = 65536u / unsigned(S) + 1u;
-      const dim3 g(seg_blocks(d.max_efix, 256 / S), unsigned(n));
-      if (P == 4) k_edge_fix_n<4><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);
-      else if (P == 2) k_edge_fix_n<2><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);
-      else k_edge_fix_n<1><<<g, 256, 0, s>>>(tab, t0, w0, S, mul);
+      const dim3 g(seg_blocks(d.max_efix * S, 256 / kFixThreads), unsigned(n));
+      if (P == 2) k_edge_fix_n<2><<<g, 256, 0, s>>>(tab, t0, w0, S);
+      else k_edge_fix_n<1><<<g, 256, 0, s>>>(tab, t0, w0, S);
     } else {
-      const dim3 g(seg_blocks(d.max_efix, 256), unsigned(S));
+      const dim3 g(seg_blocks(d.max_efix, 256 / kFixThreads), unsigned(S));
       if (P == 2) k_edge_fix_1<2><<<g, 256, 0, s>>>(single, t0, w0);
       else k_edge_fix_1<1><<<g, 256, 0, s>>>(single, t0, w0);
     }
@@ -51,8 +51,12 @@ int launch_edge_fix(const Inst& single, const Inst* tab, int n, const LaunchDims
 
 namespace {
 
-__host__ __device__ constexpr int edge_blocks(int ntr) { return ntr == 1 ? 5 : ntr == 2 ? 3 : 2; }
-__host__ __device__ constexpr int edge_batch(int) { return 1; }
+__host__ __device__ constexpr int edge_blocks(int ntr, bool) {
+  return ntr == 1 ? 5 : ntr == 2 ? 3 : 2;
+}
+__host__ __device__ constexpr int edge_batch(int, bool) {
+  return 1;
+}
 FCT_STREAM_KERNEL(k_edge_stream, stream_edge_adf, edge_blocks, edge_batch)
 
 #define FCT_COUNT(V) d.max_eseg[V]

@@ -11,8 +11,12 @@ FCT_SEG_KERNEL(k_seg_final, seg_node_final, kStageFinal)
 // mapping: 1 tracer 90 us against 102, T and S 155 against 179 (CORE2-size mesh); 8 tracers of
 // two members 1.15 ms against 1.08 of the run kernel at 2 x 2, which interleaved instances of 4
 // tracers or more therefore keep.
-__host__ __device__ constexpr int stream_blocks(int ntr) { return ntr == 1 ? 4 : ntr == 2 ? 2 : 1; }
-__host__ __device__ constexpr int slot_batch(int) { return 3; }
+__host__ __device__ constexpr int stream_blocks(int ntr, bool) {
+  return ntr == 1 ? 4 : ntr == 2 ? 2 : 1;
+}
+__host__ __device__ constexpr int slot_batch(int, bool) {
+  return 3;
+}
 FCT_STREAM_KERNEL(k_stream_final, stream_node_final, stream_blocks, slot_batch)
 
 #define FCT_COUNT(V) d.max_nseg[V]

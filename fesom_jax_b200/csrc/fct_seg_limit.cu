@@ -10,8 +10,12 @@ FCT_SEG_LIMIT_KERNEL(k_seg_limit)
 // Blocks per SM and slots per batch by tracers per thread, against the run kernel at its best
 // mapping: 1 tracer 123 us against 131, T and S 194 against 198 (CORE2-size mesh); 8 tracers of
 // two members, 4 per thread, 1.25 ms against 1.46.
-__host__ __device__ constexpr int stream_blocks(int ntr) { return ntr == 1 ? 3 : ntr == 2 ? 4 : 2; }
-__host__ __device__ constexpr int slot_batch(int ntr) { return ntr == 2 ? 1 : 3; }
+__host__ __device__ constexpr int stream_blocks(int ntr, bool il) {
+  return ntr == 1 ? (il ? 5 : 3) : ntr == 2 ? 4 : 2;
+}
+__host__ __device__ constexpr int slot_batch(int ntr, bool il) {
+  return ntr == 1 ? (il ? 1 : 3) : ntr == 2 ? (il ? 2 : 1) : 3;
+}
 FCT_STREAM_LIMIT_KERNEL(k_stream_limit, stream_blocks, slot_batch)
 
 #define FCT_COUNT(V) d.max_nseg[V]

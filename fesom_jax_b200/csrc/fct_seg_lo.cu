@@ -10,8 +10,12 @@ FCT_SEG_KERNEL(k_seg_lo, seg_node_lo, kStageLo)
 // Blocks per SM and slots per batch by tracers per thread, against the run kernel at its best
 // mapping: 1 tracer 84 us against 106, T and S 126 against 147 (CORE2-size mesh); 8 tracers of
 // two members, 4 per thread, 0.76 ms against 0.90.
-__host__ __device__ constexpr int stream_blocks(int ntr) { return ntr == 1 ? 4 : ntr == 2 ? 3 : 2; }
-__host__ __device__ constexpr int slot_batch(int ntr) { return ntr == 2 ? 2 : 3; }
+__host__ __device__ constexpr int stream_blocks(int ntr, bool il) {
+  return ntr == 1 ? 4 : ntr == 2 ? (il ? 2 : 3) : 2;
+}
+__host__ __device__ constexpr int slot_batch(int ntr, bool il) {
+  return ntr == 2 && !il ? 2 : 3;
+}
 FCT_STREAM_KERNEL(k_stream_lo, stream_node_lo, stream_blocks, slot_batch)
 
 #define FCT_COUNT(V) d.max_nseg[V]

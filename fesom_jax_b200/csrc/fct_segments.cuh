@@ -399,106 +399,81 @@ __device__ __forceinline__ void stream_edge_adf(const Inst& in, int64_t si, int6
   }
 }
 
-// node-average gradients of T at the two nodes n[0], n[1], level k (_node_avg_grad,
-// tracer_adv.py:329-341): the area-weighted mean over a node's cells wet at k, in the node's
-// cell order. The two nodes' cells go side by side, their records one ahead: the loop is a
-// chain of dependent loads, and one loop for both halves it.
-template <int NTR, bool IL>
-__device__ __forceinline__ void node_avg_grads(const Inst& in, int n1, int n2, int k, int t0,
-                                               double (&nx)[2][NTR], double (&ny)[2][NTR]) {
-  const DevMesh& m = in.m;
-  int c[2], left[2];
-  double den[2] = {0.0, 0.0};
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int4 rec = __ldg(m.nrec + (i == 0 ? n1 : n2));
-    c[i] = rec.y;
-    left[i] = int(unsigned(rec.z) >> 24);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) nx[i][t] = ny[i][t] = 0.0;
-  }
-  const int count = max(left[0], left[1]);
-  int4 sl[2];
-  unsigned r[2];
-  auto fetch = [&](int j) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const bool some = j < left[i];
-      r[i] = some ? unsigned(__ldg(m.nelr + c[i] + j)) : 0u;   // 0: no level
-      sl[i] = __ldg(m.nel4 + (some ? c[i] + j : 0));   // (a cell whose values are not used)
-    }
-  };
-  if (count > 0) fetch(0);
-  for (int j = 0; j < count; ++j) {
-    const int4 s0[2] = {sl[0], sl[1]};
-    const bool on[2] = {in_range(k, r[0]), in_range(k, r[1])};
-    if (j + 1 < count) fetch(j + 1);
-    double gx[2][NTR], gy[2][NTR], a[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      a[i] = __ldg(m.earea + s0[i].x);
-      cell_grad<NTR, IL>(in, s0[i].x, s0[i].y, s0[i].z, s0[i].w, k, t0, gx[i], gy[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (on[i]) {
-#pragma unroll
-        for (int t = 0; t < NTR; ++t) {
-          nx[i][t] += gx[i][t] * a[i];
-          ny[i][t] += gy[i][t] * a[i];
-        }
-        den[i] += a[i];
-      }
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const Rcp rdd = rcp(den[i] > 0.0 ? den[i] : 1.0);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) {
-      nx[i][t] = divr(nx[i][t], rdd);
-      ny[i][t] = divr(ny[i][t], rdd);
-    }
-  }
-}
-
 // ----------------------------------------------- adf_h on the remaining edge lanes
+// kFixThreads adjacent threads take one edge lane, one per end node: each forms its node's
+// average gradient (_node_avg_grad, tracer_adv.py:329-341: the mean over the node's cells wet
+// at the level, in the node's cell order; a chain of dependent loads, the cells' records one
+// ahead), and the first one combines them. (With one thread per lane the kernel held 128
+// registers; with eight per lane, one cell in four each, it took twice the time.) Where MFCT
+// takes the up/down cells although they do not hold the edge's nodes, each end has one cell.
+// ``i`` may lie beyond the list (the whole warp takes part in the shuffle).
+constexpr int kFixThreads = 2;
 template <int NTR, bool IL>
-__device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int t0, int w0) {
+__device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int g, int t0, int w0) {
   const DevMesh& m = in.m;
-  if (i >= m.n_efix) return;
-  const uint32_t lane = __ldg(m.efix + i);
+  const bool valid = i < m.n_efix;
+  const uint32_t lane = __ldg(m.efix + (valid ? i : 0));
   const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
   const int4 er = __ldg(m.erec + e);
-  const int n1 = er.x, n2 = er.y;
   const bool use_tri = in_range(k, unsigned(__ldg(m.etr + e)));
+  const int4 rec = __ldg(m.nrec + (g ? er.y : er.x));
+  const int count = use_tri ? 1 : int(unsigned(rec.z) >> 24);
+  double nx[NTR], ny[NTR], den = 0.0;
+#pragma unroll
+  for (int t = 0; t < NTR; ++t) nx[t] = ny[t] = 0.0;
+  int4 sl = make_int4(0, 0, 0, 0);
+  unsigned r = 0xffu << 8;   // every level
+  if (use_tri) {
+    sl = __ldg(m.eud4 + 2 * e + g);
+  } else if (count > 0) {
+    sl = __ldg(m.nel4 + rec.y);
+    r = unsigned(__ldg(m.nelr + rec.y));
+  }
+  for (int j = 0; j < count; ++j) {
+    const int4 c = sl;
+    const bool on = in_range(k, r);
+    if (j + 1 < count) {
+      sl = __ldg(m.nel4 + rec.y + j + 1);
+      r = unsigned(__ldg(m.nelr + rec.y + j + 1));
+    }
+    if (!on) continue;
+    const double a = use_tri ? 1.0 : __ldg(m.earea + c.x);
+    double gx[NTR], gy[NTR];
+    cell_grad<NTR, IL>(in, c.x, c.y, c.z, c.w, k, t0, gx, gy);
+#pragma unroll
+    for (int t = 0; t < NTR; ++t) {
+      nx[t] += gx[t] * a;
+      ny[t] += gy[t] * a;
+    }
+    den += a;
+  }
+  const Rcp rdd = rcp(den > 0.0 ? den : 1.0);
+  const double c1 = __ldg(m.ecoef + 2 * e), c2 = __ldg(m.ecoef + 2 * e + 1);
+  double X[NTR], Xo[NTR];   // c1 gx + c2 gy of this thread's end and of the other's
+#pragma unroll
+  for (int t = 0; t < NTR; ++t) {
+    X[t] = c1 * divr(nx[t], rdd) + c2 * divr(ny[t], rdd);
+    Xo[t] = __shfl_xor_sync(0xffffffffu, X[t], 1);
+  }
+  if (!valid || g != 0) return;
   const double vf = __ldg(in.ws.vflux + lq(e, L, k));
   const double avf = fabs(vf);
-  const double c1 = __ldg(m.ecoef + 2 * e), c2 = __ldg(m.ecoef + 2 * e + 1);
-  const uint32_t q1 = lq(n1, L, k), q2 = lq(n2, L, k);
+  const uint32_t q1 = lq(er.x, L, k), q2 = lq(er.y, L, k);
   const int64_t ts = in.tstride;
   const int tg = in.tg;
-  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[2][NTR], gy[2][NTR];
+  double T1[NTR], T2[NTR], O1[NTR], O2[NTR], adf[NTR];
   ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
   ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
   ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
   ldn<NTR, IL>(in.T_old, q2, t0, ts, tg, O2);
-  if (use_tri) {   // a mesh whose up/down cells do not hold the edge's nodes
-    const int4 cu = __ldg(m.eud4 + 2 * e), cd = __ldg(m.eud4 + 2 * e + 1);
-    cell_grad<NTR, IL>(in, cu.x, cu.y, cu.z, cu.w, k, t0, gx[0], gy[0]);
-    cell_grad<NTR, IL>(in, cd.x, cd.y, cd.z, cd.w, k, t0, gx[1], gy[1]);
-  } else {
-    node_avg_grads<NTR, IL>(in, n1, n2, k, t0, gx, gy);
-  }
-  double adf[NTR];
   const Rcp r6{6.0, 1.0 / 6.0, true};
 #pragma unroll
   for (int t = 0; t < NTR; ++t) {
     const double fl = -0.5 * (T1[t] * (vf + avf) + T2[t] * (vf - avf));
     const double A1 = ab2(T1[t], O1[t]), A2 = ab2(T2[t], O2[t]);
     const double diff = A2 - A1;
-    const double Tm1 = A1 + divr(2.0 * diff + c1 * gx[0][t] + c2 * gy[0][t], r6);
-    const double Tm2 = A2 - divr(2.0 * diff + c1 * gx[1][t] + c2 * gy[1][t], r6);
+    const double Tm1 = A1 + divr(2.0 * diff + X[t], r6);
+    const double Tm2 = A2 - divr(2.0 * diff + Xo[t], r6);
     const double ho = -0.5 * ((vf + avf) * Tm1 + (vf - avf) * Tm2);
     adf[t] = ho - fl;
   }
@@ -1309,38 +1284,37 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
   }
 
 // Kernels whose threads walk the segments (one level per thread): as many blocks as are
-// resident at once; the batched ones go through the instances one after the other, so the
-// gathers of all blocks stay within a few columns of each other.
+// resident at once (stream_grid).
 #define FCT_STREAM_KERNEL(name, body, blocks, batch)                                         \
   template <int NTR>                                                                     \
-  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+  __global__ void __launch_bounds__(256, blocks(NTR, false))                             \
       name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
     const int sub = int(blockIdx.y) * NTR;                                               \
-    body<NTR, false, batch(NTR)>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub); \
+    body<NTR, false, batch(NTR, false)>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub); \
   }                                                                                      \
   template <int NTR>                                                                     \
-  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+  __global__ void __launch_bounds__(256, blocks(NTR, true))                              \
       name##_n(const Inst* __restrict__ tab, int n, int t0, int w0, int S, unsigned mul) { \
     const int slots = slice_div(256, mul), slot = slice_div(int(threadIdx.x), mul);      \
     if (slot >= slots) return;                                                           \
     const int sub = (int(threadIdx.x) - slot * S) * NTR;                                 \
-    for (int i = 0; i < n; ++i)                                                          \
-      body<NTR, true, batch(NTR)>(tab[i], int64_t(blockIdx.x) * slots + slot,                     \
+    for (int i = int(blockIdx.y); i < n; i += int(gridDim.y))                            \
+      body<NTR, true, batch(NTR, true)>(tab[i], int64_t(blockIdx.x) * slots + slot,                     \
                          int64_t(gridDim.x) * slots, t0 + sub, w0 + sub);                \
   }
 #define FCT_STREAM_LIMIT_KERNEL(name, blocks, batch)                                         \
   template <int NTR>                                                                     \
-  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+  __global__ void __launch_bounds__(256, blocks(NTR, false))                             \
       name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
     __shared__ double sh[4 * NTR * 256];                                                 \
     const int tid = threadIdx.x, sub = int(blockIdx.y) * NTR;                            \
     const int64_t stride = int64_t(gridDim.x) * 254, b0 = int64_t(blockIdx.x) * 254;     \
     const int64_t rounds = (in.m.n_nseg[0] - b0 + stride - 1) / stride;                  \
-    stream_node_limit<NTR, false, batch(NTR)>(in, b0 + tid - 1, stride, rounds,                   \
+    stream_node_limit<NTR, false, batch(NTR, false)>(in, b0 + tid - 1, stride, rounds,                   \
                                      tid >= 1 && tid <= 254, t0 + sub, w0 + sub, tid, 1, sh); \
   }                                                                                      \
   template <int NTR>                                                                     \
-  __global__ void __launch_bounds__(256, blocks(NTR))                                    \
+  __global__ void __launch_bounds__(256, blocks(NTR, true))                              \
       name##_n(const Inst* __restrict__ tab, int n, int t0, int w0, int S, unsigned mul) { \
     __shared__ double sh[4 * NTR * 256];                                                 \
     const int tid = threadIdx.x;                                                         \
@@ -1348,9 +1322,9 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
     const int sub = slot < slots ? (tid - slot * S) * NTR : 0;                           \
     const int64_t stride = int64_t(gridDim.x) * (slots - 2);                             \
     const int64_t b0 = int64_t(blockIdx.x) * (slots - 2);                                \
-    for (int i = 0; i < n; ++i) {                                                        \
+    for (int i = int(blockIdx.y); i < n; i += int(gridDim.y)) {                          \
       const int64_t rounds = (tab[i].m.n_nseg[0] - b0 + stride - 1) / stride;            \
-      stream_node_limit<NTR, true, batch(NTR)>(tab[i], b0 + slot - 1, stride, rounds,             \
+      stream_node_limit<NTR, true, batch(NTR, true)>(tab[i], b0 + slot - 1, stride, rounds,             \
                                       slot >= 1 && slot <= slots - 2, t0 + sub, w0 + sub, \
                                       tid, S, sh);                                       \
       __syncthreads();                                                                   \
@@ -1363,10 +1337,10 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
       const SegSplit sp =                                                                \
           seg_split(c1 - t0, d.smap_tracers[STAGE], tab != nullptr, seg_even(d));        \
       const int P = sp.tracers, S = sp.slices, w0 = t0 - c0;                             \
-      const int64_t need = GRID(COUNT(0), tab ? S : 1), full = int64_t(148) * blocks(P); \
+      const int64_t need = GRID(COUNT(0), tab ? S : 1), full = int64_t(148) * blocks(P, tab != nullptr); \
       if (tab) {                                                                         \
         const unsigned mul = 65536u / unsigned(S) + 1u;                                  \
-        const unsigned g = unsigned(std::max<int64_t>(1, std::min(need, full)));         \
+        const dim3 g = stream_grid(need, full, n);                                       \
         if (P == 4) kern##_n<4><<<g, 256, 0, s>>>(tab, n, t0, w0, S, mul);               \
         else if (P == 2) kern##_n<2><<<g, 256, 0, s>>>(tab, n, t0, w0, S, mul);          \
         else kern##_n<1><<<g, 256, 0, s>>>(tab, n, t0, w0, S, mul);                      \

@@ -33,11 +33,17 @@ _plans: "weakref.WeakKeyDictionary[Mesh, dict]" = weakref.WeakKeyDictionary()
 _plans_lock = threading.Lock()
 
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("fesom_jax_b200 FCT needs a CUDA GPU; there is no CPU fallback")
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("fesom_jax_b200 FCT needs a CUDA GPU; there is no CPU fallback")
+        _torch_module = torch
+    return _torch_module
 
 
 class FctPlan:
@@ -54,6 +60,9 @@ class FctPlan:
                                               C.byref(h)))
         self._h = h
         self._lock = threading.Lock()
+        self._node = (mesh.nod2D, mesh.nl)
+        self._elem = (mesh.elem2D, mesh.nl)
+        self._reserved = max(1, int(max_tracers))   # tracers the workspace holds at least
 
     @property
     def handle(self) -> C.c_void_p:
@@ -68,6 +77,7 @@ class FctPlan:
 
     def reserve(self, ntr: int) -> None:
         _lib.check(_lib.lib().fct_plan_reserve(self._h, int(ntr)))
+        self._reserved = max(self._reserved, int(ntr))
 
     def health(self, stream=None) -> int:
         """Non-finite ``T_new`` values this plan's forward calls wrote since the previous
@@ -158,41 +168,33 @@ class FctPlan:
         """One FCT step on device tensors; returns ``T_new`` (same shape as ``T``).
         ``stagewise`` runs one kernel per reference stage (``fct_forward_ex``), the kernels
         the reverse pass recomputes with (needs the plan's adjoint reservation)."""
+        # (host time counts on small meshes: one pass over the arguments, no closure, the sizes
+        # and the reservation kept with the plan)
         torch = _torch()
-        m = self.mesh
-        N, E, nl = m.nod2D, m.elem2D, m.nl
+        node, elem, dev = self._node, self._elem, self.device
         ntr = 1 if T.dim() == 2 else int(T.shape[0])
-        dev = torch.device("cuda", self.device)
-
-        def chk(x, shape, name):
+        tshape = node if T.dim() == 2 else (ntr, *node)
+        if out is None:
+            out = torch.empty_like(T)
+        for x, shape, name in ((uv, (*elem, 2), "uv"), (w_e, node, "w_e"), (helem, elem, "helem"),
+                               (hnode, node, "hnode"), (hnode_new, node, "hnode_new"),
+                               (T, tshape, "T"), (T_old, tshape, "T_old"), (Z3d, node, "Z3d"),
+                               (zbar3, node, "zbar3"), (w_i, node, "w_i"), (out, tshape, "out")):
             if x is None:
-                return None
-            if not (x.is_cuda and x.dtype == torch.float64 and x.device == dev):
-                raise TypeError(f"{name}: need a float64 tensor on {dev}")
-            if tuple(x.shape) != tuple(shape):
+                continue
+            if not (x.dtype is torch.float64 and x.is_cuda and x.get_device() == dev):
+                raise TypeError(f"{name}: need a float64 tensor on cuda:{dev}")
+            if x.shape != shape:
                 raise ValueError(f"{name}: shape {tuple(x.shape)} != {tuple(shape)}")
             if not x.is_contiguous():
                 raise ValueError(f"{name}: must be contiguous")
-            return x
-
-        tshape = (N, nl) if T.dim() == 2 else (ntr, N, nl)
-        chk(uv, (E, nl, 2), "uv"); chk(w_e, (N, nl), "w_e"); chk(helem, (E, nl), "helem")
-        chk(hnode, (N, nl), "hnode"); chk(hnode_new, (N, nl), "hnode_new")
-        chk(T, tshape, "T"); chk(T_old, tshape, "T_old")
-        chk(Z3d, (N, nl), "Z3d"); chk(zbar3, (N, nl), "zbar3"); chk(w_i, (N, nl), "w_i")
-        if out is None:
-            out = torch.empty_like(T)
-        chk(out, tshape, "out")
-        if ntr > self.info()["max_tracers"]:
+        if ntr > self._reserved:
             self.reserve(ntr)
-        f = _lib.FctFields()
-        f.uv, f.w_e, f.helem = uv.data_ptr(), w_e.data_ptr(), helem.data_ptr()
-        f.hnode, f.hnode_new = hnode.data_ptr(), hnode_new.data_ptr()
-        f.T, f.T_old, f.T_new = T.data_ptr(), T_old.data_ptr(), out.data_ptr()
-        f.tracer_stride = N * nl
-        f.Z3d = Z3d.data_ptr() if Z3d is not None else None
-        f.zbar3 = zbar3.data_ptr() if zbar3 is not None else None
-        f.w_i = w_i.data_ptr() if w_i is not None else None
+        f = _lib.FctFields(uv.data_ptr(), w_e.data_ptr(), helem.data_ptr(), hnode.data_ptr(),
+                           hnode_new.data_ptr(), T.data_ptr(), T_old.data_ptr(), out.data_ptr(),
+                           node[0] * node[1], Z3d.data_ptr() if Z3d is not None else None,
+                           zbar3.data_ptr() if zbar3 is not None else None,
+                           w_i.data_ptr() if w_i is not None else None)
         s = stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
         # the library orders calls on one plan on the GPU; the lock keeps the host-side
         # enqueue of concurrent Python threads whole
@@ -213,7 +215,9 @@ class FctPlan:
 def get_plan(mesh: Mesh, device: int = 0) -> FctPlan:
     """The cached plan of ``mesh`` on ``device`` (created on first use)."""
     with _plans_lock:
-        per = _plans.setdefault(mesh, {})
+        per = _plans.get(mesh)
+        if per is None:
+            per = _plans[mesh] = {}
         p = per.get(device)
         if p is None:
             p = per[device] = FctPlan(mesh, device, max_tracers=1)   # grows on demand
