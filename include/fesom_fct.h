@@ -107,7 +107,7 @@ int fct_plan_reserve(FctPlan* plan, int max_tracers);
  * layers, max_tracers]. */
 int fct_plan_info(const FctPlan* plan, int64_t out[8]);
 /* Which stage kernels fct_forward runs: fused (1, the default: 5 launches per tracer
- * chunk over runs of consecutive levels, element gradients and cluster bounds recomputed
+ * chunk, 2 fewer on a small mesh, element gradients and cluster bounds recomputed
  * instead of stored, quotients by reciprocals and explicit FMAs) or one kernel per
  * reference stage (0: 7 launches, every intermediate written to the workspace, every
  * quotient correctly rounded; the form the reverse pass recomputes). The two give the same
@@ -115,7 +115,8 @@ int fct_plan_info(const FctPlan* plan, int64_t out[8]);
 int fct_plan_set_fused(FctPlan* plan, int fused);
 /* Thread mapping of the fused stages of this plan's fct_forward / fct_forward_noalloc and
  * of its instances in fct_serve_step: the most tracers one thread carries and the levels
- * of one node or edge column it takes (each 1, 2, 4 or 8; default 2 and 4). A tuning knob:
+ * of one node or edge column it takes (each 1, 2, 4 or 8; by default the library chooses per
+ * stage: two tracers and one level, more for large interleaved instances). A tuning knob:
  * the results do not depend on it. No reference counterpart (XLA picks its own loop
  * mapping). */
 int fct_plan_set_mapping(FctPlan* plan, int tracers_per_thread, int levels_per_thread);
@@ -360,8 +361,8 @@ typedef struct FctBatch FctBatch;
 int fct_batch_create(const FctInstance* insts, int n, int64_t workspace_budget_bytes,
                      FctBatch** out);
 int fct_batch_destroy(FctBatch* b);
-/* Tuning: the most tracers one thread carries (1, 2, 4 or 8; default: the workspace
- * chunk, at most 8). Fewer use fewer registers (higher occupancy), more share each
+/* Tuning: the most tracers one thread carries (1, 2, 4 or 8; by default the library
+ * chooses per stage). Fewer use fewer registers (higher occupancy), more share each
  * gather's index work. Drops cached graphs. */
 int fct_batch_set_chunk(FctBatch* b, int chunk);
 /* Tuning: tracers per thread (1, 2, 4 or 8; the fused stages carry at most 4) and levels
@@ -372,7 +373,9 @@ int fct_batch_set_mapping(FctBatch* b, int tracers_per_thread, int levels_per_th
 int fct_batch_set_stage_mapping(FctBatch* b, int stage, int tracers_per_thread,
                                 int levels_per_thread);
 /* [instances, groups, workspace bytes, total wet node layers x tracers,
- *  tracers per workspace chunk (largest over groups), kernel launches per step] */
+ *  tracers per workspace chunk (largest over groups), kernel launches per step (of
+ *  fct_batch_step; in an fct_batch_run the volume fluxes, and w_derived, are launched in
+ *  its first step only)] */
 int fct_batch_info(const FctBatch* b, int64_t out[6]);
 /* Copy the dry levels of buf[1] into buf[0] and buf[2] (dry levels never change). */
 int fct_batch_prepare(FctBatch* b, fct_stream_t stream);
@@ -380,7 +383,8 @@ int fct_batch_prepare(FctBatch* b, fct_stream_t stream);
 int fct_batch_step(FctBatch* b, int phase, fct_stream_t stream);
 /* ``steps`` consecutive steps starting at ``first_phase``, captured once into a CUDA
  * graph (cached per (first_phase, steps)) and launched on ``stream``. The instance that
- * holds T after the run is buf[(first_phase + steps + 1) % 3]. */
+ * holds T after the run is buf[(first_phase + steps + 1) % 3]. A run forms the volume fluxes
+ * (and w_derived) once, from the uv and helem it finds at its start. */
 int fct_batch_run(FctBatch* b, int first_phase, int steps, fct_stream_t stream);
 
 /* Health check of a batch (as fct_plan_health): per-instance counts of non-finite T_new
