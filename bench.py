@@ -36,14 +36,14 @@ FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes (read + write) per node-level update of the six kernels of the fused FCT step
 # (volume fluxes, LO, edge fluxes and their node-gradient lanes, limiter, final), from one
 # ncu capture of the small case of the batched workload (2 members x 8 tracers of the
-# CORE2-size mesh: 12.53 GB per FCT step / 48.76 M updates). Scaled to a launch by the
-# updates it does.
-TRAFFIC_B_PER_UPDATE = 257.0
+# CORE2-size mesh, 48.76 M updates, default mapping; the volume fluxes count once per 30
+# steps). Scaled to a launch by the updates it does.
+TRAFFIC_B_PER_UPDATE = 245.0
 # Warp-instructions per node-level update of the same six kernels in the same capture
 # (smsp__inst_executed.sum / updates). The kernels are latency- and issue-limited rather
 # than HBM-bound, so the line also reports this issue-rate fraction beside the HBM one:
 # achieved warp-instructions/s against 148 SMs x 4 schedulers x the sampled SM clock.
-WARP_INST_PER_UPDATE = 46.0
+WARP_INST_PER_UPDATE = 34.9
 B200_SMS, SCHEDULERS_PER_SM = 148, 4
 
 
@@ -367,7 +367,9 @@ def run_ours(args, D: Dist) -> dict | None:
     pk = peaks()
     achieved = alg / (fct_step_ms / 1e3) / 1e9
     info = ens.info()   # after tuning: launches per step depend on tracers per thread
-    n_kernels = info["launches_per_step"]
+    # a run forms the volume fluxes (and derived w) of each group in its first step only
+    once = info["groups"] * (2 if args.derive_w else 1)
+    n_kernels = (info["launches_per_step"] - once) * S + once
     gates = None
     if D.rank == 0 and not args.no_gates:
         from fesom_jax_b200.tracer_adv import get_plan
@@ -375,8 +377,8 @@ def run_ours(args, D: Dist) -> dict | None:
     out = dict(value=value, t=t, info=info, clocks=clk, prof=prof, fct_step_ms=fct_step_ms,
                finite=finite, nonfinite=int(sum(nonfinite)), gates=gates, mesh=mesh, cfg=cfg,
                alg_bytes=alg,
-               roofline=dict(bound="hbm", kernel="fused FCT step (k_vflux, k_seg_lo, k_seg_edge, "
-                                                 "k_edge_fix, k_seg_limit, k_seg_final)",
+               roofline=dict(bound="hbm", kernel="fused FCT step (volume fluxes, LO, edge fluxes and "
+                                                 "their node-gradient lanes, limiter, final)",
                              achieved=achieved, peak=pk["hbm_gbs"], unit="GB/s",
                              frac=achieved / pk["hbm_gbs"], peak_source=pk["source"],
                              traffic=TRAFFIC_B_PER_UPDATE * info["updates_per_step"],
@@ -384,7 +386,7 @@ def run_ours(args, D: Dist) -> dict | None:
                                           "capture scaled by updates",
                              alg_bytes_per_step=alg,
                              issue=issue_roofline(value / D.world, clk)),
-               gpu_launches=n_kernels * S * args.steps,
+               gpu_launches=n_kernels * args.steps,
                tuning=dict(stage_mapping={st: f"{c}x{lv}" for st, (c, lv) in
                                           zip(ens.STAGES, ens.stage_map)},
                            autotune=tune))

@@ -270,14 +270,16 @@ int fct_batch_info(const FctBatch* B, int64_t out[6]) {
   for (const auto& g : B->groups) {
     const int chunk = g.dims.chunk > 0 ? g.dims.chunk : g.dims.ntr;
     wmax = std::max<int64_t>(wmax, chunk);
-    int64_t per_chunk_launches = 0;
-    for (int c0 = 0; c0 < g.dims.ntr; c0 += chunk) {
-      const int csz = std::min(chunk, g.dims.ntr - c0);
-      per_chunk_launches += stage_launches(csz, g.dims.smap_tracers[kStageLo], seg_even(g.dims));
+    const LaunchDims& d = g.dims;
+    const bool even = seg_even(d);
+    launches += 1 + (d.any_derive_w ? 1 : 0);
+    for (int c0 = 0; c0 < d.ntr; c0 += chunk) {
+      const int csz = std::min(chunk, d.ntr - c0);
+      for (int i = 0; i < kFusedStages; ++i) launches += stage_launches(csz, d.smap_tracers[i], even);
+      if (d.max_efix > 0)
+        launches += stage_launches(csz, std::min(2, d.smap_tracers[kStageEdge]), even);
+      if (d.any_vdiff) launches += (csz + 7) / 8;
     }
-    const int stages = (g.dims.fused ? 4 + (g.dims.max_efix > 0 ? 1 : 0) : 7) +
-                       (g.dims.any_wi ? 1 : 0) + (g.dims.any_vdiff ? 1 : 0);
-    launches += 1 + (g.dims.any_derive_w ? 1 : 0) + int64_t(stages) * per_chunk_launches;
   }
   out[4] = wmax;
   out[5] = launches;

@@ -154,14 +154,31 @@ int plan_reserve_ws(FctPlan* P, int ntr, bool full) {
 
 namespace {
 
+// The plan's static arrays: offsets (256-byte aligned) in one device allocation, each array
+// copied from where the host built it (they stay alive until upload; gathered into one host
+// buffer first, they were written three times over while it grew).
 struct Blob {
-  std::vector<char> bytes;
+  struct Part {
+    const void* src;
+    size_t bytes, off;
+  };
+  std::vector<Part> parts;
+  size_t size = 0;
   template <class T>
   size_t add(const T* src, size_t n) {
-    size_t off = (bytes.size() + 255) & ~size_t(255);
-    bytes.resize(off + n * sizeof(T));
-    if (n) std::memcpy(bytes.data() + off, src, n * sizeof(T));
+    static const char zeros[sizeof(T)] = {};   // an empty array holds one zero element
+    const size_t off = (size + 255) & ~size_t(255);
+    parts.push_back({n ? static_cast<const void*>(src) : zeros, std::max(n, size_t(1)) * sizeof(T),
+                     off});
+    size = off + std::max(n, size_t(1)) * sizeof(T);
     return off;
+  }
+  cudaError_t upload(char* base) const {
+    for (const Part& p : parts) {
+      const cudaError_t e = cudaMemcpy(base + p.off, p.src, p.bytes, cudaMemcpyHostToDevice);
+      if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
   }
 };
 
@@ -380,6 +397,17 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   }
   // lanes
   std::vector<uint32_t> iface, layer, edgel, eleml, dry;
+  {   // (their sizes: no growth by copies)
+    size_t wet = 0, edge_levels = 0, elem_levels = 0;
+    for (int n = 0; n < N; ++n) wet += size_t(nzmax[n] - nzmin[n]);
+    for (int e = 0; e < Ed; ++e) edge_levels += size_t(std::max(0, ekmax[e] - ekmin[e]));
+    for (int e = 0; e < E; ++e) elem_levels += size_t(enl[e] - eul[e]);
+    layer.reserve(wet);
+    iface.reserve(wet + N);
+    dry.reserve(size_t(N) * L - wet);
+    edgel.reserve(edge_levels);
+    eleml.reserve(elem_levels);
+  }
   for (int n = 0; n < N; ++n) {
     for (int k = std::max(nzmin[n], 0); k <= std::min(nzmax[n], L - 1); ++k) {
       iface.push_back((uint32_t(n) << kLevelBits) | uint32_t(k));
@@ -446,6 +474,7 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   // the only levels where the one-kernel-per-stage forward computes them)
   std::vector<int4> nrec(static_cast<size_t>(N));
   std::vector<unsigned long long> nflags;
+  nflags.reserve(layer.size());
   for (int n = 0; n < N; ++n) {
     const int ed = ne_off[n + 1] - ne_off[n];
     const int cd = d->nod_in_elem2D_offsets[n + 1] - d->nod_in_elem2D_offsets[n];
@@ -525,6 +554,8 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   std::vector<uint32_t> nseg[kSegVariants], eseg[kSegVariants];
   for (int v = 0; v < kSegVariants; ++v) {
     const int lpt = kSegLevels[v];
+    nseg[v].reserve(layer.size() / lpt + N);
+    eseg[v].reserve(edgel.size() / lpt + Ed);
     for (int n = 0; n < N; ++n)
       for (int k = std::max(nzmin[n], 0); k < std::min(nzmax[n], L); k += lpt)
         nseg[v].push_back((uint32_t(n) << kLevelBits) | uint32_t(k));
@@ -553,12 +584,12 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   size_t o_etr = b.add(etr.data(), Ed);
   size_t o_eedge = b.add(eedge.data(), eedge.size());
   size_t o_eudoff = b.add(eud_off.data(), eud_off.size());
-  size_t o_eudidx = b.add(eud_idx.data(), std::max<size_t>(eud_idx.size(), 1));
+  size_t o_eudidx = b.add(eud_idx.data(), eud_idx.size());
   size_t o_ne4 = b.add(ne4.data(), ne4.size()), o_nel4 = b.add(nel4.data(), nel4.size());
   size_t o_nelr = b.add(nelr.data(), nelr.size());
   size_t o_Zp = b.add(Zp.data(), L), o_zbar = b.add(d->zbar, L);
   size_t o_if = b.add(iface.data(), iface.size()), o_ly = b.add(layer.data(), layer.size());
-  size_t o_dry = b.add(dry.data(), std::max<size_t>(dry.size(), 1));
+  size_t o_dry = b.add(dry.data(), dry.size());
   size_t o_ed = b.add(edgel.data(), edgel.size()), o_el = b.add(eleml.data(), eleml.size());
   size_t o_if4 = b.add(iface4.data(), iface4.size()), o_ly4 = b.add(layer4.data(), layer4.size());
   size_t o_ed4 = b.add(edge4.data(), edge4.size());
@@ -570,18 +601,18 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   size_t o_iarea0 = b.add(iarea0.data(), N), o_earea12 = b.add(earea12.data(), E);
   size_t o_ediff = b.add(ediff.data(), E);
   size_t o_emf4 = b.add(emf4.data(), emf4.size()), o_emfw = b.add(emfw.data(), emfw.size());
-  size_t o_nflags = b.add(nflags.data(), std::max<size_t>(nflags.size(), 1));
-  size_t o_efix = b.add(efix.data(), std::max<size_t>(efix.size(), 1));
+  size_t o_nflags = b.add(nflags.data(), nflags.size());
+  size_t o_efix = b.add(efix.data(), efix.size());
   size_t o_nseg[kSegVariants], o_eseg[kSegVariants];
   for (int v = 0; v < kSegVariants; ++v) {
-    o_nseg[v] = b.add(nseg[v].data(), std::max<size_t>(nseg[v].size(), 1));
-    o_eseg[v] = b.add(eseg[v].data(), std::max<size_t>(eseg[v].size(), 1));
+    o_nseg[v] = b.add(nseg[v].data(), nseg[v].size());
+    o_eseg[v] = b.add(eseg[v].data(), eseg[v].size());
   }
 
   FCT_CUDA(cudaSetDevice(device));
-  FCT_CUDA(cudaMalloc(&P->d_static, b.bytes.size()));
-  FCT_CUDA(cudaMemcpy(P->d_static, b.bytes.data(), b.bytes.size(), cudaMemcpyHostToDevice));
+  FCT_CUDA(cudaMalloc(&P->d_static, b.size));
   char* base = static_cast<char*>(P->d_static);
+  FCT_CUDA(b.upload(base));
   DevMesh& m = P->hm;
   m.N = N; m.E = E; m.Ed = Ed; m.L = L;
   m.edges_outside = 0;
