@@ -8,6 +8,7 @@
 // running sum gives w, divided by ``area`` (safe where 0) and masked to the node's
 // interfaces.
 #include <algorithm>
+#include <cstdint>
 
 #include "fct_div.cuh"
 #include "fct_host.h"
@@ -24,12 +25,20 @@ namespace {
 // CORE2-size mesh.)
 constexpr int kWColumns = 16, kWThreads = 256;
 
+// u and v of element level q: one 16-byte load, or two of 8 bytes where the caller's uv starts
+// at an odd double.
+template <bool Pairs>
+__device__ __forceinline__ double2 uv_at(const double* __restrict__ uv, uint32_t q) {
+  if constexpr (Pairs) return __ldg(reinterpret_cast<const double2*>(uv) + q);
+  return make_double2(__ldg(uv + 2 * size_t(q)), __ldg(uv + 2 * size_t(q) + 1));
+}
+
+template <bool Pairs>
 __device__ __forceinline__ void compute_w_columns(const DevMesh& m, const double* __restrict__ uv,
                                                   const double* __restrict__ helem,
                                                   double* __restrict__ w, int n0, double* sh) {
   if (n0 >= m.N) return;   // block-uniform
   const int L = m.L, stride = L | 1;
-  const double2* uv2 = reinterpret_cast<const double2*>(uv);
   for (int i = threadIdx.x; i < kWColumns * L; i += kWThreads) {
     const int col = i / L, k = i - col * L, n = n0 + col;
     if (n >= m.N) break;
@@ -51,11 +60,11 @@ __device__ __forceinline__ void compute_w_columns(const DevMesh& m, const double
       double2 U1 = make_double2(0.0, 0.0), U2 = U1;
       double h1 = 0.0, h2 = 0.0;
       if (on1) {
-        U1 = __ldg(uv2 + (uint32_t(sl.x) + uint32_t(k)));
+        U1 = uv_at<Pairs>(uv, uint32_t(sl.x) + uint32_t(k));
         h1 = __ldg(helem + (uint32_t(sl.x) + uint32_t(k)));
       }
       if (on2) {
-        U2 = __ldg(uv2 + (uint32_t(sl.y) + uint32_t(k)));
+        U2 = uv_at<Pairs>(uv, uint32_t(sl.y) + uint32_t(k));
         h2 = __ldg(helem + (uint32_t(sl.y) + uint32_t(k)));
       }
       const double t1 = on1 ? (U1.y * x1.x - U1.x * x1.y) * h1 : 0.0;
@@ -86,12 +95,13 @@ __device__ __forceinline__ void compute_w_columns(const DevMesh& m, const double
   }
 }
 
+template <bool Pairs>
 __global__ void __launch_bounds__(kWThreads) k_compute_w(const DevMesh* __restrict__ mp,
                                                          const double* __restrict__ uv,
                                                          const double* __restrict__ helem,
                                                          double* __restrict__ w) {
   __shared__ double sh[kWColumns * (kMaxLevels + 1)];
-  compute_w_columns(*mp, uv, helem, w, int(blockIdx.x) * kWColumns, sh);
+  compute_w_columns<Pairs>(*mp, uv, helem, w, int(blockIdx.x) * kWColumns, sh);
 }
 
 // batched: instance blockIdx.y of a device table derives its w into w_derived
@@ -99,7 +109,7 @@ __global__ void __launch_bounds__(kWThreads) k_compute_w_n(const Inst* __restric
   __shared__ double sh[kWColumns * (kMaxLevels + 1)];
   const Inst& in = tab[blockIdx.y];
   if (!in.w_derived) return;
-  compute_w_columns(in.m, in.uv, in.helem, in.w_derived, int(blockIdx.x) * kWColumns, sh);
+  compute_w_columns<true>(in.m, in.uv, in.helem, in.w_derived, int(blockIdx.x) * kWColumns, sh);
 }
 
 }  // namespace
@@ -122,8 +132,13 @@ extern "C" int fct_compute_w(FctPlan* P, const double* uv, const double* helem, 
   int prev = -1;
   cudaGetDevice(&prev);
   if (prev != P->device) cudaSetDevice(P->device);
-  k_compute_w<<<(P->N + kWColumns - 1) / kWColumns, kWThreads, 0,
-                static_cast<cudaStream_t>(stream)>>>(P->d_mesh, uv, helem, w);
+  const int blocks = (P->N + kWColumns - 1) / kWColumns;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // uv may start at any double; the pair loads need a 16-byte boundary
+  if (reinterpret_cast<uintptr_t>(uv) % 16 == 0)
+    k_compute_w<true><<<blocks, kWThreads, 0, s>>>(P->d_mesh, uv, helem, w);
+  else
+    k_compute_w<false><<<blocks, kWThreads, 0, s>>>(P->d_mesh, uv, helem, w);
   cudaError_t e = cudaGetLastError();
   if (prev >= 0 && prev != P->device) cudaSetDevice(prev);
   return e == cudaSuccess ? FCT_OK : cuda_error(e, "compute_w launch");
