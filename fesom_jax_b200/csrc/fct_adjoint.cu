@@ -1117,11 +1117,13 @@ int fct_forward_taped(FctPlan* P, const FctFields* f, double dt, int ntr, FctTap
   if (!(dt > 0.0)) return set_error(FCT_ERR_INVALID, "dt must be positive");
   if (tape->share_vflux && slot > 0 && !tape->recorded[0])
     return set_error(FCT_ERR_INVALID, "a tape sharing its volume fluxes records slot 0 first");
+  const bool shared = tape->share_vflux && slot > 0;   // slot 0's fluxes are this step's
+  if (!shared && (st = check_uv(f->uv))) return st;
   DeviceGuard g(P->device);
   Inst in = make_inst(P, f, dt, ntr, tape->ws[size_t(slot)]);
   in.nonfinite = P->d_health;
   LaunchDims dims = unfused_dims(P, ntr);
-  dims.skip_vflux = tape->share_vflux && slot > 0;   // slot 0's fluxes are this step's
+  dims.skip_vflux = shared;
   {
     PlanUse use(P, static_cast<cudaStream_t>(stream));
     st = use.status();
@@ -1164,6 +1166,7 @@ int fct_adjoint_ex(FctPlan* P, const FctFields* f, const double* gT_new, double 
   if (!g->gT || !g->gT_old || (!g->guv && !defer_uv) || !g->gw_e)
     return set_error(FCT_ERR_INVALID, "a gradient output pointer is NULL");
   if (!(dt > 0.0)) return set_error(FCT_ERR_INVALID, "dt must be positive");
+  if (!tape && (st = check_uv(f->uv))) return st;   // only the recomputation reads uv
   DeviceGuard guard(P->device);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   PlanUse use(P, s);

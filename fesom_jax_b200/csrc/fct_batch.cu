@@ -91,6 +91,7 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
         !q.buf[2])
       return set_error(FCT_ERR_INVALID, "instance %d: a field pointer is NULL", i);
     if (!(q.dt > 0.0)) return set_error(FCT_ERR_INVALID, "instance %d: dt <= 0", i);
+    if (const int bad = check_uv(q.uv)) return bad;
     const FctPlan* P = q.plan;
     // the workspace holds a chunk of the instance's tracers (stages run chunk by chunk):
     // up to 8, halved until one instance fits the budget
@@ -518,6 +519,7 @@ int fct_serve_step(FctServe* S, const FctInstance* insts, const int32_t* phases,
     if (!q.plan || q.plan->device != S->device || q.ntr < 1 || !q.buf[0] || !q.buf[1] ||
         !q.buf[2] || !q.uv || !q.w_e || !q.helem || !q.hnode || !q.hnode_new || !(q.dt > 0.0))
       return set_error(FCT_ERR_INVALID, "instance %d is invalid", i);
+    if (const int bad = check_uv(q.uv)) return bad;
     const int st = check_interleave(q.plan, q.ntr, q.ntr, i);
     if (st) return st;
     need += workspace_doubles_fused(q.plan->N, q.plan->Ed, q.plan->L, q.ntr);

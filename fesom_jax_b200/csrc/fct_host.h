@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <string>
 
@@ -242,6 +243,14 @@ class PlanUse {
 // Copy a device counter to the host on ``s``, wait, zero it, and return FCT_ERR_NONFINITE
 // when it was non-zero (``out`` receives the count when not NULL).
 int read_health(unsigned long long* d_counter, int n, cudaStream_t s, int64_t* out);
+
+// The volume-flux kernel reads u and v of an element level with one 16-byte load: a uv that it
+// cannot read is refused before the launch.
+inline int check_uv(const double* uv) {
+  if (reinterpret_cast<uintptr_t>(uv) % 16 != 0)
+    return set_error(FCT_ERR_INVALID, "uv must start on a 16-byte boundary");
+  return FCT_OK;
+}
 
 // Launches one fused stage takes for `csz` tracers of a workspace chunk with at most
 // `per_thread` tracers per thread.

@@ -49,6 +49,7 @@ extern "C" int fct_forward_noalloc(FctPlan* P, const FctFields* f, double dt, in
   if ((f->Z3d == nullptr) != (f->zbar3 == nullptr))
     return set_error(FCT_ERR_INVALID, "Z3d and zbar3 must be given together");
   if (!(dt > 0.0)) return set_error(FCT_ERR_INVALID, "dt must be positive");
+  if (const int bad = check_uv(f->uv)) return bad;
   if (P->device < 0 || P->device >= kMaxDevices)
     return set_error(FCT_ERR_INVALID, "device %d out of range", P->device);
   const int64_t need = workspace_doubles_fused(P->N, P->Ed, P->L, ntr);

@@ -840,6 +840,7 @@ int fct_forward_ex(FctPlan* P, const FctFields* f, double dt, int ntr, int flags
   if ((f->Z3d == nullptr) != (f->zbar3 == nullptr))
     return set_error(FCT_ERR_INVALID, "Z3d and zbar3 must be given together");
   if (!(dt > 0.0)) return set_error(FCT_ERR_INVALID, "dt must be positive");
+  if (const int bad = check_uv(f->uv)) return bad;
   Inst in{};
   in.m = P->hm;
   in.uv = f->uv; in.w_e = f->w_e; in.helem = f->helem;

@@ -80,7 +80,7 @@ typedef struct FctMeshDesc {
  * split vertical velocity (tracer_adv.py:487-529, 557-572).
  */
 typedef struct FctFields {
-  const double* uv;         /* [elem2D,nl,2] */
+  const double* uv;         /* [elem2D,nl,2], on a 16-byte boundary (checked) */
   const double* w_e;        /* [nod2D,nl] */
   const double* helem;      /* [elem2D,nl] */
   const double* hnode;      /* [nod2D,nl] */
@@ -318,7 +318,8 @@ int fct_forward_noalloc(FctPlan* plan, const FctFields* fields, double dt, int n
                         fct_stream_t stream);
 
 /* Vertical velocity at interfaces from continuity, fesom_jax/ale.py:309-365
- * (``compute_w(mesh, uv, helem)``): ``w`` [nod2D,nl] (DEVICE), all levels written. */
+ * (``compute_w(mesh, uv, helem)``): ``w`` [nod2D,nl] (DEVICE), all levels written; uv
+ * [elem2D,nl,2] may start at any double. */
 int fct_compute_w(FctPlan* plan, const double* uv, const double* helem, double* w,
                   fct_stream_t stream);
 
@@ -333,7 +334,7 @@ int fct_compute_w(FctPlan* plan, const double* uv, const double* helem, double* 
  */
 typedef struct FctInstance {
   FctPlan* plan;            /* the instance's mesh */
-  const double* uv;         /* [elem2D,nl,2] */
+  const double* uv;         /* [elem2D,nl,2], on a 16-byte boundary (checked) */
   const double* w_e;        /* [nod2D,nl] */
   const double* helem;      /* [elem2D,nl] */
   const double* hnode;      /* [nod2D,nl] */

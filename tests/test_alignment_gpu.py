@@ -39,3 +39,40 @@ def test_compute_w_takes_uv_at_any_double(torch, mesh, offset):
     want = compute_w(mesh, _at(torch, f.uv, 0), helem)
     got = compute_w(mesh, _at(torch, f.uv, offset), helem)
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+def test_step_refuses_uv_off_a_16_byte_boundary(torch, mesh):
+    """The volume-flux kernel reads (u, v) pairs: every call that launches it refuses such a
+    pointer on the host; the reverse pass of a taped step, which does not read uv, takes it."""
+    from fesom_jax_b200.adjoint import Tape, advect_one_fct_vjp
+    from fesom_jax_b200.ensemble import Ensemble
+    from fesom_jax_b200.tracer_adv import FctPlan
+    f = I.make_fields(mesh, seed=4, kind="basin")
+    uv, off = _at(torch, f.uv, 0), _at(torch, f.uv, 1)
+    rest = [_at(torch, x, 1) for x in (f.w_e, f.helem, f.hnode, f.hnode_new, f.tracers[0],
+                                       f.tracers_old[0])]
+    plan = FctPlan(mesh, 0)
+    want = plan.forward(uv, *rest, 1200.0)      # the other fields may start anywhere
+    for kw in ({}, {"stagewise": True}):
+        if kw:
+            plan.set_fused(False)
+        with pytest.raises(Exception, match="16-byte"):
+            plan.forward(off, *rest, 1200.0, **kw)
+    plan.set_fused(True)
+    assert torch.equal(plan.forward(uv, *rest, 1200.0), want)
+    plan.close()
+    ens = Ensemble()
+    ens.add_member(mesh, off, *rest[:4], rest[4], rest[5], 1200.0)
+    with pytest.raises(Exception, match="16-byte"):
+        ens.build()
+    g = torch.ones_like(rest[4])
+    with pytest.raises(Exception, match="16-byte"):
+        advect_one_fct_vjp(mesh, off, *rest, g, dt=1200.0)
+    with Tape(mesh, 1) as tape:
+        with pytest.raises(Exception, match="16-byte"):
+            tape.forward(0, off, *rest, 1200.0)
+        tape.forward(0, uv, *rest, 1200.0)
+        a = advect_one_fct_vjp(mesh, uv, *rest, g, dt=1200.0, tape=tape)
+        b = advect_one_fct_vjp(mesh, off, *rest, g, dt=1200.0, tape=tape)
+        assert all(torch.equal(x, y) for x, y in zip(a, b))
