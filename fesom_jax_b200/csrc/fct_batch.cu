@@ -146,6 +146,7 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
           carve_workspace(B->arena + off, P->N, P->E, P->Ed, P->L, wchunk[i], /*fused=*/true);
       off += ws_doubles[i];
       dims_cover(d, P);
+      d.pairs = d.pairs && buffers_paired(q);
       d.ntr = q.ntr;
       d.chunk = wchunk[i];
       B->total_updates += int64_t(q.ntr) * P->hm.n_layer;
@@ -578,6 +579,7 @@ int fct_serve_step(FctServe* S, const FctInstance* insts, const int32_t* phases,
     const FctPlan* P0 = insts[order[j0]].plan;
     while (j1 < n && insts[order[j1]].ntr == ntr && insts[order[j1]].plan == P0) {
       dims_cover(d, insts[order[j1]].plan);
+      d.pairs = d.pairs && buffers_paired(insts[order[j1]]);
       ++j1;
     }
     d.ntr = ntr;

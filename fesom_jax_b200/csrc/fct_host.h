@@ -48,6 +48,7 @@ struct LaunchDims {
   int per_thread = 8;  // most tracers one thread carries (8, 4, 2 or 1): the tuning knob
   bool any_wi;      // launch the implicit w_i stage
   bool copy_dry;    // launch the dry-level copy
+  bool pairs = true;  // the instances' interleaved tracer buffers start on 16-byte boundaries
   bool any_vdiff = false;  // launch the implicit vertical diffusion after each chunk
   bool any_derive_w = false;  // derive w_e from uv (compute_w) before the step
   bool skip_vflux = false;    // the workspace already holds this step's volume fluxes (and
@@ -132,8 +133,7 @@ inline dim3 stream_grid(int64_t need, int64_t full, int n) {
 }
 
 // Tracers per thread and tracer slices of one segment launch over ``rem`` tracers: the
-// largest compiled count (1, 2 or 4 interleaved, 1 when the interleave strides are odd and
-// pairs would not be 16-byte aligned; 1 or 2 tracer-major) of at most ``per_thread``, and as
+// largest compiled count (1, 2 or 4 interleaved, 1 when pairs are not 16-byte aligned; 1 or 2 tracer-major) of at most ``per_thread``, and as
 // many slices as whole counts fit (at most 8 interleaved). Three tracer-major tracers go one
 // per thread, in one launch instead of two.
 struct SegSplit {
@@ -154,10 +154,16 @@ inline SegSplit seg_split(int rem, int per_thread, bool interleaved, bool even) 
   if (rem == 3) P = 1;
   return {P, rem / P};
 }
-// the interleaved tracer and workspace strides are even (tracer pairs 16-byte aligned)
+// tracer pairs are 16-byte aligned: the interleaved tracer and workspace strides are even and
+// the tracer buffers start on such a boundary
 inline bool seg_even(const LaunchDims& d) {
   const int chunk = d.chunk > 0 ? d.chunk : d.ntr;
-  return d.ntr % 2 == 0 && chunk % 2 == 0;
+  return d.pairs && d.ntr % 2 == 0 && chunk % 2 == 0;
+}
+inline bool buffers_paired(const FctInstance& q) {
+  for (const double* b : q.buf)
+    if (reinterpret_cast<uintptr_t>(b) % 16 != 0) return false;
+  return true;
 }
 
 // The fused stages over the tracers [c0, c1) of a workspace chunk (fct_seg_*.cu).

@@ -76,3 +76,40 @@ def test_step_refuses_uv_off_a_16_byte_boundary(torch, mesh):
         a = advect_one_fct_vjp(mesh, uv, *rest, g, dt=1200.0, tape=tape)
         b = advect_one_fct_vjp(mesh, off, *rest, g, dt=1200.0, tape=tape)
         assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntr", [2, 4])
+def test_batch_takes_tracer_buffers_at_any_double(torch, mesh, ntr):
+    """Interleaved buffers off a 16-byte boundary: single loads instead of tracer pairs, the
+    same bits under the default mapping and a set one, batched and served."""
+    import ctypes as C
+    from fesom_jax_b200 import _lib
+    from fesom_jax_b200.ensemble import FctInstance, _bind_batch
+    from fesom_jax_b200.serve import _bind
+    from fesom_jax_b200.tracer_adv import get_plan
+    f = I.make_fields(mesh, seed=4, n_passive=2, ab2=True, kind="basin")
+    fields = [_at(torch, x, 0) for x in (f.uv, f.w_e, f.helem, f.hnode, f.hnode_new)]
+    old, T = (np.moveaxis(x[:ntr], 0, -1) for x in (f.tracers_old, f.tracers))
+    L, plan = _bind_batch(_lib.lib()), get_plan(mesh, 0)
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    got = []
+    for offset in (0, 1):
+        for run in ("batch", "mapped", "serve"):
+            buf = [_at(torch, x, offset) for x in (old, T, T)]
+            q = (FctInstance * 1)(FctInstance(
+                plan.handle.value, *(x.data_ptr() for x in fields),
+                (C.c_void_p * 3)(*(b.data_ptr() for b in buf)), ntr, 1200.0, None, None))
+            h = C.c_void_p()
+            if run == "serve":
+                _lib.check(_bind(L).fct_serve_create(0, 1, 1 << 28, C.byref(h)))
+                _lib.check(L.fct_serve_step(h, q, (C.c_int32 * 1)(0), 1, s))
+            else:
+                _lib.check(L.fct_batch_create(q, 1, 1 << 30, C.byref(h)))
+                if run == "mapped":
+                    _lib.check(L.fct_batch_set_mapping(h, 4, 2))
+                _lib.check(L.fct_batch_run(h, 0, 1, s))
+            torch.cuda.synchronize()
+            got.append(buf[2].clone())
+            (L.fct_serve_destroy if run == "serve" else L.fct_batch_destroy)(h)
+    assert all(torch.equal(g, got[0]) for g in got)
