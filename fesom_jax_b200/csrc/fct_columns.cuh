@@ -5,10 +5,11 @@
 // memory rate with 11% of the issue slots used). Here a block takes a few columns:
 //   1. all threads form the rows' coefficients and right-hand sides, levels adjacent (whole
 //      lines), into shared memory;
-//   2. one thread per column eliminates and substitutes back in shared memory (rows padded to
-//      an odd length, so that neighbouring columns use different banks), all tracers of the
-//      block in its registers: the walk's chain is the matrix recursion's, and the tracers'
-//      and the next row's loads fit beside it;
+//   2. one lane per column, or with several tracers two or four of a warp, eliminate and
+//      substitute back in shared memory (rows padded to an odd length, so that neighbouring
+//      columns use different banks), the block's tracers divided among them, in registers: the
+//      walk's chain is the matrix recursion's, and the tracers' and the next row's loads fit
+//      beside it;
 //   3. all threads write the result, levels adjacent.
 // What bounds it is that chain (about 20 dependent operations a level), so the blocks are
 // small and many: 3 + (tracers) values per row and column.
@@ -59,62 +60,127 @@ __device__ __forceinline__ double col_div(double x, double y, double r) {
 
 // Thomas algorithm over the rows [nzmin, nzmax) of every column of the block (fesom_jax/
 // ops.py:121-168; the padded rows above and below solve to exactly 0). The solutions replace
-// the right-hand sides. Every thread of the block calls it, after a barrier.
-template <int NT>
-__device__ __forceinline__ void col_solve(const DevMesh& m, const ColRows& s, int n0) {
+// the right-hand sides. Every thread of the block calls one of the two forms, after a barrier;
+// lanes of the first warp work.
+//
+// One tracer: one lane per column (more lanes would only add traffic: 201 us against 253 for
+// 127,000 nodes x 48 levels).
+__device__ __forceinline__ void col_solve_one(const DevMesh& m, const ColRows& s, int n0) {
   const int col = threadIdx.x, n = n0 + col;
   if (col < s.columns && n < m.N) {
     const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
-    const int rs = s.columns * s.stride;
-    double cp = 0.0, dp[NT], an = 0.0, bn = 1.0, cn = 0.0, rn[NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t) dp[t] = rn[t] = 0.0;
+    double cp = 0.0, dp = 0.0, an = 0.0, bn = 1.0, cn = 0.0, rn = 0.0;
     int i = s.at(col, nzmin);
     if (nzmin < nzmax) {
-      an = s.a[i]; bn = s.b[i]; cn = s.c[i];
-#pragma unroll
-      for (int t = 0; t < NT; ++t) rn[t] = s.r[t * rs + i];
+      an = s.a[i]; bn = s.b[i]; cn = s.c[i]; rn = s.r[i];
     }
     for (int k = nzmin; k < nzmax; ++k, ++i) {
-      const double a = an, c = cn, y = bn - a * cp;
-      double x[NT];
-#pragma unroll
-      for (int t = 0; t < NT; ++t) x[t] = rn[t] - a * dp[t];
+      const double a = an, c = cn, y = bn - a * cp, x = rn - a * dp;
       if (k + 1 < nzmax) {   // the next row beside this one's chain
-        an = s.a[i + 1]; bn = s.b[i + 1]; cn = s.c[i + 1];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) rn[t] = s.r[t * rs + i + 1];
+        an = s.a[i + 1]; bn = s.b[i + 1]; cn = s.c[i + 1]; rn = s.r[i + 1];
       }
-      bool ok = div_exp_ok(y) && col_div_ok(c);
-#pragma unroll
-      for (int t = 0; t < NT; ++t) ok = ok && col_div_ok(x[t]);
       const double r = __drcp_rn(y);
       cp = col_div(c, y, r);
-#pragma unroll
-      for (int t = 0; t < NT; ++t) dp[t] = col_div(x[t], y, r);
-      if (!ok) {
+      dp = col_div(x, y, r);
+      if (!(div_exp_ok(y) && col_div_ok(c) && col_div_ok(x))) {
         cp = col_div_slow(c, y);
-#pragma unroll
-        for (int t = 0; t < NT; ++t) dp[t] = col_div_slow(x[t], y);
+        dp = col_div_slow(x, y);
       }
       s.c[i] = cp;
-#pragma unroll
-      for (int t = 0; t < NT; ++t) s.r[t * rs + i] = dp[t];
+      s.r[i] = dp;
     }
-    double v[NT];
-#pragma unroll
-    for (int t = 0; t < NT; ++t) v[t] = 0.0;
+    double v = 0.0;
     for (int k = nzmax - 1; k >= nzmin; --k) {
       --i;
-      const double q = s.c[i];
-#pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        v[t] = s.r[t * rs + i] - q * v[t];
-        s.r[t * rs + i] = v[t];
-      }
+      v = s.r[i] - s.c[i] * v;
+      s.r[i] = v;
     }
   }
   __syncthreads();
+}
+
+// Several tracers: G = 32 / C lanes share a column (C columns in the block), each carries the
+// matrix recursion and TPL of the tracers, because a row's instructions bound the walk (one
+// lane per column with 8 tracers in its registers: 786 us for 30,000 nodes x 70 levels, 2,195
+// for 127,000 x 48; so 428 and 1,215; two tracers 146 and 318, so 141 and 306).
+// The lanes step through their rows together, for the longest column of the warp: a column's
+// first lane writes cp over c, after the others of the column have read it.
+template <int NT, int C>
+__device__ __forceinline__ void col_solve(const DevMesh& m, const ColRows& s, int n0) {
+  constexpr int G = 32 / C, TPL = (NT + G - 1) / G;
+  if (threadIdx.x < 32) {
+    const int col = int(threadIdx.x) % C, g = int(threadIdx.x) / C, n = n0 + col;
+    const bool in_mesh = n < m.N;
+    const int nzmin = in_mesh ? ld(m.nzmin + n) : 0;
+    const int len = in_mesh ? max(0, ld(m.nzmax + n) - nzmin) : 0;   // rows of the column
+    const int rows = __reduce_max_sync(0xffffffffu, len);
+    const int first = s.at(col, nzmin);
+    double* rt[TPL];   // the lane's right-hand sides; past the last tracer, the last again
+    bool own[TPL];     //   (read, not written)
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) {
+      own[t] = g * TPL + t < NT;
+      rt[t] = s.rhs(own[t] ? g * TPL + t : NT - 1) + first;
+    }
+    double cp = 0.0, dp[TPL], an = 0.0, bn = 1.0, cn = 0.0, rn[TPL];
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) dp[t] = rn[t] = 0.0;
+    if (len > 0) {
+      an = s.a[first]; bn = s.b[first]; cn = s.c[first];
+#pragma unroll
+      for (int t = 0; t < TPL; ++t) rn[t] = rt[t][0];
+    }
+    for (int i = 0; i < rows; ++i) {
+      const double a = an, c = cn, y = bn - a * cp;
+      double x[TPL];
+#pragma unroll
+      for (int t = 0; t < TPL; ++t) x[t] = rn[t] - a * dp[t];
+      if (i + 1 < len) {   // the next row beside this one's chain
+        an = s.a[first + i + 1]; bn = s.b[first + i + 1]; cn = s.c[first + i + 1];
+#pragma unroll
+        for (int t = 0; t < TPL; ++t) rn[t] = rt[t][i + 1];
+      }
+      if (i < len) {
+        bool ok = div_exp_ok(y) && col_div_ok(c);
+#pragma unroll
+        for (int t = 0; t < TPL; ++t) ok = ok && col_div_ok(x[t]);
+        const double r = __drcp_rn(y);
+        cp = col_div(c, y, r);
+#pragma unroll
+        for (int t = 0; t < TPL; ++t) dp[t] = col_div(x[t], y, r);
+        if (!ok) {
+          cp = col_div_slow(c, y);
+#pragma unroll
+          for (int t = 0; t < TPL; ++t) dp[t] = col_div_slow(x[t], y);
+        }
+      }
+      __syncwarp();
+      if (i < len) {
+        if (g == 0) s.c[first + i] = cp;
+#pragma unroll
+        for (int t = 0; t < TPL; ++t)
+          if (own[t]) rt[t][i] = dp[t];
+      }
+    }
+    __syncwarp();
+    double v[TPL];
+#pragma unroll
+    for (int t = 0; t < TPL; ++t) v[t] = 0.0;
+    for (int i = len - 1; i >= 0; --i) {
+      const double q = s.c[first + i];
+#pragma unroll
+      for (int t = 0; t < TPL; ++t)
+        if (own[t]) rt[t][i] = v[t] = rt[t][i] - q * v[t];
+    }
+  }
+  __syncthreads();
+}
+
+template <int NT>
+__device__ __forceinline__ void col_solve_block(const DevMesh& m, const ColRows& s, int n0) {
+  if constexpr (NT == 1) col_solve_one(m, s, n0);
+  else if (s.columns == 16) col_solve<NT, 16>(m, s, n0);
+  else col_solve<NT, 8>(m, s, n0);
 }
 
 // ------------- implicit vertical diffusion (tracer_diff.py:68-123, ops.py:121-168) of the
@@ -171,7 +237,7 @@ __device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns,
     }
   }
   __syncthreads();
-  col_solve<nt>(m, s, n0);
+  col_solve_block<nt>(m, s, n0);
   const bool copy = Tin != in.T_new;   // out of place: dry levels keep T
   if constexpr (IL) {
     for (int i = threadIdx.x; i < columns * L * nt; i += kColThreads) {
@@ -237,7 +303,7 @@ __device__ __forceinline__ void block_vert_impl(const Inst& in, int n0, int colu
     }
   }
   __syncthreads();
-  col_solve<nt>(m, s, n0);
+  col_solve_block<nt>(m, s, n0);
   for (int t = 0; t < nt; ++t)
     for (int i = threadIdx.x; i < columns * L; i += kColThreads) {
       const int col = i / L, k = i - col * L, n = n0 + col;
