@@ -485,7 +485,9 @@ __device__ __forceinline__ void body_edge_fix(const Inst& in, int64_t i, int g, 
 // the nodes of n's cells that are wet at k, padded with -BIG (+BIG) when one of n's cells
 // is dry at k (tracer_adv.py:389-405). Every cell of n has two edges at n, so those nodes
 // are n itself (when any cell is wet at k) and the edge neighbours with a wet cell at k;
-// max/min are exact, so this equals the per-cell evaluation bit for bit.
+// max/min are exact, so this equals the per-cell evaluation bit for bit. The neighbour comes
+// first in each comparison: a non-finite one (a comparison with NaN is false) leaves the bound
+// as it is instead of replacing it.
 // The a4 window (k-1, k, k+1 of the same column) crosses a run's ends: each thread leaves
 // the bounds of its run's first and last level in shared memory, and the neighbouring
 // runs of the column (the adjacent segment slots of the block: a column's runs are
@@ -566,8 +568,8 @@ __device__ __forceinline__ void seg_node_limit(const Inst& in, int64_t si, bool 
         if (on) fA.ld(F::off(uint32_t(sl.x) + uint32_t(k0 + l), wtg), a);
 #pragma unroll
         for (int t = 0; t < NTR; ++t) {
-          mx[l][t] = dmax(mx[l][t], dmax(lv[t], tv[t]));
-          mn[l][t] = dmin(mn[l][t], dmin(lv[t], tv[t]));
+          mx[l][t] = dmax(dmax(lv[t], tv[t]), mx[l][t]);
+          mn[l][t] = dmin(dmin(lv[t], tv[t]), mn[l][t]);
           const double sv = flip_sign(a[t], sl.z);   // adf_h leaves the edge's first node
           if (sv > 0.0) sp[l][t] += sv;
           if (sv < 0.0) sm[l][t] += sv;
@@ -1097,8 +1099,8 @@ __device__ __forceinline__ void stream_node_limit(const Inst& in, int64_t si, in
         const bool on = (onb >> u) & 1u;
 #pragma unroll
         for (int t = 0; t < NTR; ++t) {
-          mx[t] = dmax(mx[t], dmax(lv[u][t], tv[u][t]));
-          mn[t] = dmin(mn[t], dmin(lv[u][t], tv[u][t]));
+          mx[t] = dmax(dmax(lv[u][t], tv[u][t]), mx[t]);
+          mn[t] = dmin(dmin(lv[u][t], tv[u][t]), mn[t]);
           const double sv = flip_sign(a[u][t], sgn[u]);   // adf_h leaves the first node
           if (on && sv > 0.0) sp[t] += sv;
           if (on && sv < 0.0) sm[t] += sv;
