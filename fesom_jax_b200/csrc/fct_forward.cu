@@ -261,9 +261,13 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
 
 // -------------------------- fill_up_dn_grad + adv_flux_hor_ho - LO flux = adf_h
 // -0.5 ((vf + |vf|) Tm1 + (vf - |vf|) Tm2) is exactly -0.5 times the upwind end's term (the
-// other one is 0), so only that end's gradient is read. A thread walks the lanes i, i + stride,
-// ...: the next lane's record, volume flux and cells are loaded while this lane's gathers are
-// under way.
+// other one is 0 times a finite value), so only that end's gradient is read, and one component
+// of the other's, times 0: a non-finite value on the other cell makes the flux NaN, as it does
+// in the formula (a vertex that is not finite makes both components so; the reverse pass takes
+// it from adf_h). 10-step chain on the CORE2-size mesh: 24.3 ms without that component,
+// 24.6 with it, 24.9 with both gradients in full here and in r_edge. A thread walks the lanes
+// i, i + stride, ...: the next lane's record, volume flux and cells are loaded while this lane's
+// gathers are under way.
 template <int NTR, bool IL>
 __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t stride, int t0,
                                               int w0) {
@@ -285,7 +289,7 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t
     const double vf = vf1, avf = fabs(vf);
     const uint32_t q1 = lq(rec.y, L, k), q2 = lq(rec.z, L, k);
     const bool first = vf > 0.0;
-    double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[NTR], gy[NTR];
+    double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[NTR], gy[NTR], gd[NTR];
     ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
     ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
     ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
@@ -295,10 +299,12 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t
       const uint32_t q = lq(first ? ud1.x : ud1.y, L, k);
       ldn<NTR, IL>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
       ldn<NTR, IL>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
+      ldn<NTR, IL>(in.ws.gx, lq(first ? ud1.y : ud1.x, L, k), w0, in.ws.sE, in.wtg, gd);
     } else {
       const uint32_t q = first ? q1 : q2;
       ldn<NTR, IL>(in.ws.gnx, q, w0, in.ws.sN, in.wtg, gx);
       ldn<NTR, IL>(in.ws.gny, q, w0, in.ws.sN, in.wtg, gy);
+      ldn<NTR, IL>(in.ws.gnx, first ? q2 : q1, w0, in.ws.sN, in.wtg, gd);
     }
     const double2 c = __ldg(coef + e);
     rec = rec1;
@@ -315,7 +321,7 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t
       const double diff = A2 - A1;
       const double X = divr(2.0 * diff + c.x * gx[t] + c.y * gy[t], r6);
       const double Tm = first ? A1 + X : A2 - X;
-      const double ho = -0.5 * (cu * Tm);
+      const double ho = -0.5 * (cu * Tm) + 0.0 * gd[t];
       adf[t] = ho - fl;
     }
     stn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);

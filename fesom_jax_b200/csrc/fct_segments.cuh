@@ -292,9 +292,9 @@ __device__ __forceinline__ void seg_node_lo(const Inst& in, int64_t si, int t0, 
 // upwind end alone, with Tm = A_u + (2*(A_d - A_u) + edx*a*gx + edy*R*gy)/6 over that end's
 // cell (the up cell at the first node, the down cell at the second; its gradient is one
 // weighted vertex sum whose weights carry the sign of the end). So a level gathers the six
-// values of the upwind side instead of the eight of both. (A non-finite value on the
-// downwind cell still reaches both ends: it makes LO, hence the limiter factors, of the
-// downwind node non-finite.)
+// values of the upwind side instead of the eight of both. (A NaN on the downwind cell still
+// reaches both ends: it makes LO, hence the limiter factors, of the downwind node NaN. After an
+// infinite value one of that node's two factors may be finite, and the upwind end with it.)
 template <int NTR, int LPT, bool IL>
 __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0, int w0) {
   const DevMesh& m = in.m;

@@ -84,3 +84,66 @@ def test_fused_step_keeps_a_nan_within_its_stencil(torch, case, mapping):
         assert not np.isfinite(got[:, v, k]).any()
     bad = ~np.isfinite(got)
     assert not (bad & ~allowed[None]).any()
+
+
+def _reached(m, places):
+    """Edge levels whose flux formula holds a NaN of ``places``: a vertex of the up or down cell
+    (where MFCT takes the cells), or of a cell around either end node (elsewhere)."""
+    from oracle import fct_np
+    T = np.zeros((m.nod2D, m.nl))
+    for v, k in places:
+        T[v, k] = np.nan
+    with np.errstate(invalid="ignore"):
+        g = fct_np.fill_up_dn_grad(m, fct_np.tracer_gradient_elements(m, T))
+    hit = ~np.isfinite(np.asarray(g)).all(axis=tuple(
+        a for a in range(np.ndim(g)) if np.shape(g)[a] not in (m.edge2D, m.nl)))
+    assert hit.shape == (m.edge2D, m.nl) and hit.sum() > 100
+    k = np.arange(m.nl)[None, :]
+    wet = np.zeros(hit.shape, bool)
+    for j in range(2):
+        el = m.edge_tri[:, j]
+        wet |= (el >= 0)[:, None] & (k >= (m.ulevels[el] - 1)[:, None]) & \
+            (k < (m.nlevels[el] - 1)[:, None])
+    return hit & wet
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("stagewise", [False, True])
+def test_a_nan_of_either_gradient_reaches_both_ends(torch, case, stagewise):
+    """The flux weighs the downwind end's gradient with 0, and 0 x NaN is NaN: T_new of both
+    ends is non-finite, in the fused step (by way of LO and the limiter) and stage by stage."""
+    from fesom_jax_b200.tracer_adv import FctPlan
+    m, f, places = case
+    plan = FctPlan(m, 0, max_tracers=3)
+    plan.set_fused(not stagewise)
+    got = plan.forward(*(_dev(torch, x) for x in (f.uv, f.w_e, f.helem, f.hnode, f.hnode_new,
+                                                  _with_nan(f, places), f.tracers_old)),
+                       DT).cpu().numpy()
+    plan.close()
+    e, k = np.nonzero(_reached(m, places))
+    for end in range(2):
+        assert not np.isfinite(got[:, m.edges[e, end], k]).any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tape", [False, True])
+def test_a_nan_of_either_gradient_reaches_the_velocity_gradient(torch, case, tape):
+    """The limiter's sums of both ends have a NaN cotangent then, which the uv of every cell
+    around them receives."""
+    from fesom_jax_b200.adjoint import Tape, advect_one_fct_vjp
+    m, f, places = case
+    args = [_dev(torch, x) for x in (f.uv, f.w_e, f.helem, f.hnode, f.hnode_new,
+                                     _with_nan(f, places)[0], f.tracers_old[0])]
+    kw = {}
+    if tape:
+        kw["tape"] = Tape(m, 1)
+        kw["tape"].forward(0, *args, DT)
+    guv = advect_one_fct_vjp(m, *args, torch.ones_like(args[5]), dt=DT, **kw)[2].cpu().numpy()
+    e, k = np.nonzero(_reached(m, places))
+    near = np.zeros((m.nod2D, m.nl), bool)
+    for end in range(2):
+        near[m.edges[e, end], k] = True
+    kk = np.arange(m.nl)[None, :]
+    wet = (kk >= (m.ulevels - 1)[:, None]) & (kk < (m.nlevels - 1)[:, None])
+    cells = near[m.elem_nodes].any(axis=1) & wet
+    assert cells.sum() > 100 and not np.isfinite(guv[cells]).any()
