@@ -1,11 +1,11 @@
-"""Persistent cache of autotuned thread mappings, per (GPU model, mesh, workload shape).
+"""Persistent cache of autotuned thread mappings, per (GPU model, kernels, mesh, workload shape).
 
 The autotuners (:meth:`fesom_jax_b200.ensemble.Ensemble.autotune`,
 :meth:`fesom_jax_b200.tracer_adv.FctPlan.autotune`) time every candidate mapping of the
 fused stages, which takes seconds on a large batch. With a cache they time once per GPU
 model, mesh and workload shape, store the choice in a JSON file and apply it directly on
-later runs. The mapping only changes speed, never results, so a stale entry costs time,
-not correctness.
+later runs. The mapping only changes speed, never results. An entry holds for the kernels it
+was timed on (:data:`KERNELS`): with others it is passed over and the choice made again.
 
 Default location: ``$FESOM_FCT_TUNING_CACHE``, else
 ``~/.cache/fesom_jax_b200/tuning.json``.
@@ -20,6 +20,12 @@ import tempfile
 from pathlib import Path
 
 import numpy as np
+
+
+# Generation of the fused stages' kernels and mappings, part of every key; to be raised when a
+# change of them moves the fastest mapping. 1: runs of levels only (entries without a number);
+# 2: one level per thread on the stream kernels.
+KERNELS = 2
 
 
 def default_path() -> Path:
@@ -47,11 +53,11 @@ def gpu_name(device: int = 0) -> str:
 
 
 def key(kind: str, gpu: str, meshes, **shape) -> str:
-    """Cache key: the tuner (``kind``), the GPU model, the mesh fingerprints and the
-    workload shape (tracers, members, ...), in a stable order."""
+    """Cache key: the tuner (``kind``), the GPU model, the kernels' generation, the mesh
+    fingerprints and the workload shape (tracers, members, ...), in a stable order."""
     fp = ",".join(sorted(mesh_fingerprint(m) for m in meshes))
     sh = ",".join(f"{k}={shape[k]}" for k in sorted(shape))
-    return f"{kind}|{gpu}|{fp}|{sh}"
+    return f"{kind}|{gpu}|kernels={KERNELS}|{fp}|{sh}"
 
 
 class TuningCache:
