@@ -334,7 +334,8 @@ def run_ours(args, D: Dist) -> dict | None:
         for st, m in enumerate(parse_stage_mapping(args.stage_mapping)):
             ens.set_stage_mapping(st, *m)
     elif fixed:
-        ens.set_mapping(args.chunk or ens.chunk, args.levels or ens.levels)
+        for st, (c, lv) in enumerate(list(ens.stage_map)):   # what is not fixed stays
+            ens.set_stage_mapping(st, args.chunk or c, args.levels or lv)
     torch.cuda.synchronize()
     for _ in range(args.warmup):
         ens.run(S)

@@ -59,6 +59,17 @@ static int batch_launch_steps(FctBatch* b, int phase, int steps, cudaStream_t s)
 
 namespace {
 
+// A group's mapping by the library's rule.
+void batch_auto_map(LaunchDims& d, int count) {
+  d.auto_map(true, seg_even(d), d.max_nseg[0] * d.chunk / 4 * count);
+}
+
+// A changed mapping: the cached graphs are captured again (under graph_mu).
+void drop_graphs(FctBatch* B) {
+  for (auto& kv : B->graphs) cudaGraphExecDestroy(kv.second);
+  B->graphs.clear();
+}
+
 // The kernels index an interleaved array (entity-level x tracer slot) in 32 bits: every
 // such array of instance i must hold fewer than 2^32 elements.
 int check_interleave(const FctPlan* P, int tg, int wtg, int i) {
@@ -179,7 +190,7 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
     d.any_wi = false;
     d.copy_dry = false;
     d.per_thread = std::min(d.chunk, 2);
-    d.auto_map(true, seg_even(d), d.max_nseg[0] * d.chunk / 4 * gr.count);
+    batch_auto_map(d, gr.count);
     gr.dims = d;
   }
   e = cudaMalloc(&B->d_health, size_t(n) * sizeof(unsigned long long));
@@ -232,15 +243,36 @@ int fct_batch_set_mapping(FctBatch* B, int tracers_per_thread, int levels_per_th
     g.dims.per_thread = t;
     g.dims.set_map(t, l);
   }
-  for (auto& kv : B->graphs) cudaGraphExecDestroy(kv.second);   // recapture with the mapping
-  B->graphs.clear();
+  drop_graphs(B);
   return FCT_OK;
 }
 
 int fct_batch_set_chunk(FctBatch* B, int chunk) {
   if (!B) return set_error(FCT_ERR_INVALID, "batch is NULL");
-  const int lpt = B->groups.empty() ? 1 : B->groups[0].dims.smap_levels[kStageLimit];
-  return fct_batch_set_mapping(B, chunk, lpt);
+  if (chunk != 1 && chunk != 2 && chunk != 4 && chunk != 8)
+    return set_error(FCT_ERR_INVALID, "tracers per thread must be 1, 2, 4 or 8");
+  std::lock_guard<std::mutex> lk(B->graph_mu);
+  for (auto& g : B->groups)
+    for (int& t : g.dims.smap_tracers) t = chunk;
+  drop_graphs(B);
+  return FCT_OK;
+}
+
+int fct_batch_reset_mapping(FctBatch* B) {
+  if (!B) return set_error(FCT_ERR_INVALID, "batch is NULL");
+  std::lock_guard<std::mutex> lk(B->graph_mu);
+  for (auto& g : B->groups) batch_auto_map(g.dims, g.count);
+  drop_graphs(B);
+  return FCT_OK;
+}
+
+int fct_batch_get_stage_mapping(const FctBatch* B, int group, int stage, int out[2]) {
+  if (!B || !out) return set_error(FCT_ERR_INVALID, "NULL argument");
+  if (group < 0 || group >= int(B->groups.size()) || stage < 0 || stage >= kFusedStages)
+    return set_error(FCT_ERR_INVALID, "group %d or stage %d out of range", group, stage);
+  out[0] = B->groups[size_t(group)].dims.smap_tracers[stage];
+  out[1] = B->groups[size_t(group)].dims.smap_levels[stage];
+  return FCT_OK;
 }
 
 int fct_batch_set_stage_mapping(FctBatch* B, int stage, int tracers_per_thread,
@@ -257,8 +289,7 @@ int fct_batch_set_stage_mapping(FctBatch* B, int stage, int tracers_per_thread,
     g.dims.smap_tracers[stage] = t;
     g.dims.smap_levels[stage] = l;
   }
-  for (auto& kv : B->graphs) cudaGraphExecDestroy(kv.second);   // recapture with the mapping
-  B->graphs.clear();
+  drop_graphs(B);
   return FCT_OK;
 }
 

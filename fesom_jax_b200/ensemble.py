@@ -53,12 +53,15 @@ def _bind_batch(L):
     L.fct_batch_set_chunk.argtypes = [C.c_void_p, C.c_int]
     L.fct_batch_set_mapping.argtypes = [C.c_void_p, C.c_int, C.c_int]
     L.fct_batch_set_stage_mapping.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_int]
+    L.fct_batch_reset_mapping.argtypes = [C.c_void_p]
+    L.fct_batch_get_stage_mapping.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_int)]
     L.fct_batch_health.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_int64)]
     L.fct_batch_fill_workspace.argtypes = [C.c_void_p, C.c_int, C.c_void_p]
     for n in ("fct_batch_create", "fct_batch_destroy", "fct_batch_info", "fct_batch_prepare",
               "fct_batch_step", "fct_batch_run", "fct_batch_profile", "fct_batch_set_chunk",
               "fct_batch_health", "fct_batch_fill_workspace", "fct_batch_set_mapping",
-              "fct_batch_set_stage_mapping"):
+              "fct_batch_set_stage_mapping", "fct_batch_reset_mapping",
+              "fct_batch_get_stage_mapping"):
         getattr(L, n).restype = C.c_int
     L._batch_bound = True
     return L
@@ -92,11 +95,10 @@ class Ensemble:
         self._plans: dict[int, FctPlan] = {}
         self._h = None
         self.phase = 0
-        self.chunk = 2          # tracers per thread of the fused stages
-        self.levels = 1         # levels per thread
-        # per fused stage (LO, edge, limiter, final); until a mapping is set the library
-        # takes four tracers per thread where a large launch has them
+        # the mapping in force, from build() on: per fused stage (LO, edge, limiter, final) of
+        # the first workspace group, and the most tracers and levels per thread among them
         self.stage_map = [(2, 1)] * 4
+        self.chunk, self.levels = 2, 1
 
     # ---------------------------------------------------------------- members
     def plan(self, mesh: Mesh) -> FctPlan:
@@ -162,6 +164,7 @@ class Ensemble:
         _lib.check(L.fct_batch_create(arr, n, self.workspace_budget, C.byref(h)))
         self._h = h
         self.phase = 0
+        self._read_mapping()
         self.prepare()
 
     def info(self) -> dict:
@@ -207,23 +210,42 @@ class Ensemble:
                                                                     self._stream(stream)))
 
     def set_chunk(self, chunk: int) -> None:
-        """Tracers per thread of the fused stages (1, 2, 4 or 8)."""
-        self.set_mapping(chunk, self.levels)
+        """Tracers per thread of the fused stages (1, 2, 4 or 8); each stage keeps its levels."""
+        _lib.check(_bind_batch(_lib.lib()).fct_batch_set_chunk(self._h, int(chunk)))
+        self._read_mapping()
 
     def set_mapping(self, tracers_per_thread: int, levels_per_thread: int) -> None:
         """Thread mapping of the fused stages: tracers and column levels per thread (each
         1, 2, 4 or 8; 8 tracers with at most 2 levels). Results do not depend on it."""
         _lib.check(_bind_batch(_lib.lib()).fct_batch_set_mapping(
             self._h, int(tracers_per_thread), int(levels_per_thread)))
-        self.chunk, self.levels = int(tracers_per_thread), int(levels_per_thread)
-        self.stage_map = [(self.chunk, self.levels)] * 4
+        self._read_mapping()
 
     def set_stage_mapping(self, stage: int, tracers_per_thread: int,
                           levels_per_thread: int) -> None:
         """The mapping of one fused stage (0 LO, 1 edge, 2 limiter, 3 final)."""
         _lib.check(_bind_batch(_lib.lib()).fct_batch_set_stage_mapping(
             self._h, int(stage), int(tracers_per_thread), int(levels_per_thread)))
-        self.stage_map[int(stage)] = (int(tracers_per_thread), int(levels_per_thread))
+        self._read_mapping()
+
+    def reset_mapping(self) -> None:
+        """Back to the mapping the library chooses (each workspace group its own)."""
+        _lib.check(_bind_batch(_lib.lib()).fct_batch_reset_mapping(self._h))
+        self._read_mapping()
+
+    def group_mapping(self, group: int) -> list:
+        """``(tracers, levels)`` per thread of each fused stage in workspace group ``group``."""
+        L, out = _bind_batch(_lib.lib()), []
+        for i in range(len(self.STAGES)):
+            m = (C.c_int * 2)()
+            _lib.check(L.fct_batch_get_stage_mapping(self._h, int(group), i, m))
+            out.append((m[0], m[1]))
+        return out
+
+    def _read_mapping(self) -> None:
+        self.stage_map = self.group_mapping(0)
+        self.chunk = max(c for c, _ in self.stage_map)
+        self.levels = max(lv for _, lv in self.stage_map)
 
     # (tracers per thread, levels per thread) tried by autotune
     MAPPINGS = ((1, 1), (1, 2), (1, 4), (1, 8), (2, 1), (2, 2), (2, 4), (2, 8), (4, 1), (4, 2),
@@ -247,8 +269,9 @@ class Ensemble:
         """Pick the thread mapping of every fused stage: each (tracers, levels) per-thread
         candidate is timed stage by stage (profile_step) and each stage keeps its fastest;
         the per-stage choice is then timed against the best single mapping for all stages
-        as ``steps``-step graph runs, and the faster stays (the member state advances while
-        tuning). Returns the per-candidate stage times and the choice.
+        and the library's own choice as ``steps``-step graph runs, and the fastest stays (the
+        member state advances while tuning). Returns the per-candidate stage times and the
+        choice.
 
         ``cache``: a :class:`fesom_jax_b200.tuning.TuningCache` (or ``True`` for the default
         file). An entry for this GPU model, these meshes and this batch shape is applied
@@ -264,12 +287,16 @@ class Ensemble:
                             ntr=",".join(str(m.ntr) for m in self.members))
             hit = cache.get(ck)
             if hit:
-                for i, (c, lv) in enumerate(hit["stage_map"]):
-                    self.set_stage_mapping(i, c, lv)
+                if hit.get("chosen") == "default":
+                    self.reset_mapping()
+                else:
+                    for i, (c, lv) in enumerate(hit["stage_map"]):
+                        self.set_stage_mapping(i, c, lv)
                 return dict(cached=True, key=ck, stage_map=hit["stage_map"])
         out = self._autotune(steps, candidates, reps)
         if cache is not None:
             cache.put(ck, dict(stage_map=[list(m) for m in self.stage_map],
+                               chosen=out["chosen"], default_ms=out["default_ms"],
                                per_stage_ms=out["per_stage_ms"], uniform_ms=out["uniform_ms"]))
         return out
 
@@ -288,13 +315,17 @@ class Ensemble:
         for i, m in enumerate(best_stage):
             self.set_stage_mapping(i, *m)
         t_stage = self._graph_ms(steps, reps)
-        if t_uniform < t_stage:
-            self.set_mapping(*uniform)
+        self.reset_mapping()
+        t_default = self._graph_ms(steps, reps)
+        chosen = "default"
+        if min(t_stage, t_uniform) <= t_default:
+            chosen = "per_stage" if t_stage <= t_uniform else "uniform"
+            for i, m in enumerate(best_stage if chosen == "per_stage" else [uniform] * 4):
+                self.set_stage_mapping(i, *m)
         return dict(stage_ms={f"{c}x{lv}": prof[(c, lv)] for c, lv in cands},
                     per_stage={st: f"{m[0]}x{m[1]}" for st, m in zip(self.STAGES, best_stage)},
                     per_stage_ms=t_stage, uniform=f"{uniform[0]}x{uniform[1]}",
-                    uniform_ms=t_uniform,
-                    chosen="per_stage" if t_stage <= t_uniform else "uniform")
+                    uniform_ms=t_uniform, default_ms=t_default, chosen=chosen)
 
     def profile_step(self, stream=None) -> dict:
         """Run one step stage by stage (synchronising) and return ``{stage: ms}``."""

@@ -363,8 +363,8 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t workspace_budget_b
                      FctBatch** out);
 int fct_batch_destroy(FctBatch* b);
 /* Tuning: the most tracers one thread carries (1, 2, 4 or 8; by default the library
- * chooses per stage). Fewer use fewer registers (higher occupancy), more share each
- * gather's index work. Drops cached graphs. */
+ * chooses per stage); every stage keeps its levels per thread. Fewer use fewer registers
+ * (higher occupancy), more share each gather's index work. Drops cached graphs. */
 int fct_batch_set_chunk(FctBatch* b, int chunk);
 /* Tuning: tracers per thread (1, 2, 4 or 8; the fused stages carry at most 4) and levels
  * per thread (1, 2, 4 or 8) of the fused stages. Drops cached graphs. */
@@ -373,6 +373,11 @@ int fct_batch_set_mapping(FctBatch* b, int tracers_per_thread, int levels_per_th
  * stages are separate kernels, so each may take its own mapping). Drops cached graphs. */
 int fct_batch_set_stage_mapping(FctBatch* b, int stage, int tracers_per_thread,
                                 int levels_per_thread);
+/* Back to the mapping that the library chooses, each workspace group its own. */
+int fct_batch_reset_mapping(FctBatch* b);
+/* The mapping in force of a stage in workspace group ``group``: out = [most tracers per
+ * thread, levels per thread]. */
+int fct_batch_get_stage_mapping(const FctBatch* b, int group, int stage, int out[2]);
 /* [instances, groups, workspace bytes, total wet node layers x tracers,
  *  tracers per workspace chunk (largest over groups), kernel launches per step (of
  *  fct_batch_step; in an fct_batch_run the volume fluxes, and w_derived, are launched in
