@@ -19,8 +19,8 @@
 //
 // Each thread owns one lane and NTR tracers (a compile-time chunk of the instance's
 // tracers, which share its velocities): mesh indices, geometry and velocity terms are
-// loaded once per lane and every neighbour gather issues NTR independent loads (one
-// contiguous chunk in the interleaved layout), so the gathers overlap.
+// loaded once per lane and every neighbour gather issues NTR independent loads, so the
+// gathers overlap.
 #include <algorithm>
 
 #include "fct_columns.cuh"
@@ -70,21 +70,21 @@ __device__ __forceinline__ void body_vflux(const Inst& in, int64_t i, int64_t st
   }
 }
 
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_elem_grad(const Inst& in, int64_t i, int t0, int w0) {
   const DevMesh& m = in.m;
   if (i >= m.n_elem) return;
   const uint32_t lane = ld(m.elem_lanes + i);
   const int e = lane_ent(lane), k = lane_lev(lane), L = m.L;
   double gx[NTR], gy[NTR];
-  cell_grad<NTR, IL>(in, e, k, t0, gx, gy);
+  cell_grad<NTR, false>(in, e, k, t0, gx, gy);
   const uint32_t q = lq(e, L, k);
-  stn<NTR, IL>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
-  stn<NTR, IL>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
+  stn<NTR, false>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
+  stn<NTR, false>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
 }
 
 // -------------------------------- LO solution, node-average gradient, adf_v
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, int w0) {
   const DevMesh& m = in.m;
   if (i >= m.n_iface) return;
@@ -103,8 +103,8 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
   const int tg = in.tg;
 
   double Tc[NTR], Ta[NTR];   // T[k], T[k-1]
-  ldn<NTR, IL>(in.T, qn, t0, ts, tg, Tc);
-  ldn<NTR, IL>(in.T, base + km1, t0, ts, tg, Ta);
+  ldn<NTR, false>(in.T, qn, t0, ts, tg, Tc);
+  ldn<NTR, false>(in.T, base + km1, t0, ts, tg, Ta);
   double fvk[NTR];
 #pragma unroll
   for (int t = 0; t < NTR; ++t) fvk[t] = layer ? vflux_up(Tc[t], Ta[t], w, area_k) : 0.0;
@@ -119,7 +119,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
     if (layer1) {
       const double w1 = ld(in.w_e + qn + 1), area1 = ld(m.area + qn + 1);
       double Tb[NTR];
-      ldn<NTR, IL>(in.T, qn + 1, t0, ts, tg, Tb);
+      ldn<NTR, false>(in.T, qn + 1, t0, ts, tg, Tb);
 #pragma unroll
       for (int t = 0; t < NTR; ++t) fvk1[t] = vflux_up(Tb[t], Tc[t], w1, area1);
     } else {
@@ -141,7 +141,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
       // the face flux with the node's own value first (a + b == b + a exactly)
       const double cown = sl.z ? vf - avf : vf + avf, coth = sl.z ? vf + avf : vf - avf;
       double To[NTR];
-      ldn<NTR, IL>(in.T, uint32_t(sl.y) + uint32_t(k), t0, ts, tg, To);
+      ldn<NTR, false>(in.T, uint32_t(sl.y) + uint32_t(k), t0, ts, tg, To);
 #pragma unroll
       for (int t = 0; t < NTR; ++t) {
         const double fl = -0.5 * (Tc[t] * cown + To[t] * coth);
@@ -155,7 +155,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
     for (int t = 0; t < NTR; ++t)
       lo[t] = valid ? divr(Tc[t] * hn + divr((div[t] + (fvk[t] - fvk1[t])) * dt, rav), rhn)
                     : 0.0;
-    stn<NTR, IL>(in.ws.lo, qn, w0, in.ws.sN, in.wtg, lo);
+    stn<NTR, false>(in.ws.lo, qn, w0, in.ws.sN, in.wtg, lo);
     // _node_avg_grad: area-weighted mean over the node's active elements, at the levels
     // where an edge of the node takes it (kGradBit; its readers, the edge stage's and the
     // reverse pass's node-gradient lanes, read no other level)
@@ -170,8 +170,8 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
           const double a = ld(m.earea + el);
           const uint32_t qe = lq(el, L, k);
           double gx[NTR], gy[NTR];
-          ldn<NTR, IL>(in.ws.gx, qe, w0, in.ws.sE, in.wtg, gx);
-          ldn<NTR, IL>(in.ws.gy, qe, w0, in.ws.sE, in.wtg, gy);
+          ldn<NTR, false>(in.ws.gx, qe, w0, in.ws.sE, in.wtg, gx);
+          ldn<NTR, false>(in.ws.gy, qe, w0, in.ws.sE, in.wtg, gy);
 #pragma unroll
           for (int t = 0; t < NTR; ++t) {
             nx[t] += gx[t] * a;
@@ -187,8 +187,8 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
         nx[t] = divr(nx[t], rdd);
         ny[t] = divr(ny[t], rdd);
       }
-      stn<NTR, IL>(in.ws.gnx, qn, w0, in.ws.sN, in.wtg, nx);
-      stn<NTR, IL>(in.ws.gny, qn, w0, in.ws.sN, in.wtg, ny);
+      stn<NTR, false>(in.ws.gnx, qn, w0, in.ws.sN, in.wtg, nx);
+      stn<NTR, false>(in.ws.gny, qn, w0, in.ws.sN, in.wtg, ny);
     }
   }
 
@@ -198,15 +198,15 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
   for (int t = 0; t < NTR; ++t) hi[t] = 0.0;
   if (k == nzmin) {
     double To[NTR];
-    ldn<NTR, IL>(in.T_old, qn, t0, ts, tg, To);
+    ldn<NTR, false>(in.T_old, qn, t0, ts, tg, To);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) hi[t] = -ab2(Tc[t], To[t]) * Wf * area_k;
   } else if (k == nzmax) {
     // bottom interface: no flux
   } else if (k == nzmin + 1 || k == nzmax - 1) {
     double To[NTR], Tom[NTR];
-    ldn<NTR, IL>(in.T_old, qn, t0, ts, tg, To);
-    ldn<NTR, IL>(in.T_old, qn - 1, t0, ts, tg, Tom);
+    ldn<NTR, false>(in.T_old, qn, t0, ts, tg, To);
+    ldn<NTR, false>(in.T_old, qn - 1, t0, ts, tg, Tom);
 #pragma unroll
     for (int t = 0; t < NTR; ++t)
       hi[t] = -0.5 * (ab2(Ta[t], Tom[t]) + ab2(Tc[t], To[t])) * Wf * area_k;
@@ -232,12 +232,12 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
     }
     const Rcp r3{3.0, 1.0 / 3.0, true};
     double To[NTR], Tom[NTR], Tm2[NTR], Tom2[NTR], Tp[NTR], Top[NTR];
-    ldn<NTR, IL>(in.T_old, qn, t0, ts, tg, To);
-    ldn<NTR, IL>(in.T_old, qn - 1, t0, ts, tg, Tom);
-    ldn<NTR, IL>(in.T, qn - 2, t0, ts, tg, Tm2);
-    ldn<NTR, IL>(in.T_old, qn - 2, t0, ts, tg, Tom2);
-    ldn<NTR, IL>(in.T, qn + 1, t0, ts, tg, Tp);
-    ldn<NTR, IL>(in.T_old, qn + 1, t0, ts, tg, Top);
+    ldn<NTR, false>(in.T_old, qn, t0, ts, tg, To);
+    ldn<NTR, false>(in.T_old, qn - 1, t0, ts, tg, Tom);
+    ldn<NTR, false>(in.T, qn - 2, t0, ts, tg, Tm2);
+    ldn<NTR, false>(in.T_old, qn - 2, t0, ts, tg, Tom2);
+    ldn<NTR, false>(in.T, qn + 1, t0, ts, tg, Tp);
+    ldn<NTR, false>(in.T_old, qn + 1, t0, ts, tg, Top);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
       const double A0 = ab2(Tc[t], To[t]), Am1 = ab2(Ta[t], Tom[t]);
@@ -256,7 +256,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
     const double lo_v = in.w_i ? (layer ? vflux_up(Tc[t], Ta[t], Wf, area_k) : 0.0) : fvk[t];
     adf[t] = hi[t] - lo_v;
   }
-  stn<NTR, IL>(in.ws.adfv, qn, w0, in.ws.sN, in.wtg, adf);
+  stn<NTR, false>(in.ws.adfv, qn, w0, in.ws.sN, in.wtg, adf);
 }
 
 // -------------------------- fill_up_dn_grad + adv_flux_hor_ho - LO flux = adf_h
@@ -268,7 +268,7 @@ __device__ __forceinline__ void body_node_lo(const Inst& in, int64_t i, int t0, 
 // 24.6 with it, 24.9 with both gradients in full here and in r_edge. A thread walks the lanes
 // i, i + stride, ...: the next lane's record, volume flux and cells are loaded while this lane's
 // gathers are under way.
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t stride, int t0,
                                               int w0) {
   const DevMesh& m = in.m;
@@ -290,21 +290,21 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t
     const uint32_t q1 = lq(rec.y, L, k), q2 = lq(rec.z, L, k);
     const bool first = vf > 0.0;
     double T1[NTR], T2[NTR], O1[NTR], O2[NTR], gx[NTR], gy[NTR], gd[NTR];
-    ldn<NTR, IL>(in.T, q1, t0, ts, tg, T1);
-    ldn<NTR, IL>(in.T, q2, t0, ts, tg, T2);
-    ldn<NTR, IL>(in.T_old, q1, t0, ts, tg, O1);
-    ldn<NTR, IL>(in.T_old, q2, t0, ts, tg, O2);
+    ldn<NTR, false>(in.T, q1, t0, ts, tg, T1);
+    ldn<NTR, false>(in.T, q2, t0, ts, tg, T2);
+    ldn<NTR, false>(in.T_old, q1, t0, ts, tg, O1);
+    ldn<NTR, false>(in.T_old, q2, t0, ts, tg, O2);
     if (use_tri) {
       // both cells are wet at k here (k is above every adjacent cell's bottom)
       const uint32_t q = lq(first ? ud1.x : ud1.y, L, k);
-      ldn<NTR, IL>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
-      ldn<NTR, IL>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
-      ldn<NTR, IL>(in.ws.gx, lq(first ? ud1.y : ud1.x, L, k), w0, in.ws.sE, in.wtg, gd);
+      ldn<NTR, false>(in.ws.gx, q, w0, in.ws.sE, in.wtg, gx);
+      ldn<NTR, false>(in.ws.gy, q, w0, in.ws.sE, in.wtg, gy);
+      ldn<NTR, false>(in.ws.gx, lq(first ? ud1.y : ud1.x, L, k), w0, in.ws.sE, in.wtg, gd);
     } else {
       const uint32_t q = first ? q1 : q2;
-      ldn<NTR, IL>(in.ws.gnx, q, w0, in.ws.sN, in.wtg, gx);
-      ldn<NTR, IL>(in.ws.gny, q, w0, in.ws.sN, in.wtg, gy);
-      ldn<NTR, IL>(in.ws.gnx, first ? q2 : q1, w0, in.ws.sN, in.wtg, gd);
+      ldn<NTR, false>(in.ws.gnx, q, w0, in.ws.sN, in.wtg, gx);
+      ldn<NTR, false>(in.ws.gny, q, w0, in.ws.sN, in.wtg, gy);
+      ldn<NTR, false>(in.ws.gnx, first ? q2 : q1, w0, in.ws.sN, in.wtg, gd);
     }
     const double2 c = __ldg(coef + e);
     rec = rec1;
@@ -324,12 +324,12 @@ __device__ __forceinline__ void body_edge_adf(const Inst& in, int64_t i, int64_t
       const double ho = -0.5 * (cu * Tm) + 0.0 * gd[t];
       adf[t] = ho - fl;
     }
-    stn<NTR, IL>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);
+    stn<NTR, false>(in.ws.adfh, lq(e, L, k), w0, in.ws.sEd, in.wtg, adf);
   }
 }
 
 // ------------------------ zalesak a2: element max/min of the LO/T window
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_elem_bounds(const Inst& in, int64_t i, int t0, int w0) {
   const DevMesh& m = in.m;
   if (i >= m.n_elem) return;
@@ -344,8 +344,8 @@ __device__ __forceinline__ void body_elem_bounds(const Inst& in, int64_t i, int 
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
     double a[NTR], b[NTR];
-    ldn<NTR, IL>(in.ws.lo, q[v], w0, in.ws.sN, in.wtg, a);
-    ldn<NTR, IL>(in.T, q[v], t0, in.tstride, in.tg, b);
+    ldn<NTR, false>(in.ws.lo, q[v], w0, in.ws.sN, in.wtg, a);
+    ldn<NTR, false>(in.T, q[v], t0, in.tstride, in.tg, b);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
       hi[v][t] = fmax(a[t], b[t]);
@@ -362,15 +362,15 @@ __device__ __forceinline__ void body_elem_bounds(const Inst& in, int64_t i, int 
       cx[t] = (hi[0][t] == mx[t]) + (hi[1][t] == mx[t]) + (hi[2][t] == mx[t]);
       cn[t] = (lw[0][t] == mn[t]) + (lw[1][t] == mn[t]) + (lw[2][t] == mn[t]);
     }
-    stc<NTR, IL>(in.ws.ecx, qe, w0, in.ws.sE, in.wtg, cx);
-    stc<NTR, IL>(in.ws.ecn, qe, w0, in.ws.sE, in.wtg, cn);
+    stc<NTR, false>(in.ws.ecx, qe, w0, in.ws.sE, in.wtg, cx);
+    stc<NTR, false>(in.ws.ecn, qe, w0, in.ws.sE, in.wtg, cn);
   }
-  stn<NTR, IL>(in.ws.amax, qe, w0, in.ws.sE, in.wtg, mx);
-  stn<NTR, IL>(in.ws.amin, qe, w0, in.ws.sE, in.wtg, mn);
+  stn<NTR, false>(in.ws.amax, qe, w0, in.ws.sE, in.wtg, mx);
+  stn<NTR, false>(in.ws.amin, qe, w0, in.ws.sE, in.wtg, mn);
 }
 
 // ------------------------ zalesak a3: node cluster max/min over elements
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int t0, int w0) {
   const DevMesh& m = in.m;
   if (i >= m.n_layer) return;
@@ -385,8 +385,8 @@ __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int
     if (k >= ld(m.eul + el) && k < ld(m.enl + el)) {
       const uint32_t q = lq(el, L, k);
       double a[NTR], b[NTR];
-      ldn<NTR, IL>(in.ws.amax, q, w0, in.ws.sE, in.wtg, a);
-      ldn<NTR, IL>(in.ws.amin, q, w0, in.ws.sE, in.wtg, b);
+      ldn<NTR, false>(in.ws.amax, q, w0, in.ws.sE, in.wtg, a);
+      ldn<NTR, false>(in.ws.amin, q, w0, in.ws.sE, in.wtg, b);
 #pragma unroll
       for (int t = 0; t < NTR; ++t) {
         mx[t] = fmax(mx[t], a[t]);
@@ -401,8 +401,8 @@ __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int
     }
   }
   const uint32_t qn = lq(n, L, k);
-  stn<NTR, IL>(in.ws.tvmax, qn, w0, in.ws.sN, in.wtg, mx);
-  stn<NTR, IL>(in.ws.tvmin, qn, w0, in.ws.sN, in.wtg, mn);
+  stn<NTR, false>(in.ws.tvmax, qn, w0, in.ws.sN, in.wtg, mx);
+  stn<NTR, false>(in.ws.tvmin, qn, w0, in.ws.sN, in.wtg, mn);
   // cells attaining the cluster bounds (padded values included), for the reverse pass
   int cx[NTR], cn[NTR];
 #pragma unroll
@@ -412,8 +412,8 @@ __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int
     double a[NTR], b[NTR];
     if (k >= ld(m.eul + el) && k < ld(m.enl + el)) {
       const uint32_t q = lq(el, L, k);
-      ldn<NTR, IL>(in.ws.amax, q, w0, in.ws.sE, in.wtg, a);
-      ldn<NTR, IL>(in.ws.amin, q, w0, in.ws.sE, in.wtg, b);
+      ldn<NTR, false>(in.ws.amax, q, w0, in.ws.sE, in.wtg, a);
+      ldn<NTR, false>(in.ws.amin, q, w0, in.ws.sE, in.wtg, b);
     } else {
 #pragma unroll
       for (int t = 0; t < NTR; ++t) { a[t] = -kBig; b[t] = kBig; }
@@ -424,12 +424,12 @@ __device__ __forceinline__ void body_node_cluster(const Inst& in, int64_t i, int
       cn[t] += b[t] == mn[t];
     }
   }
-  stc<NTR, IL>(in.ws.ccx, qn, w0, in.ws.sN, in.wtg, cx);
-  stc<NTR, IL>(in.ws.ccn, qn, w0, in.ws.sN, in.wtg, cn);
+  stc<NTR, false>(in.ws.ccx, qn, w0, in.ws.sN, in.wtg, cx);
+  stc<NTR, false>(in.ws.ccn, qn, w0, in.ws.sN, in.wtg, cn);
 }
 
 // ------------------- zalesak a4 + b1 + b2: admissible window, sums, factors
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int t0, int w0) {
   const DevMesh& m = in.m;
   if (i >= m.n_layer) return;
@@ -447,14 +447,14 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
   const double dt = in.dt;
   const int64_t sN = in.ws.sN;
   double tmax[NTR], tmin[NTR];
-  ldn<NTR, IL>(in.ws.tvmax, qn, w0, sN, in.wtg, tmax);
-  ldn<NTR, IL>(in.ws.tvmin, qn, w0, sN, in.wtg, tmin);
+  ldn<NTR, false>(in.ws.tvmax, qn, w0, sN, in.wtg, tmax);
+  ldn<NTR, false>(in.ws.tvmin, qn, w0, sN, in.wtg, tmin);
   if (!use_own) {   // interior: max/min over k-1, k, k+1 (all layers of this column)
     double am[NTR], an[NTR], bm[NTR], bn[NTR];
-    ldn<NTR, IL>(in.ws.tvmax, qn - 1, w0, sN, in.wtg, am);
-    ldn<NTR, IL>(in.ws.tvmin, qn - 1, w0, sN, in.wtg, an);
-    ldn<NTR, IL>(in.ws.tvmax, qn + 1, w0, sN, in.wtg, bm);
-    ldn<NTR, IL>(in.ws.tvmin, qn + 1, w0, sN, in.wtg, bn);
+    ldn<NTR, false>(in.ws.tvmax, qn - 1, w0, sN, in.wtg, am);
+    ldn<NTR, false>(in.ws.tvmin, qn - 1, w0, sN, in.wtg, an);
+    ldn<NTR, false>(in.ws.tvmax, qn + 1, w0, sN, in.wtg, bm);
+    ldn<NTR, false>(in.ws.tvmin, qn + 1, w0, sN, in.wtg, bn);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
       tmax[t] = fmax(fmax(am[t], tmax[t]), bm[t]);
@@ -462,9 +462,9 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
     }
   }
   double lo[NTR], ft[NTR], fb[NTR];
-  ldn<NTR, IL>(in.ws.lo, qn, w0, sN, in.wtg, lo);
-  ldn<NTR, IL>(in.ws.adfv, qn, w0, sN, in.wtg, ft);
-  ldn<NTR, IL>(in.ws.adfv, qn + 1, w0, sN, in.wtg, fb);   // k+1 <= nzmax < L
+  ldn<NTR, false>(in.ws.lo, qn, w0, sN, in.wtg, lo);
+  ldn<NTR, false>(in.ws.adfv, qn, w0, sN, in.wtg, ft);
+  ldn<NTR, false>(in.ws.adfv, qn + 1, w0, sN, in.wtg, fb);   // k+1 <= nzmax < L
   double sp[NTR], sm[NTR];
 #pragma unroll
   for (int t = 0; t < NTR; ++t) sp[t] = sm[t] = 0.0;
@@ -474,7 +474,7 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
     const int4 sl = __ldg(m.ns4 + j);
     if (!(onb & 1u)) continue;   // no flux on this level
     double a[NTR];
-    ldn<NTR, IL>(in.ws.adfh, uint32_t(sl.x) + uint32_t(k), w0, in.ws.sEd, in.wtg, a);
+    ldn<NTR, false>(in.ws.adfh, uint32_t(sl.x) + uint32_t(k), w0, in.ws.sEd, in.wtg, a);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
       const double s = sl.z ? -a[t] : a[t];
@@ -498,14 +498,14 @@ __device__ __forceinline__ void body_node_factors(const Inst& in, int64_t i, int
       mf[t] = fmin(1.0, (tmin[t] - lo[t]) / flux_neg);
     }
   }
-  stn<NTR, IL>(in.ws.pf, qn, w0, sN, in.wtg, pf);
-  stn<NTR, IL>(in.ws.mf, qn, w0, sN, in.wtg, mf);
-  stn<NTR, IL>(in.ws.fplus, qn, w0, sN, in.wtg, pl);    // kept for the reverse pass
-  stn<NTR, IL>(in.ws.fminus, qn, w0, sN, in.wtg, mi);
+  stn<NTR, false>(in.ws.pf, qn, w0, sN, in.wtg, pf);
+  stn<NTR, false>(in.ws.mf, qn, w0, sN, in.wtg, mf);
+  stn<NTR, false>(in.ws.fplus, qn, w0, sN, in.wtg, pl);    // kept for the reverse pass
+  stn<NTR, false>(in.ws.fminus, qn, w0, sN, in.wtg, mi);
 }
 
 // ---------- zalesak b3 + flux2dtracer_fct + ale_reconstruct: T_new on layers
-template <int NTR, bool IL>
+template <int NTR>
 __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t0, int w0) {
   const DevMesh& m = in.m;
   if (i >= m.n_layer) return;
@@ -523,9 +523,9 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
   const int64_t sN = in.ws.sN;
   // own limiter factors at k (and k-1 / k+1 for the vertical fluxes)
   double pf0[NTR], mf0[NTR], ft[NTR];
-  ldn<NTR, IL>(in.ws.pf, qn, w0, sN, in.wtg, pf0);
-  ldn<NTR, IL>(in.ws.mf, qn, w0, sN, in.wtg, mf0);
-  ldn<NTR, IL>(in.ws.adfv, qn, w0, sN, in.wtg, ft);
+  ldn<NTR, false>(in.ws.pf, qn, w0, sN, in.wtg, pf0);
+  ldn<NTR, false>(in.ws.mf, qn, w0, sN, in.wtg, mf0);
+  ldn<NTR, false>(in.ws.adfv, qn, w0, sN, in.wtg, ft);
   // limited vertical flux at the top interface k (tracer_adv.py:453-459)
   double vt[NTR];
   if (k == nzmin) {
@@ -533,8 +533,8 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
     for (int t = 0; t < NTR; ++t) vt[t] = (ft[t] >= 0.0 ? pf0[t] : mf0[t]) * ft[t];
   } else {
     double pfa[NTR], mfa[NTR];
-    ldn<NTR, IL>(in.ws.pf, qn - 1, w0, sN, in.wtg, pfa);
-    ldn<NTR, IL>(in.ws.mf, qn - 1, w0, sN, in.wtg, mfa);
+    ldn<NTR, false>(in.ws.pf, qn - 1, w0, sN, in.wtg, pfa);
+    ldn<NTR, false>(in.ws.mf, qn - 1, w0, sN, in.wtg, mfa);
 #pragma unroll
     for (int t = 0; t < NTR; ++t)
       vt[t] = (ft[t] >= 0.0 ? fmin(mfa[t], pf0[t]) : fmin(pfa[t], mf0[t])) * ft[t];
@@ -546,9 +546,9 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
     for (int t = 0; t < NTR; ++t) vb[t] = 0.0;
   } else {
     double fb[NTR], pfb[NTR], mfb[NTR];
-    ldn<NTR, IL>(in.ws.adfv, qn + 1, w0, sN, in.wtg, fb);
-    ldn<NTR, IL>(in.ws.pf, qn + 1, w0, sN, in.wtg, pfb);
-    ldn<NTR, IL>(in.ws.mf, qn + 1, w0, sN, in.wtg, mfb);
+    ldn<NTR, false>(in.ws.adfv, qn + 1, w0, sN, in.wtg, fb);
+    ldn<NTR, false>(in.ws.pf, qn + 1, w0, sN, in.wtg, pfb);
+    ldn<NTR, false>(in.ws.mf, qn + 1, w0, sN, in.wtg, mfb);
 #pragma unroll
     for (int t = 0; t < NTR; ++t)
       vb[t] = (fb[t] >= 0.0 ? fmin(mf0[t], pfb[t]) : fmin(pf0[t], mfb[t])) * fb[t];
@@ -564,9 +564,9 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
     if (!(onb & 1u)) continue;   // no flux on this level
     const uint32_t qo = uint32_t(sl.y) + uint32_t(k);
     double a[NTR], pfo[NTR], mfo[NTR];
-    ldn<NTR, IL>(in.ws.adfh, uint32_t(sl.x) + uint32_t(k), w0, in.ws.sEd, in.wtg, a);
-    ldn<NTR, IL>(in.ws.pf, qo, w0, sN, in.wtg, pfo);
-    ldn<NTR, IL>(in.ws.mf, qo, w0, sN, in.wtg, mfo);
+    ldn<NTR, false>(in.ws.adfh, uint32_t(sl.x) + uint32_t(k), w0, in.ws.sEd, in.wtg, a);
+    ldn<NTR, false>(in.ws.pf, qo, w0, sN, in.wtg, pfo);
+    ldn<NTR, false>(in.ws.mf, qo, w0, sN, in.wtg, mfo);
 #pragma unroll
     for (int t = 0; t < NTR; ++t) {
       // ae = a >= 0 ? min(plus(n1), minus(n2)) : min(minus(n1), plus(n2)): the own plus and
@@ -578,8 +578,8 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
     }
   }
   double Tv[NTR], lo[NTR], out[NTR];
-  ldn<NTR, IL>(in.T, qn, t0, in.tstride, tg, Tv);
-  ldn<NTR, IL>(in.ws.lo, qn, w0, sN, in.wtg, lo);
+  ldn<NTR, false>(in.T, qn, t0, in.tstride, tg, Tv);
+  ldn<NTR, false>(in.ws.lo, qn, w0, sN, in.wtg, lo);
 #pragma unroll
   for (int t = 0; t < NTR; ++t) {
     const double lo_trans = -Tv[t] * hn + lo[t] * hnn;
@@ -588,16 +588,14 @@ __device__ __forceinline__ void body_node_final(const Inst& in, int64_t i, int t
     d = d + Tv[t] * (hn - hnn);
     out[t] = Tv[t] + (hnn > 0.0 ? divr(d, rhn) : 0.0);
   }
-  stn<NTR, IL>(in.T_new, qn, t0, in.tstride, tg, out);
+  stn<NTR, false>(in.T_new, qn, t0, in.tstride, tg, out);
   count_nonfinite<NTR>(in.nonfinite, out);
 }
 
-// Kernel wrappers: ``_1`` takes one instance by value (tracer-major layout, the
-// single-call path); ``_n`` reads instance blockIdx.y of a device table (interleaved
-// layout, the batched path). A launch covers S = 2^lg tracer slices of NTR tracers each:
-// in ``_n`` the S threads of a lane are adjacent (slice = thread index mod S), so they
-// read one contiguous run of S*NTR interleaved tracers together; in ``_1`` the slice is
-// blockIdx.y, so lanes stay contiguous along x within each tracer plane.
+// Kernel wrappers: ``_1`` takes one instance by value, ``_n`` reads instance blockIdx.y of a
+// device table (interleaved layout, the batched path). The stage-by-stage kernels take one
+// instance (tracer-major); a launch covers S = 2^lg tracer slices of NTR tracers each, the
+// slice is blockIdx.y, so lanes stay contiguous along x within each tracer plane.
 // Resident 256-thread blocks per SM the compiler must fit (registers capped
 // accordingly): latency hiding pays more than the spills it costs (one tracer, the
 // adjoint's taped forward on the CORE2-size mesh: 11.1 ms for 10 steps at 6 blocks,
@@ -610,17 +608,8 @@ constexpr int kMinBlocks = NTR == 1 ? 7 : NTR == 2 ? 5 : NTR == 4 ? 4 : 2;
   __global__ void __launch_bounds__(256, kMinBlocks<NTR>) name##_1(                       \
       const __grid_constant__ Inst in, int t0, int w0) {                                \
     const int sub = int(blockIdx.y) * NTR;                                              \
-    body<NTR, false>(in, lane_index(), t0 + sub, w0 + sub);                             \
-  }                                                                                     \
-  template <int NTR>                                                                    \
-  __global__ void __launch_bounds__(256, kMinBlocks<NTR>) name##_n(                     \
-      const Inst* __restrict__ tab, int t0,                                             \
-                                                  int w0, int lg) {                     \
-    const int64_t g = lane_index();                                                     \
-    const int sub = int(g & ((int64_t(1) << lg) - 1)) * NTR;                            \
-    body<NTR, true>(tab[blockIdx.y], g >> lg, t0 + sub, w0 + sub);                      \
+    body<NTR>(in, lane_index(), t0 + sub, w0 + sub);                                    \
   }
-
 
 // unfused stages (every intermediate in the workspace; the reverse pass reads them)
 FCT_KERNEL_T(k_elem_grad, body_elem_grad)
@@ -632,7 +621,7 @@ template <int NTR>
 __global__ void __launch_bounds__(256, kWalkBlocks<NTR>) k_edge_adf_1(
     const __grid_constant__ Inst in, int t0, int w0) {
   const int sub = int(blockIdx.y) * NTR;
-  body_edge_adf<NTR, false>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub);
+  body_edge_adf<NTR>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub);
 }
 FCT_KERNEL_T(k_elem_bounds, body_elem_bounds)
 FCT_KERNEL_T(k_node_cluster, body_node_cluster)
@@ -684,13 +673,7 @@ const char* const kStageNames[kNumStages] = {
 // power of two (at most 8) with S*NTR tracers left; the workspace index of tracer t is
 // t - c0.
 #define FCT_STAGE_AS(name, lanes, P)                                                    \
-  do {                                                                                  \
-    if (tab)                                                                            \
-      name##_n<P><<<dim3(xblocks(int64_t(lanes) << lg), unsigned(n)), B, 0, s>>>(        \
-          tab, t0, w0, lg);                                                             \
-    else                                                                                \
-      name##_1<P><<<dim3(xblocks(lanes), 1u << lg), B, 0, s>>>(single, t0, w0);          \
-  } while (0)
+  name##_1<P><<<dim3(xblocks(lanes), 1u << lg), B, 0, s>>>(single, t0, w0)
 
 #define FCT_SPLIT(AS, name, lanes)                                                      \
   do {                                                                                  \
@@ -709,7 +692,7 @@ const char* const kStageNames[kNumStages] = {
     }                                                                                   \
   } while (0)
 #define FCT_STAGE(name, lanes) FCT_SPLIT(FCT_STAGE_AS, name, lanes)
-// a stage whose threads walk its lanes (single instances: the reverse pass's stages)
+// a stage whose threads walk its lanes
 #define FCT_WALK_AS(name, lanes, P)                                                     \
   name##_1<P><<<dim3(unsigned(std::min<int64_t>(xblocks(lanes), 148 * kWalkBlocks<P>)),  \
                      1u << lg), B, 0, s>>>(single, t0, w0)
@@ -783,6 +766,8 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
     return unsigned(std::max<int64_t>(1, (lanes + B - 1) / B));
   };
   auto grid = [&](int64_t lanes) { return dim3(xblocks(lanes), unsigned(n), 1); };
+  if (tab && !d.fused)   // (their kernels read ``single``)
+    return set_error(FCT_ERR_INVALID, "the stage-by-stage kernels take one instance");
   const int chunk = d.chunk > 0 ? d.chunk : d.ntr;
   const int nchunks = (d.ntr + chunk - 1) / chunk;
   // the dry-level copy on the side stream, beside the stages (190 of 9,200 us of a step of
