@@ -1004,7 +1004,7 @@ LaunchDims unfused_dims(const FctPlan* P, int ntr) {
   d.max_elem = P->hm.n_elem; d.max_dense = int64_t(P->N) * P->L; d.max_nodes = P->N;
   d.max_dry = P->hm.n_dry;
   d.max_levels = P->L;
-  d.ntr = ntr; d.chunk = 0; d.per_thread = 8; d.any_wi = false; d.copy_dry = true;
+  d.ntr = ntr; d.chunk = 0; d.any_wi = false; d.copy_dry = true;
   d.fused = false;   // the reverse kernels read every stage's intermediates
   return d;
 }

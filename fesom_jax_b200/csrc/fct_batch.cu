@@ -189,7 +189,6 @@ int fct_batch_create(const FctInstance* insts, int n, int64_t budget, FctBatch**
     }
     d.any_wi = false;
     d.copy_dry = false;
-    d.per_thread = std::min(d.chunk, 2);
     batch_auto_map(d, gr.count);
     gr.dims = d;
   }
@@ -239,10 +238,7 @@ int fct_batch_set_mapping(FctBatch* B, int tracers_per_thread, int levels_per_th
   if ((t != 1 && t != 2 && t != 4 && t != 8) || (l != 1 && l != 2 && l != 4 && l != 8))
     return set_error(FCT_ERR_INVALID, "tracers and levels per thread must be 1, 2, 4 or 8");
   std::lock_guard<std::mutex> lk(B->graph_mu);
-  for (auto& g : B->groups) {
-    g.dims.per_thread = t;
-    g.dims.set_map(t, l);
-  }
+  for (auto& g : B->groups) g.dims.set_map(t, l);
   drop_graphs(B);
   return FCT_OK;
 }
@@ -615,7 +611,6 @@ int fct_serve_step(FctServe* S, const FctInstance* insts, const int32_t* phases,
     }
     d.ntr = ntr;
     d.chunk = 0;
-    d.per_thread = 2;   // (the diffusion epilogue's split)
     if (P0->per_thread > 0) d.set_map(P0->per_thread, P0->lpt);
     else d.auto_map(true, seg_even(d), P0->hm.n_layer * ntr / 4 * (j1 - j0));
     for (int j = j0; j < j1; ++j)

@@ -150,33 +150,6 @@ __device__ __forceinline__ void cell_grad(const Inst& in, int el, int v0, int v1
   cell_grad_vals<NTR>(in, el, a0, a1, a2, gx, gy);
 }
 
-// The same gradient when the tracer values at the lane's own node (vertex `pos` of the
-// cell) are already in registers: only the other two vertices are gathered.
-template <int NTR, bool IL>
-__device__ __forceinline__ void cell_grad_own(const Inst& in, int el, int v0, int v1, int v2,
-                                              int pos, const double (&own)[NTR], int k, int t0,
-                                              double (&gx)[NTR], double (&gy)[NTR]) {
-  const int L = in.m.L;
-  double a0[NTR], a1[NTR], a2[NTR];
-  if (pos == 0) {
-    ldn<NTR, IL>(in.T, lq(v1, L, k), t0, in.tstride, in.tg, a1);
-    ldn<NTR, IL>(in.T, lq(v2, L, k), t0, in.tstride, in.tg, a2);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) a0[t] = own[t];
-  } else if (pos == 1) {
-    ldn<NTR, IL>(in.T, lq(v0, L, k), t0, in.tstride, in.tg, a0);
-    ldn<NTR, IL>(in.T, lq(v2, L, k), t0, in.tstride, in.tg, a2);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) a1[t] = own[t];
-  } else {
-    ldn<NTR, IL>(in.T, lq(v0, L, k), t0, in.tstride, in.tg, a0);
-    ldn<NTR, IL>(in.T, lq(v1, L, k), t0, in.tstride, in.tg, a1);
-#pragma unroll
-    for (int t = 0; t < NTR; ++t) a2[t] = own[t];
-  }
-  cell_grad_vals<NTR>(in, el, a0, a1, a2, gx, gy);
-}
-
 template <int NTR, bool IL>
 __device__ __forceinline__ void cell_grad(const Inst& in, int el, int k, int t0,
                                           double (&gx)[NTR], double (&gy)[NTR]) {

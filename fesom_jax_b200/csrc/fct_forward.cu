@@ -668,10 +668,9 @@ const char* const kStageNames[kNumStages] = {
     "vflux", "elem_grad", "node_lo", "vert_impl", "edge_adf", "elem_bounds",
     "node_cluster", "node_factors", "node_final", "copy_dry"};
 
-// One stage over the tracers [c0, c1) of a workspace chunk: launches of S slices x NTR
-// tracers, NTR in {8, 4, 2, 1} (largest first, at most d.per_thread) and S the largest
-// power of two (at most 8) with S*NTR tracers left; the workspace index of tracer t is
-// t - c0.
+// One stage-by-stage stage over the tracers [c0, c1) of a workspace chunk: launches of S slices
+// x NTR tracers, NTR in {8, 4, 2, 1} (largest first) and S the largest power of two (at most 8)
+// with S*NTR tracers left; the workspace index of tracer t is t - c0.
 #define FCT_STAGE_AS(name, lanes, P)                                                    \
   name##_1<P><<<dim3(xblocks(lanes), 1u << lg), B, 0, s>>>(single, t0, w0)
 
@@ -679,8 +678,7 @@ const char* const kStageNames[kNumStages] = {
   do {                                                                                  \
     for (int t0 = c0; t0 < c1;) {                                                       \
       const int rem = c1 - t0;                                                          \
-      const int lim = std::min(rem, d.per_thread);                                      \
-      const int P = lim >= 8 ? 8 : lim >= 4 ? 4 : lim >= 2 ? 2 : 1;                     \
+      const int P = rem >= 8 ? 8 : rem >= 4 ? 4 : rem >= 2 ? 2 : 1;                     \
       int lg = 0;                                                                       \
       while (lg < 3 && (P << (lg + 1)) <= rem) ++lg;                                    \
       const int w0 = t0 - c0;                                                           \

@@ -45,7 +45,6 @@ struct LaunchDims {
   int ntr;           // tracers per instance (every instance of a launch has the same)
   int chunk = 0;     // tracers whose intermediates share the workspace (0 = all ntr);
                      // stages run chunk by chunk
-  int per_thread = 8;  // most tracers one thread carries (8, 4, 2 or 1): the tuning knob
   bool any_wi;      // launch the implicit w_i stage
   bool copy_dry;    // launch the dry-level copy
   bool pairs = true;  // the instances' interleaved tracer buffers start on 16-byte boundaries

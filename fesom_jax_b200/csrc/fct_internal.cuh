@@ -74,11 +74,6 @@ struct DevMesh {
   // nodes
   const int* nzmin;      // ulevels_nod2D - 1
   const int* nzmax;      // nlevels_nod2D - 1 (exclusive layer bound; bottom interface)
-  const int* ulmax;      // ulevels_nod2D_max
-  const int* nlmin;      // nlevels_nod2D_min
-  const int* ne_off;     // node -> incident edges CSR, ascending edge id
-  const int* ne_idx;     //   entry = 2*edge + (node is the edge's second node)
-  const int* ne_oth;     //   the edge's other node, aligned with ne_idx
   const int* nel_off;    // node -> elements CSR (nod_in_elem2D, element-ascending)
   const int* nel_idx;
   const double* area;    // [N,L]
@@ -91,29 +86,27 @@ struct DevMesh {
   const double* earea;   // [E]
   // edges
   const int* edges;      // [Ed,2]
-  const int* etri;       // [Ed,2]
   const int* eupdn;      // [Ed,2]
   const double* cross;   // [Ed,4]
   const double* ecoef;   // [Ed,2]: edx*a, edy*R  (a = R*cos, averaged over the two cells)
   const int* eedge;      // [E,3] the element's edges: 2*edge + (element is edge_tri[:,1])
   const int* eud_off;    // element -> edges that use it as MFCT up/down triangle (CSR)
   const int* eud_idx;    //   entry = 2*edge + slot (edge_up_dn_tri[edge, slot] == element)
-  const int* ekmin;      // [Ed] first level of the edge's lanes (union of its cells' layers)
-  const int* ekmax;      // [Ed] one past the last such level
   const int* etr;        // [Ed] levels where MFCT uses the up/down cells' gradients
                          //   (fill_up_dn_grad, tracer_adv.py:344-368), packed
-                         //   kmin | kmax << 8 and clipped to [ekmin, ekmax); empty
+                         //   kmin | kmax << 8 and clipped to the edge's levels (the
+                         //   union of its cells' layers); empty
                          //   when a cell is missing
   // packed CSR slots for the fused stage kernels (one 16-byte load per neighbour)
   const int4* ne4;       // per node->edge slot: {2*edge + second, other node,
-                         //   ekmin | ekmax << 8, cell layer ranges (see pack_tri)}
+                         //   the edge's levels kmin | kmax << 8, cell layer ranges (see pack_tri)}
   const int4* nel4;      // per node->element slot: {element, its three nodes}
   const int* nelr;       // per node->element slot: eul | enl << 8 | (node's vertex index) << 16
   // vertical
   const double* Zp;      // [L]  Z padded with Z[L-2] (tracer_adv.py:233)
   const double* zbar;    // [L]
   // lanes
-  const uint32_t* iface_lanes;  int64_t n_iface;   // nodes, k in [nzmin, nzmax]
+  int64_t n_iface;   // node lanes, k in [nzmin, nzmax] (iface4)
   const uint32_t* layer_lanes;  int64_t n_layer;   // nodes, k in [nzmin, nzmax)
   const uint32_t* dry_lanes;    int64_t n_dry;     // nodes, k outside [nzmin, nzmax)
   const uint32_t* edge_lanes;   int64_t n_edge;    // edges, k in the union of cell layers

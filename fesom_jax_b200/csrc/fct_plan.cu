@@ -567,20 +567,16 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   Blob b;
   const int nie = d->nod_in_elem2D_offsets[N];
   size_t o_nzmin = b.add(nzmin.data(), N), o_nzmax = b.add(nzmax.data(), N);
-  size_t o_ulmax = b.add(d->ulevels_nod2D_max, N), o_nlmin = b.add(d->nlevels_nod2D_min, N);
-  size_t o_neoff = b.add(ne_off.data(), N + 1), o_neidx = b.add(ne_idx.data(), ne_idx.size());
-  size_t o_neoth = b.add(ne_oth.data(), ne_oth.size());
   size_t o_neloff = b.add(d->nod_in_elem2D_offsets, N + 1);
   size_t o_nelidx = b.add(d->nod_in_elem2D, nie);
   size_t o_area = b.add(d->area, size_t(N) * L), o_av = b.add(d->areasvol, size_t(N) * L);
   size_t o_en = b.add(d->elem_nodes, 3 * size_t(E));
   size_t o_eul = b.add(eul.data(), E), o_enl = b.add(enl.data(), E);
   size_t o_gs = b.add(d->gradient_sca, 6 * size_t(E)), o_ea = b.add(d->elem_area, E);
-  size_t o_edges = b.add(d->edges, 2 * size_t(Ed)), o_etri = b.add(d->edge_tri, 2 * size_t(Ed));
+  size_t o_edges = b.add(d->edges, 2 * size_t(Ed));
   size_t o_eud = b.add(d->edge_up_dn_tri, 2 * size_t(Ed));
   size_t o_cross = b.add(d->edge_cross_dxdy, 4 * size_t(Ed));
   size_t o_ecoef = b.add(ecoef.data(), ecoef.size());
-  size_t o_ekmin = b.add(ekmin.data(), Ed), o_ekmax = b.add(ekmax.data(), Ed);
   size_t o_etr = b.add(etr.data(), Ed);
   size_t o_eedge = b.add(eedge.data(), eedge.size());
   size_t o_eudoff = b.add(eud_off.data(), eud_off.size());
@@ -588,7 +584,7 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   size_t o_ne4 = b.add(ne4.data(), ne4.size()), o_nel4 = b.add(nel4.data(), nel4.size());
   size_t o_nelr = b.add(nelr.data(), nelr.size());
   size_t o_Zp = b.add(Zp.data(), L), o_zbar = b.add(d->zbar, L);
-  size_t o_if = b.add(iface.data(), iface.size()), o_ly = b.add(layer.data(), layer.size());
+  size_t o_ly = b.add(layer.data(), layer.size());
   size_t o_dry = b.add(dry.data(), dry.size());
   size_t o_ed = b.add(edgel.data(), edgel.size()), o_el = b.add(eleml.data(), eleml.size());
   size_t o_if4 = b.add(iface4.data(), iface4.size()), o_ly4 = b.add(layer4.data(), layer4.size());
@@ -623,11 +619,6 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
     }
   m.nzmin = (const int*)(base + o_nzmin);
   m.nzmax = (const int*)(base + o_nzmax);
-  m.ulmax = (const int*)(base + o_ulmax);
-  m.nlmin = (const int*)(base + o_nlmin);
-  m.ne_off = (const int*)(base + o_neoff);
-  m.ne_idx = (const int*)(base + o_neidx);
-  m.ne_oth = (const int*)(base + o_neoth);
   m.nel_off = (const int*)(base + o_neloff);
   m.nel_idx = (const int*)(base + o_nelidx);
   m.area = (const double*)(base + o_area);
@@ -638,22 +629,19 @@ static int plan_build(const FctMeshDesc* d, int device, FctPlan* P) {
   m.gsca = (const double*)(base + o_gs);
   m.earea = (const double*)(base + o_ea);
   m.edges = (const int*)(base + o_edges);
-  m.etri = (const int*)(base + o_etri);
   m.eupdn = (const int*)(base + o_eud);
   m.cross = (const double*)(base + o_cross);
   m.ecoef = (const double*)(base + o_ecoef);
-  m.ekmin = (const int*)(base + o_ekmin);
   m.eedge = (const int*)(base + o_eedge);
   m.eud_off = (const int*)(base + o_eudoff);
   m.eud_idx = (const int*)(base + o_eudidx);
-  m.ekmax = (const int*)(base + o_ekmax);
   m.etr = (const int*)(base + o_etr);
   m.ne4 = (const int4*)(base + o_ne4);
   m.nel4 = (const int4*)(base + o_nel4);
   m.nelr = (const int*)(base + o_nelr);
   m.Zp = (const double*)(base + o_Zp);
   m.zbar = (const double*)(base + o_zbar);
-  m.iface_lanes = (const uint32_t*)(base + o_if);  m.n_iface = int64_t(iface.size());
+  m.n_iface = int64_t(iface.size());
   m.layer_lanes = (const uint32_t*)(base + o_ly);  m.n_layer = int64_t(layer.size());
   m.dry_lanes = (const uint32_t*)(base + o_dry);  m.n_dry = int64_t(dry.size());
   m.edge_lanes = (const uint32_t*)(base + o_ed);   m.n_edge = int64_t(edgel.size());

@@ -54,10 +54,9 @@ namespace {
 __host__ __device__ constexpr int edge_blocks(int ntr, bool) {
   return ntr == 1 ? 5 : ntr == 2 ? 3 : 2;
 }
-__host__ __device__ constexpr int edge_batch(int, bool) {
-  return 1;
-}
-FCT_STREAM_KERNEL(k_edge_stream, stream_edge_adf, edge_blocks, edge_batch)
+#define FCT_BODY(NTR, IL) stream_edge_adf<NTR, IL>
+FCT_STREAM_KERNEL(k_edge_stream, FCT_BODY, edge_blocks)
+#undef FCT_BODY
 
 #define FCT_COUNT(V) d.max_eseg[V]
 FCT_STREAM_LAUNCHER(launch_stream, k_edge_stream, FCT_COUNT, FCT_GRID, kStageEdge, edge_blocks)

@@ -17,7 +17,9 @@ __host__ __device__ constexpr int stream_blocks(int ntr, bool) {
 __host__ __device__ constexpr int slot_batch(int, bool) {
   return 3;
 }
-FCT_STREAM_KERNEL(k_stream_final, stream_node_final, stream_blocks, slot_batch)
+#define FCT_BODY(NTR, IL) stream_node_final<NTR, IL, slot_batch(NTR, IL)>
+FCT_STREAM_KERNEL(k_stream_final, FCT_BODY, stream_blocks)
+#undef FCT_BODY
 
 #define FCT_COUNT(V) d.max_nseg[V]
 FCT_STREAM_LAUNCHER(launch_stream, k_stream_final, FCT_COUNT, FCT_GRID, kStageFinal, stream_blocks)

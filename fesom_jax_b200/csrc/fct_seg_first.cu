@@ -19,7 +19,7 @@ __global__ void __launch_bounds__(256, 2) k_seg_first_1(const __grid_constant__ 
     stream_node_lo<NTR, false, 3>(in, int64_t(b) * 256 + tid, int64_t(nlo) * 256, t0 + sub,
                                   w0 + sub);
   } else if ((b -= nlo) < nedge) {
-    stream_edge_adf<NTR, false, 1>(in, int64_t(b) * 256 + tid, int64_t(nedge) * 256, t0 + sub,
+    stream_edge_adf<NTR, false>(in, int64_t(b) * 256 + tid, int64_t(nedge) * 256, t0 + sub,
                                    w0 + sub);
   } else if (blockIdx.y == 0) {
     body_copy_dry<false>(in, int64_t(b - nedge) * 256 + tid);

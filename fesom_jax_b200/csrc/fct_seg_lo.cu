@@ -16,7 +16,9 @@ __host__ __device__ constexpr int stream_blocks(int ntr, bool il) {
 __host__ __device__ constexpr int slot_batch(int ntr, bool il) {
   return ntr == 2 && !il ? 2 : 3;
 }
-FCT_STREAM_KERNEL(k_stream_lo, stream_node_lo, stream_blocks, slot_batch)
+#define FCT_BODY(NTR, IL) stream_node_lo<NTR, IL, slot_batch(NTR, IL)>
+FCT_STREAM_KERNEL(k_stream_lo, FCT_BODY, stream_blocks)
+#undef FCT_BODY
 
 #define FCT_COUNT(V) d.max_nseg[V]
 FCT_STREAM_LAUNCHER(launch_stream, k_stream_lo, FCT_COUNT, FCT_GRID, kStageLo, stream_blocks)

@@ -346,7 +346,7 @@ __device__ __forceinline__ void seg_edge_adf(const Inst& in, int64_t si, int t0,
 // two members, 4 per thread: 0.82 -> 0.66 ms), for a thread that walks the segments si, si + stride, ...: the
 // next level's records and volume flux are loaded while this level's gathers are under way, so
 // a level costs one memory round trip instead of three in a row (segment, records, gathers).
-template <int NTR, bool IL, int U>
+template <int NTR, bool IL>
 __device__ __forceinline__ void stream_edge_adf(const Inst& in, int64_t si, int64_t stride, int t0,
                                                 int w0) {
   const DevMesh& m = in.m;
@@ -1286,13 +1286,13 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
   }
 
 // Kernels whose threads walk the segments (one level per thread): as many blocks as are
-// resident at once (stream_grid).
-#define FCT_STREAM_KERNEL(name, body, blocks, batch)                                         \
+// resident at once (stream_grid). ``BODY(NTR, IL)`` names the body's instantiation.
+#define FCT_STREAM_KERNEL(name, BODY, blocks)                                            \
   template <int NTR>                                                                     \
   __global__ void __launch_bounds__(256, blocks(NTR, false))                             \
       name##_1(const __grid_constant__ Inst in, int t0, int w0) {                        \
     const int sub = int(blockIdx.y) * NTR;                                               \
-    body<NTR, false, batch(NTR, false)>(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub); \
+    BODY(NTR, false)(in, lane_index(), int64_t(gridDim.x) * 256, t0 + sub, w0 + sub);    \
   }                                                                                      \
   template <int NTR>                                                                     \
   __global__ void __launch_bounds__(256, blocks(NTR, true))                              \
@@ -1301,8 +1301,8 @@ inline unsigned seg_blocks(int64_t lanes, int per_block) {
     if (slot >= slots) return;                                                           \
     const int sub = (int(threadIdx.x) - slot * S) * NTR;                                 \
     for (int i = int(blockIdx.y); i < n; i += int(gridDim.y))                            \
-      body<NTR, true, batch(NTR, true)>(tab[i], int64_t(blockIdx.x) * slots + slot,                     \
-                         int64_t(gridDim.x) * slots, t0 + sub, w0 + sub);                \
+      BODY(NTR, true)(tab[i], int64_t(blockIdx.x) * slots + slot,                        \
+                      int64_t(gridDim.x) * slots, t0 + sub, w0 + sub);                   \
   }
 #define FCT_STREAM_LIMIT_KERNEL(name, blocks, batch)                                         \
   template <int NTR>                                                                     \
