@@ -81,7 +81,7 @@ class Member:
     hnode_new: object
     buf: object         # torch [3, N, nl, ntr] (tracers interleaved innermost)
     Kv: object = None   # torch [N, nl] or None (no vertical diffusion)
-    derive_w: bool = False   # w_e recomputed from uv each step (into w_e)
+    derive_w: bool = False   # w_e recomputed from uv each step() and run() (into w_e)
 
 
 class Ensemble:
@@ -112,8 +112,9 @@ class Ensemble:
         """Add a member (host numpy or device tensors); ``T``/``T_old`` are ``[ntr, N, nl]``.
         With ``Kv`` (``[N, nl]``) every step is followed by the implicit vertical diffusion
         of fesom_jax/tracer_diff.py:68-123 (step.py:452), in the same graph. With
-        ``derive_w`` every step first derives ``w_e = compute_w(uv, helem)``
-        (fesom_jax/ale.py:309-365, step.py:367) on the GPU and ``w_e`` may be None."""
+        ``derive_w`` every :meth:`step`, and every :meth:`run` once at its start, first derives
+        ``w_e = compute_w(uv, helem)`` (fesom_jax/ale.py:309-365, step.py:367) on the GPU and
+        ``w_e`` may be None."""
         if self._h is not None:
             raise RuntimeError("members must be added before the ensemble is built")
         t = self.torch
@@ -189,7 +190,8 @@ class Ensemble:
         self.phase += 1
 
     def run(self, steps: int, stream=None) -> None:
-        """``steps`` FCT steps of every member as one CUDA graph launch."""
+        """``steps`` FCT steps of every member as one CUDA graph launch. The volume fluxes (and
+        derived ``w_e``) are formed once, from the ``uv`` and ``helem`` at its start."""
         _lib.check(_bind_batch(_lib.lib()).fct_batch_run(self._h, self.phase % 3, int(steps),
                                                          self._stream(stream)))
         self.phase += int(steps)

@@ -75,7 +75,7 @@ def _run(mesh: Mesh, T, Kv, hnode_new, dt, bc_surf, sw_3d, Z3d, sw_tracer=0, out
     f.sw_tracer = sw_tracer
     L = _bind(_lib.lib())
     s = torch.cuda.current_stream(dev).cuda_stream
-    with plan._lock:   # the plan workspace holds the elimination factors
+    with plan._lock:   # the library orders calls on one plan; their enqueue stays whole
         _lib.check(L.fct_vert_diff(plan.handle, C.byref(f), float(dt), ntr, C.c_void_p(int(s))))
     return out.cpu().numpy() if host else out
 

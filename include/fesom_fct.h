@@ -344,9 +344,10 @@ typedef struct FctInstance {
   double dt;
   const double* Kv;         /* optional [nod2D,nl]: implicit vertical diffusion after each
                                step (tracer_diff.py:68-123, step.py:452; NULL = off) */
-  double* w_derived;        /* optional [nod2D,nl]: each step first derives w_e =
-                               compute_w(uv, helem) (ale.py:309-365, step.py:367) into this
-                               buffer and advects with it (w_e is then ignored); NULL = off */
+  double* w_derived;        /* optional [nod2D,nl]: w_e = compute_w(uv, helem) (ale.py:309-365,
+                               step.py:367) is derived into this buffer, by every
+                               fct_batch_step and fct_serve_step and once at the start of an
+                               fct_batch_run, and advects (w_e is then ignored); NULL = off */
   unsigned long long* nonfinite; /* optional DEVICE counter: each step adds the number of
                                non-finite T_new values it writes (NULL: the batch's own
                                per-instance counter, or the serve engine's counter) */
