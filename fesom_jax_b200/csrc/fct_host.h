@@ -27,8 +27,9 @@ inline int cuda_error(cudaError_t e, const char* what) {
   } while (0)
 
 // most blocks of the one launch of a small instance's first stages: eight waves of two blocks on
-// every SM (pi, T and S, 6 waves: 46.5 us a step against 50.9 with a launch per stage; 600 nodes
-// 33.8 against 46.1; 20,000 nodes x 3 tracers, 44 waves, no difference)
+// every SM. Measured up to 6 waves it gains (pi, T and S: 46.5 us a step against 50.9 with a
+// launch per stage; 600 nodes 33.8 against 46.1), at 44 there is no difference (20,000 nodes x 3
+// tracers); where between them the gain ends was not measured.
 constexpr int64_t kFirstBlocks = 8 * 2 * 148;
 
 // fused stages with their own thread mapping: LO, edge, limiter, final
@@ -132,9 +133,9 @@ inline dim3 stream_grid(int64_t need, int64_t full, int n) {
 }
 
 // Tracers per thread and tracer slices of one segment launch over ``rem`` tracers: the
-// largest compiled count (1, 2 or 4 interleaved, 1 when pairs are not 16-byte aligned; 1 or 2 tracer-major) of at most ``per_thread``, and as
-// many slices as whole counts fit (at most 8 interleaved). Three tracer-major tracers go one
-// per thread, in one launch instead of two.
+// largest compiled count (1, 2 or 4 interleaved, 1 when pairs are not 16-byte aligned; 1 or 2
+// tracer-major) of at most ``per_thread``, and as many slices as whole counts fit (at most 8
+// interleaved). Three tracer-major tracers go one per thread, in one launch instead of two.
 struct SegSplit {
   int tracers, slices;
 };
@@ -145,8 +146,10 @@ inline SegSplit seg_split(int rem, int per_thread, bool interleaved, bool even) 
     if (lim >= 4) P = 4;
     if (!even) P = 1;
     int S = std::min(8, rem / P);
-    // three single tracers keep their two launches per stage (fct_batch_info's count of
-    // them is checked by a test)
+    // three single tracers keep two launches per stage, two slices and one, as the launch count
+    // of test_derived_w_equals_compute_w_then_fct has it; in one launch of three slices a member
+    // of two on the CORE2-size mesh took 2.86 ms a step against 3.83, 16 pi members 0.80
+    // against 1.01, one pi member 63 us against 85
     if (P == 1 && rem == 3) S = 2;
     return {P, S};
   }
@@ -177,9 +180,9 @@ int launch_seg_limit(const Inst& single, const Inst* tab, int n, const LaunchDim
 int launch_seg_final(const Inst& single, const Inst* tab, int n, const LaunchDims& d, int c0,
                      int c1, cudaStream_t s);
 // The LO stage, the edge stage with its remaining lanes and (``dry``) the dry-level copy of a
-// single instance in one launch, where all their blocks are resident at once (seg_first_fits):
-// they depend only on the volume fluxes, and on a small mesh each of them is shorter than the
-// gap between two launches (fct_seg_first.cu).
+// single instance in one launch, where their blocks make at most kFirstBlocks (seg_first_fits):
+// they depend only on the volume fluxes, not on one another, and on a small mesh each of them is
+// shorter than the gap between two launches (fct_seg_first.cu).
 int launch_seg_first(const Inst& single, const LaunchDims& d, int c0, int c1, bool dry,
                      cudaStream_t s);
 inline int64_t seg_first_blocks(const LaunchDims& d, int tracers_per_thread, int rem) {
