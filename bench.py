@@ -44,9 +44,12 @@ TRAFFIC_B_PER_UPDATE = 245.0
 # issue-limited rather than HBM-bound, so the line also reports this issue-rate fraction
 # beside the HBM one: achieved warp-instructions/s against 148 SMs x 4 schedulers x the
 # sampled SM clock. The first is the earlier segment kernels' count (9.87 G updates/s ran
-# on them) and the arithmetic's default; the second is what the timed step executes now.
+# on them) and the arithmetic's default; the second is the stream kernels' under the default
+# mapping, CAPTURED_MAPPING (the autotuner may take another, whose count it only approximates:
+# the line says which it is).
 WARP_INST_PER_UPDATE = 46.0
 STREAM_WARP_INST_PER_UPDATE = 34.9
+CAPTURED_MAPPING = ((4, 1), (4, 1), (4, 1), (2, 2))   # LO, edge, limiter, final
 B200_SMS, SCHEDULERS_PER_SM = 148, 4
 
 
@@ -390,8 +393,12 @@ def run_ours(args, D: Dist) -> dict | None:
                              traffic_note="ncu DRAM bytes of the step's 6 kernels, small-case "
                                           "capture scaled by updates",
                              alg_bytes_per_step=alg,
-                             issue=issue_roofline(value / D.world, clk,
-                                                  STREAM_WARP_INST_PER_UPDATE)),
+                             issue=dict(issue_roofline(value / D.world, clk,
+                                                       STREAM_WARP_INST_PER_UPDATE),
+                                        counted_mapping=[f"{c}x{lv}" for c, lv in
+                                                         CAPTURED_MAPPING],
+                                        mapping_is_counted=tuple(ens.stage_map) ==
+                                        CAPTURED_MAPPING)),
                gpu_launches=n_kernels * args.steps,
                tuning=dict(stage_mapping={st: f"{c}x{lv}" for st, (c, lv) in
                                           zip(ens.STAGES, ens.stage_map)},
