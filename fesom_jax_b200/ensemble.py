@@ -318,7 +318,13 @@ class Ensemble:
             self.set_stage_mapping(i, *m)
         t_stage = self._graph_ms(steps, reps)
         self.reset_mapping()
-        t_default = self._graph_ms(steps, reps)
+        default = [self.group_mapping(g) for g in range(self.info()["groups"])]
+        if all(m == best_stage for m in default):      # timed already
+            t_default = t_stage
+        elif all(m == [uniform] * 4 for m in default):
+            t_default = t_uniform
+        else:
+            t_default = self._graph_ms(steps, reps)
         chosen = "default"
         if min(t_stage, t_uniform) <= t_default:
             chosen = "per_stage" if t_stage <= t_uniform else "uniform"
