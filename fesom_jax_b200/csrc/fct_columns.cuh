@@ -260,6 +260,90 @@ __device__ __forceinline__ void block_vdiff(const Inst& in, int n0, int columns,
   }
 }
 
+// The same for eight interleaved tracers of many columns, in place, straight from memory: a
+// thread walks a column with a tracer pair, the four pairs of a column are adjacent, so each
+// level is one whole line, and many walks hide each other's loads. It needs the threads: above
+// half of the resident ones (kPairColumns) it wins (us a step, walks / shared memory: 127,000
+// nodes x 48 levels 499 / 793, four such members 1,953 / 3,126, 16 pi members 290 / 352, 8
+// 151 / 183, 30,000 x 70 levels 232 / 288; 20,000 columns the same, 4 pi members 133 / 100).
+// With four tracers, half a line, the two are equal on large members and shared memory wins on
+// the others. cp and dp wait in the workspace's adfv and lo, which the step has finished with; a
+// batch has no surface flux and no shortwave.
+constexpr int kPairTracers = 8, kPairBlocks = 5;
+constexpr int64_t kPairColumns = int64_t(148) * kPairBlocks * 256 / 2 / (kPairTracers / 2);
+__device__ __forceinline__ void pair_vdiff(const Inst& in, int64_t n, int t0, int w0) {
+  const DevMesh& m = in.m;
+  if (n >= m.N || !in.Kv) return;
+  const int L = m.L;
+  const int nzmin = ld(m.nzmin + n), nzmax = ld(m.nzmax + n);
+  const uint32_t base = lq(int(n), L, 0);
+  const int tg = in.tg;
+  double* __restrict__ T = in.T_new;
+  double* __restrict__ lo = in.ws.lo;
+  double* __restrict__ cps = in.ws.adfv;
+  auto get = [](const double* p, uint32_t q, int t, int g, double (&v)[2]) {
+    const double2 x = *reinterpret_cast<const double2*>(p + (q * uint32_t(g) + uint32_t(t)));
+    v[0] = x.x;
+    v[1] = x.y;
+  };
+  auto put = [](double* p, uint32_t q, int t, int g, const double (&v)[2]) {
+    *reinterpret_cast<double2*>(p + (q * uint32_t(g) + uint32_t(t))) = make_double2(v[0], v[1]);
+  };
+  const int wtg = in.wtg;
+  if (nzmax <= nzmin) return;
+  const double dt = in.dt;
+  const double* Zc = in.vd_Z3d ? in.vd_Z3d + base : m.Zp;
+  double cprev = 0.0, dprev[2] = {0.0, 0.0}, Tm[2], Tc[2], Tp[2];
+  get(T, base + uint32_t(nzmin), t0, tg, Tc);
+  get(T, base + uint32_t(nzmin > 0 ? nzmin - 1 : 0), t0, tg, Tm);
+  for (int k = nzmin; k < nzmax; ++k) {
+    const uint32_t q = base + uint32_t(k);
+    const bool last = k + 1 >= L;
+    Tp[0] = Tp[1] = 0.0;
+    if (!last) get(T, q + 1, t0, tg, Tp);
+    double dzu = k == 0 ? 0.0 : ld(Zc + k - 1) - ld(Zc + k);
+    double dzd = ld(Zc + k) - (last ? 0.0 : ld(Zc + k + 1));
+    dzu = dzu == 0.0 ? 1.0 : dzu;
+    dzd = dzd == 0.0 ? 1.0 : dzd;
+    const double av = ld(m.areasvol + q);
+    const double sav = av > 0.0 ? av : 1.0;
+    const double ar = ld(m.area + q), arp = last ? 0.0 : ld(m.area + q + 1);
+    const double kv = ld(in.Kv + q), kvp = last ? 0.0 : ld(in.Kv + q + 1);
+    const double a_full = -kv * dt / dzu * (ar / sav);
+    const double c_full = -kvp * dt / dzd * (arp / sav);
+    const double a = k == nzmin ? 0.0 : a_full;
+    const double c = k == nzmax - 1 ? 0.0 : c_full;
+    const double b = -a - c + ld(in.hnode_new + q);
+    const Rcp rm = rcp(b - a * cprev);
+    cprev = divr(c, rm);
+    cps[q * uint32_t(wtg) + uint32_t(w0)] = cprev;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const double rhs = a * (Tc[t] - Tm[t]) + c * (Tc[t] - Tp[t]);
+      dprev[t] = divr(rhs - a * dprev[t], rm);
+      Tm[t] = Tc[t];
+      Tc[t] = Tp[t];
+    }
+    put(lo, q, w0, wtg, dprev);
+  }
+  double x[2] = {0.0, 0.0}, Tn[2];
+  get(T, base + uint32_t(nzmax - 1), t0, tg, Tn);
+#pragma unroll 2
+  for (int k = nzmax - 1; k >= nzmin; --k) {
+    const uint32_t q = base + uint32_t(k);
+    double d[2], Tv[2] = {Tn[0], Tn[1]};
+    const double c = cps[q * uint32_t(wtg) + uint32_t(w0)];
+    get(lo, q, w0, wtg, d);
+    if (k > nzmin) get(T, q - 1, t0, tg, Tn);   // ahead of the store
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      x[t] = d[t] - c * x[t];
+      Tv[t] = Tv[t] + x[t];
+    }
+    put(T, q, t0, tg, Tv);
+  }
+}
+
 // ---------------------------- adv_tra_vert_impl (tracer_adv.py:487-529): implicit w_i
 // advection of LO, the tracers' workspace slots [w0, w0 + nt)
 template <int nt, bool IL>

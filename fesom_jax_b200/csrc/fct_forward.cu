@@ -645,6 +645,12 @@ FCT_KERNEL_T(k_node_final, body_node_final)
 // implicit vertical diffusion (the epilogue of the batched step and fct_vert_diff)
 FCT_KERNEL_COL(k_vdiff, block_vdiff)
 FCT_KERNEL_COL(k_vert_impl, block_vert_impl)
+__global__ void __launch_bounds__(256, kPairBlocks) k_vdiff_pairs_n(
+    const Inst* __restrict__ tab, int t0) {
+  const int64_t g = lane_index();
+  const int sub = int(g % (kPairTracers / 2)) * 2;
+  pair_vdiff(tab[blockIdx.y], g / (kPairTracers / 2), t0 + sub, sub);
+}
 
 constexpr int kVfluxBlocks = 5;
 __global__ void __launch_bounds__(256, kVfluxBlocks) k_vflux_1(const __grid_constant__ Inst in) {
@@ -845,8 +851,10 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
           if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, s>>>(tab);
           else k_copy_dry_1<<<grid(d.max_dry), B, 0, s>>>(single);
         }
-        if ((st = launch_columns(FCT_COL_TABLE(k_vdiff), single, tab, n, d.max_nodes, d.max_levels,
-                                 c0, c1 - c0, s, "vertical diffusion launch")))
+        if (tab && seg_even(d) && c1 - c0 == kPairTracers && n * d.max_nodes >= kPairColumns)
+          k_vdiff_pairs_n<<<grid(d.max_nodes * (kPairTracers / 2)), B, 0, s>>>(tab, c0);
+        else if ((st = launch_columns(FCT_COL_TABLE(k_vdiff), single, tab, n, d.max_nodes,
+                                      d.max_levels, c0, c1 - c0, s, "vertical diffusion launch")))
           return st;
       }
       mark();

@@ -122,3 +122,36 @@ def test_batched_epilogue_of_members_of_different_depth(torch, meshes, ntr):
         got, old = ens.state(i)
         assert torch.equal(got, T) and torch.equal(old, To)
     ens.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ntr", [8, 10, 16])
+def test_batched_epilogue_of_many_columns(torch, meshes, ntr):
+    """Enough columns for the walks of eight tracers (chunks of 8, 8 + 2 and 8 + 8), members of
+    12 to 128 levels and a cavity in one launch: the bits of plain steps and diffusion calls."""
+    from fesom_jax_b200.ensemble import Ensemble
+    from fesom_jax_b200.tracer_adv import get_plan
+    from fesom_jax_b200.tracer_diff import impl_vert_diff_one
+    ens, want = Ensemble(), []
+    order = ("cavity", 128, 12, "cavity", 48, 70, "cavity", 12)
+    assert len(order) * meshes["cavity"].nod2D >= 148 * 5 * 256 // 8
+    for i, nl in enumerate(order):
+        m = meshes[nl]
+        f = I.make_fields(m, seed=i, n_passive=ntr - 2, ab2=True,
+                          kind="psi" if nl == "cavity" else "basin")
+        a = [_dev(torch, x) for x in (f.uv, f.w_e, f.helem, f.hnode, f.hnode_new)]
+        T, To = (_dev(torch, x) for x in (f.tracers, f.tracers_old))
+        Kv = _dev(torch, _Kv(m, np.random.default_rng(i)))
+        ens.add_member(m, *a, T, To, DT, Kv=Kv)
+        for _ in range(2):
+            T, To = impl_vert_diff_one(m, get_plan(m, 0).forward(*a, T, To, DT), Kv, a[4],
+                                       dt=DT), T
+        want.append((T, To))
+    ens.build()
+    ens.fill_workspace(0xFF)
+    ens.run(2)
+    assert ens.info()["groups"] == 1
+    for i, (T, To) in enumerate(want):
+        got, old = ens.state(i)
+        assert torch.equal(got, T) and torch.equal(old, To)
+    ens.close()
