@@ -122,14 +122,19 @@ inline void dims_map(LaunchDims& d, const FctPlan* P) {
 // Grid of a kernel whose threads walk its lanes, for ``n`` instances of at most ``need`` blocks
 // when ``full`` blocks are resident at once. Large instances go one after the other, so that
 // the gathers of all blocks stay within a few columns of each other; where one gives a thread
-// fewer than kWalk lanes they go side by side (grid.y), with as many blocks each as fill the
-// chip together (16 pi-size members x 30 steps: 17.3 ms one after the other, 14.8 with every
-// block of every instance in the grid and no walk, 12.8 so).
+// fewer than kWalk lanes they go side by side (grid.y), with about as many blocks each as fill
+// the chip together (16 pi-size members x 30 steps: 17.3 ms one after the other, 14.8 with every
+// block of every instance in the grid and no walk, 12.8 so): full / n blocks each, rounded to
+// the side with fewer waves per block. Rounded up always, a few blocks ran in a wave of their
+// own (volume fluxes of 64 pi members, 768 blocks on 740 places: 202 us against 130; two and
+// eight tracers of 24 pi members, all stages: 733 and 2,420 us a step against 627 and 2,054).
 constexpr int kWalk = 4;
 inline dim3 stream_grid(int64_t need, int64_t full, int n) {
   if (need >= kWalk * full) return dim3(unsigned(full), 1);
-  const int64_t x = std::max<int64_t>(1, std::min(need, (full + n - 1) / n));
-  return dim3(unsigned(x), unsigned(n));
+  auto waves = [&](int64_t x) { return (x * n + full - 1) / full; };
+  const int64_t lo = std::max<int64_t>(1, full / n), hi = (full + n - 1) / n;
+  const int64_t x = waves(hi) * lo <= waves(lo) * hi ? hi : lo;
+  return dim3(unsigned(std::max<int64_t>(1, std::min(need, x))), unsigned(n));
 }
 
 // Tracers per thread and tracer slices of one segment launch over ``rem`` tracers: the
