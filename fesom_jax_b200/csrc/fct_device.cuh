@@ -48,7 +48,8 @@ __device__ __forceinline__ void ldn(const double* __restrict__ p, uint32_t q, in
 
 // ldn/stn for the segment kernels: in the interleaved layout with an even NTR the host
 // guarantees 16-byte alignment (even tracer strides and offsets, tracer buffers on 16-byte
-// boundaries, seg_even; workspace fields on 256-byte boundaries), so the tracer pairs load and store as double2 without a test.
+// boundaries, seg_even; workspace fields on 256-byte boundaries), so the tracer pairs load and
+// store as double2 without a test.
 template <int NTR, bool IL>
 __device__ __forceinline__ void ldv(const double* __restrict__ p, uint32_t q, int t0,
                                     int64_t stride, int tg, double (&v)[NTR]) {

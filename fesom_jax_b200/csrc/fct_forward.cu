@@ -851,6 +851,7 @@ int launch_forward_events(const Inst& single, const Inst* tab, int n, const Laun
           if (tab) k_copy_dry_n<<<grid(d.max_dry), B, 0, s>>>(tab);
           else k_copy_dry_1<<<grid(d.max_dry), B, 0, s>>>(single);
         }
+        // eight aligned tracers of many columns walk them from memory (pair_vdiff)
         if (tab && seg_even(d) && c1 - c0 == kPairTracers && n * d.max_nodes >= kPairColumns)
           k_vdiff_pairs_n<<<grid(d.max_nodes * (kPairTracers / 2)), B, 0, s>>>(tab, c0);
         else if ((st = launch_columns(FCT_COL_TABLE(k_vdiff), single, tab, n, d.max_nodes,

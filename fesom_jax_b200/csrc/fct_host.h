@@ -152,9 +152,9 @@ inline SegSplit seg_split(int rem, int per_thread, bool interleaved, bool even) 
     if (!even) P = 1;
     int S = std::min(8, rem / P);
     // three single tracers keep two launches per stage, two slices and one, as the launch count
-    // of test_derived_w_equals_compute_w_then_fct has it; in one launch of three slices a member
-    // of two on the CORE2-size mesh took 2.86 ms a step against 3.83, 16 pi members 0.80
-    // against 1.01, one pi member 63 us against 85
+    // of test_derived_w_equals_compute_w_then_fct has it; in one launch of three slices two
+    // CORE2-size members took 2.86 ms a step against 3.83, 16 pi members 0.80 against 1.01, one
+    // pi member 63 us against 85
     if (P == 1 && rem == 3) S = 2;
     return {P, S};
   }

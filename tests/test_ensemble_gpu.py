@@ -129,7 +129,7 @@ def test_chunked_workspace_equals_plain(torch, pi, per_thread):
 
 
 def test_derived_w_equals_compute_w_then_fct(torch, pi):
-    """A member with derive_w runs compute_w(uv, helem) inside every step's graph; it
+    """A member with derive_w runs compute_w(uv, helem) at the start of a run's graph; it
     equals the plain compute_w call followed by the plain FCT calls, bit for bit."""
     from fesom_jax_b200.ale import compute_w
     from fesom_jax_b200.ensemble import Ensemble
